@@ -26,7 +26,8 @@ struct portal_batch {
     std::string err;
 
     bool prepared = false;
-    int nch = 0, n_depth = 0, kmax = 0, max_lines = 0;
+    int nch = 0, n_depth = 0, kmax = 0;
+    std::vector<int> lines;             // per model
     bool dust = false;
     std::vector<RFArgs> rf;
     std::vector<SEArgs> se;
@@ -69,6 +70,21 @@ void drop_graph(portal_batch *b) {
     b->graph = nullptr;
 }
 
+// the radiation-field launch over these items with line groups of at most nlg
+RFBatch rf_batch(portal_batch *b, const int2 *items, long long n_items, int nlg) {
+    RFBatch rb{};
+    rb.models = b->d_rf.p;
+    rb.items = items;
+    rb.n_items = n_items;
+    rb.queue = b->queue.p;
+    rb.walk = b->walk.p;
+    rb.n_depth = b->n_depth;
+    rb.chq = b->rf[0].chq;
+    rb.chw = b->rf[0].chw;
+    rf_batch_shape(&rb, b->lines.data(), (int)b->lines.size(), b->nch, b->dust, nlg, false);
+    return rb;
+}
+
 // the whole pass on the batch stream: per-model line tables and zeroed
 // outputs, one radiation-field launch, zeroed SE outputs, one SE launch
 int enqueue_pass(portal_batch *b, const int2 *items, long long n_items) {
@@ -77,8 +93,8 @@ int enqueue_pass(portal_batch *b, const int2 *items, long long n_items) {
         if ((rc = rf_pass(b->models[m], b->rf[m], b->stream)))
             return bfail(b, rc, "model " + std::to_string(m) + ": " + b->models[m]->err);
     BCHECK(b, cudaMemsetAsync(b->queue.p, 0, 2 * sizeof(unsigned long long), b->stream));
-    RFBatch rb{b->d_rf.p, items, n_items, b->queue.p, b->walk.p, b->n_depth};
-    if ((rc = rf_batch_launch(b->stream, b->rf_bps * b->sm_count, b->nch, b->dust, b->nlg, b->max_lines, rb)))
+    const RFBatch rb = rf_batch(b, items, n_items, b->nlg);
+    if ((rc = rf_batch_launch(b->stream, b->rf_bps * b->sm_count, b->dust, rb)))
         return bfail(b, rc, "radiation-field launch failed");
     for (size_t m = 0; m < b->models.size(); m++)
         if ((rc = se_pass(b->models[m], b->stream)))
@@ -162,7 +178,7 @@ extern "C" int portal_batch_prepare(portal_batch *b, int nth, int nph, int nvel,
     b->rf.assign(M, RFArgs{});
     b->se.assign(M, SEArgs{});
     b->dust = false;
-    b->max_lines = 0;
+    b->lines.clear();
     size_t wb = 0;
     b->se_a64_stride = 0;
     std::vector<double> cost(M);
@@ -177,7 +193,7 @@ extern "C" int portal_batch_prepare(portal_batch *b, int nth, int nph, int nvel,
         wb = std::max(wb, w);
         b->se_a64_stride = std::max(b->se_a64_stride, se_matrix_doubles(c));
         b->dust = b->dust || c->has_dust;
-        b->max_lines = std::max(b->max_lines, c->r_num);
+        b->lines.push_back(c->r_num);
         // per-node cost ~ lines x cells per ray ~ L N^(1/3)
         cost[m] = (double)c->r_num * std::cbrt((double)c->N);
     }
@@ -203,23 +219,32 @@ extern "C" int portal_batch_prepare(portal_batch *b, int nth, int nph, int nvel,
     BCHECK(b, cudaMemcpyAsync(b->sample.p, sm.data(), sizeof(int2) * sm.size(), cudaMemcpyHostToDevice, b->stream));
     BCHECK(b, cudaStreamSynchronize(b->stream));
 
-    // candidate launch shapes: radiation field (line group, blocks per SM),
-    // SE (warps per block; blocks per SM from the occupancy)
+    // candidate launch shapes: radiation field (widest line group, blocks per
+    // SM: all that fit, or half), SE (warps per block; blocks per SM from the
+    // occupancy)
     struct RFC { int nlg, bps; };
     std::vector<RFC> rfc;
-    const void *seen = nullptr;
+    size_t rf_grid = 0;
     for (int nlg : {5, 10}) {
-        // layouts with the lanes-over-lines remainder channel have one line
-        // group; do not time the same kernel twice
-        const void *k = rf_batch_kernel_ptr(b->nch, b->dust, nlg, b->max_lines);
-        if (k == seen) continue;
-        seen = k;
         int mx = 0;
-        if (rf_batch_blocks_per_sm(b->nch, b->dust, nlg, b->max_lines, &mx))
+        if (rf_batch_blocks_per_sm(rf_batch(b, nullptr, 0, nlg), b->dust, &mx))
             return bfail(b, PORTAL_ERR_CUDA, "occupancy query");
-        for (int bps = 1; bps <= std::min(mx, 2); bps++) rfc.push_back({nlg, bps});
+        if (mx < 1) continue;
+        rfc.push_back({nlg, mx});
+        if (mx > 1) rfc.push_back({nlg, (mx + 1) / 2});
+        rf_grid = std::max(rf_grid, (size_t)mx * b->sm_count);
     }
     if (rfc.empty()) return bfail(b, PORTAL_ERR_CUDA, "radiation-field kernel does not fit on an SM");
+    // the dynamic shared-memory limit of the largest candidate
+    auto raise_rf_limit = [&]() {
+        int most = 0;
+        for (const RFC &c : rfc)
+            if (rf_batch(b, nullptr, 0, c.nlg).warp_bytes > rf_batch(b, nullptr, 0, rfc[most].nlg).warp_bytes)
+                most = (int)(&c - rfc.data());
+        int mx = 0;
+        return rf_batch_blocks_per_sm(rf_batch(b, nullptr, 0, rfc[most].nlg), b->dust, &mx);
+    };
+    if (raise_rf_limit()) return bfail(b, PORTAL_ERR_CUDA, "occupancy query");
     std::vector<int> sec;
     for (int w : {2, 4, 8})
         if (wb * w <= 200 * 1024) sec.push_back(w);
@@ -239,8 +264,7 @@ extern "C" int portal_batch_prepare(portal_batch *b, int nth, int nph, int nvel,
         if (b->se_a64.reserve(most * b->se_a64_stride)) return bfail(b, PORTAL_ERR_NOMEM, "SE matrix scratch");
     }
     // walk scratch for the largest grid
-    const size_t warps = (size_t)2 * b->sm_count * 8;
-    if (b->walk.reserve(warps * 32 * (size_t)n_depth)) return bfail(b, PORTAL_ERR_NOMEM, "walk scratch");
+    if (b->walk.reserve(rf_grid * RF_BATCH_WARPS * rf_walk_records(n_depth))) return bfail(b, PORTAL_ERR_NOMEM, "walk scratch");
 
     b->tune.clear();
     if (autotune) {
@@ -250,10 +274,9 @@ extern "C" int portal_batch_prepare(portal_batch *b, int nth, int nph, int nvel,
             if (int rc = rf_pass(b->models[m], b->rf[m], b->stream)) return bfail(b, rc, b->models[m]->err);
         double best = 1e300;
         for (const RFC &c : rfc) {
-            RFBatch rb{b->d_rf.p, b->sample.p, b->n_sample, b->queue.p, b->walk.p, n_depth};
+            const RFBatch rb = rf_batch(b, b->sample.p, b->n_sample, c.nlg);
             double ms = 0.0;
-            int rc = time_launch(b, [&]() { return rf_batch_launch(b->stream, c.bps * b->sm_count, b->nch, b->dust,
-                                                                  c.nlg, b->max_lines, rb); }, &ms);
+            int rc = time_launch(b, [&]() { return rf_batch_launch(b->stream, c.bps * b->sm_count, b->dust, rb); }, &ms);
             if (rc) return rc;
             b->tune.insert(b->tune.end(), {(double)c.nlg, (double)c.bps, ms});
             if (ms < best) { best = ms; b->nlg = c.nlg; b->rf_bps = c.bps; }
@@ -272,10 +295,8 @@ extern "C" int portal_batch_prepare(portal_batch *b, int nth, int nph, int nvel,
         }
         se_batch_blocks_per_sm(sec.back(), wb, b->se_a64_stride, &dummy);
     } else {
-        b->nlg = 5;
-        b->rf_bps = 1;
-        for (const RFC &c : rfc)
-            if (c.nlg == 5) b->rf_bps = std::max(b->rf_bps, c.bps);
+        b->nlg = rfc[0].nlg;
+        b->rf_bps = rfc[0].bps;
         b->se_warps = sec.back();
         int bps = 0;
         se_batch_blocks_per_sm(b->se_warps, wb, b->se_a64_stride, &bps);

@@ -35,6 +35,14 @@ struct RFArgs {
     float *kmom;                      // (6, N) second moment sum w I n n of line 1 (xx yy zz xy xz yz) or null
     int2 *walk;
     unsigned long long *counters;
+    // ray-range items (small clouds): rays per item (0: one item per node), and
+    // what the items leave for k_rf_finish -- per (node, ray, line) channel sums
+    // (three planes with a split field), ray directions, segments per item (-1:
+    // a walk past n_depth)
+    int rays_per_item;
+    float *vray;
+    float4 *dray;
+    int *iseg;
 };
 
 // Everything the SE kernel reads or writes for one model.
@@ -89,7 +97,12 @@ struct RFBatch {
     unsigned long long *queue;   // [0] next item, [1] segments walked
     int2 *walk;                  // per warp: 32 rays x n_depth
     int n_depth;
-    int rem_lines;               // lines of the remainder channel's shared table (largest model)
+    int nch;                     // velocity channels and their tables (the same for every model)
+    const float *chq, *chw;
+    int max_group;               // widest line group
+    int rt;                      // remainder channel integrated lanes-over-lines
+    int split;                   // the models have split fields
+    size_t warp_bytes;           // dynamic shared memory per warp (largest model)
 };
 struct SEBatch {
     const SEArgs *models;
@@ -104,9 +117,16 @@ struct SEBatch {
 int rf_prepare(portal_ctx *c, int nth, int nph, int nvel, const double *gvec, double dx, int n_depth,
                bool split, RFArgs *a);
 int rf_pass(portal_ctx *c, const RFArgs &a, cudaStream_t s);
-int rf_batch_blocks_per_sm(int nch, bool dust, int nlg, int max_lines, int *blocks);
-const void *rf_batch_kernel_ptr(int nch, bool dust, int nlg, int max_lines);  // identity of the variant
-int rf_batch_launch(cudaStream_t s, int grid, int nch, bool dust, int nlg, int max_lines, const RFBatch &bw);
+const void *rf_kernel_narrow(int nlg);   // the single-model kernel for groups of nlg lines: 1..5,
+const void *rf_kernel_wide(int nlg);     // 6..10,
+const void *rf_kernel_dust(int nlg);     // with dust, 1..5
+size_t rf_walk_records(int n_depth);     // walk scratch per warp, int2 records
+// the batched launch: its shape for these models (max_group: the widest line
+// group wanted), and the blocks per SM the kernel reaches with it
+void rf_batch_shape(RFBatch *bw, const int *lines, int n_models, int nch, bool dust, int max_group, bool split);
+int rf_batch_blocks_per_sm(const RFBatch &bw, bool dust, int *blocks);
+int rf_batch_launch(cudaStream_t s, int grid, bool dust, const RFBatch &bw);
+constexpr int RF_BATCH_WARPS = 4;        // warps per block of the batched launch
 // se.cu
 int se_prepare(portal_ctx *c, int kmax, SEArgs *a, size_t *warp_bytes);
 int se_pass(portal_ctx *c, cudaStream_t s);

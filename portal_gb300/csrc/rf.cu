@@ -87,70 +87,130 @@ int upload_lines(portal_ctx *c) {
     return PORTAL_OK;
 }
 
-// Warps per block of the radiation-field kernel: 8, or PORTAL_RF_WARPS (4..8)
-// -- fewer warps per block let a register-heavy variant keep two blocks on
-// an SM.
+// Warps per block of the radiation-field kernel: 4, or PORTAL_RF_WARPS (4..8).
 inline int rf_warps() {
     const char *e = getenv("PORTAL_RF_WARPS");
-    const int v = e ? atoi(e) : 8;
-    return (v >= 4 && v <= 8) ? v : 8;
+    const int v = e ? atoi(e) : 4;
+    return (v >= 4 && v <= 8) ? v : 4;
 }
 
-template <int NS, int NLG, bool DUST, int RT>
-int launch_rf(portal_ctx *c, RFArgs &a, int n_depth) {
-    auto kern = k_radiation_field<NS, NLG, DUST, false, RT>;
-    const int wpb = rf_warps();
-    // the remainder channel's (cell, line) tables, one per warp
-    const size_t dyn = RT ? (size_t)wpb * 32 * rem_row_stride(a.L) * sizeof(float2) : 0;
-    if (dyn) PCHECK(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
-    int nb = 0;
-    PCHECK(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, 32 * wpb, dyn));
-    if (nb < 1) nb = 1;
-    int grid = nb * c->sm_count;
-    size_t nslots = (size_t)grid * wpb;
-    if (c->walk.reserve(nslots * 32 * (size_t)n_depth) != cudaSuccess)
-        return set_err(c, PORTAL_ERR_NOMEM, "walk scratch allocation failed");
-    a.walk = c->walk.p;
-    PCHECK(c, cudaMemsetAsync(c->counters.p, 0, 8 * sizeof(unsigned long long), c->stream));
-    timer_start(c, T_RF);
-    kern<<<grid, 32 * wpb, dyn, c->stream>>>(a, RFBatch{});
-    timer_stop(c, T_RF);
-    PCHECK(c, cudaGetLastError());
-    return PORTAL_OK;
-}
-
-// Line-group width: lines whose intensities one lane keeps in registers at
-// once.  Lines are padded to whole groups, and a padding line costs as much
-// as a real one, so the width is the one of 5, 4, 3 with the fewest padded
-// lines (the larger on ties: fewer passes over the walk lists); 10 saves
-// profile evaluations but needs more than 128 registers (one block per SM).
-// PORTAL_RF_LINE_GROUP=3|4|5|10 overrides the choice.
-inline int line_group(int L) {
+// The widest line group: lines are split into the fewest groups of at most
+// this many, of equal width.  PORTAL_RF_LINE_GROUP=3|4|5|10 overrides.
+inline int max_line_group() {
     const char *e = getenv("PORTAL_RF_LINE_GROUP");
     if (e) {
         const int v = atoi(e);
         if (v == 3 || v == 4 || v == 5 || v == 10) return v;
     }
-    int best = 5, slots = 1 << 30;
-    for (int g : {5, 4, 3}) {
-        const int sl = ((L + g - 1) / g) * g;
-        if (sl < slots) { slots = sl; best = g; }
-    }
-    return best;
+    return RF_MAX_GROUP;
 }
 
-template <int NS, int RT>
-int dispatch_nlg(portal_ctx *c, RFArgs &a, int n_depth) {
-    if (c->has_dust) {  // the dust variants: groups of 5 (or 10), whole slots
-        return line_group(a.L) == 10 ? launch_rf<NS, 10, true, 0>(c, a, n_depth)
-                                     : launch_rf<NS, 5, true, 0>(c, a, n_depth);
+// Ray-range items: sums the items' per-ray channel sums of every node in ray
+// order (one warp per node, lane = line), as the whole-node items do.
+__global__ void __launch_bounds__(128) k_rf_finish(RFArgs a, int per_node, int split) {
+    const int lane = threadIdx.x & 31;
+    const int node = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
+    if (node >= a.bulk) return;
+    int st = 0, seg = 0;
+    for (int p = 0; p < per_node; p++) {
+        const int s = a.iseg[(size_t)node * per_node + p];
+        if (s < 0) {   // the walks stop at this item, as the whole-node loop does
+            st = PORTAL_NODE_DEPTH;
+            break;
+        }
+        seg += s;
     }
-    switch (line_group(a.L)) {
-    case 3: return launch_rf<NS, 3, false, RT>(c, a, n_depth);
-    case 4: return launch_rf<NS, 4, false, RT>(c, a, n_depth);
-    case 10: return RT ? launch_rf<NS, 5, false, RT>(c, a, n_depth) : launch_rf<NS, 10, false, 0>(c, a, n_depth);
-    default: return launch_rf<NS, 5, false, RT>(c, a, n_depth);
+    const bool on = st == 0 && a.ab[node] > 0.0;
+    const int L = a.L;
+    const size_t ray0 = (size_t)node * a.ndir, plane = (size_t)a.bulk * a.ndir * L;
+    float km = 0.f;
+    for (int l = lane; l - lane < L; l += 32) {
+        NodeSum s;
+        const int line = min(l, L - 1);
+        for (int r0 = 0; on && r0 < a.ndir; r0 += 32) {
+            const int nr = min(32, a.ndir - r0);
+            const double *dr = a.dirs + 6 * (size_t)(r0 + min(lane, nr - 1));
+            const float w = (float)dr[4], w2 = (float)dr[5];
+            const float *v = a.vray + (ray0 + r0) * L + line;
+#pragma unroll 8
+            for (int r = 0; r < nr; r++) {
+                const float2 wt = make_float2(__shfl_sync(0xffffffffu, w, r), __shfl_sync(0xffffffffu, w2, r));
+                s.add(wt, v[(size_t)r * L]);
+                if (split) s.add_split(wt.x, v[plane + (size_t)r * L], v[2 * plane + (size_t)r * L]);
+            }
+            if (l == lane && lane < 6) {
+                const float *v0 = a.vray + (ray0 + r0) * L;
+                for (int r = 0; r < nr; r++)
+                    km = moment_add(km, lane, (float)a.dirs[6 * (size_t)(r0 + r) + 4], v0[(size_t)r * L],
+                                    a.dray[ray0 + r0 + r]);
+            }
+        }
+        if (l >= L) continue;
+        a.J0[(size_t)node * L + l] = on ? s.j0.value() : 0.0;
+        a.J2[(size_t)node * L + l] = on ? s.j2.value() : 0.0;
+        if (split) {
+            a.JE[(size_t)node * L + l] = on ? s.je.value() : 0.0;
+            a.LS[(size_t)node * L + l] = on ? s.ls.value() : 0.0;
+        }
     }
+    if (a.kmom && lane < 6) a.kmom[(size_t)lane * a.N + node] = on ? km : 0.f;
+    if (lane == 0) {
+        a.status[node] = st;
+        if (a.segs) a.segs[node] = seg;
+        atomicAdd(&a.counters[1], (unsigned long long)seg);
+    }
+}
+
+// Rays per item: 0 (a warp per node) for clouds of many nodes; smaller ones
+// are split into ray ranges, so that every resident warp has several items
+// and the last ones to finish do not leave the GPU idle.
+inline int rays_per_item(const RFArgs &a, bool split, long long resident) {
+    if (a.bulk >= 16 * resident || a.ndir <= 8) return 0;
+    if ((double)a.bulk * a.ndir * (a.L * (split ? 3 : 1) * 4 + 16) > 2e9) return 0;   // scratch limit
+    for (int r : {32, 16})
+        if ((long long)a.bulk * ((a.ndir + r - 1) / r) >= 4 * resident) return r;
+    return 8;
+}
+
+int launch_rf(portal_ctx *c, RFArgs &a, int n_depth) {
+    const bool dust = c->has_dust, split = a.JE != nullptr;
+    const int rt = rf_remainder(a.nch, dust, a.L);
+    RFShape sh = rf_shape(a.L, max_line_group(), a.nch, dust, rt, split);
+    const void *kern = dust ? rf_kernel_dust(sh.nlg) : sh.nlg <= 5 ? rf_kernel_narrow(sh.nlg) : rf_kernel_wide(sh.nlg);
+    const size_t table = (a.nch * sizeof(float2) + 15) & ~(size_t)15;
+    int wpb = rf_warps();
+    while (wpb > 1 && table + (size_t)wpb * sh.bytes > 200 * 1024) wpb--;   // many lines and channels
+    const size_t dyn = table + (size_t)wpb * sh.bytes;
+    PCHECK(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+    int nb = 0;
+    PCHECK(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, 32 * wpb, dyn));
+    if (nb < 1) nb = 1;
+    // fewer blocks per SM where the device cannot hold the walk scratch of all
+    while (c->walk.reserve((size_t)nb * c->sm_count * wpb * rf_walk_records(n_depth)) != cudaSuccess) {
+        cudaGetLastError();
+        if (--nb < 1) return set_err(c, PORTAL_ERR_NOMEM, "walk scratch allocation failed");
+    }
+    const int grid = nb * c->sm_count;
+    const size_t nslots = (size_t)grid * wpb;
+    a.walk = c->walk.p;
+    a.rays_per_item = rays_per_item(a, split, (long long)nslots);
+    const int per_node = a.rays_per_item ? (a.ndir + a.rays_per_item - 1) / a.rays_per_item : 1;
+    if (a.rays_per_item) {
+        const size_t rays = (size_t)a.bulk * a.ndir;
+        if (c->vray.reserve(rays * a.L * (split ? 3 : 1)) || c->dray.reserve(rays) ||
+            c->iseg.reserve((size_t)a.bulk * per_node))
+            return set_err(c, PORTAL_ERR_NOMEM, "ray sums");
+        a.vray = c->vray.p; a.dray = c->dray.p; a.iseg = c->iseg.p;
+    }
+    PCHECK(c, cudaMemsetAsync(c->counters.p, 0, 8 * sizeof(unsigned long long), c->stream));
+    timer_start(c, T_RF);
+    RFBatch none{};
+    void *args[] = {&a, &none, &sh};
+    PCHECK(c, cudaLaunchKernel(kern, dim3(grid), dim3(32 * wpb), args, dyn, c->stream));
+    if (a.rays_per_item && a.bulk > 0) k_rf_finish<<<(a.bulk + 3) / 4, 128, 0, c->stream>>>(a, per_node, split);
+    timer_stop(c, T_RF);
+    PCHECK(c, cudaGetLastError());
+    return PORTAL_OK;
 }
 
 // Star mode: the node loop through the batched kernel with one model.  Its
@@ -158,13 +218,14 @@ int dispatch_nlg(portal_ctx *c, RFArgs &a, int n_depth) {
 // single-model kernel leaves that code out, which keeps its registers for the
 // integration (1 % faster on the benchmark sphere).
 int launch_rf_star(portal_ctx *c, RFArgs &a, int n_depth) {
-    const int nlg = (c->has_dust && line_group(a.L) == 10) ? 10 : 5;
+    RFBatch bw{};
+    rf_batch_shape(&bw, &a.L, 1, a.nch, c->has_dust, max_line_group(), a.JE != nullptr);
     int nb = 0;
-    if (rf_batch_blocks_per_sm(a.nch, c->has_dust, nlg, a.L, &nb))
+    if (rf_batch_blocks_per_sm(bw, c->has_dust, &nb))
         return set_err(c, PORTAL_ERR_CUDA, "star mode: occupancy query failed");
     if (nb < 1) nb = 1;
     const int grid = nb * c->sm_count;
-    if (c->walk.reserve((size_t)grid * 8 * 32 * (size_t)n_depth) != cudaSuccess)
+    if (c->walk.reserve((size_t)grid * RF_BATCH_WARPS * rf_walk_records(n_depth)) != cudaSuccess)
         return set_err(c, PORTAL_ERR_NOMEM, "walk scratch allocation failed");
     if (c->star_model.reserve(sizeof(RFArgs)) || c->star_items.reserve(c->bulk > 0 ? c->bulk : 1))
         return set_err(c, PORTAL_ERR_NOMEM, "star-mode work items");
@@ -179,15 +240,16 @@ int launch_rf_star(portal_ctx *c, RFArgs &a, int n_depth) {
     a.walk = c->walk.p;
     PCHECK(c, cudaMemcpyAsync(c->star_model.p, &a, sizeof(RFArgs), cudaMemcpyHostToDevice, c->stream));
     PCHECK(c, cudaMemsetAsync(c->counters.p, 0, 8 * sizeof(unsigned long long), c->stream));
-    RFBatch bw;
     bw.models = reinterpret_cast<const RFArgs *>(c->star_model.p);
     bw.items = c->star_items.p;
     bw.n_items = c->bulk;
     bw.queue = c->counters.p;  // [0] next item, [1] segments, as the single-model kernel's counters
     bw.walk = c->walk.p;
     bw.n_depth = n_depth;
+    bw.chq = a.chq;
+    bw.chw = a.chw;
     timer_start(c, T_RF);
-    const int rc = rf_batch_launch(c->stream, grid, a.nch, c->has_dust, nlg, a.L, bw);
+    const int rc = rf_batch_launch(c->stream, grid, c->has_dust, bw);
     timer_stop(c, T_RF);
     if (rc) return set_err(c, rc, std::string("star mode: ") + cudaGetErrorString(cudaGetLastError()));
     // the argument block is read by the kernel: keep it until the stream passes here
@@ -196,28 +258,14 @@ int launch_rf_star(portal_ctx *c, RFArgs &a, int n_depth) {
 }
 
 int dispatch_rf(portal_ctx *c, RFArgs &a, int n_depth) {
-    if (a.star) return launch_rf_star(c, a, n_depth);
-    const ChanLayout cl = chan_layout(a.nch, c->has_dust, a.L);
-    if (cl.rt) {
-        switch (cl.ns) {
-        case 1: return dispatch_nlg<1, 1>(c, a, n_depth);
-        case 2: return dispatch_nlg<2, 1>(c, a, n_depth);
-        case 4: return dispatch_nlg<4, 1>(c, a, n_depth);
-        default: return dispatch_nlg<8, 1>(c, a, n_depth);
-        }
-    }
-    switch (cl.ns) {
-    case 1: return dispatch_nlg<1, 0>(c, a, n_depth);
-    case 2: return dispatch_nlg<2, 0>(c, a, n_depth);
-    case 3: return dispatch_nlg<3, 0>(c, a, n_depth);
-    case 5: return dispatch_nlg<5, 0>(c, a, n_depth);
-    default: return dispatch_nlg<9, 0>(c, a, n_depth);
-    }
+    return a.star ? launch_rf_star(c, a, n_depth) : launch_rf(c, a, n_depth);
 }
 
 }  // namespace
 
 namespace portal {
+
+size_t rf_walk_records(int n_depth) { return (size_t)1024 * (size_t)((n_depth + 31) / 32); }
 
 // Validates the call, uploads the molecule's line constants and the
 // direction / channel tables, sizes the outputs and fills the kernel's
@@ -289,6 +337,8 @@ int rf_prepare(portal_ctx *c, int nth, int nph, int nvel, const double *gvec, do
     a.JE = split ? c->JE.p : nullptr;
     a.LS = split ? c->LS.p : nullptr;
     a.walk = nullptr;
+    a.rays_per_item = 0;
+    a.vray = nullptr; a.dray = nullptr; a.iseg = nullptr;
     // the line table's transfer step (main_para.f90:135 dx times r_max)
     c->rf_dxp = c->tx * dx;
     *out = a;

@@ -7,6 +7,8 @@
 
 #include <cmath>
 
+#include <algorithm>
+
 #include "internal.cuh"
 
 using namespace portal;
@@ -53,36 +55,6 @@ struct KahanF {
     __device__ __forceinline__ double value() const { return (double)s - (double)c; }
 };
 
-// Row stride (float2 per cell) of the remainder channel's (cell, line)
-// table: odd, so the staging lanes' 64-bit row stores of a half-warp fall in
-// distinct banks.
-__host__ __device__ __forceinline__ int rem_row_stride(int lines) { return lines | 1; }
-
-// Line groups up to these widths run the cell loop two cells per iteration,
-// and instantiate it for every count of Taylor-only lines; wider groups one
-// cell per iteration, all or none of the lines Taylor-only (the larger
-// bodies cost more in instruction fetch than they gain).
-constexpr int UNROLL_MAX_NLG = 4;
-constexpr int SUFFIX_MAX_NLG = 3;
-
-// f(std::integral_constant<int, k>) for the run-time count k in [0, NLG] of
-// Taylor-only lines: every k for groups up to SUFFIX_MAX_NLG lines, 0 or NLG
-// for wider ones, 0 alone with dust
-template <int NLG, bool DUST, int K = 0, typename F>
-__device__ __forceinline__ void with_thin_lines(int k, F &f) {
-    if constexpr (DUST) {
-        f(std::integral_constant<int, 0>{});
-    } else if constexpr (NLG > SUFFIX_MAX_NLG) {
-        if (k == NLG) f(std::integral_constant<int, NLG>{});
-        else f(std::integral_constant<int, 0>{});
-    } else if constexpr (K < NLG) {
-        if (k == K) f(std::integral_constant<int, K>{});
-        else with_thin_lines<NLG, DUST, K + 1>(k, f);
-    } else {
-        f(std::integral_constant<int, NLG>{});
-    }
-}
-
 __device__ __forceinline__ float ex2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -121,34 +93,6 @@ __global__ void k_line_table(int N, int L, double dxp, const LineConst *__restri
     // FP32 denormals
     ltab[t] = make_float4((float)(kv * phif), (float)(kv != 0.0 ? ev / kv : 0.0), (float)Ad, (float)(Ad * Ibb));
 }
-
-template <int NLG, bool DUST>
-struct CellRec {
-    float2 qd[32];       // profile argument at channel 0 and its step per channel, times sqrt(log2 e)
-    float2 AS[32][NLG];  // (A * steps, S) without dust, (A * steps, E * steps) with dust
-    float Ad[32][DUST ? NLG : 1];   // dust tau per cell (dust only)
-    float Jd[32][DUST ? NLG : 1];   // dust emissivity * steps (dust only)
-};
-
-// Per-warp shared state of the node being processed and its current batch of
-// (up to) 32 rays (RayBatch; RayBatchStar in the batched kernel).
-struct RayBatch {
-    double frame[13];    // b(3), x(3), w(3), node position(3), |p|^2
-    float4 dir[32];      // (d_x, d_y, d_z, v_node . d) per ray
-    int K[32];           // segments per ray (-1: n_depth overflow)
-    float km[6];         // the node's second moment of line 1 (lane 0 accumulates)
-};
-// The batched kernel's: also the per-node ray sets of star mode.
-struct RayBatchStar {
-    double frame[13];
-    double sk[7];        // star direction k(3), th_star, dth_star, dth_rest, th_i
-    int sn[2];           // star rays, all rays of the node (-1: more than nth nph)
-    unsigned smask;      // star rays of the batch
-    float4 dir[32];
-    float2 wts[32];      // (w, w c_in / sqrt 2) per ray
-    int K[32];
-    float km[6];
-};
 
 constexpr double PI_D = 3.141592653589793;  // acos(-1.d0)
 
@@ -272,40 +216,607 @@ __device__ __noinline__ double star_exit(double sexit, double px, double py, dou
     return sexit;
 }
 
-// NS channel slots per lane, NLG lines per register group.
-// RT = 0: nch <= 32 NS, every channel in a slot.  RT = 1: nch = 32 NS + 1
-// (the reference's 2 nvel + 1 channels with nvel a multiple of 16): the
-// last channel (nv = +nvel) is integrated lanes-over-lines (lane = line,
-// L <= 32) in the first line-group pass instead of costing a whole slot of
-// 32 lanes for one channel.  Its transfer weights (1 - e^-tau, S) per (cell,
-// line) are formed by the staging lanes (lane = cell) into a per-warp table
-// of dynamic shared memory, rem_row_stride(L) float2 per cell; the
-// lanes-over-lines pass then only runs the recurrence.
+// Per-warp state of the node being processed and its current batch of (up
+// to) 32 rays.
+struct RayBatch {
+    double frame[13];    // b(3), x(3), w(3), node position(3), |p|^2
+    float4 dir[32];      // (d_x, d_y, d_z, v_node . d) per ray
+    float2 wts[32];      // (w, w c_in / sqrt 2) per ray
+    int K[32];           // segments per ray
+    int st0[32];         // trace steps in the node's own cell
+    float km[6];         // the node's second moment of line 1
+};
+// The batched kernel's: also the per-node ray sets of star mode.
+struct RayBatchStar : RayBatch {
+    double sk[7];        // star direction k(3), th_star, dth_star, dth_rest, th_i
+    int sn[2];           // star rays, all rays of the node (-1: more than nth nph)
+    unsigned smask;      // star rays of the batch
+};
+constexpr int RF_RAYS_BYTES = (sizeof(RayBatchStar) + 15) & ~15;   // at the start of the warp's shared memory
+
+// ---- shape of a launch: line groups and the warp's shared-memory layout ----
+// Lines are integrated in groups of nlg (the group's intensities of one pass
+// over the channels live in registers).  A pass covers two slots of 32
+// channels (the last one, when the slot count is odd, a single slot); the
+// intensities of the passes not running wait in shared memory between two
+// chunks of 32 cells.  Without dust, lines are handled in packs of two on the
+// packed FP32x2 pipe (the last line of an odd group packs its two channel
+// slots instead); with dust one by one.
+struct RFShape {
+    int L, nlg, groups, npk, nslot, rt, split;
+    int rec_ld, om_ld;                    // row strides: float4 per cell, float per cell
+    int o_rec, o_qd, o_om, o_I, o_part, o_v, o_acc, o_row, o_bb, bytes;   // byte offsets in the warp's block
+};
+constexpr int RF_MAX_GROUP = 10;          // lines per group without dust
+constexpr int RF_MAX_GROUP_DUST = 5;      // with dust (a wider body costs more in registers than it gains)
+
+// The remainder channel: 2 nvel + 1 channels with nvel a multiple of 16 are
+// whole slots and one channel more, which the lanes-over-lines pass takes (no
+// dust, at most 32 lines); any other count is padded to whole slots.
+__host__ __device__ inline int rf_remainder(int nch, bool dust, int max_lines) {
+    const int k = nch / 32;
+    return (!dust && max_lines <= 32 && nch % 32 == 1 && (k == 1 || k == 2 || k == 4 || k == 8)) ? 1 : 0;
+}
+
+__host__ __device__ inline RFShape rf_shape(int L, int max_group, int nch, bool dust, int rt, bool split) {
+    RFShape s;
+    const int cap = dust ? (max_group < RF_MAX_GROUP_DUST ? max_group : RF_MAX_GROUP_DUST) : max_group;
+    s.L = L;
+    s.groups = (L + cap - 1) / cap;
+    s.nlg = (L + s.groups - 1) / s.groups;
+    s.npk = (s.nlg + 1) / 2;
+    s.rt = rt;
+    s.split = split;
+    s.nslot = (nch - rt + 31) / 32;
+    s.rec_ld = (dust ? s.nlg : s.npk) | 1;
+    s.om_ld = s.nlg | 1;
+    const int nq = split ? 3 : 1;
+    int o = RF_RAYS_BYTES;
+    s.o_rec = o; o += 32 * s.rec_ld * 16;
+    s.o_qd = o; o += 32 * 16;
+    s.o_I = o; o += ((s.nslot / 2) * s.nlg + (s.nslot & 1) * s.npk) * 32 * 8;
+    s.o_part = o; o += nq * s.npk * 32 * 8;
+    s.o_row = o; o += s.groups * (dust ? s.nlg : s.npk) * 16;
+    s.o_bb = o; o += 2 * s.groups * 2 * s.npk * 4;
+    s.o_om = o; o += rt ? 32 * s.om_ld * 4 : 0;
+    s.o_v = o; o += nq * 32 * L * 4;
+    s.o_acc = o; o += (split ? 8 : 4) * L * 4;
+    s.bytes = (o + 15) & ~15;
+    return s;
+}
+
+// Index of record k of a ray in its warp's walk scratch: blocks of 32
+// records, the 32 rays' blocks side by side, so that a warp's live part of
+// the scratch is a few consecutive kilobytes (not 32 streams n_depth records
+// apart) and a chunk of 32 cells is read from two such blocks at most.
+__device__ __forceinline__ int walk_at(int k, int ray) { return ((k >> 5) << 10) + (ray << 5) + (k & 31); }
+
+// f(std::integral_constant<int, k>) for the run-time count k of the group's
+// trailing packs that take the Taylor form alone
+template <int NPK, int K = 0, typename F>
+__device__ __forceinline__ void with_thin_packs(int k, F &f) {
+    if constexpr (K < NPK) {
+        if (k == K) f(std::integral_constant<int, K>{});
+        else with_thin_packs<NPK, K + 1>(k, f);
+    } else {
+        f(std::integral_constant<int, NPK>{});
+    }
+}
+
+// I' = I + (1 - e^-tau)(S - I) for two updates on the packed pipe, x = tau
+// log2 e >= 0 (lines with kv <= 0 and padding lines carry A = S = 0).  The
+// Taylor value is overwritten by 1 - e where x reaches the switch: a compare
+// and a predicated subtraction per element, one issue slot less than forming
+// 1 - e for both and selecting (the same value: one_minus_exp2).
+// thin is a compile-time constant once the pack loops are unrolled.
+__device__ __forceinline__ void transfer2(bool thin, float2 &I, float2 A2, float2 S2, float2 g2) {
+    const float2 x = __fmul2_rn(A2, g2);
+    float2 om = om_taylor2(x);
+    if (!thin) {
+        const float e0 = ex2(-x.x), e1 = ex2(-x.y);
+        asm("{\n .reg .pred p;\n setp.ge.f32 p, %1, %3;\n @p sub.rn.f32 %0, %4, %2;\n}"
+            : "+f"(om.x) : "f"(x.x), "f"(e0), "f"(OM_TAYLOR_X), "f"(1.f));
+        asm("{\n .reg .pred p;\n setp.ge.f32 p, %1, %3;\n @p sub.rn.f32 %0, %4, %2;\n}"
+            : "+f"(om.y) : "f"(x.y), "f"(e1), "f"(OM_TAYLOR_X), "f"(1.f));
+    }
+    I = __ffma2_rn(om, __ffma2_rn(I, make_float2(-1.f, -1.f), S2), I);
+}
+__device__ __forceinline__ void transfer1(bool thin, float &I, float A, float S, float g) {
+    const float x = A * g;
+    const float om = thin ? om_taylor(x) : one_minus_exp(x, ex2(-x));
+    I = fmaf(om, S - I, I);
+}
+
+// Sums of N per-lane values over the warp, value l's sum on every lane whose
+// low bits name it (sum_line).  Each butterfly step halves the values a lane
+// carries while there are two or more left; every sum adds the same partners
+// in the same order as N separate butterflies over 16, 8, 4, 2, 1 would.
+template <int N>
+__device__ __forceinline__ float sum_lines(const float (&v)[N], int o, int lane) {
+    if constexpr (N == 1) {
+        float x = v[0];
+        for (; o >= 1; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        return x;
+    } else {
+        constexpr int H = (N + 1) / 2;
+        float w[H];
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < H; i++) {
+            const float b = (2 * i + 1 < N) ? v[2 * i + 1 < N ? 2 * i + 1 : 0] : 0.f;
+            const float keep = up ? b : v[2 * i], send = up ? v[2 * i] : b;
+            w[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+        return sum_lines<H>(w, o >> 1, lane);
+    }
+}
+template <int N>
+__device__ __forceinline__ int sum_line(int lane) {
+    int l = 0, bit = 0;
+    for (int n = N, o = 16; n > 1; n = (n + 1) / 2, o >>= 1, bit++)
+        if (lane & o) l |= 1 << bit;
+    return l;
+}
+
+// Everything of one warp in shared memory.
+struct WarpMem {
+    unsigned char *p;
+    __device__ __forceinline__ float4 *rec(const RFShape &s) const { return (float4 *)(p + s.o_rec); }
+    __device__ __forceinline__ float4 *qd(const RFShape &s) const { return (float4 *)(p + s.o_qd); }
+    __device__ __forceinline__ float *om(const RFShape &s) const { return (float *)(p + s.o_om); }
+    __device__ __forceinline__ float2 *I(const RFShape &s) const { return (float2 *)(p + s.o_I); }
+    __device__ __forceinline__ float2 *part(const RFShape &s) const { return (float2 *)(p + s.o_part); }
+    __device__ __forceinline__ float4 *row(const RFShape &s) const { return (float4 *)(p + s.o_row); }
+    __device__ __forceinline__ float *bb(const RFShape &s) const { return (float *)(p + s.o_bb); }
+    __device__ __forceinline__ float *v(const RFShape &s) const { return (float *)(p + s.o_v); }
+    __device__ __forceinline__ float *acc(const RFShape &s) const { return (float *)(p + s.o_acc); }
+};
+
+// One pass over NSL channel slots (from slot s0) of a chunk of nc cells for
+// the line group g without dust: tk of the group's trailing packs take the
+// Taylor form alone.  first: the intensities start from the background bb;
+// last: the central cell and the weighted channel sums follow, else the
+// intensities go back to shared memory.
+template <int NLG, int NSL>
+__device__ __forceinline__ void channel_pass(const RFShape &sh, const WarpMem &m, const float2 *chtab, int nch,
+                                             int nvel, int lane, int g, int s0, int nc, int tk, bool first,
+                                             bool last, const float *bb, float fst0) {
+    constexpr int NP = NLG / 2, ODD = NLG & 1, NPK = NP + ODD;
+    float2 I[NSL][NP > 0 ? NP : 1], Io;   // Io: the odd line's slots
+    float2 *sv = m.I(sh) + (size_t)(s0 / 2) * NLG * 32 + lane;
+    if (first) {
+#pragma unroll
+        for (int k = 0; k < NP; k++)
+#pragma unroll
+            for (int s = 0; s < NSL; s++) I[s][k] = make_float2(bb[2 * k], bb[2 * k + 1]);
+        if (ODD) Io = make_float2(bb[NLG - 1], bb[NLG - 1]);
+    } else {
+#pragma unroll
+        for (int s = 0; s < NSL; s++)
+#pragma unroll
+            for (int k = 0; k < NP; k++) I[s][k] = sv[(s * NP + k) * 32];
+        if (ODD) Io = sv[NSL * NP * 32];
+    }
+    const float4 *rec = m.rec(sh), *qd = m.qd(sh);
+    const float2 ch2 = make_float2((float)(lane + 32 * s0 - nvel), (float)(lane + 32 * (s0 + 1) - nvel));
+    auto run = [&](auto tag) {
+        constexpr int TK = decltype(tag)::value;
+        auto cell = [&](int u) {
+            const float4 q4 = qd[u];
+            // Gaussian profile of the cell at the lane's channels, exp(-q^2) =
+            // 2^(-q'^2) with q' = q sqrt(log2 e) (staged scaled)
+            float gs[2];
+            if (NSL == 2) {
+                const float2 q = __ffma2_rn(make_float2(q4.z, q4.w), ch2, make_float2(q4.x, q4.y));
+                const float2 t = __fmul2_rn(q, q);
+                gs[0] = ex2(-t.x);
+                gs[1] = ex2(-t.y);
+            } else {
+                const float q = fmaf(q4.z, ch2.x, q4.x);
+                gs[0] = gs[1] = ex2(-(q * q));
+            }
+            const float4 *r = rec + u * sh.rec_ld;
+#pragma unroll
+            for (int k = 0; k < NP; k++) {
+                const float4 v = r[k];
+#pragma unroll
+                for (int s = 0; s < NSL; s++)
+                    transfer2(k >= NPK - TK, I[s][k], make_float2(v.x, v.y), make_float2(v.z, v.w),
+                              make_float2(gs[s], gs[s]));
+            }
+            if (ODD) {
+                const float4 v = r[NP];
+                if (NSL == 2)
+                    transfer2(TK >= 1, Io, make_float2(v.x, v.y), make_float2(v.z, v.w), make_float2(gs[0], gs[1]));
+                else
+                    transfer1(TK >= 1, Io.x, v.x, v.z, gs[0]);
+            }
+        };
+        // enough independent updates in flight per iteration: narrow groups
+        // run several cells at once (their weights do not depend on each other)
+        constexpr int U = NSL * NLG >= 10 ? 1 : NSL * NLG >= 5 ? 2 : 4;
+#pragma unroll U
+        for (int u = 0; u < nc; u++) cell(u);
+    };
+    with_thin_packs<NPK>(tk, run);
+    if (!last) {
+#pragma unroll
+        for (int s = 0; s < NSL; s++)
+#pragma unroll
+            for (int k = 0; k < NP; k++) sv[(s * NP + k) * 32] = I[s][k];
+        if (ODD) sv[NSL * NP * 32] = Io;
+        return;
+    }
+    // central cell (inverse_rt.f90:320-339): no gate, profile at the node's own
+    // b, then the weighted channel sum, slot by slot
+    float2 *part = m.part(sh) + lane;
+    const float4 *row = m.row(sh) + g * NPK;
+    const int np32 = sh.npk * 32;
+    auto weigh = [&](float2 &I2, float4 v, float2 g0, float2 &om, float2 &Ie) {
+        const float2 x = __fmul2_rn(__fmul2_rn(__fmul2_rn(make_float2(v.x, v.y), g0), make_float2(fst0, fst0)),
+                                    make_float2(LOG2E_F, LOG2E_F));
+        om = one_minus_exp2(x, ex2(-x.x), ex2(-x.y));
+        const float2 mI = __fmul2_rn(I2, make_float2(-1.f, -1.f));
+        Ie = __ffma2_rn(om, mI, I2);
+        return __ffma2_rn(om, __fadd2_rn(make_float2(v.z, v.w), mI), I2);
+    };
+#pragma unroll
+    for (int s = 0; s < NSL; s++) {
+        const int ch = lane + 32 * (s0 + s);
+        const bool valid = ch < nch - sh.rt;
+        const float2 ct = chtab[valid ? ch : 0];
+        const float2 g0 = make_float2(ct.x, ct.x), w2 = make_float2(ct.y, ct.y);
+#pragma unroll
+        for (int k = 0; k < NP; k++) {
+            float2 om, Ie;
+            const float2 o = weigh(I[s][k], row[k], g0, om, Ie);
+            if (valid) part[k * 32] = __ffma2_rn(w2, o, part[k * 32]);
+            if (sh.split && valid) {
+                part[np32 + k * 32] = __ffma2_rn(w2, Ie, part[np32 + k * 32]);
+                part[2 * np32 + k * 32] = __ffma2_rn(w2, om, part[2 * np32 + k * 32]);
+            }
+        }
+    }
+    if (ODD) {
+        const int ch = lane + 32 * s0;
+        const bool v0 = ch < nch - sh.rt, v1 = NSL == 2 && ch + 32 < nch - sh.rt;
+        const float2 c0 = chtab[v0 ? ch : 0], c1 = chtab[v1 ? ch + 32 : 0];
+        float2 om, Ie;
+        const float2 o = weigh(Io, row[NP], make_float2(c0.x, c1.x), om, Ie);
+        auto add = [&](float2 *q, float2 y) {
+            if (v0) q->x = fmaf(c0.y, y.x, q->x);
+            if (v1) q->x = fmaf(c1.y, y.y, q->x);
+        };
+        add(part + NP * 32, o);
+        if (sh.split) {
+            add(part + np32 + NP * 32, Ie);
+            add(part + 2 * np32 + NP * 32, om);
+        }
+    }
+}
+
+// The same with dust: line by line, tau = (kv phi + alpha) dx n, S = (ev phi
+// + j) / (kv phi + alpha), with ray_in's gate tau > 1e-30
+// (inverse_rt.f90:308).
+template <int NLG, int NSL>
+__device__ __forceinline__ void channel_pass_dust(const RFShape &sh, const WarpMem &m, const float2 *chtab, int nch,
+                                                  int nvel, int lane, int g, int s0, int nc, bool first, bool last,
+                                                  const float *bb, float fst0) {
+    float I[NSL][NLG];
+    float *sv = (float *)m.I(sh) + (size_t)s0 * NLG * 32 + lane;
+#pragma unroll
+    for (int s = 0; s < NSL; s++)
+#pragma unroll
+        for (int l = 0; l < NLG; l++) I[s][l] = first ? bb[l] : sv[(s * NLG + l) * 32];
+    const float4 *rec = m.rec(sh), *qd = m.qd(sh);
+    const float ch0 = (float)(lane + 32 * s0 - nvel), ch1 = (float)(lane + 32 * (s0 + 1) - nvel);
+#pragma unroll 1
+    for (int u = 0; u < nc; u++) {
+        const float4 q4 = qd[u];
+        float gs[2];
+        {
+            const float q = fmaf(q4.z, ch0, q4.x);
+            gs[0] = ex2(-(q * q));
+            gs[1] = 0.f;
+        }
+        if (NSL == 2) {
+            const float q = fmaf(q4.z, ch1, q4.x);
+            gs[1] = ex2(-(q * q));
+        }
+        const float4 *r = rec + u * sh.rec_ld;
+#pragma unroll
+        for (int l = 0; l < NLG; l++) {
+            const float4 v = r[l];
+#pragma unroll
+            for (int s = 0; s < NSL; s++) {
+                const float tau = fmaf(v.x, gs[s], v.z);
+                const float Sv = fmaf(v.y, gs[s], v.w) / tau;
+                const float x = tau * LOG2E_F;
+                const float om = one_minus_exp(x, ex2(-x));
+                const float In = fmaf(om, Sv - I[s][l], I[s][l]);
+                I[s][l] = (tau > 1e-30f) ? In : I[s][l];
+            }
+        }
+    }
+    if (!last) {
+#pragma unroll
+        for (int s = 0; s < NSL; s++)
+#pragma unroll
+            for (int l = 0; l < NLG; l++) sv[(s * NLG + l) * 32] = I[s][l];
+        return;
+    }
+    float *part = (float *)m.part(sh) + lane;     // [line][lane]
+    const float4 *row = m.row(sh) + g * NLG;
+    const int np32 = 2 * sh.npk * 32;
+#pragma unroll
+    for (int s = 0; s < NSL; s++) {
+        const int ch = lane + 32 * (s0 + s);
+        if (ch >= nch) continue;
+        const float2 ct = chtab[ch];
+#pragma unroll
+        for (int l = 0; l < NLG; l++) {
+            const float4 v = row[l];
+            const float kap = fmaf(v.x, ct.x, v.z);
+            const float tau = kap * fst0;
+            const float Sv = fmaf(v.y * v.x, ct.x, v.w) / kap;
+            const float x = tau * LOG2E_F;
+            const float om = one_minus_exp(x, ex2(-x));
+            const float Io = fmaf(om, Sv - I[s][l], I[s][l]);
+            part[l * 32] = fmaf(ct.y, Io, part[l * 32]);
+            if (sh.split) {
+                const float lf = v.x * ct.x / kap;   // line share of the opacity
+                const float Sd = v.w / kap;          // dust emission share of S
+                part[np32 + l * 32] = fmaf(ct.y, fmaf(om, Sd - I[s][l], I[s][l]), part[np32 + l * 32]);
+                part[2 * np32 + l * 32] = fmaf(ct.y, lf * om, part[2 * np32 + l * 32]);
+            }
+        }
+    }
+}
+
+// The channel integration of a warp's batch of nr walked rays: per ray and
+// line the weighted channel sum at the node (v), with split also those of
+// J_eff and L*.  One chunk of up to 32 cells at a time is staged in shared
+// memory (lane = cell); then lanes run over channels, pass by pass.
+template <int NLG, bool DUST, bool STAR>
+__device__ __forceinline__ void integrate_batch(const RFArgs &a, const RFShape &sh, const WarpMem &m,
+                                                const RayBatch &B, unsigned smask, const float2 *chtab,
+                                                const int2 *walk, int nr, float dqfac, int lane) {
+    const unsigned FULL = 0xffffffffu;
+    constexpr int NP = NLG / 2, ODD = NLG & 1, NPK = NP + ODD;
+    const int L = a.L, nch = a.nch, nvel = a.nvel;
+    float4 *rec = m.rec(sh) + lane * sh.rec_ld;
+    // walk records of a chunk (lane = cell), the next chunk's -- of this ray,
+    // the next line group or the next ray -- loaded while one is integrated
+    int2 wcp = make_int2(0, 0);
+    {
+        const int h = B.K[0] - 1;
+        if (lane < min(32, h)) wcp = walk[walk_at(h - lane, 0)];
+    }
+    for (int rr = 0; rr < nr; rr++) {
+        const int Kr = B.K[rr];
+        const float4 d4 = B.dir[rr];
+        const float fst0 = (float)B.st0[rr];
+        const float *bb0 = m.bb(sh) + ((STAR && ((smask >> rr) & 1u)) ? sh.groups * 2 * NPK : 0);
+        for (int g = 0; g < sh.groups; g++) {
+            const int l0 = g * NLG;
+            const float *bb = bb0 + g * 2 * NPK;
+            // the remainder channel of this lane's line (lane = line of the group)
+            float Irem = (sh.rt && lane < NLG) ? bb[lane] : 0.f;
+            {
+                float2 *part = m.part(sh) + lane;
+                for (int k = 0; k < (sh.split ? 3 : 1) * NPK; k++) part[k * 32] = make_float2(0.f, 0.f);
+            }
+            for (int hi = Kr - 1, first = 1;; hi -= 32, first = 0) {
+                const int nc = max(0, min(32, hi));
+                const bool last = hi <= 32;
+                const int2 wc = wcp;
+                {
+                    int nh, nrr = rr;
+                    if (!last) nh = hi - 32;
+                    else if (g + 1 < sh.groups) nh = Kr - 1;
+                    else if (rr + 1 < nr) { nrr = rr + 1; nh = B.K[rr + 1] - 1; }
+                    else nh = 0;
+                    if (lane < min(32, nh)) wcp = walk[walk_at(nh - lane, nrr)];
+                }
+                __syncwarp();
+                unsigned thin = (1u << NPK) - 1u;   // the packs thin in this cell
+                if (lane < nc) {
+                    const float4 cv = a.cellv[wc.x];
+                    const float4 *lt = a.ltab + (size_t)wc.x * L;
+                    const float fst = (float)wc.y;
+                    const float vp = fmaf(cv.z, d4.z, fmaf(cv.y, d4.y, __fmul_rn(cv.x, d4.x)));
+                    const float ib = SQL2E_F * (1.f / cv.w);
+                    const float2 qdl = make_float2((d4.w - vp) * ib, dqfac * ib);
+                    m.qd(sh)[lane] = make_float4(qdl.x, qdl.x, qdl.y, qdl.y);
+                    if constexpr (DUST) {
+#pragma unroll
+                        for (int l = 0; l < NLG; l++) {
+                            const float4 v = lt[min(l0 + l, L - 1)];
+                            rec[l] = make_float4(v.x * fst, v.y * v.x * fst, v.z * fst, v.w * fst);
+                        }
+                    } else {
+                        // optical depth at unit profile in log2 units (ex2 takes
+                        // it as is) and the source function.  A cell line with kv
+                        // <= 0 fails ray_in's gate tau > 1e-30 in every channel
+                        // (inverse_rt.f90:308), and so does a padding line of the
+                        // last group: both get A = S = 0, which leaves I unchanged
+                        // exactly; 0 < tau < 2^-54 rounds to a zero weight as in
+                        // FP64, so the gate needs no test.
+                        float2 v[NLG];
+#pragma unroll
+                        for (int l = 0; l < NLG; l++)
+                            v[l] = *reinterpret_cast<const float2 *>(lt + min(l0 + l, L - 1));
+#pragma unroll
+                        for (int l = 0; l < NLG; l++) {
+                            const bool on = v[l].x > 0.f && l0 + l < L;
+                            v[l].x = on ? v[l].x * fst * LOG2E_F : 0.f;
+                            v[l].y = on ? v[l].y : 0.f;
+                            if (!(v[l].x < OM_THIN_A)) thin &= ~(1u << (l / 2));
+                        }
+#pragma unroll
+                        for (int k = 0; k < NP; k++)
+                            rec[k] = make_float4(v[2 * k].x, v[2 * k + 1].x, v[2 * k].y, v[2 * k + 1].y);
+                        if (ODD) rec[NP] = make_float4(v[NLG - 1].x, v[NLG - 1].x, v[NLG - 1].y, v[NLG - 1].y);
+                        if (sh.rt) {
+                            // the remainder channel's transfer weight of this
+                            // cell for the group's lines
+                            const float q = fmaf(qdl.y, (float)(nch - 1 - nvel), qdl.x);
+                            const float gr = ex2(-(q * q));
+                            float *om = m.om(sh) + lane * sh.om_ld;
+#pragma unroll
+                            for (int l = 0; l < NLG; l++) {
+                                const float x = v[l].x * gr;
+                                om[l] = one_minus_exp(x, ex2(-x));
+                            }
+                        }
+                    }
+                }
+                // Packs whose lines' line-centre optical depth is below OM_THIN_A
+                // in every cell of the chunk take the Taylor form of 1 - e^-tau
+                // alone in every channel: the full update would pick exactly that
+                // value.  Decided per chunk, uniform over the warp, for the
+                // group's trailing packs (a rotor's higher lines are the thinner).
+                const int tk = DUST ? 0 : __clz(~(__reduce_and_sync(FULL, thin) << (32 - NPK)));
+                __syncwarp();
+                if (!DUST && sh.rt && lane < NLG) {
+                    const float *om = m.om(sh) + lane;
+                    const float *S = reinterpret_cast<const float *>(m.rec(sh) + (lane >> 1)) + 2 + (lane & 1);
+#pragma unroll 4
+                    for (int u = 0; u < nc; u++) Irem = fmaf(om[u * sh.om_ld], S[u * sh.rec_ld * 4] - Irem, Irem);
+                }
+                int s0 = 0;
+                for (; s0 + 1 < sh.nslot; s0 += 2) {
+                    if constexpr (DUST)
+                        channel_pass_dust<NLG, 2>(sh, m, chtab, nch, nvel, lane, g, s0, nc, first, last, bb, fst0);
+                    else
+                        channel_pass<NLG, 2>(sh, m, chtab, nch, nvel, lane, g, s0, nc, tk, first, last, bb, fst0);
+                }
+                if (s0 < sh.nslot) {
+                    if constexpr (DUST)
+                        channel_pass_dust<NLG, 1>(sh, m, chtab, nch, nvel, lane, g, s0, nc, first, last, bb, fst0);
+                    else
+                        channel_pass<NLG, 1>(sh, m, chtab, nch, nvel, lane, g, s0, nc, tk, first, last, bb, fst0);
+                }
+                if (last) break;
+            }
+            // the channel sums over the lanes, the remainder channel's share
+            // added last
+            const int line = l0 + sum_line<NLG>(lane);
+            for (int q = 0; q < (sh.split ? 3 : 1); q++) {
+                const float2 *part = m.part(sh) + q * NPK * 32 + lane;
+                float v[NLG];
+                if constexpr (DUST) {
+#pragma unroll
+                    for (int l = 0; l < NLG; l++) v[l] = reinterpret_cast<const float *>(part - lane)[l * 32 + lane];
+                } else {
+#pragma unroll
+                    for (int k = 0; k < NP; k++) {
+                        const float2 p = part[k * 32];
+                        v[2 * k] = p.x;
+                        v[2 * k + 1] = p.y;
+                    }
+                    if (ODD) v[NLG - 1] = part[NP * 32].x;
+                }
+                const float t = sum_lines<NLG>(v, 16, lane);
+                float *dst = m.v(sh) + (q * 32 + rr) * L;
+                if (line < min(l0 + NLG, L)) dst[line] = t;
+                if (!DUST && sh.rt) {
+                    __syncwarp();
+                    if (lane < NLG && l0 + lane < L) {
+                        const float *row = reinterpret_cast<const float *>(m.row(sh) + g * NPK + (lane >> 1)) + (lane & 1);
+                        const float2 ct = chtab[nch - 1];
+                        const float x = row[0] * ct.x * fst0 * LOG2E_F;
+                        const float om = one_minus_exp(x, ex2(-x));
+                        const float r = (q == 0) ? fmaf(om, row[2] - Irem, Irem) : (q == 1) ? fmaf(om, -Irem, Irem) : om;
+                        dst[l0 + lane] = __fadd_rn(dst[l0 + lane], __fmul_rn(ct.y, r));
+                    }
+                }
+            }
+        }
+    }
+    __syncwarp();
+}
+
+// integrate_batch for a run-time group width (the batched kernel: models of
+// any line count in one launch)
+template <int NLG, bool DUST>
+__device__ __noinline__ void integrate_any_width(const RFArgs &a, const RFShape &sh, const WarpMem &m, const RayBatch &B,
+                                        unsigned smask, const float2 *chtab, const int2 *walk, int nr, float dqfac,
+                                        int lane) {
+    integrate_batch<NLG, DUST, true>(a, sh, m, B, smask, chtab, walk, nr, dqfac, lane);
+}
+
+// FP32 sums over rays, in ray order.
+struct NodeSum {
+    KahanF j0, j2, je, ls;
+    __device__ __forceinline__ void add(float2 w, float v) {
+        j0.add(__fmul_rn(w.x, v));
+        j2.add(__fmul_rn(w.y, v));
+    }
+    __device__ __forceinline__ void add_split(float w, float ve, float vl) {
+        je.add(__fmul_rn(w, ve));
+        ls.add(__fmul_rn(w, vl));
+    }
+};
+// second moment of line 1's field, sum w I n n (xx yy zz xy xz yz), whose
+// traceless part is J^2_Q in any frame: one ray's term of component k
+__device__ __forceinline__ float moment_add(float km, int k, float w, float v, float4 d) {
+    const float wv = __fmul_rn(w, v);
+    const float p = (k == 0 || k == 3 || k == 4) ? d.x : (k == 2) ? d.z : d.y;
+    const float q = (k == 0) ? d.x : (k == 1 || k == 3) ? d.y : d.z;
+    return fmaf(wv * p, q, km);
+}
+
+// NLG: lines per group (0: the model's own, BATCH only).
 // BATCH: the work items are (model, node) pairs of many models (RFBatch);
 // each warp copies the argument block of its current model into shared
-// memory.  Otherwise the nodes of the one model a0.
-template <int NS, int NLG, bool DUST, bool BATCH, int RT>
-__global__ void __launch_bounds__(256, (NLG <= 5 && NS <= 5) ? 2 : 1) k_radiation_field(RFArgs a0, RFBatch bw) {
+// memory.  Otherwise the nodes of the one model a0, or -- a0.rays_per_item >
+// 0 -- their ray ranges: small clouds have too few nodes to fill the GPU with
+// a warp per node, so each item is a part of a node's rays and stores their
+// per-line channel sums, which k_rf_finish adds up in ray order afterwards
+// (the same sums in the same order).
+template <int NLG, bool DUST, bool BATCH>
+__global__ void __launch_bounds__(256, (NLG >= 1 && NLG <= 4) ? 3 : 2) k_radiation_field(RFArgs a0, RFBatch bw, RFShape sh0) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     const long long gw = (long long)blockIdx.x * (blockDim.x >> 5) + wib;
     const int n_depth = BATCH ? bw.n_depth : a0.n_depth;
-    int2 *const wbase = (BATCH ? bw.walk : a0.walk) + (size_t)gw * 32 * (size_t)n_depth;
-    __shared__ CellRec<NLG, DUST> recs[8];
+    int2 *const walk = (BATCH ? bw.walk : a0.walk) + (size_t)gw * 1024 * (size_t)((n_depth + 31) / 32);
     using RB = typename std::conditional<BATCH, RayBatchStar, RayBatch>::type;
-    __shared__ RB rbs[8];
-    __shared__ RFArgs margs[BATCH ? 8 : 1];
-    extern __shared__ float2 rem_dyn[];
-    CellRec<NLG, DUST> &R = recs[wib];
-    RB &B = rbs[wib];
-    const int rem_ld = rem_row_stride(BATCH ? bw.rem_lines : a0.L);
-    float2 *const remS = rem_dyn + (size_t)wib * 32 * rem_ld;   // RT: this warp's (cell, line) table
+    __shared__ RFArgs margs[BATCH ? RF_BATCH_WARPS : 1];
+    __shared__ RFShape mshape[BATCH ? RF_BATCH_WARPS : 1];
+    extern __shared__ __align__(16) unsigned char dyn[];
+    // per channel: the central cell's profile exp(-q0^2) and the channel weight
+    const int nch = BATCH ? bw.nch : a0.nch;
+    float2 *chtab = reinterpret_cast<float2 *>(dyn);
+    const float *chq = BATCH ? bw.chq : a0.chq, *chw = BATCH ? bw.chw : a0.chw;
+    for (int i = threadIdx.x; i < nch; i += blockDim.x) {
+        const float q0c = chq[i];
+        chtab[i] = make_float2(ex2(-q0c * q0c * LOG2E_F), chw[i]);
+    }
+    WarpMem m;
+    m.p = dyn + ((nch * sizeof(float2) + 15) & ~(size_t)15) + (size_t)wib * (BATCH ? bw.warp_bytes : sh0.bytes);
+    RB &B = *reinterpret_cast<RB *>(m.p);
+    auto fill_bb = [&](const RFArgs &a, const RFShape &sh) {
+        float *bb = m.bb(sh);
+        const int per = 2 * sh.npk, n = sh.groups * per;
+        for (int i = lane; i < n; i += 32) {
+            const int l = (i / per) * sh.nlg + i % per;
+            const bool on = i % per < sh.nlg && l < sh.L;
+            bb[i] = on ? a.bb[l] : 0.f;
+            bb[n + i] = (BATCH && on) ? a.bbs[l] : 0.f;
+        }
+    };
+    if (!BATCH) fill_bb(a0, sh0);
+    __syncthreads();
 
+    const int rpi = BATCH ? 0 : a0.rays_per_item;
+    const int per_node = rpi ? (a0.ndir + rpi - 1) / rpi : 1;
     unsigned long long nseg = 0;
     int cur_model = -1;
     for (;;) {
-        int node = 0;
+        int node = 0, part = 0;
         if (BATCH) {
             long long item = 0;
             if (lane == 0) item = (long long)atomicAdd(&bw.queue[0], 1ULL);
@@ -318,20 +829,24 @@ __global__ void __launch_bounds__(256, (NLG <= 5 && NS <= 5) ? 2 : 1) k_radiatio
                 int *dst = reinterpret_cast<int *>(&margs[wib]);
                 for (int k = lane; k < (int)(sizeof(RFArgs) / sizeof(int)); k += 32) dst[k] = src[k];
                 __syncwarp();
+                if (lane == 0) mshape[wib] = rf_shape(margs[wib].L, bw.max_group, nch, DUST, bw.rt, bw.split);
+                __syncwarp();
+                fill_bb(margs[wib], mshape[wib]);
                 cur_model = wi.x;
             }
             node = wi.y;
         } else {
-            if (lane == 0) node = (int)atomicAdd(&a0.counters[0], 1ULL);
-            node = __shfl_sync(FULL, node, 0);
-            if (node >= a0.bulk) break;
+            long long item = 0;
+            if (lane == 0) item = (long long)atomicAdd(&a0.counters[0], 1ULL);
+            item = __shfl_sync(FULL, item, 0);
+            if (item >= (long long)a0.bulk * per_node) break;
+            node = (int)(item / per_node);
+            part = (int)(item - (long long)node * per_node);
         }
         const RFArgs &a = BATCH ? margs[wib] : a0;
-        KahanF acc0a, acc0b, acc2a, acc2b;  // lines lane and lane+32, compensated FP32
-        KahanF accEa, accEb, accLa, accLb;  // J_eff and L* of the same lines (split field only)
-        const bool split = (a.JE != nullptr);
+        const RFShape &sh = BATCH ? mshape[wib] : sh0;
         int st = 0;
-        int node_seg = 0;   // the node's ray segments (sum of node_count over its rays)
+        int node_seg = 0;   // the item's ray segments (sum of node_count over its rays)
         if (a.ab[node] > 0.0) {
             if (lane == 0) {
                 // node frame (find_dir miscellaneous.f90:48-82): x = b x g / |b x g|,
@@ -357,31 +872,42 @@ __global__ void __launch_bounds__(256, (NLG <= 5 && NS <= 5) ? 2 : 1) k_radiatio
                     }
                 }
             }
-            __syncwarp();
-            // star mode runs in the batched kernel only: its node's ray count lives in
-            // shared memory (read where used, holding no register through the
-            // integration); the single-model kernel uses the common direction table
-            const volatile int *vsn = nullptr;
-            if constexpr (BATCH) {
-                vsn = B.sn;
-                if (vsn[1] < 0) st |= PORTAL_NODE_STAR;
+            // the node's own line row, packed as the staged cells are
+            {
+                const float4 *lt = a.ltab + (size_t)node * sh.L;
+                float4 *row = m.row(sh);
+                const int per = DUST ? sh.nlg : sh.npk;
+                for (int i = lane; i < sh.groups * per; i += 32) {
+                    const int l0 = (i / per) * sh.nlg, k = i % per;
+                    if (DUST) {
+                        row[i] = lt[min(l0 + k, sh.L - 1)];
+                    } else {
+                        const float4 v = lt[min(l0 + 2 * k, sh.L - 1)];
+                        const float4 w = lt[min(l0 + min(2 * k + 1, sh.nlg - 1), sh.L - 1)];
+                        row[i] = make_float4(v.x, w.x, v.y, w.y);
+                    }
+                }
+                for (int i = lane; i < (sh.split ? 8 : 4) * sh.L; i += 32) m.acc(sh)[i] = 0.f;
             }
-            auto n_rays = [&]() -> int {
-                if constexpr (BATCH) return vsn[1];
-                else return a.ndir;
-            };
+            __syncwarp();
+            int n_rays = a.ndir;
+            if constexpr (BATCH) {
+                n_rays = B.sn[1];
+                if (n_rays < 0) st |= PORTAL_NODE_STAR;
+            }
             const float4 cvn = a.cellv[node];
             const float dqfac = 2.f * cvn.w / (float)a.nvel;
+            const int kfirst = part * rpi, kend = rpi ? min(n_rays, kfirst + rpi) : n_rays;
 
-            for (int k0 = 0; st == 0 && k0 < n_rays(); k0 += 32) {
-                const int nr = min(32, n_rays() - k0);
+            for (int k0 = kfirst; st == 0 && k0 < kend; k0 += 32) {
+                const int nr = min(32, kend - k0);
                 // ---- (1)+(2) set-up and walk, one lane per ray ----
                 int K = 0;
                 bool over = false;
                 bool sray = false;
                 unsigned smask = 0u;
                 if constexpr (BATCH) {
-                    sray = a.star && lane < nr && k0 + lane < vsn[0];
+                    sray = a.star && lane < nr && k0 + lane < B.sn[0];
                     smask = __ballot_sync(FULL, sray);
                 }
                 if (lane < nr) {
@@ -390,7 +916,7 @@ __global__ void __launch_bounds__(256, (NLG <= 5 && NS <= 5) ? 2 : 1) k_radiatio
                     bool tab = true;
                     if constexpr (BATCH) {
                         if (a.star) {
-                            const RayDir r = star_ray(B.sk, vsn[0], k0 + lane, a.nth, a.nph, a.gx, a.gy, a.gz, f,
+                            const RayDir r = star_ray(B.sk, B.sn[0], k0 + lane, a.nth, a.nph, a.gx, a.gy, a.gz, f,
                                                       &B.wts[lane]);
                             mu = r.ct; sth = r.st; cph = r.cp; sph = r.sp;
                             tab = false;
@@ -399,7 +925,7 @@ __global__ void __launch_bounds__(256, (NLG <= 5 && NS <= 5) ? 2 : 1) k_radiatio
                     if (tab) {
                         const double *dr = a.dirs + 6 * (size_t)(k0 + lane);
                         mu = dr[0]; sth = dr[1]; cph = dr[2]; sph = dr[3];
-                        if constexpr (BATCH) B.wts[lane] = make_float2((float)dr[4], (float)dr[5]);
+                        B.wts[lane] = make_float2((float)dr[4], (float)dr[5]);
                     }
                     const double dx = mu * f[0] + sth * (cph * f[6] + sph * f[3]);
                     const double dy = mu * f[1] + sth * (cph * f[7] + sph * f[4]);
@@ -410,7 +936,6 @@ __global__ void __launch_bounds__(256, (NLG <= 5 && NS <= 5) ? 2 : 1) k_radiatio
                     }
                     const float fdx = (float)dx, fdy = (float)dy, fdz = (float)dz;
                     B.dir[lane] = make_float4(fdx, fdy, fdz, cvn.x * fdx + cvn.y * fdy + cvn.z * fdz);
-                    int2 *wl = wbase + (size_t)lane * n_depth;
                     // distance left to the sphere exit as an unevaluated float pair
                     // (rh + rl), decremented exactly by each step
                     float rh = (float)sexit, rl = (float)(sexit - (double)rh);
@@ -422,22 +947,31 @@ __global__ void __launch_bounds__(256, (NLG <= 5 && NS <= 5) ? 2 : 1) k_radiatio
                         // check_neigh_fast's scan: best starts at the sphere exit, a
                         // neighbour replaces it when FACE_EPS < t <= best (so among equal
                         // t the later neighbour wins).  t = num/den compared by cross
-                        // multiplication (den > 0).
+                        // multiplication (den > 0).  Eight neighbours' records are loaded
+                        // before they are compared: the loads are scattered L2 reads.
                         float bnum = tsph, bden = 1.f;
                         int bj = -1;
-                        for (int j = 0; j < deg; j++) {
-                            const float4 e = a.edge[o + j];
-                            const float den = e.x * fdx + e.y * fdy + e.z * fdz;
-                            const float num = e.w - (e.x * rx + e.y * ry + e.z * rz);
-                            if (den > 0.f && num > FACE_EPS * den && num * bden <= bnum * den) {
-                                bnum = num;
-                                bden = den;
-                                bj = j;
+                        for (int j0 = 0; j0 < deg; j0 += 8) {
+                            float4 e8[8];
+#pragma unroll
+                            for (int i = 0; i < 8; i++) e8[i] = a.edge[o + min(j0 + i, deg - 1)];
+#pragma unroll
+                            for (int i = 0; i < 8; i++) {
+                                const float4 e = e8[i];
+                                const float den = e.x * fdx + e.y * fdy + e.z * fdz;
+                                const float num = e.w - (e.x * rx + e.y * ry + e.z * rz);
+                                if (j0 + i < deg && den > 0.f && num > FACE_EPS * den && num * bden <= bnum * den) {
+                                    bnum = num;
+                                    bden = den;
+                                    bj = j0 + i;
+                                }
                             }
                         }
                         const float delta = (bj < 0) ? tsph : bnum / bden;
                         if (K >= n_depth) { over = true; break; }
-                        wl[K] = make_int2(c, (int)roundf(delta / a.dx32));  // nint(delta_x/dx)
+                        const int steps = (int)roundf(delta / a.dx32);   // nint(delta_x/dx)
+                        walk[walk_at(K, lane)] = make_int2(c, steps);
+                        if (K == 0) B.st0[lane] = steps;
                         K++;
                         if (bj < 0) break;
                         const float4 e = a.edge[o + bj];
@@ -454,398 +988,93 @@ __global__ void __launch_bounds__(256, (NLG <= 5 && NS <= 5) ? 2 : 1) k_radiatio
                         rz = fmaf(delta, fdz, rz) - e.z;
                         c = a.idx[o + bj];
                     }
-                }
-                B.K[lane] = over ? -1 : K;
-                if constexpr (BATCH) {
-                    if (lane == 0) B.smask = smask;
+                    B.K[lane] = K;
                 }
                 if (__any_sync(FULL, over)) { st |= PORTAL_NODE_DEPTH; break; }
+                node_seg += __reduce_add_sync(FULL, lane < nr ? K : 0);
                 __syncwarp();
 
-                // ---- (3)+(4) channel integration of each ray of the batch ----
-                for (int rr = 0; rr < nr; rr++) {
-                    const int Kr = B.K[rr];
-                    const int2 *wl = wbase + (size_t)rr * n_depth;
-                    const float4 d4 = B.dir[rr];
-                    float wgt, wgt2;
-                    if constexpr (BATCH) {
-                        const float2 wt = B.wts[rr];
-                        wgt = wt.x;
-                        wgt2 = wt.y;
-                    } else {
-                        const double *dr = a.dirs + 6 * (size_t)(k0 + rr);
-                        wgt = (float)dr[4];
-                        wgt2 = (float)dr[5];
-                    }
-                    // the incoming intensity: B(T_star) for a star ray (inverse_rt.f90:113-118),
-                    // the ray's flag read from shared memory where it is used
-                    auto bb_in = [&](int l) -> float {
-                        if constexpr (BATCH) {
-                            const volatile unsigned *vsm = &B.smask;
-                            return ((*vsm >> rr) & 1u) ? a.bbs[l] : a.bb[l];
+                // ---- (3)+(4) channel integration of the batch's rays ----
+                if constexpr (NLG > 0) {
+                    integrate_batch<NLG, DUST, BATCH>(a, sh, m, B, smask, chtab, walk, nr, dqfac, lane);
+                } else {
+                    switch (sh.nlg) {
+#define RF_WIDTH(n)                                                                                        \
+    case n: integrate_any_width<n, DUST>(a, sh, m, B, smask, chtab, walk, nr, dqfac, lane); break;
+                        RF_WIDTH(1) RF_WIDTH(2) RF_WIDTH(3) RF_WIDTH(4)
+                    default:
+                        if constexpr (DUST) {
+                            integrate_any_width<5, DUST>(a, sh, m, B, smask, chtab, walk, nr, dqfac, lane);
                         } else {
-                            return a.bb[l];
-                        }
-                    };
-                    node_seg += Kr;
-                    const int2 w0 = wl[0];
-                    // the remainder channel of this lane's line (RT): intensity, and
-                    // its central-cell contributions to J0 (and J_eff, L*)
-                    float Irem = 0.f, remJ = 0.f, remE = 0.f, remL = 0.f;
-                    if (RT && lane < a.L) Irem = bb_in(lane);
-                    for (int l0 = 0; l0 < a.L; l0 += NLG) {
-                        // intensities of the lane's channels: slot pairs (s, s+1) in one
-                        // float2 (packed FP32x2 arithmetic), an odd last slot in .x
-                        float2 I2[(NS + 1) / 2][NLG];
-#define IV(s, l) (((s) & 1) ? I2[(s) >> 1][l].y : I2[(s) >> 1][l].x)
-#pragma unroll
-                        for (int l = 0; l < NLG; l++) {
-                            const float bb = (l0 + l < a.L) ? bb_in(l0 + l) : 0.f;
-#pragma unroll
-                            for (int s2 = 0; s2 < NS; s2++) IV(s2, l) = bb;
-                        }
-                        // walk records of the chunk (lane = cell), the next chunk's
-                        // loaded while this one is integrated
-                        int2 wcp = make_int2(0, 0);
-                        if (lane < min(32, Kr - 1)) wcp = wl[Kr - 1 - lane];
-                        for (int hi = Kr - 1; hi >= 1; hi -= 32) {
-                            const int nc = min(32, hi);
-                            const int2 wc = wcp;
-                            if (lane < min(32, hi - 32)) wcp = wl[hi - 32 - lane];
-                            __syncwarp();
-                            unsigned thin_m = (1u << NLG) - 1u;   // the group's lines thin in this cell
-                            if (lane < nc) {
-                                const float4 cv = a.cellv[wc.x];
-                                const float vp = fmaf(cv.z, d4.z, fmaf(cv.y, d4.y, __fmul_rn(cv.x, d4.x)));
-                                const float ib = SQL2E_F * (1.f / cv.w);
-                                const float2 qdl = make_float2((d4.w - vp) * ib, dqfac * ib);
-                                R.qd[lane] = qdl;
-                                const float fst = (float)wc.y;
-                                if (RT && l0 == 0) {
-                                    // the remainder channel's transfer weight and source
-                                    // function of this cell for every line
-                                    const float q = fmaf(qdl.y, (float)(32 * NS - a.nvel), qdl.x);
-                                    const float gr = ex2(-(q * q));
-                                    const float2 *lr = reinterpret_cast<const float2 *>(a.ltab + (size_t)wc.x * a.L);
-                                    float2 *dst = remS + lane * rem_ld;
-#pragma unroll 4
-                                    for (int l = 0; l < a.L; l++) {
-                                        const float2 v = lr[2 * l];
-                                        const float As = (v.x > 0.f) ? v.x * fst * LOG2E_F : 0.f;
-                                        const float Ss = (v.x > 0.f) ? v.y : 0.f;
-                                        const float x = As * gr;
-                                        dst[l] = make_float2(one_minus_exp(x, ex2(-x)), Ss);
-                                    }
-                                }
-                                const float4 *lt = a.ltab + (size_t)wc.x * a.L + l0;
-#pragma unroll
-                                for (int l = 0; l < NLG; l++) {
-                                    if (DUST) {
-                                        if (l0 + l < a.L) {
-                                            const float4 v = lt[l];
-                                            R.AS[lane][l] = make_float2(v.x * fst, v.y * v.x * fst);   // emissivity x steps
-                                            R.Ad[lane][DUST ? l : 0] = v.z * fst;
-                                            R.Jd[lane][DUST ? l : 0] = v.w * fst;
-                                        }
-                                    } else {
-                                        // optical depth at unit profile in log2 units (ex2
-                                        // takes it as is) and the source function.  A cell
-                                        // line with kv <= 0 fails ray_in's gate tau > 1e-30
-                                        // in every channel (inverse_rt.f90:308), and so does
-                                        // a padding line of the last group: both get A = S
-                                        // = 0, which leaves I unchanged exactly.
-                                        float As = 0.f, Ss = 0.f;
-                                        if (l0 + l < a.L) {
-                                            const float4 v = lt[l];
-                                            if (v.x > 0.f) {
-                                                As = v.x * fst * LOG2E_F;
-                                                Ss = v.y;
-                                            }
-                                        }
-                                        R.AS[lane][l] = make_float2(As, Ss);
-                                        if (!(As < OM_THIN_A)) thin_m &= ~(1u << l);
-                                    }
-                                }
-                            }
-                            // A line whose line-centre optical depth is below OM_THIN_A
-                            // in every cell of the chunk takes the Taylor form of
-                            // 1 - e^-tau in every channel: the branch-free update would
-                            // select exactly that value, so it skips the ex2 and the
-                            // select.  Decided per chunk of 32 cells, uniform over the
-                            // warp, for the group's last tk lines (a rotor's higher lines
-                            // are the thinner ones); the cell loop is instantiated per tk
-                            // (groups of at most 5 lines; wider groups: none or all).
-                            int tk = 0;
-                            if (!DUST) {
-                                const unsigned tm = __reduce_and_sync(FULL, thin_m);
-                                tk = __clz(~(tm << (32 - NLG)));   // trailing run of thin lines
-                                if (NLG > SUFFIX_MAX_NLG && tk != NLG) tk = 0;
-                            }
-                            __syncwarp();
-                            if (RT && l0 == 0 && lane < a.L) {
-                                // the remainder channel, lane = line, the same cells inward
-                                for (int u = 0; u < nc; u++) {
-                                    const float2 r = remS[u * rem_ld + lane];
-                                    Irem = fmaf(r.x, r.y - Irem, Irem);
-                                }
-                            }
-                            // one cell's update of the group's lines in every channel slot
-                            auto cell_step = [&](auto tk_tag, int u) {
-                                constexpr int TK = decltype(tk_tag)::value;   // the last TK lines: Taylor only
-                                const float2 qd = R.qd[u];
-                                const float q0 = qd.x, dq = qd.y;
-                                // Gaussian profile of the cell at the lane's channels,
-                                // exp(-q^2) = 2^(-q'^2) with q' = q sqrt(log2 e) (staged
-                                // scaled); slot pairs on the packed pipe (the same
-                                // roundings per slot as the odd slot's scalar form)
-                                float g[NS];
-#pragma unroll
-                                for (int s2 = 0; s2 + 1 < NS; s2 += 2) {
-                                    const float2 ch2 = make_float2((float)(lane + 32 * s2 - a.nvel),
-                                                                   (float)(lane + 32 * (s2 + 1) - a.nvel));
-                                    const float2 q = __ffma2_rn(make_float2(dq, dq), ch2, make_float2(q0, q0));
-                                    const float2 t = __fmul2_rn(q, q);
-                                    g[s2] = ex2(-t.x);
-                                    g[s2 + 1] = ex2(-t.y);
-                                }
-                                if (NS & 1) {
-                                    const float q = fmaf(dq, (float)(lane + 32 * (NS - 1) - a.nvel), q0);
-                                    g[NS - 1] = ex2(-(q * q));
-                                }
-#pragma unroll
-                                for (int l = 0; l < NLG; l++) {
-                                    const float2 ASu = R.AS[u][l];
-                                    const float Au = ASu.x;
-                                    const float Su = ASu.y;
-                                    if (DUST) {
-                                        if (l0 + l < a.L) {
-                                            const float Adu = R.Ad[u][DUST ? l : 0], Jdu = R.Jd[u][DUST ? l : 0];
-#pragma unroll
-                                            for (int s2 = 0; s2 < NS; s2++) {
-                                                // tau = (kv phi + alpha) dx n, S = (ev phi + j)/(kv phi + alpha)
-                                                const float tau = fmaf(Au, g[s2], Adu);
-                                                const float Sv = fmaf(Su, g[s2], Jdu) / tau;
-                                                const float x = tau * LOG2E_F;
-                                                const float om = one_minus_exp(x, ex2(-x));
-                                                const float In = fmaf(om, Sv - IV(s2, l), IV(s2, l));
-                                                IV(s2, l) = (tau > 1e-30f) ? In : IV(s2, l);
-                                            }
-                                        }
-                                    } else {
-                                        // I' = I + (1 - e^-tau)(S - I) with 1 - e^-tau accurate
-                                        // down to tau = 0 and rounded as the reference's FP64
-                                        // (one_minus_exp).  ray_in's gate tau > 1e-30
-                                        // (inverse_rt.f90:308) needs no test: lines with kv <= 0
-                                        // carry A = S = 0 and leave I unchanged exactly, and
-                                        // 0 < tau < 2^-54 rounds to a zero weight as in FP64.
-                                        // Branch-free inside a cell, so the NS x NLG update
-                                        // chains interleave: a warp-uniform branch per cell to
-                                        // a Taylor-only path measured 24 % slower in spite of
-                                        // skipping the ex2 (1.45e9 against 1.90e9 segments/s);
-                                        // decided once per chunk of 32 cells (TK) it gains
-                                        // (1.96e9 -> 2.03e9).  Channel-slot pairs go through
-                                        // the packed FP32x2 pipe (one issue slot for two
-                                        // updates).
-                                        const float2 A2 = make_float2(Au, Au), S2 = make_float2(Su, Su);
-#pragma unroll
-                                        for (int s2 = 0; s2 + 1 < NS; s2 += 2) {
-                                            const float2 x = __fmul2_rn(A2, make_float2(g[s2], g[s2 + 1]));
-                                            const float2 om = (l >= NLG - TK) ? om_taylor2(x)
-                                                                              : one_minus_exp2(x, ex2(-x.x), ex2(-x.y));
-                                            float2 &Ip = I2[s2 >> 1][l];
-                                            Ip = __ffma2_rn(om, __ffma2_rn(Ip, make_float2(-1.f, -1.f), S2), Ip);
-                                        }
-                                        if (NS & 1) {
-                                            const float x = Au * g[NS - 1];
-                                            const float om = (l >= NLG - TK) ? om_taylor(x) : one_minus_exp(x, ex2(-x));
-                                            float &Is = I2[NS >> 1][l].x;
-                                            Is = fmaf(om, Su - Is, Is);
-                                        }
-                                    }
-                                }
-                            };
-                            // two cells per iteration: the second cell's profile and
-                            // transfer weights do not depend on the first's update and
-                            // fill its dependency stalls (2.10e9 -> 2.22e9 segments/s on
-                            // the benchmark sphere with the walk-record prefetch above;
-                            // 4 cells per iteration: 2.21e9)
-                            auto run = [&](auto tk_tag) {
-                                if constexpr (NLG <= UNROLL_MAX_NLG) {
-#pragma unroll 2
-                                    for (int u = 0; u < nc; u++) cell_step(tk_tag, u);
-                                } else {
-#pragma unroll 1
-                                    for (int u = 0; u < nc; u++) cell_step(tk_tag, u);
-                                }
-                            };
-                            with_thin_lines<NLG, DUST>(tk, run);
-                        }
-                        // central cell (inverse_rt.f90:320-339): no gate, profile at
-                        // the node's own b, then the weighted channel sum
-                        const float fst0 = (float)w0.y;
-                        if (RT && l0 == 0 && lane < a.L) {
-                            const int ch = 32 * NS;
-                            const float4 v = a.ltab[(size_t)node * a.L + lane];
-                            const float q0c = a.chq[ch];
-                            const float g0 = ex2(-q0c * q0c * LOG2E_F);
-                            const float x = v.x * g0 * fst0 * LOG2E_F;
-                            const float om = one_minus_exp(x, ex2(-x));
-                            remJ = __fmul_rn(a.chw[ch], fmaf(om, v.y - Irem, Irem));
-                            if (split) {
-                                remE = __fmul_rn(a.chw[ch], fmaf(om, -Irem, Irem));
-                                remL = __fmul_rn(a.chw[ch], om);
+                            switch (sh.nlg) {
+                                RF_WIDTH(5) RF_WIDTH(6) RF_WIDTH(7) RF_WIDTH(8) RF_WIDTH(9)
+                            default: integrate_any_width<10, DUST>(a, sh, m, B, smask, chtab, walk, nr, dqfac, lane);
                             }
                         }
-                        float part[NLG], pe[NLG], pl[NLG];
-#pragma unroll
-                        for (int l = 0; l < NLG; l++) {
-                            part[l] = 0.f;
-                            pe[l] = 0.f;
-                            pl[l] = 0.f;
-                            if (l0 + l < a.L) {
-                                const float4 v = a.ltab[(size_t)node * a.L + l0 + l];
-#pragma unroll
-                                for (int s2 = 0; s2 < NS; s2++) {
-                                    const int ch = lane + 32 * s2;
-                                    if (ch < a.nch) {
-                                        const float q0c = a.chq[ch];
-                                        const float g0 = ex2(-q0c * q0c * LOG2E_F);
-                                        float tau, Sv, lf = 1.f, Sd = 0.f;
-                                        if (DUST) {
-                                            const float kap = fmaf(v.x, g0, v.z);
-                                            tau = kap * fst0;
-                                            Sv = fmaf(v.y * v.x, g0, v.w) / kap;
-                                            lf = v.x * g0 / kap;   // line share of the opacity
-                                            Sd = v.w / kap;        // dust emission share of S
-                                        } else {
-                                            tau = v.x * g0 * fst0;
-                                            Sv = v.y;
-                                        }
-                                        const float x = tau * LOG2E_F;
-                                        const float e = ex2(-x);
-                                        const float om = one_minus_exp(x, e);
-                                        const float Io = fmaf(om, Sv - IV(s2, l), IV(s2, l));
-                                        part[l] = fmaf(a.chw[ch], Io, part[l]);
-                                        if (split) {
-                                            pe[l] = fmaf(a.chw[ch], fmaf(om, Sd - IV(s2, l), IV(s2, l)), pe[l]);
-                                            pl[l] = fmaf(a.chw[ch], lf * om, pl[l]);
-                                        }
-                                    }
-                                }
-                            }
+                    }
+#undef RF_WIDTH
+                }
+                const float *v = m.v(sh);
+                const int L = sh.L;
+                if (rpi) {   // the rays' channel sums and directions for k_rf_finish
+                    const size_t ray0 = (size_t)node * a.ndir + k0, plane = (size_t)a.bulk * a.ndir * L;
+                    for (int q = 0; q < (sh.split ? 3 : 1); q++)
+                        for (int i = lane; i < nr * L; i += 32) a.vray[q * plane + ray0 * L + i] = v[q * 32 * L + i];
+                    if (lane < nr) a.dray[ray0 + lane] = B.dir[lane];
+                } else {
+                    for (int l = lane; l < L; l += 32) {
+                        float *acc = m.acc(sh) + l;
+                        NodeSum s;
+                        s.j0.s = acc[0]; s.j0.c = acc[L]; s.j2.s = acc[2 * L]; s.j2.c = acc[3 * L];
+                        for (int r = 0; r < nr; r++) s.add(B.wts[r], v[r * L + l]);
+                        acc[0] = s.j0.s; acc[L] = s.j0.c; acc[2 * L] = s.j2.s; acc[3 * L] = s.j2.c;
+                        if (sh.split) {
+                            s.je.s = acc[4 * L]; s.je.c = acc[5 * L]; s.ls.s = acc[6 * L]; s.ls.c = acc[7 * L];
+                            for (int r = 0; r < nr; r++)
+                                s.add_split(B.wts[r].x, v[(32 + r) * L + l], v[(64 + r) * L + l]);
+                            acc[4 * L] = s.je.s; acc[5 * L] = s.je.c; acc[6 * L] = s.ls.s; acc[7 * L] = s.ls.c;
                         }
-#pragma unroll
-                        for (int l = 0; l < NLG; l++) {
-                            float v = part[l];
-#pragma unroll
-                            for (int o2 = 16; o2 >= 1; o2 >>= 1) v += __shfl_xor_sync(FULL, v, o2);
-                            const int line = l0 + l;
-                            if (line < a.L && (line & 31) == lane) {
-                                if (line < 32) {
-                                    if (RT) v = __fadd_rn(v, remJ);   // this lane's line: its remainder channel
-                                    acc0a.add(__fmul_rn(wgt, v));
-                                    acc2a.add(__fmul_rn(wgt2, v));
-                                    if (line == 0) {
-                                        // the full second moment of line 1's field, sum w I n n,
-                                        // whose traceless part is J^2_Q in any frame
-                                        const float wv = __fmul_rn(wgt, v);
-                                        B.km[0] = fmaf(wv * d4.x, d4.x, B.km[0]);
-                                        B.km[1] = fmaf(wv * d4.y, d4.y, B.km[1]);
-                                        B.km[2] = fmaf(wv * d4.z, d4.z, B.km[2]);
-                                        B.km[3] = fmaf(wv * d4.x, d4.y, B.km[3]);
-                                        B.km[4] = fmaf(wv * d4.x, d4.z, B.km[4]);
-                                        B.km[5] = fmaf(wv * d4.y, d4.z, B.km[5]);
-                                    }
-                                } else {
-                                    acc0b.add(__fmul_rn(wgt, v));
-                                    acc2b.add(__fmul_rn(wgt2, v));
-                                }
-                            }
-                        }
-                        if (split) {
-#pragma unroll
-                            for (int l = 0; l < NLG; l++) {
-                                float ve = pe[l], vl = pl[l];
-#pragma unroll
-                                for (int o2 = 16; o2 >= 1; o2 >>= 1) {
-                                    ve += __shfl_xor_sync(FULL, ve, o2);
-                                    vl += __shfl_xor_sync(FULL, vl, o2);
-                                }
-                                const int line = l0 + l;
-                                if (line < a.L && (line & 31) == lane) {
-                                    if (line < 32) {
-                                        if (RT) {
-                                            ve = __fadd_rn(ve, remE);
-                                            vl = __fadd_rn(vl, remL);
-                                        }
-                                        accEa.add(__fmul_rn(wgt, ve));
-                                        accLa.add(__fmul_rn(wgt, vl));
-                                    } else {
-                                        accEb.add(__fmul_rn(wgt, ve));
-                                        accLb.add(__fmul_rn(wgt, vl));
-                                    }
-                                }
-                            }
-                        }
+                    }
+                    if (lane < 6) {
+                        float km = B.km[lane];
+                        for (int r = 0; r < nr; r++) km = moment_add(km, lane, B.wts[r].x, v[r * L], B.dir[r]);
+                        B.km[lane] = km;
                     }
                 }
                 __syncwarp();
             }
         }
-#undef IV
-        if (lane < a.L) {
-            a.J0[(size_t)node * a.L + lane] = (st == 0) ? acc0a.value() : 0.0;
-            a.J2[(size_t)node * a.L + lane] = (st == 0) ? acc2a.value() : 0.0;
+        if (rpi) {
+            if (lane == 0) a.iseg[(size_t)node * per_node + part] = st ? -1 : node_seg;
+            __syncwarp();
+            continue;
         }
-        if (lane + 32 < a.L) {
-            a.J0[(size_t)node * a.L + lane + 32] = (st == 0) ? acc0b.value() : 0.0;
-            a.J2[(size_t)node * a.L + lane + 32] = (st == 0) ? acc2b.value() : 0.0;
-        }
-        if (split) {
-            if (lane < a.L) {
-                a.JE[(size_t)node * a.L + lane] = (st == 0) ? accEa.value() : 0.0;
-                a.LS[(size_t)node * a.L + lane] = (st == 0) ? accLa.value() : 0.0;
+        {
+            const int L = a.L;
+            const bool on = st == 0 && a.ab[node] > 0.0;
+            const float *acc = m.acc(sh);
+            auto value = [&](int q, int l) { return on ? (double)acc[2 * q * L + l] - (double)acc[(2 * q + 1) * L + l] : 0.0; };
+            for (int l = lane; l < L; l += 32) {
+                a.J0[(size_t)node * L + l] = value(0, l);
+                a.J2[(size_t)node * L + l] = value(1, l);
+                if (sh.split) {
+                    a.JE[(size_t)node * L + l] = value(2, l);
+                    a.LS[(size_t)node * L + l] = value(3, l);
+                }
             }
-            if (lane + 32 < a.L) {
-                a.JE[(size_t)node * a.L + lane + 32] = (st == 0) ? accEb.value() : 0.0;
-                a.LS[(size_t)node * a.L + lane + 32] = (st == 0) ? accLb.value() : 0.0;
+            if (lane == 0) {
+                a.status[node] = st;
+                if (a.segs) a.segs[node] = node_seg;
+                if (a.kmom)
+                    for (int k = 0; k < 6; k++) a.kmom[(size_t)k * a.N + node] = on ? B.km[k] : 0.f;
             }
-        }
-        if (lane == 0) {
-            a.status[node] = st;
-            if (a.segs) a.segs[node] = node_seg;
-            if (a.kmom)
-                for (int k = 0; k < 6; k++)
-                    a.kmom[(size_t)k * a.N + node] = (st == 0 && a.ab[node] > 0.0) ? B.km[k] : 0.f;
         }
         nseg += (unsigned long long)node_seg;
         __syncwarp();
     }
-    // segment count (every lane holds the same count)
-    if (lane == 0) atomicAdd(BATCH ? &bw.queue[1] : &a0.counters[1], nseg);
+    // segment count (every lane holds the same count; k_rf_finish counts ray-range items)
+    if (lane == 0 && !rpi) atomicAdd(BATCH ? &bw.queue[1] : &a0.counters[1], nseg);
 }
 
-}  // namespace
-
-namespace {
-
-// Channel layout: (slots per lane, remainder channel).  2 nvel + 1 channels
-// with nvel a multiple of 16 take 2 nvel / 32 full slots plus the
-// lanes-over-lines remainder channel (no dust, at most 32 lines); any other
-// count is padded to whole slots.
-struct ChanLayout {
-    int ns, rt;
-};
-inline ChanLayout chan_layout(int nch, bool dust, int max_lines) {
-    if (!dust && max_lines <= 32 && nch > 32 && nch % 32 == 1) {
-        const int k = nch / 32;
-        if (k == 1 || k == 2 || k == 4 || k == 8) return {k, 1};
-    }
-    if (nch <= 32) return {1, 0};
-    if (nch <= 64) return {2, 0};
-    if (nch <= 96) return {3, 0};
-    if (nch <= 160) return {5, 0};
-    return {9, 0};
-}
 
 }  // namespace
