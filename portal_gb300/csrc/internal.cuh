@@ -12,6 +12,7 @@ struct RFArgs {
     float dx32;
     const double *__restrict__ pos;
     const double *__restrict__ bvec;
+    double *frames;                   // (N, 13) node frames (k_line_table)
     const double *__restrict__ ab;
     const float4 *__restrict__ cellv;
     const int *__restrict__ off;

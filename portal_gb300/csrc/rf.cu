@@ -309,7 +309,7 @@ int rf_prepare(portal_ctx *c, int nth, int nph, int nvel, const double *gvec, do
     }
     if (c->dirtab.reserve(dt.size()) || c->chtab.reserve(ct.size()) ||
         c->ltab.reserve((size_t)L * N) || c->J0.reserve((size_t)L * N) || c->J2.reserve((size_t)L * N) ||
-        c->nodeseg.reserve((size_t)N) || c->kmom.reserve((size_t)6 * N))
+        c->nodeseg.reserve((size_t)N) || c->frames.reserve(FRAME_N * (size_t)N) || c->kmom.reserve((size_t)6 * N))
         return set_err(c, PORTAL_ERR_NOMEM, "radiation-field buffers");
     if (split && (c->JE.reserve((size_t)L * N) || c->LS.reserve((size_t)L * N)))
         return set_err(c, PORTAL_ERR_NOMEM, "split-field buffers");
@@ -337,6 +337,7 @@ int rf_prepare(portal_ctx *c, int nth, int nph, int nvel, const double *gvec, do
     a.JE = split ? c->JE.p : nullptr;
     a.LS = split ? c->LS.p : nullptr;
     a.walk = nullptr;
+    a.frames = c->frames.p;
     a.rays_per_item = 0;
     a.vray = nullptr; a.dray = nullptr; a.iseg = nullptr;
     // the line table's transfer step (main_para.f90:135 dx times r_max)
@@ -359,9 +360,10 @@ int rf_pass(portal_ctx *c, const RFArgs &a, cudaStream_t s) {
         PCHECK(c, cudaMemsetAsync(c->LS.p, 0, (size_t)L * N * sizeof(double), s));
     }
     const long long tot = (long long)N * L;
-    k_line_table<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(
+    const int table_blocks = (int)((tot + 255) / 256);
+    k_line_table<<<table_blocks + (a.bulk + 255) / 256, 256, 0, s>>>(
         N, L, c->rf_dxp, reinterpret_cast<const LineConst *>(c->linebuf.p), c->levp.p, c->nlev, c->b64.p,
-        c->dustp.p, c->tdust.p, c->ltab.p);
+        c->dustp.p, c->tdust.p, c->ltab.p, a, table_blocks);
     PCHECK(c, cudaGetLastError());
     return PORTAL_OK;
 }

@@ -61,11 +61,63 @@ __device__ __forceinline__ float ex2(float x) {
     return y;
 }
 
-// Line table: one thread per (node, line).
+// A node's frame, the part of the ray set-up that all its rays share: b(3), x
+// = b x g / |b x g| (3), x x b (3), its position p(3), |p|^2 - 1 as
+// pos_quadratic forms it.  One thread per bulk node (the FP64 pipe takes a
+// warp's instruction in 16 cycles whether one lane or all use it: formed by
+// one lane per item, the frames took a tenth of a 4,096-point pass).
+constexpr int FRAME_N = 13;
+__device__ __forceinline__ void node_frame(int node, const double *__restrict__ bvec, const double *__restrict__ pos,
+                                           double gx, double gy, double gz, double *__restrict__ frames) {
+    // find_dir miscellaneous.f90:48-82:
+    // dir = R(b,ph) R(x,th) b = cos th b + sin th (cos ph (x x b) + sin ph x)
+    const double bx = bvec[3 * (size_t)node], by = bvec[3 * (size_t)node + 1], bz = bvec[3 * (size_t)node + 2];
+    double xx = by * gz - bz * gy, xy = bz * gx - bx * gz, xz = bx * gy - by * gx;
+    const double xn = sqrt(xx * xx + xy * xy + xz * xz);
+    xx /= xn; xy /= xn; xz /= xn;
+    const double px = pos[3 * (size_t)node], py = pos[3 * (size_t)node + 1], pz = pos[3 * (size_t)node + 2];
+    const double np = __dsqrt_rn(dsum3sq(px, py, pz));
+    double *f = frames + FRAME_N * (size_t)node;
+    f[0] = bx; f[1] = by; f[2] = bz; f[3] = xx; f[4] = xy; f[5] = xz;
+    f[6] = xy * bz - xz * by; f[7] = xz * bx - xx * bz; f[8] = xx * by - xy * bx;
+    f[9] = px; f[10] = py; f[11] = pz; f[12] = __dsub_rn(__dmul_rn(np, np), 1.0);
+}
+
+// sphere_exit for a direction of unit length up to rounding, with c = |p|^2 -
+// 1 given: the same values with a third of the FP64 instructions.  With s =
+// |d|^2 = 1 + e, e a few ulp, sqrt(s) = 1 + e/2 - e^2/8 lies just below 1 +
+// e/2, which is a double or halfway between two: rounding 1 + e/2 downwards
+// rounds sqrt(s) correctly.  The quotient by 2 a = 2 (1 + h), h a few ulp, is
+// q = n/2 corrected by its exact residual (n - 2 a q)/2; and of the two roots
+// only the one taken is divided.
+__device__ __forceinline__ double sphere_exit_unit(double px, double py, double pz, double c, double dx, double dy,
+                                                   double dz) {
+    const double s = dsum3sq(dx, dy, dz), e = __dsub_rn(s, 1.0);
+    const bool unit = fabs(e) < 0x1p-40;
+    const double nd = unit ? __dadd_rd(1.0, __dmul_rn(0.5, e)) : __dsqrt_rn(s);
+    const double a = __dmul_rn(nd, nd);
+    const double b = __dmul_rn(2.0, ddot3(px, py, pz, dx, dy, dz));
+    const double dis = __dsub_rn(__dmul_rn(b, b), __dmul_rn(__dmul_rn(4.0, a), c));
+    if (!(dis > 0.0)) return 0.0;
+    const double sq = __dsqrt_rn(dis);
+    const double n2 = __dsub_rn(-b, sq), n = (n2 > 0.0) ? n2 : __dadd_rn(-b, sq);
+    const double a2 = __dmul_rn(2.0, a);
+    if (!unit) return __ddiv_rn(n, a2);
+    const double q = __dmul_rn(0.5, n);
+    return __fma_rn(__fma_rn(-q, a2, n), 0.5, q);
+}
+
+// Line table, one thread per (node, line), and -- the blocks after its own --
+// the node frames, one thread per node.
 __global__ void k_line_table(int N, int L, double dxp, const LineConst *__restrict__ lines,
                              const double *__restrict__ levp, int nlev, const double *__restrict__ b,
                              const double *__restrict__ dustp, const double *__restrict__ tdust,
-                             float4 *__restrict__ ltab) {
+                             float4 *__restrict__ ltab, RFArgs a, int table_blocks) {
+    if ((int)blockIdx.x >= table_blocks) {
+        const int node = (int)((blockIdx.x - table_blocks) * blockDim.x + threadIdx.x);
+        if (node < a.bulk) node_frame(node, a.bvec, a.pos, a.gx, a.gy, a.gz, a.frames);
+        return;
+    }
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (long long)N * L) return;
     int n = (int)(t / L), l = (int)(t - (long long)n * L);
@@ -219,7 +271,7 @@ __device__ __noinline__ double star_exit(double sexit, double px, double py, dou
 // Per-warp state of the node being processed and its current batch of (up
 // to) 32 rays.
 struct RayBatch {
-    double frame[13];    // b(3), x(3), w(3), node position(3), |p|^2
+    double frame[FRAME_N];
     float4 dir[32];      // (d_x, d_y, d_z, v_node . d) per ray
     float2 wts[32];      // (w, w c_in / sqrt 2) per ray
     int K[32];           // segments per ray
@@ -848,24 +900,14 @@ __global__ void __launch_bounds__(256, (NLG >= 1 && NLG <= 4) ? 3 : 2) k_radiati
         int st = 0;
         int node_seg = 0;   // the item's ray segments (sum of node_count over its rays)
         if (a.ab[node] > 0.0) {
-            if (lane == 0) {
-                // node frame (find_dir miscellaneous.f90:48-82): x = b x g / |b x g|,
-                // dir = R(b,ph) R(x,th) b = cos th b + sin th (cos ph (x x b) + sin ph x)
-                const double bx = a.bvec[3 * (size_t)node], by = a.bvec[3 * (size_t)node + 1],
-                             bz = a.bvec[3 * (size_t)node + 2];
-                double xx = by * a.gz - bz * a.gy, xy = bz * a.gx - bx * a.gz, xz = bx * a.gy - by * a.gx;
-                const double xn = sqrt(xx * xx + xy * xy + xz * xz);
-                xx /= xn; xy /= xn; xz /= xn;
-                const double px = a.pos[3 * (size_t)node], py = a.pos[3 * (size_t)node + 1],
-                             pz = a.pos[3 * (size_t)node + 2];
-                double *f = B.frame;
-                f[0] = bx; f[1] = by; f[2] = bz; f[3] = xx; f[4] = xy; f[5] = xz;
-                f[6] = xy * bz - xz * by; f[7] = xz * bx - xx * bz; f[8] = xx * by - xy * bx;
-                f[9] = px; f[10] = py; f[11] = pz; f[12] = px * px + py * py + pz * pz;
-                for (int k = 0; k < 6; k++) B.km[k] = 0.f;
-                if constexpr (BATCH) {
+            if (lane < FRAME_N) B.frame[lane] = a.frames[FRAME_N * (size_t)node + lane];
+            if (lane < 6) B.km[lane] = 0.f;
+            __syncwarp();
+            if constexpr (BATCH) {
+                if (lane == 0) {
                     if (a.star) {
-                        star_node(B.sk, B.sn, a.xs, a.ys, a.zs, a.Rs, a.nth, a.nph, px, py, pz);
+                        star_node(B.sk, B.sn, a.xs, a.ys, a.zs, a.Rs, a.nth, a.nph, B.frame[9], B.frame[10],
+                                  B.frame[11]);
                     } else {
                         B.sn[0] = 0;
                         B.sn[1] = a.ndir;
@@ -930,7 +972,7 @@ __global__ void __launch_bounds__(256, (NLG >= 1 && NLG <= 4) ? 3 : 2) k_radiati
                     const double dx = mu * f[0] + sth * (cph * f[6] + sph * f[3]);
                     const double dy = mu * f[1] + sth * (cph * f[7] + sph * f[4]);
                     const double dz = mu * f[2] + sth * (cph * f[8] + sph * f[5]);
-                    double sexit = sphere_exit(f[9], f[10], f[11], dx, dy, dz);
+                    double sexit = sphere_exit_unit(f[9], f[10], f[11], f[12], dx, dy, dz);
                     if constexpr (BATCH) {
                         if (sray) sexit = star_exit(sexit, f[9], f[10], f[11], dx, dy, dz, a.xs, a.ys, a.zs, a.Rs);
                     }
