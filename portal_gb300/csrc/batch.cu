@@ -219,9 +219,9 @@ extern "C" int portal_batch_prepare(portal_batch *b, int nth, int nph, int nvel,
     BCHECK(b, cudaMemcpyAsync(b->sample.p, sm.data(), sizeof(int2) * sm.size(), cudaMemcpyHostToDevice, b->stream));
     BCHECK(b, cudaStreamSynchronize(b->stream));
 
-    // candidate launch shapes: radiation field (widest line group, blocks per
-    // SM: all that fit, or half), SE (warps per block; blocks per SM from the
-    // occupancy)
+    // candidate launch shapes: radiation field (widest line group), SE (warps
+    // per block); blocks per SM from the occupancy (the sample is too small to
+    // fill the GPU, so timing fewer blocks on it would flatter them)
     struct RFC { int nlg, bps; };
     std::vector<RFC> rfc;
     size_t rf_grid = 0;
@@ -231,7 +231,6 @@ extern "C" int portal_batch_prepare(portal_batch *b, int nth, int nph, int nvel,
             return bfail(b, PORTAL_ERR_CUDA, "occupancy query");
         if (mx < 1) continue;
         rfc.push_back({nlg, mx});
-        if (mx > 1) rfc.push_back({nlg, (mx + 1) / 2});
         rf_grid = std::max(rf_grid, (size_t)mx * b->sm_count);
     }
     if (rfc.empty()) return bfail(b, PORTAL_ERR_CUDA, "radiation-field kernel does not fit on an SM");
