@@ -14,27 +14,39 @@
 //                absorption coefficients, stored as per-trace-step factors at
 //                the profile peak (float4), plus per-node Stokes-rotation
 //                constants.
-//   k_image      one warp per 32 pixels (persistent):
-//                 (1) one lane per pixel: the start node (argmin of the FP64
-//                     distance, lowest index on ties) and the fixed-step
-//                     march along +z.  The step at which a neighbour becomes
-//                     nearer is predicted from the bisector-plane crossing,
-//                     the photon's z is advanced by the reference's own
-//                     sequence of FP64 additions (computed in exact jumps,
-//                     add_steps), and check_neigh is replayed exactly (FP64,
-//                     strict <, list order) around each predicted change and
-//                     at the exit -- over the neighbours that can come within
-//                     1e-12 of the current node's squared distance before the
-//                     next predicted change, the others being unable to win
-//                     -- so the recorded (node, step) list is the reference's;
+//   k_im_dust    per (node, line): the dust's Planck function.
+//   k_image      one block per 32 pixels (persistent):
+//                 (1) the first warp marches, one lane per pixel: the start
+//                     node (argmin of the FP64 distance, lowest index on
+//                     ties) and the fixed-step march along +z.  The step at
+//                     which a neighbour becomes nearer is predicted from the
+//                     bisector-plane crossings: FP32 with rounding bounds
+//                     picks the few neighbours that can cross next, FP64
+//                     places their crossings.  The photon's z is advanced to
+//                     just before it by the reference's own sequence of FP64
+//                     additions (computed in exact jumps, add_steps), and
+//                     check_neigh is replayed exactly (FP64, strict <, list
+//                     order) from there and at the exit -- over the
+//                     neighbours that can come within 1e-12 of the current
+//                     node's squared distance, the others being unable to
+//                     win -- so the recorded (node, step) list is the
+//                     reference's.  What bounds it: the FP64 pipe (16 cycles
+//                     a warp instruction) and the scattered loads; FP64 for
+//                     every neighbour and a replay from three steps before
+//                     took 10.2 ms for 257 x 257 x 129 of a 32,768-point
+//                     sphere, this 4.1 ms;
 //                 (2) per pixel, lanes over velocity channels, lines looped:
 //                     the polarized propagation in the numerically stable
 //                     form o11 = (phi(p)+phi(m))/2, o12 = -(phi(p)-phi(m))/2,
 //                     e ch = (E_p+E_m)/2, e sh = (E_p-E_m)/2 with p, m =
 //                     tau_I -/+ tau_Q, E = exp(-.), phi(x) = (1-e^-x)/x,
 //                     algebraically identical to raytrace.f90:41-53; the
-//                     optical depth summed with compensation; the
-//                     channel-independent dust terms once per pixel.
+//                     optical depth summed with compensation; cell records
+//                     staged in shared memory 32 at a time;
+//                 (3) the channel-independent dust terms (FP64), lane =
+//                     pixel, a line per warp (every lane alike they took most
+//                     of the per-node maps of a dusty cloud: 25.1 ms for
+//                     9,001 nodes x 3 lines, now 1.2 ms).
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -154,14 +166,17 @@ struct ImArgs {
     int N, npx, im_pix, nlines, nvel, nch, n_depth;
     int mode, nrays;         // 0: pixel grid, nrays = npx^2; 1: one ray per bulk node
     int star;                // star mode: rays starting on the star's disc start at its front
+    int dust;                // the cloud has dust
     double Rs, sx, sy, sz;   // R_star / tx and the rotated star position
-    double im_size, dx, tdx, alpha, dvel, v0;
+    double im_size, dx, inv_dx, tdx, alpha, dvel, v0;
+    float R[9];              // the rotation (column-major), for directions in the unrotated frame
     const double *xyz;       // rotated (3,N)
     const double *nrm2;      // |X|^2 per node
     const int *off, *idx;    // neighbour CSR
+    const float4 *edge;      // (e, |e|^2/2) per directed edge, unrotated
     const float4 *cellv, *cellb, *coef;
-    const double *dust_p, *tdust;
-    int2 *walk;              // per warp: 32 pixels x n_depth
+    const double *dust_p, *ibb;   // dust density; Planck function of the dust (nlines, N)
+    int2 *walk;              // per block: 32 rays x n_depth
     unsigned long long *counters;
     int *status;
     float *out[8];           // (npx, npx, nch, nlines) or (nrays, nch, nlines) each, or null
@@ -197,11 +212,13 @@ __device__ __forceinline__ int lsb_exp(double v) {
 // dx is the REAL*4 step, a 24-bit mantissa, and m < 2^29).  Only a sum that
 // enters a binade whose spacing exceeds g can round; that one addition is
 // made as the reference makes it, after which z lies on the coarser grid.
-__device__ double add_steps(double z, long long n, double dx, int e_dx) {
+// (The quotient only places m, two short of the limit: a product with 1/dx
+// serves.)
+__device__ double add_steps(double z, long long n, double dx, double inv_dx, int e_dx) {
     while (n > 0) {
         const int eg = min(lsb_exp(z), e_dx);
-        const double L = ldexp(1.0, eg + 53);
-        long long m = (long long)floor(__ddiv_rn(__dsub_rn(L, z), dx)) - 2;  // z + m dx < L, with margin
+        const double L = __longlong_as_double((long long)(min(eg + 53, 1022) + 1023) << 52);
+        long long m = (long long)floor((L - z) * inv_dx) - 2;  // z + m dx < L, with margin
         if (m > n) m = n;
         if (m > 0) {
             z = __fma_rn((double)m, dx, z);
@@ -220,232 +237,307 @@ __device__ double black_body(double T, double nu) {
     return 1.4744995e-50 * nu * nu * nu / (exp(4.79924e-11 / T * nu) - 1.0);
 }
 
-template <int NS>
-__global__ void __launch_bounds__(128, 1) k_image(ImArgs a) {
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const long long gw = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    int2 *const wbase = a.walk + (size_t)gw * 32 * (size_t)a.n_depth;
-    const int npix = a.nrays;
-    const int e_dx = lsb_exp(a.dx);
-    for (;;) {
-        int p0 = 0;
-        if (lane == 0) p0 = (int)atomicAdd(&a.counters[0], 32ULL);
-        p0 = __shfl_sync(FULL, p0, 0);
-        if (p0 >= npix) break;
-        // ---- (1) march, one lane per pixel ----
-        // Work index w -> the reference's pixel p = a npx + b (para_finish.f90:
-        // 369-376) with a = w mod npx: consecutive work items step along the
-        // cube's first (fastest) index, so the batch's stores of a channel fill
-        // whole sectors instead of one float every npx^2 (mode 1: w is the node)
-        const int w = p0 + lane;
-        const int p = (a.mode == 1 || w >= npix) ? w : (w % a.npx) * a.npx + w / a.npx;
-        int nc = 0, st = 0, fs = 0;  // fs: the ray starts on the star
-        if (p < npix) {
-            double x, y;
-            if (a.mode == 1) {  // the node's rotated sky position (para_finish.f90:296)
-                x = a.xyz[3 * (size_t)p];
-                y = a.xyz[3 * (size_t)p + 1];
-            } else {
-                const int ia = p / a.npx - a.im_pix, ib = p % a.npx - a.im_pix;
-                x = ia * a.im_size / a.im_pix;
-                y = ib * a.im_size / a.im_pix;
-            }
-            // the oracle's FP64 arithmetic, without FMA contraction, throughout the march
-            const double zs0 = -1.0 * __dsqrt_rn(__dsub_rn(__dsub_rn(1.0, __dmul_rn(x, x)), __dmul_rn(y, y)));
-            double z0 = zs0;
-            if (a.star) {  // raytrace.f90:103-115: on the star's disc, start at its front
-                const double xc = __dsub_rn(x, a.sx), yc = __dsub_rn(y, a.sy);
-                if (__dsqrt_rn(__dadd_rn(__dmul_rn(xc, xc), __dmul_rn(yc, yc))) < a.Rs) {
-                    z0 = __dadd_rn(a.sz, a.Rs);
-                    fs = 1;
+// the dust's Planck function per (line, node)
+__global__ void k_im_dust(int N, int nlines, const double *__restrict__ tdust, double *__restrict__ ibb) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (long long)N * nlines) return;
+    ibb[t] = black_body(tdust[t % N], c_im[t / N].nu0);
+}
+
+// Index of record k of ray r in a block's march scratch (blocks of 32 records,
+// the rays' blocks side by side).
+__device__ __forceinline__ int march_at(int k, int r) { return ((k >> 5) << 10) + (r << 5) + (k & 31); }
+
+constexpr int IM_WARPS = 4;        // warps per block
+constexpr double IM_NEAR = 1e-12;  // squared distances closer than this are compared in FP64 at every step
+
+// The start node (raytrace.f90:126-134 scans all nodes; strict <, so the
+// lowest index wins) and its distance.  The same argmin by greedy descent on
+// the Delaunay graph: a node that is not the nearest has a neighbour at most
+// as far (the segment to the point leaves its Voronoi cell through a face
+// shared with that neighbour), so descending in (distance, index) order ends
+// at the nearest node with the lowest index, from any start.  The descent
+// runs in FP32 on the edge records (nearer by e.r > |e|^2/2); FP64 distances,
+// computed exactly as the reference's norm2, decide between the last node and
+// the neighbours that FP32 cannot tell from it.
+__device__ int start_node(const ImArgs &a, int c, double x, double y, double z0, double *best_out) {
+    auto dist = [&](int i) {
+        return __dsqrt_rn(dsum3sq(x - a.xyz[3 * (size_t)i], y - a.xyz[3 * (size_t)i + 1],
+                                  z0 - a.xyz[3 * (size_t)i + 2]));
+    };
+    auto offset = [&](int i, float &rx, float &ry, float &rz) {   // point - node, unrotated frame
+        const float ux = (float)(x - a.xyz[3 * (size_t)i]), uy = (float)(y - a.xyz[3 * (size_t)i + 1]),
+                    uz = (float)(z0 - a.xyz[3 * (size_t)i + 2]);
+        rx = a.R[0] * ux + a.R[1] * uy + a.R[2] * uz;
+        ry = a.R[3] * ux + a.R[4] * uy + a.R[5] * uz;
+        rz = a.R[6] * ux + a.R[7] * uy + a.R[8] * uz;
+    };
+    double best = 0.0;
+    float rx, ry, rz;
+    offset(c, rx, ry, rz);
+    bool fine = false;
+    for (int hop = 0; hop < 2 * a.N; hop++) {
+        const int o = a.off[c], deg = a.off[c + 1] - o;
+        float g = 0.f;
+        int bj = -1;
+        unsigned long long close = 0ULL;   // (first 64) neighbours not certainly farther
+        const float r2 = rx * rx + ry * ry + rz * rz;
+        for (int j0 = 0; j0 < deg; j0 += 8) {
+            float4 e8[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) e8[i] = a.edge[o + min(j0 + i, deg - 1)];
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const float4 e = e8[i];
+                const float gain = e.x * rx + e.y * ry + e.z * rz - e.w, tol = 1e-6f * (2.f * e.w + r2);
+                if (j0 + i >= deg) continue;
+                if (gain > tol + g) {
+                    g = gain - tol;
+                    bj = j0 + i;
                 }
-            }
-            int2 *dl = wbase + (size_t)lane * a.n_depth;
-            // nearest node to the start point (raytrace.f90:126-134 scans all
-            // nodes; strict <, so the lowest index wins).  The same argmin by
-            // greedy descent on the Delaunay graph: a node that is not the
-            // nearest has a neighbour at most as far (the segment to the point
-            // leaves its Voronoi cell through a face shared with that
-            // neighbour), so descending in (distance, index) order from node 0
-            // ends at the nearest node with the lowest index; distances are
-            // computed exactly as the reference's norm2.
-            auto dist = [&](int i) {
-                return __dsqrt_rn(dsum3sq(x - a.xyz[3 * (size_t)i], y - a.xyz[3 * (size_t)i + 1],
-                                          z0 - a.xyz[3 * (size_t)i + 2]));
-            };
-            int c = 0;
-            double best = dist(0);
-            for (int hop = 0; hop < a.N; hop++) {
-                int nbest = c;
-                double dbest = best;
-                for (int q = a.off[c]; q < a.off[c + 1]; q++) {
-                    const int nb = a.idx[q];
-                    const double d = dist(nb);
-                    if (d < dbest || (d == dbest && nb < nbest)) { dbest = d; nbest = nb; }
-                }
-                if (nbest == c) break;
-                c = nbest;
-                best = dbest;
-            }
-            if (!(best < 10.0)) { c = -1; st = 3; }  // start point outside the unit sphere (NaN; rsave = 10)
-            double z = z0;
-            int k = 0;
-            const double zexit = -zs0;
-            while (st == 0) {
-                // predicted first step at which a neighbour is nearer than c
-                const double cx = a.xyz[3 * (size_t)c], cy = a.xyz[3 * (size_t)c + 1],
-                             cz = a.xyz[3 * (size_t)c + 2];
-                const double cc = a.nrm2[c];
-                const int o = a.off[c], deg = a.off[c + 1] - o;
-                // Candidates of the replay below: the neighbours (of the first 64)
-                // that come within 1e-12 of c's squared distance somewhere up to
-                // z_lim.  Every other neighbour stays farther than c by more than
-                // the FP64 rounding of both squared distances (~1e-15), so it
-                // cannot win check_neigh's strict comparison and skipping it leaves
-                // the scan's outcome unchanged.
-                const double WIN = 6.0 * a.dx;
-                unsigned long long cand = 0ULL;
-                // the predicted crossing zt = tn / td, the minimum of A / (2 dzn) kept
-                // as a fraction (compared by cross-multiplication, one division at the end)
-                double tn = zexit, td = 1.0;
-                for (int j = 0; j < deg; j++) {
-                    const int nb = a.idx[o + j];
-                    const double nx = a.xyz[3 * (size_t)nb], ny = a.xyz[3 * (size_t)nb + 1],
-                                 nz = a.xyz[3 * (size_t)nb + 2];
-                    // |P-X_n|^2 - |P-X_c|^2 = A - 2 z dzn along the ray
-                    const double dzn = nz - cz;
-                    const double A = a.nrm2[nb] - cc - 2.0 * x * (nx - cx) - 2.0 * y * (ny - cy);
-                    if (A - 2.0 * z * dzn < 1e-12) {   // already (nearly) nearer: replay now
-                        tn = z;
-                        td = 1.0;
-                        if (j < 64) cand |= 1ULL << j;
-                    } else if (dzn > 0.0) {
-                        const double d2 = 2.0 * dzn;
-                        if (A * td < tn * d2) {
-                            tn = A;
-                            td = d2;
-                        }
-                        // A - 2 z' dzn <= 1e-12 for some z' <= zt + WIN (zt only falls
-                        // further in this loop, so the set is a superset)
-                        if (j < 64 && (A - 1e-12) * td <= d2 * (tn + WIN * td)) cand |= 1ULL << j;
-                    }
-                }
-                const double zt = tn / td;
-                const double z_lim = zt + WIN;
-                long long kt = (long long)floor((zt - z0) / a.dx) - 3;
-                if ((long long)k < kt) {  // the reference's own additions, in jumps
-                    z = add_steps(z, kt - k, a.dx, e_dx);
-                    k = (int)kt;
-                }
-                // exact replay of trace_out_raytrace's loop until c changes or the ray exits
-                bool done = false, changed = false;
-                while (!done && !changed) {
-                    z = z + a.dx;
-                    k++;
-                    const bool exited = __dsqrt_rn(dsum3sq(x, y, z)) > 1.0;  // norm2(X_phot) > 1
-                    if (exited) {
-                        if (nc >= a.n_depth) { st = 1; break; }
-                        dl[nc++] = make_int2(c, k);
-                        done = true;
-                    }
-                    // check_neigh miscellaneous.f90:1-46, in list order: the candidates
-                    // while z <= z_lim (and every neighbour past the 64th), else all
-                    double d0 = dsum3sq(x - cx, y - cy, z - cz);
-                    int nn = c;
-                    auto probe = [&](int j) {
-                        const int nb = a.idx[o + j];
-                        const double ex = x - a.xyz[3 * (size_t)nb], ey = y - a.xyz[3 * (size_t)nb + 1],
-                                     ez = z - a.xyz[3 * (size_t)nb + 2];
-                        const double dd = dsum3sq(ex, ey, ez);
-                        if (dd < d0) { d0 = dd; nn = nb; }
-                    };
-                    if (z <= z_lim) {
-                        for (unsigned long long m = cand; m; m &= m - 1ULL) probe(__ffsll((long long)m) - 1);
-                        for (int j = 64; j < deg; j++) probe(j);
-                    } else {
-                        for (int j = 0; j < deg; j++) probe(j);
-                    }
-                    if (nn != c) {
-                        if (nc >= a.n_depth) { st = 1; break; }
-                        dl[nc++] = make_int2(nn, k);
-                        c = nn;
-                        changed = true;
-                    }
-                }
-                if (done || st) break;
+                if (j0 + i < 64 && gain > -tol) close |= 1ULL << (j0 + i);
             }
         }
-        if (p < npix && a.status) a.status[p] = st;
-        __syncwarp();
-        // ---- (2) integration of each pixel of the batch, lanes over channels ----
+        if (!fine && bj >= 0) {
+            c = a.idx[o + bj];
+            offset(c, rx, ry, rz);
+            continue;
+        }
+        // FP64: (distance, index) order over the neighbours in doubt
+        if (!fine) best = dist(c);
+        fine = true;
+        int nbest = c;
+        double dbest = best;
+        auto probe = [&](int j) {
+            const int nb = a.idx[o + j];
+            const double d = dist(nb);
+            if (d < dbest || (d == dbest && nb < nbest)) { dbest = d; nbest = nb; }
+        };
+        for (unsigned long long m = close; m; m &= m - 1ULL) probe(__ffsll((long long)m) - 1);
+        for (int j = 64; j < deg; j++) probe(j);
+        if (nbest == c) break;
+        c = nbest;
+        best = dbest;
+        offset(c, rx, ry, rz);
+    }
+    *best_out = best;
+    return c;
+}
+
+// The fixed-step march of one ray along +z (trace_out_raytrace): records
+// (node, step) at every change of the nearest node and at the exit.
+// Returns the record count; *st: 1 more than n_depth records, 3 the start
+// point is outside the unit sphere.
+__device__ int march(const ImArgs &a, int ray, int lane, int2 *dl, int *hint, int *st_out, int *fs_out, int e_dx) {
+    const int p = ray;
+    double x, y;
+    if (a.mode == 1) {  // the node's rotated sky position (para_finish.f90:296)
+        x = a.xyz[3 * (size_t)p];
+        y = a.xyz[3 * (size_t)p + 1];
+    } else {
+        const int ia = p / a.npx - a.im_pix, ib = p % a.npx - a.im_pix;
+        x = ia * a.im_size / a.im_pix;
+        y = ib * a.im_size / a.im_pix;
+    }
+    // the oracle's FP64 arithmetic, without FMA contraction, throughout the march
+    const double zs0 = -1.0 * __dsqrt_rn(__dsub_rn(__dsub_rn(1.0, __dmul_rn(x, x)), __dmul_rn(y, y)));
+    double z0 = zs0;
+    if (a.star) {  // raytrace.f90:103-115: on the star's disc, start at its front
+        const double xc = __dsub_rn(x, a.sx), yc = __dsub_rn(y, a.sy);
+        if (__dsqrt_rn(__dadd_rn(__dmul_rn(xc, xc), __dmul_rn(yc, yc))) < a.Rs) {
+            z0 = __dadd_rn(a.sz, a.Rs);
+            *fs_out = 1;
+        }
+    }
+    double best;
+    int c = start_node(a, *hint, x, y, z0, &best);
+    if (!(best < 10.0)) {  // start point outside the unit sphere (NaN; rsave = 10)
+        *st_out = 3;
+        return 0;
+    }
+    *hint = c;
+    double z = z0;
+    int k = 0, nc = 0;
+    const double zexit = -zs0;
+    const float nx = a.R[2], ny = a.R[5], nz = a.R[8];   // the ray's direction, unrotated frame
+    for (;;) {
+        // Where the nearest node can change next: in FP32 on the edge records,
+        // with bounds on their rounding.  Half the difference of the squared
+        // distances to neighbour j and to c at a distance s ahead is num - s
+        // den, num = |e|^2/2 - e.r and den = e.n; |num| is off by less than B =
+        // 1e-6 (|e|^2 + |r|^2), den by less than D = 4e-7 |e|.  So a crossing
+        // lies before s_up = min (num + B)/(den - D), and only neighbours with
+        // num - B - s (den + D) <= IM_NEAR up to s = s_up + window can win
+        // check_neigh's strict comparison there; FP64 then looks at those alone.
+        const double cx = a.xyz[3 * (size_t)c], cy = a.xyz[3 * (size_t)c + 1], cz = a.xyz[3 * (size_t)c + 2];
+        const int o = a.off[c], deg = a.off[c + 1] - o;
+        const float ux = (float)(x - cx), uy = (float)(y - cy), uz = (float)(z - cz);
+        const float rx = a.R[0] * ux + a.R[1] * uy + a.R[2] * uz;
+        const float ry = a.R[3] * ux + a.R[4] * uy + a.R[5] * uz;
+        const float rz = a.R[6] * ux + a.R[7] * uy + a.R[8] * uz;
+        const float r2 = rx * rx + ry * ry + rz * rz;
+        const double WIN = 6.0 * a.dx;
+        const float win = 8.f * (float)a.dx;
+        unsigned long long cand = 0ULL;   // of the first 64 neighbours
+        float un = fmaxf((float)(zexit - z), 0.f) + win, ud = 1.f;   // s_up
+        for (int j0 = 0; j0 < deg; j0 += 8) {
+            float4 e8[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) e8[i] = a.edge[o + min(j0 + i, deg - 1)];
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const float4 e = e8[i];
+                if (j0 + i >= deg) continue;
+                const float num = e.w - (e.x * rx + e.y * ry + e.z * rz), den = e.x * nx + e.y * ny + e.z * nz;
+                const float B = 1e-6f * (2.f * e.w + r2), D = 4e-7f * sqrtf(2.f * e.w);
+                const float hn = fmaxf(num + B, 0.f), hd = den - D;
+                if (hd > 0.f && hn * ud < un * hd) {
+                    un = hn;
+                    ud = hd;
+                }
+                // (s_up only falls further in this loop: the set is a superset)
+                if (j0 + i < 64 && (num - B - 1e-12f) * ud <= (den + D) * (un + win * ud)) cand |= 1ULL << (j0 + i);
+                if (j0 + i < 64 && num - B <= 1e-12f) cand |= 1ULL << (j0 + i);
+            }
+        }
+        // the FP64 crossings of the candidates: the steps before kt are those at
+        // which every neighbour is farther than c by IM_NEAR or more, which
+        // exceeds the FP64 rounding of both squared distances (~1e-15)
+        double tn = zexit, td = 1.0;
+        bool now = false;
+        const double cc = a.nrm2[c];
+        auto cross = [&](int j) {
+            const int nb = a.idx[o + j];
+            const double gx = a.xyz[3 * (size_t)nb], gy = a.xyz[3 * (size_t)nb + 1], gz = a.xyz[3 * (size_t)nb + 2];
+            // |P-X_n|^2 - |P-X_c|^2 = A - 2 z dzn along the ray
+            const double d2 = 2.0 * (gz - cz);
+            const double A = a.nrm2[nb] - cc - 2.0 * x * (gx - cx) - 2.0 * y * (gy - cy) - IM_NEAR;
+            if (A - z * d2 < 0.0) now = true;   // already (nearly) nearer: replay now
+            else if (d2 > 0.0 && A * td < tn * d2) {
+                tn = A;
+                td = d2;
+            }
+        };
+        {
+            const float s_lim = un / ud + win;
+            unsigned long long keep = 0ULL;
+            for (unsigned long long m = cand; m; m &= m - 1ULL) {
+                const int j = __ffsll((long long)m) - 1;
+                const float4 e = a.edge[o + j];
+                const float num = e.w - (e.x * rx + e.y * ry + e.z * rz), den = e.x * nx + e.y * ny + e.z * nz;
+                const float B = 1e-6f * (2.f * e.w + r2), D = 4e-7f * sqrtf(2.f * e.w);
+                if (num - B - 1e-12f > 0.f && num - B - 1e-12f > s_lim * (den + D)) continue;
+                keep |= 1ULL << j;
+                cross(j);
+            }
+            cand = keep;
+            for (int j = 64; j < deg; j++) cross(j);
+        }
+        const double zt = now ? z : tn / td;
+        const double z_lim = fmin(zt, zexit) + WIN;
+        if (!now) {
+            // z after k steps is z0 + k dx to ~1e-12, far within the 1e-6 of a step
+            // left here; the exit is replayed from three steps before
+            const long long kt = min((long long)floor((zt - z0) * a.inv_dx - 1e-6),
+                                     (long long)floor((zexit - z0) * a.inv_dx) - 3);
+            if ((long long)k < kt) {  // the reference's own additions, in jumps
+                z = add_steps(z, kt - k, a.dx, a.inv_dx, e_dx);
+                k = (int)kt;
+            }
+        }
+        // exact replay of trace_out_raytrace's loop until c changes or the ray exits
+        bool done = false, changed = false;
+        while (!done && !changed) {
+            z = z + a.dx;
+            k++;
+            // norm2(X_phot) > 1: the rounded root of s exceeds 1 when s exceeds 1 + 2^-52
+            if (dsum3sq(x, y, z) > 1.0 + 0x1p-52) {
+                if (nc >= a.n_depth) { *st_out = 1; return nc; }
+                dl[march_at(nc++, lane)] = make_int2(c, k);
+                done = true;
+            }
+            // check_neigh miscellaneous.f90:1-46, in list order: the candidates
+            // while z <= z_lim (and every neighbour past the 64th), else all
+            double d0 = dsum3sq(x - cx, y - cy, z - cz);
+            int nn = c;
+            auto probe = [&](int j) {
+                const int nb = a.idx[o + j];
+                const double ex = x - a.xyz[3 * (size_t)nb], ey = y - a.xyz[3 * (size_t)nb + 1],
+                             ez = z - a.xyz[3 * (size_t)nb + 2];
+                const double dd = dsum3sq(ex, ey, ez);
+                if (dd < d0) { d0 = dd; nn = nb; }
+            };
+            if (z <= z_lim) {
+                for (unsigned long long m = cand; m; m &= m - 1ULL) probe(__ffsll((long long)m) - 1);
+                for (int j = 64; j < deg; j++) probe(j);
+            } else {
+                for (int j = 0; j < deg; j++) probe(j);
+            }
+            if (nn != c) {
+                if (nc >= a.n_depth) { *st_out = 1; return nc; }
+                dl[march_at(nc++, lane)] = make_int2(nn, k);
+                c = nn;
+                changed = true;
+            }
+        }
+        if (done) break;
+    }
+    return nc;
+}
+
+// One block per 32 rays (persistent): the first warp marches them, lane = ray;
+// then every warp integrates its share of the rays, lanes over channels, from
+// cell records staged 32 at a time, and the dust terms -- independent of the
+// channel, FP64 -- are summed lane = ray, one line per warp.
+template <int NS>
+__global__ void __launch_bounds__(32 * IM_WARPS, NS <= 5 ? 4 : 3) k_image(ImArgs a) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int2 *const dl = a.walk + (size_t)blockIdx.x * 1024 * (size_t)((a.n_depth + 31) / 32);
+    __shared__ float4 s_cv[IM_WARPS][32], s_cf[IM_WARPS][32];
+    __shared__ float s_dk[IM_WARPS][32];
+    __shared__ float4 s_dust[IM_MAX_LINES][32];
+    __shared__ int s_nc[32], s_st[32], s_fs[32], s_p0;
+    const int npix = a.nrays;
+    const int e_dx = lsb_exp(a.dx);
+    int hint = 0;
+    // Work index w -> the reference's pixel p = a npx + b (para_finish.f90:
+    // 369-376) with a = w mod npx: consecutive work items step along the
+    // cube's first (fastest) index, so the batch's stores of a channel fill
+    // whole sectors instead of one float every npx^2 (mode 1: w is the node)
+    auto ray_of = [&](int w) { return (a.mode == 1) ? w : (w % a.npx) * a.npx + w / a.npx; };
+    for (;;) {
+        if (threadIdx.x == 0) s_p0 = (int)atomicAdd(&a.counters[0], 32ULL);
+        __syncthreads();
+        const int p0 = s_p0;
+        if (p0 >= npix) break;
+        if (warp == 0) {
+            int nc = 0, st = 0, fs = 0;
+            if (p0 + lane < npix) {
+                const int p = ray_of(p0 + lane);
+                nc = march(a, p, lane, dl, &hint, &st, &fs, e_dx);
+                if (a.status) a.status[p] = st;
+            }
+            s_nc[lane] = nc;
+            s_st[lane] = st;
+            s_fs[lane] = fs;
+        }
+        __syncthreads();
         const int npx_b = min(32, npix - p0);
-        for (int rr = 0; rr < npx_b; rr++) {
-            const int ncr = __shfl_sync(FULL, nc, rr);
-            const int str = __shfl_sync(FULL, st, rr);
-            const int fsr = __shfl_sync(FULL, fs, rr);
-            const int wr = p0 + rr;
-            const int pix = (a.mode == 1) ? wr : (wr % a.npx) * a.npx + wr / a.npx;
-            const int2 *dl = wbase + (size_t)rr * a.n_depth;
-            for (int j = 0; j < a.nlines; j++) {
+        // dust terms (raytrace.f90:268-290, finish :301-317): one line per warp
+        if (a.out[4] || a.out[5] || a.out[6] || a.out[7])
+            for (int j = IM_WARPS - 1 - warp; j < a.nlines; j += IM_WARPS) {
                 const ImLine L = c_im[j];
-                float I[NS], Q[NS], U[NS], tau[NS], tauc[NS];
-                const double Iin_d = fsr ? L.bb_star : L.bb_cmb;  // I_in (raytrace.f90:97-115)
-                const float Iin = (float)Iin_d;
-#pragma unroll
-                for (int s = 0; s < NS; s++) { I[s] = Iin; Q[s] = 0.f; U[s] = 0.f; tau[s] = 0.f; tauc[s] = 0.f; }
-                // dust terms: channel independent, FP64, every lane alike
-                double Id = Iin_d, sig0 = 0.0, sig2 = 0.0, Qd = 0.0, Ud = 0.0, taud = 0.0;
-                for (int i = 0; i + 1 < ncr && str == 0; i++) {
-                    const int2 e0 = dl[i], e1 = dl[i + 1];
-                    const int cell = e0.x;
-                    const int dk = e1.y - e0.y;
-                    const float4 cv = a.cellv[cell];
-                    const float4 cf = a.coef[(size_t)j * a.N + cell];
-                    const float fdk = (float)dk;
-#pragma unroll
-                    for (int s = 0; s < NS; s++) {
-                        const int ch = lane + 32 * s;
-                        if (ch < a.nch) {
-                            const float vobs = (float)((ch - a.nvel) * a.dvel + a.v0);
-                            const float q = (vobs - cv.x) * cv.y;
-                            const float vc = expf(-q * q) * fdk;
-                            const float ta = cf.x * vc, tq = cf.y * vc, ei = cf.z * vc, eq = cf.w * vc;
-                            if (ta > 1e-30f) {  // raytrace.f90:260
-                                // rot_stokes into the node frame
-                                const float Qn = Q[s] * cv.z + U[s] * cv.w;
-                                const float Un = U[s] * cv.z - Q[s] * cv.w;
-                                const float pm = ta - tq, pp = ta + tq;
-                                const float Ep = expf(-pm), Em = expf(-pp);
-                                const float fp = phi1(pm), fm = phi1(pp);
-                                const float o11 = 0.5f * (fp + fm), o12 = -0.5f * (fp - fm);
-                                const float ech = 0.5f * (Ep + Em), esh = 0.5f * (Ep - Em);
-                                const float In = o11 * ei + o12 * eq + (ech * I[s] - esh * Qn);
-                                const float Qo = o12 * ei + o11 * eq + (-esh * I[s] + ech * Qn);
-                                const float Uo = Un * expf(-ta);
-                                I[s] = In;
-                                // rot_stokes_back
-                                Q[s] = Qo * cv.z - Uo * cv.w;
-                                U[s] = Uo * cv.z + Qo * cv.w;
-                                // compensated tau sum
-                                const float yk = ta - tauc[s];
-                                const float tk = tau[s] + yk;
-                                tauc[s] = (tk - tau[s]) - yk;
-                                tau[s] = tk;
-                            } else if (cv.z != cv.z) {
-                                // the reference rotates Q, U into the node frame and back at
-                                // every cell; a field along the line of sight has no frame
-                                // (NaN angle), which makes them NaN there too
-                                Q[s] = cv.z;
-                                U[s] = cv.z;
-                            }
-                        }
-                    }
-                    // dust (raytrace.f90:268-290)
+                const double Iin = s_fs[lane] ? L.bb_star : L.bb_cmb;
+                double Id = Iin, sig0 = 0.0, sig2 = 0.0, Qd = 0.0, Ud = 0.0, taud = 0.0;
+                const int ncr = (a.dust && s_st[lane] == 0) ? s_nc[lane] : 0;
+                for (int i = 0; i + 1 < ncr; i++) {
+                    const int2 e0 = dl[march_at(i, lane)];
+                    const int cell = e0.x, dk = dl[march_at(i + 1, lane)].y - e0.y;
                     const double tau_d = L.kd * a.dust_p[cell] * (a.tdx * (double)dk);
                     if (tau_d > 1e-30) {
                         const float4 cb = a.cellb[cell];
-                        const double Ibb = black_body(a.tdust[cell], L.nu0);
+                        const double Ibb = a.ibb[(size_t)j * a.N + cell];
                         const double ed = exp(-tau_d);
                         const double mu2 = cb.x;
                         const double sI = 0.5 * a.alpha * (mu2 - 2.0 / 3.0), sQ = a.alpha * mu2;
@@ -457,14 +549,82 @@ __global__ void __launch_bounds__(128, 1) k_image(ImArgs a) {
                         taud = taud + tau_d;
                     }
                 }
-                // finish (raytrace.f90:301-317)
-                const double Ic = L.bb_cmb;
-                double Idf = Id - Ic, Qdf = 0.0, Udf = 0.0, tdf = 0.0;
+                double Idf = Id - L.bb_cmb, Qdf = 0.0, Udf = 0.0, tdf = 0.0;
                 if (Idf != 0.0) {
                     Qdf = Idf * Qd / (sig0 - sig2);
                     Udf = Idf * Ud / (sig0 - sig2);
                     tdf = taud;
                 }
+                s_dust[j][lane] = make_float4((float)Idf, (float)Qdf, (float)Udf, (float)tdf);
+            }
+        __syncthreads();
+        for (int rr = warp; rr < npx_b; rr += IM_WARPS) {
+            const bool bad = s_st[rr] != 0;
+            const int ncr = bad ? 0 : s_nc[rr];
+            const int pix = ray_of(p0 + rr);
+            for (int j = 0; j < a.nlines; j++) {
+                const double Ic = c_im[j].bb_cmb;
+                float I[NS], Q[NS], U[NS], tau[NS], tauc[NS];
+                const float Iin = (float)(s_fs[rr] ? c_im[j].bb_star : Ic);  // I_in (raytrace.f90:97-115)
+#pragma unroll
+                for (int s = 0; s < NS; s++) { I[s] = Iin; Q[s] = 0.f; U[s] = 0.f; tau[s] = 0.f; tauc[s] = 0.f; }
+                for (int i0 = 0; i0 + 1 < ncr; i0 += 32) {
+                    const int n = min(32, ncr - 1 - i0);
+                    __syncwarp();
+                    if (lane < n) {
+                        const int2 e0 = dl[march_at(i0 + lane, rr)];
+                        const int k1 = dl[march_at(i0 + lane + 1, rr)].y;
+                        s_cv[warp][lane] = a.cellv[e0.x];
+                        s_cf[warp][lane] = a.coef[(size_t)j * a.N + e0.x];
+                        s_dk[warp][lane] = (float)(k1 - e0.y);
+                    }
+                    __syncwarp();
+                    for (int i = 0; i < n; i++) {
+                        const float4 cv = s_cv[warp][i];
+                        const float4 cf = s_cf[warp][i];
+                        const float fdk = s_dk[warp][i];
+#pragma unroll
+                        for (int s = 0; s < NS; s++) {
+                            const int ch = lane + 32 * s;
+                            if (ch < a.nch) {
+                                const float vobs = (float)((ch - a.nvel) * a.dvel + a.v0);
+                                const float q = (vobs - cv.x) * cv.y;
+                                const float vc = expf(-q * q) * fdk;
+                                const float ta = cf.x * vc, tq = cf.y * vc, ei = cf.z * vc, eq = cf.w * vc;
+                                if (ta > 1e-30f) {  // raytrace.f90:260
+                                    // rot_stokes into the node frame
+                                    const float Qn = Q[s] * cv.z + U[s] * cv.w;
+                                    const float Un = U[s] * cv.z - Q[s] * cv.w;
+                                    const float pm = ta - tq, pp = ta + tq;
+                                    const float Ep = expf(-pm), Em = expf(-pp);
+                                    const float fp = phi1(pm), fm = phi1(pp);
+                                    const float o11 = 0.5f * (fp + fm), o12 = -0.5f * (fp - fm);
+                                    const float ech = 0.5f * (Ep + Em), esh = 0.5f * (Ep - Em);
+                                    const float In = o11 * ei + o12 * eq + (ech * I[s] - esh * Qn);
+                                    const float Qo = o12 * ei + o11 * eq + (-esh * I[s] + ech * Qn);
+                                    const float Uo = Un * expf(-ta);
+                                    I[s] = In;
+                                    // rot_stokes_back
+                                    Q[s] = Qo * cv.z - Uo * cv.w;
+                                    U[s] = Uo * cv.z + Qo * cv.w;
+                                    // compensated tau sum
+                                    const float yk = ta - tauc[s];
+                                    const float tk = tau[s] + yk;
+                                    tauc[s] = (tk - tau[s]) - yk;
+                                    tau[s] = tk;
+                                } else if (cv.z != cv.z) {
+                                    // the reference rotates Q, U into the node frame and back at
+                                    // every cell; a field along the line of sight has no frame
+                                    // (NaN angle), which makes them NaN there too
+                                    Q[s] = cv.z;
+                                    U[s] = cv.z;
+                                }
+                            }
+                        }
+                    }
+                }
+                const float4 ds = (a.out[4] || a.out[5] || a.out[6] || a.out[7]) ? s_dust[j][rr]
+                                                                                 : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
                 for (int s = 0; s < NS; s++) {
                     const int ch = lane + 32 * s;
@@ -477,11 +637,10 @@ __global__ void __launch_bounds__(128, 1) k_image(ImArgs a) {
                             o = (size_t)ia + (size_t)a.npx * ((size_t)ib + (size_t)a.npx *
                                                               ((size_t)ch + (size_t)a.nch * j));
                         }
-                        const bool bad = (str != 0);
                         const float vals[8] = {bad ? NAN : (float)((double)I[s] - Ic), bad ? NAN : Q[s],
                                                bad ? NAN : U[s], bad ? NAN : tau[s],
-                                               bad ? NAN : (float)Idf, bad ? NAN : (float)Qdf,
-                                               bad ? NAN : (float)Udf, bad ? NAN : (float)tdf};
+                                               bad ? NAN : ds.x, bad ? NAN : ds.y,
+                                               bad ? NAN : ds.z, bad ? NAN : ds.w};
 #pragma unroll
                         for (int q2 = 0; q2 < 8; q2++)
                             if (a.out[q2]) a.out[q2][o] = vals[q2];
@@ -489,7 +648,7 @@ __global__ void __launch_bounds__(128, 1) k_image(ImArgs a) {
                 }
             }
         }
-        __syncwarp();
+        __syncthreads();
     }
 }
 
@@ -568,7 +727,7 @@ static int image_call(portal_ctx *c, const double *pol_pops, int nlines, const i
             na.R[i + 3 * j] = s;
         }
     // device buffers
-    DevBuf<double> xyz_r, pops_d, vel_d, nrm2;
+    DevBuf<double> xyz_r, pops_d, vel_d, nrm2, ibb;
     DevBuf<int> jl;
     DevBuf<float4> cellv, cellb, coef;
     DevBuf<float> outd;
@@ -593,6 +752,12 @@ static int image_call(portal_ctx *c, const double *pol_pops, int nlines, const i
     k_im_nodes<<<(N + 127) / 128, 128, 0, c->stream>>>(na);
     timer_stop(c, T_EMCOEF);
     PCHECK(c, cudaGetLastError());
+    if (c->has_dust) {
+        if (ibb.reserve((size_t)nlines * N)) return set_err(c, PORTAL_ERR_NOMEM, "dust emission");
+        const long long tot = (long long)nlines * N;
+        k_im_dust<<<(unsigned)((tot + 127) / 128), 128, 0, c->stream>>>(N, nlines, c->tdust.p, ibb.p);
+        PCHECK(c, cudaGetLastError());
+    }
     // outputs on the device
     int nout = 0;
     for (int q = 0; q < 8; q++) nout += dout[q] ? 1 : 0;
@@ -612,24 +777,30 @@ static int image_call(portal_ctx *c, const double *pol_pops, int nlines, const i
     }
     ia.n_depth = n_depth_rt; ia.im_size = im_size; ia.dx = dx; ia.tdx = c->tx * dx; ia.alpha = alpha; ia.dvel = dvel; ia.v0 = v0;
     ia.xyz = xyz_r.p; ia.nrm2 = nrm2.p; ia.off = c->nb_off.p; ia.idx = c->nb_idx.p; ia.cellv = cellv.p; ia.cellb = cellb.p;
-    ia.coef = coef.p; ia.dust_p = c->dustp.p; ia.tdust = c->tdust.p; ia.status = stat.p;
+    ia.coef = coef.p; ia.dust_p = c->dustp.p; ia.ibb = ibb.p; ia.dust = c->has_dust; ia.status = stat.p;
+    ia.edge = c->edge.p; ia.inv_dx = 1.0 / dx;
+    for (int i = 0; i < 9; i++) ia.R[i] = (float)na.R[i];
     {
         int q2 = 0;
         for (int q = 0; q < 8; q++) ia.out[q] = dout[q] ? outd.p + cube * (q2++) : nullptr;
     }
-    int grid = c->sm_count * 4;
-    size_t nslots = (size_t)grid * 4;
-    if (c->walk.reserve(nslots * 32 * (size_t)n_depth_rt) != cudaSuccess)
+    const void *kern = nch <= 32    ? (const void *)k_image<1>
+                       : nch <= 64  ? (const void *)k_image<2>
+                       : nch <= 96  ? (const void *)k_image<3>
+                       : nch <= 160 ? (const void *)k_image<5>
+                                    : (const void *)k_image<9>;
+    int nb = 0;
+    PCHECK(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, 32 * IM_WARPS, 0));
+    const int grid = (int)std::min<long long>((long long)std::max(1, nb) * c->sm_count,
+                                              std::max(1, (nrays + 31) / 32));
+    if (c->walk.reserve((size_t)grid * 1024 * (size_t)((n_depth_rt + 31) / 32)) != cudaSuccess)
         return set_err(c, PORTAL_ERR_NOMEM, "image walk scratch");
     ia.walk = c->walk.p;
     ia.counters = c->counters.p;
     PCHECK(c, cudaMemsetAsync(c->counters.p, 0, sizeof(unsigned long long), c->stream));
     timer_start(c, T_IMWALK);
-    if (nch <= 32) k_image<1><<<grid, 128, 0, c->stream>>>(ia);
-    else if (nch <= 64) k_image<2><<<grid, 128, 0, c->stream>>>(ia);
-    else if (nch <= 96) k_image<3><<<grid, 128, 0, c->stream>>>(ia);
-    else if (nch <= 160) k_image<5><<<grid, 128, 0, c->stream>>>(ia);
-    else k_image<9><<<grid, 128, 0, c->stream>>>(ia);
+    void *args[] = {&ia};
+    PCHECK(c, cudaLaunchKernel(kern, dim3(grid), dim3(32 * IM_WARPS), args, 0, c->stream));
     timer_stop(c, T_IMWALK);
     PCHECK(c, cudaGetLastError());
     for (int q = 0; q < 8; q++)
