@@ -15,38 +15,38 @@
 //                the profile peak (float4), plus per-node Stokes-rotation
 //                constants.
 //   k_im_dust    per (node, line): the dust's Planck function.
-//   k_image      one block per 32 pixels (persistent):
-//                 (1) the first warp marches, one lane per pixel: the start
-//                     node (argmin of the FP64 distance, lowest index on
-//                     ties) and the fixed-step march along +z.  The step at
-//                     which a neighbour becomes nearer is predicted from the
-//                     bisector-plane crossings: FP32 with rounding bounds
-//                     picks the few neighbours that can cross next, FP64
-//                     places their crossings.  The photon's z is advanced to
-//                     just before it by the reference's own sequence of FP64
-//                     additions (computed in exact jumps, add_steps), and
-//                     check_neigh is replayed exactly (FP64, strict <, list
-//                     order) from there and at the exit -- over the
-//                     neighbours that can come within 1e-12 of the current
-//                     node's squared distance, the others being unable to
-//                     win -- so the recorded (node, step) list is the
-//                     reference's.  What bounds it: the FP64 pipe (16 cycles
-//                     a warp instruction) and the scattered loads; FP64 for
-//                     every neighbour and a replay from three steps before
-//                     took 10.2 ms for 257 x 257 x 129 of a 32,768-point
-//                     sphere, this 4.1 ms;
-//                 (2) per pixel, lanes over velocity channels, lines looped:
-//                     the polarized propagation in the numerically stable
-//                     form o11 = (phi(p)+phi(m))/2, o12 = -(phi(p)-phi(m))/2,
-//                     e ch = (E_p+E_m)/2, e sh = (E_p-E_m)/2 with p, m =
-//                     tau_I -/+ tau_Q, E = exp(-.), phi(x) = (1-e^-x)/x,
-//                     algebraically identical to raytrace.f90:41-53; the
-//                     optical depth summed with compensation; cell records
-//                     staged in shared memory 32 at a time;
-//                 (3) the channel-independent dust terms (FP64), lane =
-//                     pixel, a line per warp (every lane alike they took most
-//                     of the per-node maps of a dusty cloud: 25.1 ms for
-//                     9,001 nodes x 3 lines, now 1.2 ms).
+//   k_im_march   one lane per pixel: the start node (argmin of the FP64
+//                distance, lowest index on ties) and the fixed-step march
+//                along +z.  The step at which a neighbour becomes nearer is
+//                predicted from the bisector-plane crossings: FP32 with
+//                rounding bounds picks the few neighbours that can cross
+//                next, FP64 places their crossings.  The photon's z is
+//                advanced to just before it by the reference's own sequence of
+//                FP64 additions (computed in exact jumps, add_steps), and
+//                check_neigh is replayed exactly (FP64, strict <, list order)
+//                from there and at the exit -- over the neighbours that can
+//                come within 1e-12 of the current node's squared distance,
+//                the others being unable to win -- so the recorded (node,
+//                step) list is the reference's.  Bound by the FP64 pipe (16
+//                cycles a warp instruction; 70 % busy): 1.26 ms for 257 x 257
+//                pixels of a 32,768-point sphere.
+//   k_im_stokes, k_im_stokes_tail   per (pixel, line), lanes over velocity
+//                channels (whole slots of 32, cell records staged in shared
+//                memory 32 at a time) or, for the few channels left over,
+//                lanes over pixels: the polarized propagation in the
+//                numerically stable form o11 = (phi(p)+phi(m))/2, o12 =
+//                -(phi(p)-phi(m))/2, e ch = (E_p+E_m)/2, e sh = (E_p-E_m)/2
+//                with p, m = tau_I -/+ tau_Q, E = exp(-.), phi(x) =
+//                (1-e^-x)/x, algebraically identical to raytrace.f90:41-53;
+//                the optical depth summed with compensation.  Bound by
+//                instruction issue (FMA pipe 62 %): 1.32 ms for the 128 whole
+//                channels of that cube, 0.04 ms for the last one.
+//   k_im_dust, k_im_dust_maps   the dust's Planck function per (node, line)
+//                and the channel-independent dust terms per (pixel, line),
+//                FP64.
+// March and integration in one kernel, 32 pixels to a warp or block, took
+// 10.2 ms and (marching warp beside three waiting ones) 4.06 ms on that cube;
+// apart 2.62 ms.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -176,8 +176,10 @@ struct ImArgs {
     const float4 *edge;      // (e, |e|^2/2) per directed edge, unrotated
     const float4 *cellv, *cellb, *coef;
     const double *dust_p, *ibb;   // dust density; Planck function of the dust (nlines, N)
-    int2 *walk;              // per block: 32 rays x n_depth
-    unsigned long long *counters;
+    int ray0, rays;          // this launch's rays [ray0, ray0 + rays), of nrays
+    int2 *walk;              // march lists, per batch of 32 rays of the launch: 32 x n_depth
+    int *cnt;                // per ray of the launch: records, -1 the start lies outside, -2 n_depth overflow
+    unsigned char *on_star;  // per ray of the launch: it starts on the star
     int *status;
     float *out[8];           // (npx, npx, nch, nlines) or (nrays, nch, nlines) each, or null
 };
@@ -244,11 +246,25 @@ __global__ void k_im_dust(int N, int nlines, const double *__restrict__ tdust, d
     ibb[t] = black_body(tdust[t % N], c_im[t / N].nu0);
 }
 
-// Index of record k of ray r in a block's march scratch (blocks of 32 records,
-// the rays' blocks side by side).
+// Index of record k of ray r (of its batch of 32) in the batch's march list:
+// blocks of 32 records, the rays' blocks side by side.
 __device__ __forceinline__ int march_at(int k, int r) { return ((k >> 5) << 10) + (r << 5) + (k & 31); }
+__device__ __forceinline__ const int2 *march_list(const ImArgs &a, int i) {
+    return a.walk + (size_t)(i >> 5) * 1024 * (size_t)((a.n_depth + 31) / 32);
+}
+// Work index w -> the reference's pixel p = a npx + b (para_finish.f90:
+// 369-376) with a = w mod npx: consecutive work items step along the cube's
+// first (fastest) index (mode 1: w is the node).
+__device__ __forceinline__ int ray_of(const ImArgs &a, int w) {
+    return (a.mode == 1) ? w : (w % a.npx) * a.npx + w / a.npx;
+}
+// where channel ch of line j of ray p goes in the output arrays
+__device__ __forceinline__ size_t cube_at(const ImArgs &a, int p, int ch, int j) {
+    if (a.mode == 1) return (size_t)p + (size_t)a.nrays * ((size_t)ch + (size_t)a.nch * j);
+    const int ia = p / a.npx, ib = p % a.npx;
+    return (size_t)ia + (size_t)a.npx * ((size_t)ib + (size_t)a.npx * ((size_t)ch + (size_t)a.nch * j));
+}
 
-constexpr int IM_WARPS = 4;        // warps per block
 constexpr double IM_NEAR = 1e-12;  // squared distances closer than this are compared in FP64 at every step
 
 // The start node (raytrace.f90:126-134 scans all nodes; strict <, so the
@@ -260,7 +276,8 @@ constexpr double IM_NEAR = 1e-12;  // squared distances closer than this are com
 // runs in FP32 on the edge records (nearer by e.r > |e|^2/2); FP64 distances,
 // computed exactly as the reference's norm2, decide between the last node and
 // the neighbours that FP32 cannot tell from it.
-__device__ int start_node(const ImArgs &a, int c, double x, double y, double z0, double *best_out) {
+__device__ int start_node(const ImArgs &a, double x, double y, double z0, double *best_out) {
+    int c = 0;
     auto dist = [&](int i) {
         return __dsqrt_rn(dsum3sq(x - a.xyz[3 * (size_t)i], y - a.xyz[3 * (size_t)i + 1],
                                   z0 - a.xyz[3 * (size_t)i + 2]));
@@ -328,7 +345,7 @@ __device__ int start_node(const ImArgs &a, int c, double x, double y, double z0,
 // (node, step) at every change of the nearest node and at the exit.
 // Returns the record count; *st: 1 more than n_depth records, 3 the start
 // point is outside the unit sphere.
-__device__ int march(const ImArgs &a, int ray, int lane, int2 *dl, int *hint, int *st_out, int *fs_out, int e_dx) {
+__device__ int march(const ImArgs &a, int ray, int lane, int2 *dl, int *st_out, int *fs_out, int e_dx) {
     const int p = ray;
     double x, y;
     if (a.mode == 1) {  // the node's rotated sky position (para_finish.f90:296)
@@ -350,15 +367,14 @@ __device__ int march(const ImArgs &a, int ray, int lane, int2 *dl, int *hint, in
         }
     }
     double best;
-    int c = start_node(a, *hint, x, y, z0, &best);
+    int c = start_node(a, x, y, z0, &best);
     if (!(best < 10.0)) {  // start point outside the unit sphere (NaN; rsave = 10)
         *st_out = 3;
         return 0;
     }
-    *hint = c;
     double z = z0;
     int k = 0, nc = 0;
-    const double zexit = -zs0;
+    const double zexit = -zs0, z_inside = zexit - 4.0 * a.dx;   // between -zexit and here no step can exit
     const float nx = a.R[2], ny = a.R[5], nz = a.R[8];   // the ray's direction, unrotated frame
     for (;;) {
         // Where the nearest node can change next: in FP32 on the edge records,
@@ -433,7 +449,10 @@ __device__ int march(const ImArgs &a, int ray, int lane, int2 *dl, int *hint, in
             cand = keep;
             for (int j = 64; j < deg; j++) cross(j);
         }
-        const double zt = now ? z : tn / td;
+        // (the quotient from an FP32 reciprocal and one Newton step: to 1e-13, it
+        // only places the replay)
+        const double rtd = (double)(1.f / (float)td), q0 = tn * rtd;
+        const double zt = now ? z : q0 + (tn - q0 * td) * rtd;
         const double z_lim = fmin(zt, zexit) + WIN;
         if (!now) {
             // z after k steps is z0 + k dx to ~1e-12, far within the 1e-6 of a step
@@ -451,7 +470,7 @@ __device__ int march(const ImArgs &a, int ray, int lane, int2 *dl, int *hint, in
             z = z + a.dx;
             k++;
             // norm2(X_phot) > 1: the rounded root of s exceeds 1 when s exceeds 1 + 2^-52
-            if (dsum3sq(x, y, z) > 1.0 + 0x1p-52) {
+            if (!(z > zs0 && z < z_inside) && dsum3sq(x, y, z) > 1.0 + 0x1p-52) {
                 if (nc >= a.n_depth) { *st_out = 1; return nc; }
                 dl[march_at(nc++, lane)] = make_int2(c, k);
                 done = true;
@@ -485,172 +504,199 @@ __device__ int march(const ImArgs &a, int ray, int lane, int2 *dl, int *hint, in
     return nc;
 }
 
-// One block per 32 rays (persistent): the first warp marches them, lane = ray;
-// then every warp integrates its share of the rays, lanes over channels, from
-// cell records staged 32 at a time, and the dust terms -- independent of the
-// channel, FP64 -- are summed lane = ray, one line per warp.
-template <int NS>
-__global__ void __launch_bounds__(32 * IM_WARPS, NS <= 5 ? 4 : 3) k_image(ImArgs a) {
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int2 *const dl = a.walk + (size_t)blockIdx.x * 1024 * (size_t)((a.n_depth + 31) / 32);
-    __shared__ float4 s_cv[IM_WARPS][32], s_cf[IM_WARPS][32];
-    __shared__ float s_dk[IM_WARPS][32];
-    __shared__ float4 s_dust[IM_MAX_LINES][32];
-    __shared__ int s_nc[32], s_st[32], s_fs[32], s_p0;
-    const int npix = a.nrays;
-    const int e_dx = lsb_exp(a.dx);
-    int hint = 0;
-    // Work index w -> the reference's pixel p = a npx + b (para_finish.f90:
-    // 369-376) with a = w mod npx: consecutive work items step along the
-    // cube's first (fastest) index, so the batch's stores of a channel fill
-    // whole sectors instead of one float every npx^2 (mode 1: w is the node)
-    auto ray_of = [&](int w) { return (a.mode == 1) ? w : (w % a.npx) * a.npx + w / a.npx; };
-    for (;;) {
-        if (threadIdx.x == 0) s_p0 = (int)atomicAdd(&a.counters[0], 32ULL);
-        __syncthreads();
-        const int p0 = s_p0;
-        if (p0 >= npix) break;
-        if (warp == 0) {
-            int nc = 0, st = 0, fs = 0;
-            if (p0 + lane < npix) {
-                const int p = ray_of(p0 + lane);
-                nc = march(a, p, lane, dl, &hint, &st, &fs, e_dx);
-                if (a.status) a.status[p] = st;
-            }
-            s_nc[lane] = nc;
-            s_st[lane] = st;
-            s_fs[lane] = fs;
+// The marches of the launch's rays, one lane per ray, `per` rays to a warp:
+// with few rays a full warp's serial chain (the longest of its 32 marches) is
+// the launch's time, and more warps of fewer rays run beside each other.
+__global__ void __launch_bounds__(64) k_im_march(ImArgs a, int per) {
+    const int i = (blockIdx.x * 2 + (threadIdx.x >> 5)) * per + (threadIdx.x & 31);
+    if ((int)(threadIdx.x & 31) >= per || i >= a.rays) return;
+    const int p = ray_of(a, a.ray0 + i);
+    int st = 0, fs = 0;
+    const int nc = march(a, p, i & 31, const_cast<int2 *>(march_list(a, i)), &st, &fs, lsb_exp(a.dx));
+    a.cnt[i] = st == 0 ? nc : st == 3 ? -1 : -2;
+    a.on_star[i] = (unsigned char)fs;
+    if (a.status) a.status[p] = st;
+}
+
+// The dust maps (raytrace.f90:268-290, finish :301-317): independent of the
+// channel, FP64, one thread per (ray, line).
+__global__ void __launch_bounds__(64) k_im_dust_maps(ImArgs a) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y;
+    if (i >= a.rays) return;
+    const ImLine L = c_im[j];
+    const int ncr = a.cnt[i];
+    const int2 *dl = march_list(a, i);
+    const double Iin = a.on_star[i] ? L.bb_star : L.bb_cmb;
+    double Id = Iin, sig0 = 0.0, sig2 = 0.0, Qd = 0.0, Ud = 0.0, taud = 0.0;
+    for (int k = 0; a.dust && k + 1 < ncr; k++) {
+        const int2 e0 = dl[march_at(k, i & 31)];
+        const int cell = e0.x, dk = dl[march_at(k + 1, i & 31)].y - e0.y;
+        const double tau_d = L.kd * a.dust_p[cell] * (a.tdx * (double)dk);
+        if (tau_d > 1e-30) {
+            const float4 cb = a.cellb[cell];
+            const double Ibb = a.ibb[(size_t)j * a.N + cell];
+            const double ed = exp(-tau_d);
+            const double mu2 = cb.x;
+            const double sI = 0.5 * a.alpha * (mu2 - 2.0 / 3.0), sQ = a.alpha * mu2;
+            Id = Id * ed + Ibb * (1 - ed);
+            sig0 = sig0 * ed + Ibb * (1 - ed);
+            sig2 = sig2 * ed + sI * Ibb * (1 - ed);
+            Qd = Qd * ed + sQ * Ibb * (1 - ed) * cb.y;
+            Ud = Ud * ed + sQ * Ibb * (1 - ed) * cb.z;
+            taud = taud + tau_d;
         }
-        __syncthreads();
-        const int npx_b = min(32, npix - p0);
-        // dust terms (raytrace.f90:268-290, finish :301-317): one line per warp
-        if (a.out[4] || a.out[5] || a.out[6] || a.out[7])
-            for (int j = IM_WARPS - 1 - warp; j < a.nlines; j += IM_WARPS) {
-                const ImLine L = c_im[j];
-                const double Iin = s_fs[lane] ? L.bb_star : L.bb_cmb;
-                double Id = Iin, sig0 = 0.0, sig2 = 0.0, Qd = 0.0, Ud = 0.0, taud = 0.0;
-                const int ncr = (a.dust && s_st[lane] == 0) ? s_nc[lane] : 0;
-                for (int i = 0; i + 1 < ncr; i++) {
-                    const int2 e0 = dl[march_at(i, lane)];
-                    const int cell = e0.x, dk = dl[march_at(i + 1, lane)].y - e0.y;
-                    const double tau_d = L.kd * a.dust_p[cell] * (a.tdx * (double)dk);
-                    if (tau_d > 1e-30) {
-                        const float4 cb = a.cellb[cell];
-                        const double Ibb = a.ibb[(size_t)j * a.N + cell];
-                        const double ed = exp(-tau_d);
-                        const double mu2 = cb.x;
-                        const double sI = 0.5 * a.alpha * (mu2 - 2.0 / 3.0), sQ = a.alpha * mu2;
-                        Id = Id * ed + Ibb * (1 - ed);
-                        sig0 = sig0 * ed + Ibb * (1 - ed);
-                        sig2 = sig2 * ed + sI * Ibb * (1 - ed);
-                        Qd = Qd * ed + sQ * Ibb * (1 - ed) * cb.y;
-                        Ud = Ud * ed + sQ * Ibb * (1 - ed) * cb.z;
-                        taud = taud + tau_d;
-                    }
-                }
-                double Idf = Id - L.bb_cmb, Qdf = 0.0, Udf = 0.0, tdf = 0.0;
-                if (Idf != 0.0) {
-                    Qdf = Idf * Qd / (sig0 - sig2);
-                    Udf = Idf * Ud / (sig0 - sig2);
-                    tdf = taud;
-                }
-                s_dust[j][lane] = make_float4((float)Idf, (float)Qdf, (float)Udf, (float)tdf);
-            }
-        __syncthreads();
-        for (int rr = warp; rr < npx_b; rr += IM_WARPS) {
-            const bool bad = s_st[rr] != 0;
-            const int ncr = bad ? 0 : s_nc[rr];
-            const int pix = ray_of(p0 + rr);
-            for (int j = 0; j < a.nlines; j++) {
-                const double Ic = c_im[j].bb_cmb;
-                float I[NS], Q[NS], U[NS], tau[NS], tauc[NS];
-                const float Iin = (float)(s_fs[rr] ? c_im[j].bb_star : Ic);  // I_in (raytrace.f90:97-115)
+    }
+    double Idf = Id - L.bb_cmb, Qdf = 0.0, Udf = 0.0, tdf = 0.0;
+    if (Idf != 0.0) {
+        Qdf = Idf * Qd / (sig0 - sig2);
+        Udf = Idf * Ud / (sig0 - sig2);
+        tdf = taud;
+    }
+    const bool bad = ncr < 0;
+    const float v[4] = {bad ? NAN : (float)Idf, bad ? NAN : (float)Qdf, bad ? NAN : (float)Udf, bad ? NAN : (float)tdf};
+    const int p = ray_of(a, a.ray0 + i);
+    for (int ch = 0; ch < a.nch; ch++) {
+        const size_t o = cube_at(a, p, ch, j);
 #pragma unroll
-                for (int s = 0; s < NS; s++) { I[s] = Iin; Q[s] = 0.f; U[s] = 0.f; tau[s] = 0.f; tauc[s] = 0.f; }
-                for (int i0 = 0; i0 + 1 < ncr; i0 += 32) {
-                    const int n = min(32, ncr - 1 - i0);
-                    __syncwarp();
-                    if (lane < n) {
-                        const int2 e0 = dl[march_at(i0 + lane, rr)];
-                        const int k1 = dl[march_at(i0 + lane + 1, rr)].y;
-                        s_cv[warp][lane] = a.cellv[e0.x];
-                        s_cf[warp][lane] = a.coef[(size_t)j * a.N + e0.x];
-                        s_dk[warp][lane] = (float)(k1 - e0.y);
-                    }
-                    __syncwarp();
-                    for (int i = 0; i < n; i++) {
-                        const float4 cv = s_cv[warp][i];
-                        const float4 cf = s_cf[warp][i];
-                        const float fdk = s_dk[warp][i];
-#pragma unroll
-                        for (int s = 0; s < NS; s++) {
-                            const int ch = lane + 32 * s;
-                            if (ch < a.nch) {
-                                const float vobs = (float)((ch - a.nvel) * a.dvel + a.v0);
-                                const float q = (vobs - cv.x) * cv.y;
-                                const float vc = expf(-q * q) * fdk;
-                                const float ta = cf.x * vc, tq = cf.y * vc, ei = cf.z * vc, eq = cf.w * vc;
-                                if (ta > 1e-30f) {  // raytrace.f90:260
-                                    // rot_stokes into the node frame
-                                    const float Qn = Q[s] * cv.z + U[s] * cv.w;
-                                    const float Un = U[s] * cv.z - Q[s] * cv.w;
-                                    const float pm = ta - tq, pp = ta + tq;
-                                    const float Ep = expf(-pm), Em = expf(-pp);
-                                    const float fp = phi1(pm), fm = phi1(pp);
-                                    const float o11 = 0.5f * (fp + fm), o12 = -0.5f * (fp - fm);
-                                    const float ech = 0.5f * (Ep + Em), esh = 0.5f * (Ep - Em);
-                                    const float In = o11 * ei + o12 * eq + (ech * I[s] - esh * Qn);
-                                    const float Qo = o12 * ei + o11 * eq + (-esh * I[s] + ech * Qn);
-                                    const float Uo = Un * expf(-ta);
-                                    I[s] = In;
-                                    // rot_stokes_back
-                                    Q[s] = Qo * cv.z - Uo * cv.w;
-                                    U[s] = Uo * cv.z + Qo * cv.w;
-                                    // compensated tau sum
-                                    const float yk = ta - tauc[s];
-                                    const float tk = tau[s] + yk;
-                                    tauc[s] = (tk - tau[s]) - yk;
-                                    tau[s] = tk;
-                                } else if (cv.z != cv.z) {
-                                    // the reference rotates Q, U into the node frame and back at
-                                    // every cell; a field along the line of sight has no frame
-                                    // (NaN angle), which makes them NaN there too
-                                    Q[s] = cv.z;
-                                    U[s] = cv.z;
-                                }
-                            }
-                        }
-                    }
-                }
-                const float4 ds = (a.out[4] || a.out[5] || a.out[6] || a.out[7]) ? s_dust[j][rr]
-                                                                                 : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-                for (int s = 0; s < NS; s++) {
-                    const int ch = lane + 32 * s;
-                    if (ch < a.nch) {
-                        size_t o;
-                        if (a.mode == 1) {
-                            o = (size_t)pix + (size_t)a.nrays * ((size_t)ch + (size_t)a.nch * j);
-                        } else {
-                            const int ia = pix / a.npx, ib = pix % a.npx;
-                            o = (size_t)ia + (size_t)a.npx * ((size_t)ib + (size_t)a.npx *
-                                                              ((size_t)ch + (size_t)a.nch * j));
-                        }
-                        const float vals[8] = {bad ? NAN : (float)((double)I[s] - Ic), bad ? NAN : Q[s],
-                                               bad ? NAN : U[s], bad ? NAN : tau[s],
-                                               bad ? NAN : ds.x, bad ? NAN : ds.y,
-                                               bad ? NAN : ds.z, bad ? NAN : ds.w};
-#pragma unroll
-                        for (int q2 = 0; q2 < 8; q2++)
-                            if (a.out[q2]) a.out[q2][o] = vals[q2];
-                    }
-                }
-            }
-        }
-        __syncthreads();
+        for (int q = 0; q < 4; q++)
+            if (a.out[4 + q]) a.out[4 + q][o] = v[q];
     }
 }
+
+// Stokes state of one (ray, line, channel) along its march.
+struct Stokes {
+    float I, Q, U, tau, tauc;
+    __device__ __forceinline__ void start(float Iin) { I = Iin; Q = 0.f; U = 0.f; tau = 0.f; tauc = 0.f; }
+    // a cell: cv (v_z, 1/b, cos 2 alpha, sin 2 alpha), cf the line's
+    // coefficients, fdk trace steps, vobs the channel's velocity
+    __device__ __forceinline__ void cell(float4 cv, float4 cf, float fdk, float vobs) {
+        const float q = (vobs - cv.x) * cv.y;
+        const float vc = expf(-q * q) * fdk;
+        const float ta = cf.x * vc, tq = cf.y * vc, ei = cf.z * vc, eq = cf.w * vc;
+        if (ta > 1e-30f) {  // raytrace.f90:260
+            // rot_stokes into the node frame
+            const float Qn = Q * cv.z + U * cv.w;
+            const float Un = U * cv.z - Q * cv.w;
+            const float pm = ta - tq, pp = ta + tq;
+            const float Ep = expf(-pm), Em = expf(-pp);
+            const float fp = phi1(pm), fm = phi1(pp);
+            const float o11 = 0.5f * (fp + fm), o12 = -0.5f * (fp - fm);
+            const float ech = 0.5f * (Ep + Em), esh = 0.5f * (Ep - Em);
+            const float In = o11 * ei + o12 * eq + (ech * I - esh * Qn);
+            const float Qo = o12 * ei + o11 * eq + (-esh * I + ech * Qn);
+            const float Uo = Un * expf(-ta);
+            I = In;
+            // rot_stokes_back
+            Q = Qo * cv.z - Uo * cv.w;
+            U = Uo * cv.z + Qo * cv.w;
+            // compensated tau sum
+            const float yk = ta - tauc;
+            const float tk = tau + yk;
+            tauc = (tk - tau) - yk;
+            tau = tk;
+        } else if (cv.z != cv.z) {
+            // the reference rotates Q, U into the node frame and back at
+            // every cell; a field along the line of sight has no frame
+            // (NaN angle), which makes them NaN there too
+            Q = cv.z;
+            U = cv.z;
+        }
+    }
+    __device__ __forceinline__ void store(const ImArgs &a, int p, int ch, int j, bool bad) const {
+        const size_t o = cube_at(a, p, ch, j);
+        const float v[4] = {bad ? NAN : (float)((double)I - c_im[j].bb_cmb), bad ? NAN : Q, bad ? NAN : U,
+                            bad ? NAN : tau};
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            if (a.out[q]) a.out[q][o] = v[q];
+    }
+};
+__device__ __forceinline__ float channel_velocity(const ImArgs &a, int ch) {
+    return (float)((ch - a.nvel) * a.dvel + a.v0);
+}
+
+// Whole slots of 32 channels: a warp takes NS slots (from slot s0) of one
+// line of one ray, lanes over channels, the cells' records staged 32 at a
+// time.  The rays of a block of warps are neighbours in the image, so the
+// stores of a channel fill sectors.
+constexpr int IM_WARPS = 8;
+template <int NS>
+__global__ void __launch_bounds__(32 * IM_WARPS) k_im_stokes(ImArgs a, int s0) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __shared__ float4 s_cv[IM_WARPS][32], s_cf[IM_WARPS][32];
+    __shared__ float s_dk[IM_WARPS][32];
+    const int i = blockIdx.x * IM_WARPS + warp, j = blockIdx.y;
+    if (i >= a.rays) return;
+    const int cnt = a.cnt[i], ncr = max(cnt, 0);
+    const int2 *dl = march_list(a, i);
+    const float Iin = (float)(a.on_star[i] ? c_im[j].bb_star : c_im[j].bb_cmb);  // I_in (raytrace.f90:97-115)
+    Stokes st[NS];
+    float vobs[NS];
+#pragma unroll
+    for (int s = 0; s < NS; s++) {
+        st[s].start(Iin);
+        vobs[s] = channel_velocity(a, min(lane + 32 * (s0 + s), a.nch - 1));
+    }
+    for (int k0 = 0; k0 + 1 < ncr; k0 += 32) {
+        const int n = min(32, ncr - 1 - k0);
+        __syncwarp();
+        if (lane < n) {
+            const int2 e0 = dl[march_at(k0 + lane, i & 31)];
+            const int k1 = dl[march_at(k0 + lane + 1, i & 31)].y;
+            s_cv[warp][lane] = a.cellv[e0.x];
+            s_cf[warp][lane] = a.coef[(size_t)j * a.N + e0.x];
+            s_dk[warp][lane] = (float)(k1 - e0.y);
+        }
+        __syncwarp();
+        for (int k = 0; k < n; k++) {
+            const float4 cv = s_cv[warp][k], cf = s_cf[warp][k];
+            const float fdk = s_dk[warp][k];
+#pragma unroll
+            for (int s = 0; s < NS; s++) st[s].cell(cv, cf, fdk, vobs[s]);
+        }
+    }
+    const int p = ray_of(a, a.ray0 + i);
+#pragma unroll
+    for (int s = 0; s < NS; s++) {
+        const int ch = lane + 32 * (s0 + s);
+        if (ch < a.nch) st[s].store(a, p, ch, j, cnt < 0);
+    }
+}
+
+// The channels past the whole slots (ch0 on), lanes over rays: a thread takes
+// up to 4 of one line of one ray.  One such channel would otherwise cost a
+// slot of 32 lanes (the reference's 2 nvel + 1 channels always leave some).
+__global__ void __launch_bounds__(64) k_im_stokes_tail(ImArgs a, int ch0) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, c0 = ch0 + 4 * blockIdx.z;
+    if (i >= a.rays) return;
+    const int cnt = a.cnt[i], n = min(4, a.nch - c0);
+    const int2 *dl = march_list(a, i);
+    const float Iin = (float)(a.on_star[i] ? c_im[j].bb_star : c_im[j].bb_cmb);
+    Stokes st[4];
+    float vobs[4];
+#pragma unroll
+    for (int s = 0; s < 4; s++) {
+        st[s].start(Iin);
+        vobs[s] = channel_velocity(a, min(c0 + s, a.nch - 1));
+    }
+    int2 e0 = (cnt > 0) ? dl[march_at(0, i & 31)] : make_int2(0, 0);
+    for (int k = 0; k + 1 < cnt; k++) {
+        const int2 e1 = dl[march_at(k + 1, i & 31)];
+        const float4 cv = a.cellv[e0.x], cf = a.coef[(size_t)j * a.N + e0.x];
+        const float fdk = (float)(e1.y - e0.y);
+#pragma unroll
+        for (int s = 0; s < 4; s++)
+            if (s < n) st[s].cell(cv, cf, fdk, vobs[s]);
+        e0 = e1;
+    }
+    const int p = ray_of(a, a.ray0 + i);
+#pragma unroll
+    for (int s = 0; s < 4; s++)
+        if (s < n) st[s].store(a, p, c0 + s, j, cnt < 0);
+}
+// Leftover channels up to this many go to the tail kernel, more to a padded
+// slot.
+constexpr int IM_TAIL = 16;
 
 }  // namespace
 
@@ -784,23 +830,45 @@ static int image_call(portal_ctx *c, const double *pol_pops, int nlines, const i
         int q2 = 0;
         for (int q = 0; q < 8; q++) ia.out[q] = dout[q] ? outd.p + cube * (q2++) : nullptr;
     }
-    const void *kern = nch <= 32    ? (const void *)k_image<1>
-                       : nch <= 64  ? (const void *)k_image<2>
-                       : nch <= 96  ? (const void *)k_image<3>
-                       : nch <= 160 ? (const void *)k_image<5>
-                                    : (const void *)k_image<9>;
-    int nb = 0;
-    PCHECK(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, 32 * IM_WARPS, 0));
-    const int grid = (int)std::min<long long>((long long)std::max(1, nb) * c->sm_count,
-                                              std::max(1, (nrays + 31) / 32));
-    if (c->walk.reserve((size_t)grid * 1024 * (size_t)((n_depth_rt + 31) / 32)) != cudaSuccess)
+    // Rays per launch: as many as keep the march lists (n_depth_rt records per
+    // ray) within 6 GB, fewer where the device cannot hold that.
+    const size_t list = 1024 * (size_t)((n_depth_rt + 31) / 32);   // int2 records per batch of 32 rays
+    long long batches = std::max(1, (nrays + 31) / 32);
+    batches = std::min(batches, std::max<long long>(c->sm_count, (long long)(6e9 / (list * sizeof(int2)))));
+    while (c->walk.reserve(batches * list) != cudaSuccess) {
+        cudaGetLastError();
+        if ((batches /= 2) < 1) return set_err(c, PORTAL_ERR_NOMEM, "image walk scratch");
+    }
+    DevBuf<int> cnt;
+    DevBuf<unsigned char> on_star;
+    if (cnt.reserve(32 * batches) || on_star.reserve(32 * batches))
         return set_err(c, PORTAL_ERR_NOMEM, "image walk scratch");
     ia.walk = c->walk.p;
-    ia.counters = c->counters.p;
-    PCHECK(c, cudaMemsetAsync(c->counters.p, 0, sizeof(unsigned long long), c->stream));
+    ia.cnt = cnt.p;
+    ia.on_star = on_star.p;
+    const bool stokes = dout[0] || dout[1] || dout[2] || dout[3], dustmaps = dout[4] || dout[5] || dout[6] || dout[7];
+    const int left = nch % 32, tail = left <= IM_TAIL ? left : 0, slots = (nch - tail + 31) / 32;
     timer_start(c, T_IMWALK);
-    void *args[] = {&ia};
-    PCHECK(c, cudaLaunchKernel(kern, dim3(grid), dim3(32 * IM_WARPS), args, 0, c->stream));
+    for (ia.ray0 = 0; ia.ray0 < nrays; ia.ray0 += ia.rays) {
+        ia.rays = (int)std::min<long long>(nrays - ia.ray0, 32 * batches);
+        // rays per marching warp: fewer while that leaves at most 8 warps per SM
+        // (3,000 rays: 0.49 ms with 32 a warp, 0.36 with 4; 9,001: 0.97 with
+        // 32, 0.88 with 8; beyond that the FP64 pipe is full and whole warps win:
+        // 66,049 rays 2.6 ms with 32, 3.1 with 16)
+        int per = 32;
+        while (per > 4 && ia.rays / (per / 2) <= 8 * c->sm_count) per /= 2;
+        k_im_march<<<(ia.rays + 2 * per - 1) / (2 * per), 64, 0, c->stream>>>(ia, per);
+        if (dustmaps) k_im_dust_maps<<<dim3((ia.rays + 63) / 64, nlines), 64, 0, c->stream>>>(ia);
+        const dim3 grid((ia.rays + IM_WARPS - 1) / IM_WARPS, nlines);
+        for (int s0 = 0; stokes && s0 < slots; s0 += 4) switch (std::min(4, slots - s0)) {
+            case 1: k_im_stokes<1><<<grid, 32 * IM_WARPS, 0, c->stream>>>(ia, s0); break;
+            case 2: k_im_stokes<2><<<grid, 32 * IM_WARPS, 0, c->stream>>>(ia, s0); break;
+            case 3: k_im_stokes<3><<<grid, 32 * IM_WARPS, 0, c->stream>>>(ia, s0); break;
+            default: k_im_stokes<4><<<grid, 32 * IM_WARPS, 0, c->stream>>>(ia, s0);
+            }
+        if (stokes && tail)
+            k_im_stokes_tail<<<dim3((ia.rays + 63) / 64, nlines, (tail + 3) / 4), 64, 0, c->stream>>>(ia, nch - tail);
+    }
     timer_stop(c, T_IMWALK);
     PCHECK(c, cudaGetLastError());
     for (int q = 0; q < 8; q++)
