@@ -287,6 +287,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(int M, int N, int K, 
                 }
             }
         }
+        __syncthreads();   // the transpose buffers share the A tile's memory: all warps are done with them
     }
     umma::fence_before_sync();
     __syncthreads();

@@ -103,3 +103,21 @@ def test_training_fits_and_predict_matches_oracle(built_lib):
     shapes = om.layer_shapes(8, 64, 3, 6)
     Yo = om.predict(p, st, shapes, Xt, bf16=True)
     assert np.abs(Yp - Yo).max() <= 2e-3 * np.abs(Yo).max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(8, 256, 3, 40), (300, 64, 2, 40)])
+def test_predict_many_rows_equals_pieces(built_lib, shape):
+    """More row tiles than SMs: a CTA that starts its next tile while warps of
+    it are still in the last one's epilogue must not disturb them (a call of
+    40,000 rows once differed by 4 % from run to run).  Rows do not depend on
+    each other, so a long call equals its pieces bit for bit, twice."""
+    import portal_gb300 as pg
+
+    rng = np.random.default_rng(1)
+    X = rng.normal(size=(40000, shape[0])).astype(np.float32)
+    with pg.MLP(*shape, seed=1) as m:
+        whole = m.predict(X)
+        pieces = np.concatenate([m.predict(X[i:i + 8000]) for i in range(0, 40000, 8000)])
+        np.testing.assert_array_equal(whole, pieces)
+        np.testing.assert_array_equal(m.predict(X), whole)
