@@ -36,7 +36,8 @@ struct portal_batch {
     DevBuf<int2> items, sample;
     long long n_items = 0, n_sample = 0;
     size_t se_wb = 0;
-    size_t se_a64_stride = 0;           // largest model's c_dim^2
+    size_t se_a64_stride = 0;           // largest model's matrix slot
+    int se_max_dim = 0;                 // largest model's c_dim
     DevBuf<double> se_a64;              // FP64 SE matrices, one per resident warp
     DevBuf<int2> walk;
     DevBuf<unsigned long long> queue;   // [0] next item, [1] segments
@@ -99,7 +100,7 @@ int enqueue_pass(portal_batch *b, const int2 *items, long long n_items) {
     for (size_t m = 0; m < b->models.size(); m++)
         if ((rc = se_pass(b->models[m], b->stream)))
             return bfail(b, rc, "model " + std::to_string(m) + ": " + b->models[m]->err);
-    SEBatch sb{b->d_se.p, items, n_items, b->se_wb, b->se_a64.p, b->se_a64_stride};
+    SEBatch sb{b->d_se.p, items, n_items, b->se_wb, b->se_a64.p, b->se_a64_stride, b->se_max_dim};
     if ((rc = se_batch_launch(b->stream, b->se_bps * b->sm_count, b->se_warps, sb)))
         return bfail(b, rc, "SE launch failed");
     return PORTAL_OK;
@@ -181,6 +182,7 @@ extern "C" int portal_batch_prepare(portal_batch *b, int nth, int nph, int nvel,
     b->lines.clear();
     size_t wb = 0;
     b->se_a64_stride = 0;
+    b->se_max_dim = 0;
     std::vector<double> cost(M);
     for (int m = 0; m < M; m++) {
         portal_ctx *c = b->models[m];
@@ -192,6 +194,7 @@ extern "C" int portal_batch_prepare(portal_batch *b, int nth, int nph, int nvel,
             return bfail(b, rc, "model " + std::to_string(m) + ": " + c->err);
         wb = std::max(wb, w);
         b->se_a64_stride = std::max(b->se_a64_stride, se_matrix_doubles(c));
+        b->se_max_dim = std::max(b->se_max_dim, c->c_dim);
         b->dust = b->dust || c->has_dust;
         b->lines.push_back(c->r_num);
         // per-node cost ~ lines x cells per ray ~ L N^(1/3)
@@ -249,17 +252,17 @@ extern "C" int portal_batch_prepare(portal_batch *b, int nth, int nph, int nvel,
         if (wb * w <= 200 * 1024) sec.push_back(w);
     if (sec.empty()) return bfail(b, PORTAL_ERR_ARG, "SE system too large for shared memory");
     int dummy = 0;
-    if (se_batch_blocks_per_sm(sec.back(), wb, b->se_a64_stride, &dummy))  // raises the smem limit to the largest candidate
+    if (se_batch_blocks_per_sm(sec.back(), wb, b->se_max_dim, &dummy))  // raises the smem limit to the largest candidate
         return bfail(b, PORTAL_ERR_CUDA, "SE occupancy query");
     // FP64 matrix slots for the largest SE grid among the candidates
     {
         size_t most = 0;
         for (int w : sec) {
             int bps = 0;
-            if (se_batch_blocks_per_sm(w, wb, b->se_a64_stride, &bps)) return bfail(b, PORTAL_ERR_CUDA, "SE occupancy query");
+            if (se_batch_blocks_per_sm(w, wb, b->se_max_dim, &bps)) return bfail(b, PORTAL_ERR_CUDA, "SE occupancy query");
             most = std::max(most, (size_t)std::max(1, bps) * b->sm_count * w);
         }
-        se_batch_blocks_per_sm(sec.back(), wb, b->se_a64_stride, &dummy);
+        se_batch_blocks_per_sm(sec.back(), wb, b->se_max_dim, &dummy);
         if (b->se_a64.reserve(most * b->se_a64_stride)) return bfail(b, PORTAL_ERR_NOMEM, "SE matrix scratch");
     }
     // walk scratch for the largest grid
@@ -283,22 +286,22 @@ extern "C" int portal_batch_prepare(portal_batch *b, int nth, int nph, int nvel,
         best = 1e300;
         for (int w : sec) {
             int bps = 0;
-            if (se_batch_blocks_per_sm(w, wb, b->se_a64_stride, &bps)) return bfail(b, PORTAL_ERR_CUDA, "SE occupancy query");
+            if (se_batch_blocks_per_sm(w, wb, b->se_max_dim, &bps)) return bfail(b, PORTAL_ERR_CUDA, "SE occupancy query");
             bps = std::max(1, bps);
-            SEBatch sb{b->d_se.p, b->sample.p, b->n_sample, wb, b->se_a64.p, b->se_a64_stride};
+            SEBatch sb{b->d_se.p, b->sample.p, b->n_sample, wb, b->se_a64.p, b->se_a64_stride, b->se_max_dim};
             double ms = 0.0;
             int rc = time_launch(b, [&]() { return se_batch_launch(b->stream, bps * b->sm_count, w, sb); }, &ms);
             if (rc) return rc;
             b->tune.insert(b->tune.end(), {(double)w, (double)bps, ms});
             if (ms < best) { best = ms; b->se_warps = w; b->se_bps = bps; }
         }
-        se_batch_blocks_per_sm(sec.back(), wb, b->se_a64_stride, &dummy);
+        se_batch_blocks_per_sm(sec.back(), wb, b->se_max_dim, &dummy);
     } else {
         b->nlg = rfc[0].nlg;
         b->rf_bps = rfc[0].bps;
         b->se_warps = sec.back();
         int bps = 0;
-        se_batch_blocks_per_sm(b->se_warps, wb, b->se_a64_stride, &bps);
+        se_batch_blocks_per_sm(b->se_warps, wb, b->se_max_dim, &bps);
         b->se_bps = std::max(1, bps);
     }
 

@@ -77,14 +77,17 @@ struct SEArgs {
     const int *__restrict__ pack;       // (2 nlev) rho index or -1
     const int *__restrict__ row_off;    // (c_dim + 1) entries of each matrix row,
     const int *__restrict__ row_ent;    // ascending column (the rates' summation order)
-    const int4 *__restrict__ asm_rec;   // the entries with terms: (pos, first term, end, 0)
-    int n_asm;
+    const int4 *__restrict__ sp_rec;    // the matrix's entries row by row: (pos, first term, end, -1), row 1
+                                        // the normalisation's (pos, 0, 0, level)
+    const int *__restrict__ sp_off;     // (c_dim + 1) their row offsets,
+    const int *__restrict__ sp_col;     // columns
+    int nnz;
     double *pops;                       // (N, 2 nlev) column-major
     double *jj20;                       // (N, L) or null
     double *rates;                      // (N, 3, 2 nlev) column-major or null
     int *status;
     int *nfail;
-    double *a64;                        // FP64 matrices, one slot of a64_stride doubles per team
+    double *a64;                        // FP64 matrices (entries, then dense), one slot of a64_stride doubles per team
     size_t a64_stride;
     int fp64_only;                      // factorise every system in FP64 (no FP32 LU)
 };
@@ -111,7 +114,8 @@ struct SEBatch {
     long long n_items;
     size_t warp_bytes;           // dynamic shared memory per warp (largest model)
     double *a64;                 // FP64 matrices, one slot of a64_stride doubles per warp
-    size_t a64_stride;           // largest model's c_dim^2
+    size_t a64_stride;           // largest model's nnz + c_dim^2
+    int max_dim;                 // largest model's c_dim
 };
 
 // rf.cu
@@ -132,7 +136,7 @@ constexpr int RF_BATCH_WARPS = 4;        // warps per block of the batched launc
 int se_prepare(portal_ctx *c, int kmax, SEArgs *a, size_t *warp_bytes);
 int se_pass(portal_ctx *c, cudaStream_t s);
 int se_batch_launch(cudaStream_t s, int grid, int warps_per_block, const SEBatch &bw);
-int se_batch_blocks_per_sm(int warps_per_block, size_t warp_bytes, size_t a64_stride, int *blocks);
-size_t se_matrix_doubles(const portal_ctx *c);  // c_dim^2 of the prepared SE program
+int se_batch_blocks_per_sm(int warps_per_block, size_t warp_bytes, int max_dim, int *blocks);
+size_t se_matrix_doubles(const portal_ctx *c);  // matrix slot of the prepared SE program
 
 }  // namespace portal

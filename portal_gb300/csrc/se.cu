@@ -235,10 +235,12 @@ __device__ bool team_lu(int n, T *M, int *piv, int tid, double *red_v, int *red_
 // Dynamic shared memory per team (one warp, or the block's team of warps):
 //   feat [n_feat] double | x, r [n] double | LU32 [n*n] float | d32 [n] float
 //   | scale [n] float | piv [n] int
-// The FP64 matrix A64 [n*n] (assembly, residuals, the FP64 fallback) sits in
-// a per-team slot of global memory instead (L2-resident: the grid's teams x
-// n^2 doubles); kept out of shared memory it lets 3x more warps share an SM,
-// and the kernel is latency-bound.
+// The FP64 matrix is kept as its entries only, row by row (a fifth of the
+// 74 x 74 systems, a third of the 34 x 34: collisions couple the K = 0
+// components of all levels, radiation only neighbouring levels): assembly, row
+// scaling and the refinement's residuals run over them.  They sit in a
+// per-team slot of global memory, followed by the dense matrix of the FP64
+// fallback: kept out of shared memory they let 3x more warps share an SM.
 constexpr int NF = 7;  // features per transition
 
 __host__ __device__ inline size_t se_warp_bytes(int n, int n_feat) {
@@ -291,7 +293,7 @@ __global__ void __launch_bounds__(TW == 1 ? 256 : 32 * TW, TW == 1 ? 3 : 24 / TW
     const long long n_items = BATCH ? bw.n_items : (long long)a0.bulk;
     const size_t wbytes = BATCH ? bw.warp_bytes : se_warp_bytes(a0.c_dim, a0.n_feat);
     unsigned char *base = smem + wbytes * team;
-    double *const A64 = (BATCH ? bw.a64 : a0.a64) +
+    double *const val = (BATCH ? bw.a64 : a0.a64) +
                         (size_t)((long long)blockIdx.x * teams + team) * (BATCH ? bw.a64_stride : a0.a64_stride);
     int cur_model = -1;
 
@@ -380,32 +382,29 @@ __global__ void __launch_bounds__(TW == 1 ? 256 : 32 * TW, TW == 1 ? 3 : 24 / TW
                 if (a.depol == 2) feat[NF * (size_t)a.n_trans + a.n_dep + d] = v;
             }
         }
-        for (int i = tid; i < n * n; i += TS) A64[i] = 0.0;
+        if (!a.fp64_only)
+            for (int i = tid; i < n * n; i += TS) LU[i] = 0.f;
         tsync();
-        // ---- assembly (setup_stateq) ----
-        // entries with terms, four records per thread in flight; each entry's
-        // terms summed in program order
-        for (int e0 = tid; e0 < a.n_asm; e0 += 4 * TS) {
+        // ---- assembly (setup_stateq), row 1 replaced by the normalisation
+        // (em_coefs.f90:158-164): four records per thread in flight; each
+        // entry's terms summed in program order
+        for (int e0 = tid; e0 < a.nnz; e0 += 4 * TS) {
             int4 rec[4];
 #pragma unroll
             for (int u = 0; u < 4; u++) {
                 const int e = e0 + u * TS;
-                rec[u] = (e < a.n_asm) ? a.asm_rec[e] : make_int4(-1, 0, 0, 0);
+                rec[u] = (e < a.nnz) ? a.sp_rec[e] : make_int4(-1, 0, 0, 0);
             }
 #pragma unroll
             for (int u = 0; u < 4; u++) {
                 if (rec[u].x < 0) continue;
                 double v = 0.0;
-                for (int q = rec[u].y; q < rec[u].z; q++) v = fma(a.term_c[q], feat[a.term_f[q]], v);
-                A64[rec[u].x] = v;
+                if (rec[u].w >= 0) v = a.norm_val[rec[u].w];
+                else
+                    for (int q = rec[u].y; q < rec[u].z; q++) v = fma(a.term_c[q], feat[a.term_f[q]], v);
+                val[e0 + u * TS] = v;
             }
         }
-        tsync();
-        // ---- normalisation row (em_coefs.f90:158-164) ----
-        for (int j = tid; j < n; j += TS) A64[(size_t)n * j] = 0.0;
-        tsync();
-        if (tid == 0)
-            for (int i = 0; i < a.nlev; i++) A64[(size_t)n * a.norm_col[i]] = a.norm_val[i];
         tsync();
         // ---- FP32 LU of the row-scaled matrix (skipped in FP64 mode) ----
         int st = 0;
@@ -413,10 +412,11 @@ __global__ void __launch_bounds__(TW == 1 ? 256 : 32 * TW, TW == 1 ? 3 : 24 / TW
         if (!a.fp64_only) {
             for (int i = tid; i < n; i += TS) {
                 double m = 0.0;
-                for (int j = 0; j < n; j++) m = fmax(m, fabs(A64[i + (size_t)n * j]));
+                for (int q = a.sp_off[i]; q < a.sp_off[i + 1]; q++) m = fmax(m, fabs(val[q]));
                 const float sc = (m > 0.0) ? (float)(1.0 / m) : 1.f;
                 scl[i] = sc;
-                for (int j = 0; j < n; j++) LU[i + (size_t)n * j] = (float)(A64[i + (size_t)n * j] * (double)sc);
+                for (int q = a.sp_off[i]; q < a.sp_off[i + 1]; q++)
+                    LU[i + (size_t)n * a.sp_col[q]] = (float)(val[q] * (double)sc);
             }
             tsync();
             ok = team_lu<float, TW, MR>(n, LU, piv, tid, red_v, red_i);
@@ -428,9 +428,15 @@ __global__ void __launch_bounds__(TW == 1 ? 256 : 32 * TW, TW == 1 ? 3 : 24 / TW
             for (int it = 0; it < 10; it++) {
                 // r = e_1 - A x (FP64)
                 for (int i = tid; i < n; i += TS) {
-                    double s = (i == 0) ? 1.0 : 0.0;
-                    for (int j = 0; j < n; j++) s -= A64[i + (size_t)n * j] * x[j];
-                    d32[i] = (float)(s * (double)scl[i]);
+                    double s = (i == 0) ? 1.0 : 0.0, s1 = 0.0;   // two chains of dependent FP64 sums
+                    int q = a.sp_off[i];
+                    const int q1 = a.sp_off[i + 1];
+                    for (; q + 1 < q1; q += 2) {
+                        s -= val[q] * x[a.sp_col[q]];
+                        s1 -= val[q + 1] * x[a.sp_col[q + 1]];
+                    }
+                    if (q < q1) s -= val[q] * x[a.sp_col[q]];
+                    d32[i] = (float)((s + s1) * (double)scl[i]);
                 }
                 tsync();
                 if (TW == 1 || wib == 0) warp_lu_solve<float, float, MR>(n, LU, piv, d32, lane);
@@ -454,9 +460,12 @@ __global__ void __launch_bounds__(TW == 1 ? 256 : 32 * TW, TW == 1 ? 3 : 24 / TW
             }
         }
         if (!conv) {
-            // FP64 LU on the device (reuses LU32 + d32 storage as FP64 space
-            // is not available; re-assemble into A64 in place)
-            double *M = A64;
+            // FP64 LU on the device, dense
+            double *M = val + a.nnz;
+            for (int i = tid; i < n * n; i += TS) M[i] = 0.0;
+            tsync();
+            for (int q = tid; q < a.nnz; q += TS) M[a.sp_rec[q].x] = val[q];
+            tsync();
             st |= ok ? PORTAL_NODE_REFINE : 0;
             bool ok64 = team_lu<double, TW, MR>(n, M, piv, tid, red_v, red_i);
             if (!ok64) {
@@ -792,14 +801,29 @@ int prepare_se(portal_ctx *c, int kmax) {
     size_t o_rad = putI(P.tr_rad), o_col = putI(P.tr_col), o_eoff = putI(P.ent_off),
            o_epos = putI(P.ent_pos), o_tf = putI(P.term_f), o_nc = putI(P.count_array),
            o_pack = putI(P.pack), o_roff = putI(P.row_off), o_rent = putI(P.row_ent);
-    // the assembly's records (pos, first term, end, 0) of the entries that have
-    // terms, 16-byte aligned for one load each (the matrix is zeroed first)
-    std::vector<int> asm_rec;
-    for (size_t e = 0; e < P.ent_pos.size(); e++)
-        if (P.ent_off[e + 1] > P.ent_off[e])
-            asm_rec.insert(asm_rec.end(), {P.ent_pos[e], P.ent_off[e], P.ent_off[e + 1], 0});
+    // the matrix's entries row by row in ascending column order: records (pos,
+    // first term, end, -1), row 1 replaced by the normalisation's (pos, 0, 0,
+    // level); 16-byte aligned for one load each
+    std::vector<int> sp_rec, sp_off(1, 0), sp_col;
+    for (int i = 0; i < P.c_dim; i++) {
+        if (i == 0) {
+            for (int l = 0; l < c->nlev; l++) {
+                sp_rec.insert(sp_rec.end(), {P.c_dim * P.count_array[l], 0, 0, l});
+                sp_col.push_back(P.count_array[l]);
+            }
+        } else {
+            for (int q = P.row_off[i]; q < P.row_off[i + 1]; q++) {
+                const int e = P.row_ent[q];
+                if (P.ent_off[e + 1] == P.ent_off[e]) continue;
+                sp_rec.insert(sp_rec.end(), {P.ent_pos[e], P.ent_off[e], P.ent_off[e + 1], -1});
+                sp_col.push_back(P.ent_pos[e] / P.c_dim);
+            }
+        }
+        sp_off.push_back((int)sp_col.size());
+    }
+    const size_t o_soff = putI(sp_off), o_scol = putI(sp_col);
     while (I.size() % 4) I.push_back(0);
-    const size_t o_asm = putI(asm_rec);
+    const size_t o_asm = putI(sp_rec);
     size_t o_nu = putD(P.tr_nu), o_A = putD(P.tr_A), o_B = putD(P.tr_B21), o_tc = putD(P.term_c),
            o_nv = putD(norm_val), o_ct = putD(c->col_temps), o_C = putD(c->Cji), o_dep = putD(P.dep_tab);
     if (c->se_ints.reserve(I.size()) || c->se_dbls.reserve(D.size()))
@@ -818,7 +842,8 @@ int prepare_se(portal_ctx *c, int kmax) {
     c->se_offs[7] = o_nu; c->se_offs[8] = o_A; c->se_offs[9] = o_B; c->se_offs[10] = o_tc;
     c->se_offs[11] = o_nv; c->se_offs[12] = o_ct; c->se_offs[13] = o_C;
     c->se_offs[14] = o_roff; c->se_offs[15] = o_rent; c->se_offs[16] = o_dep; c->se_offs[17] = o_asm;
-    c->se_nasm = (int)(asm_rec.size() / 4);
+    c->se_offs[18] = o_soff; c->se_offs[19] = o_scol;
+    c->se_nnz = (int)sp_col.size();
     c->n_dep = P.n_dep;
     c->n_feat = NF * P.n_trans + (c->depol == 2 ? 2 : 1) * P.n_dep;
     return PORTAL_OK;
@@ -854,8 +879,9 @@ int se_prepare(portal_ctx *c, int kmax, SEArgs *out, size_t *warp_bytes) {
     a.term_c = D + c->se_offs[10]; a.norm_val = D + c->se_offs[11]; a.col_temps = D + c->se_offs[12];
     a.Cji = D + c->se_offs[13];
     a.row_off = I + c->se_offs[14]; a.row_ent = I + c->se_offs[15];
-    a.asm_rec = reinterpret_cast<const int4 *>(I + c->se_offs[17]);
-    a.n_asm = c->se_nasm;
+    a.sp_rec = reinterpret_cast<const int4 *>(I + c->se_offs[17]);
+    a.sp_off = I + c->se_offs[18]; a.sp_col = I + c->se_offs[19];
+    a.nnz = c->se_nnz;
     a.dep_tab = c->n_dep ? D + c->se_offs[16] : nullptr;
     a.pops = c->pops.p; a.jj20 = c->jj20.p; a.status = c->status.p;
     a.rates = nullptr;
@@ -880,17 +906,17 @@ int se_pass(portal_ctx *c, cudaStream_t s) {
     return PORTAL_OK;
 }
 
-size_t se_matrix_doubles(const portal_ctx *c) { return (size_t)c->c_dim * c->c_dim; }
+size_t se_matrix_doubles(const portal_ctx *c) { return (size_t)c->se_nnz + (size_t)c->c_dim * c->c_dim; }
 
-// The batched kernel's instance for the batch's largest system (a64_stride =
-// its c_dim^2): 3 rows per lane up to 96 unknowns, SE_MAX_ROWS above.
-static const void *se_batch_kernel(size_t a64_stride) {
-    return a64_stride <= 96 * 96 ? (const void *)k_solve_se<1, true, 3> : (const void *)k_solve_se<1, true, SE_MAX_ROWS>;
+// The batched kernel's instance for the batch's largest system: 3 rows per
+// lane up to 96 unknowns, SE_MAX_ROWS above.
+static const void *se_batch_kernel(int max_dim) {
+    return max_dim <= 96 ? (const void *)k_solve_se<1, true, 3> : (const void *)k_solve_se<1, true, SE_MAX_ROWS>;
 }
 
-int se_batch_blocks_per_sm(int warps_per_block, size_t warp_bytes, size_t a64_stride, int *blocks) {
+int se_batch_blocks_per_sm(int warps_per_block, size_t warp_bytes, int max_dim, int *blocks) {
     const size_t smem = warp_bytes * warps_per_block;
-    const void *k = se_batch_kernel(a64_stride);
+    const void *k = se_batch_kernel(max_dim);
     *blocks = 0;
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return PORTAL_ERR_CUDA;
@@ -906,7 +932,7 @@ int se_batch_launch(cudaStream_t s, int grid, int warps_per_block, const SEBatch
     SEArgs a0{};
     SEBatch b = bw;
     void *args[] = {&a0, &b};
-    if (cudaLaunchKernel(se_batch_kernel(bw.a64_stride), dim3(grid), dim3(32 * warps_per_block), args, smem, s) !=
+    if (cudaLaunchKernel(se_batch_kernel(bw.max_dim), dim3(grid), dim3(32 * warps_per_block), args, smem, s) !=
         cudaSuccess)
         return PORTAL_ERR_CUDA;
     return cudaGetLastError() == cudaSuccess ? PORTAL_OK : PORTAL_ERR_CUDA;
@@ -958,7 +984,7 @@ int run_solve_se(portal_ctx *c, int kmax, int *n_singular, bool rates) {
         a.rates = c->rates.p;
     }
     if ((rc = se_pass(c, c->stream))) return rc;
-    a.a64_stride = (size_t)c->c_dim * c->c_dim;
+    a.a64_stride = se_matrix_doubles(c);
     const bool few_rows = c->c_dim <= 96;
     if (se_team_warps(c->c_dim) == 4)
         rc = few_rows ? launch_se<4, 3>(c, a, wb) : launch_se<4, SE_MAX_ROWS>(c, a, wb);
