@@ -121,3 +121,43 @@ def test_predict_many_rows_equals_pieces(built_lib, shape):
         pieces = np.concatenate([m.predict(X[i:i + 8000]) for i in range(0, 40000, 8000)])
         np.testing.assert_array_equal(whole, pieces)
         np.testing.assert_array_equal(m.predict(X), whole)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,B", [((1, 1, 1, 1), 1), ((5, 40, 1, 3), 31), ((17, 100, 2, 130), 33),
+                                     ((200, 256, 3, 256), 65), ((8, 16, 16, 48), 130)])
+def test_whole_network_kernels_at_their_edges(built_lib, shape, B):
+    """One row, one feature, widths that are not multiples of 16 or 128, the
+    widest layers and the deepest network, batches around the CTA's 32 rows
+    and the gradient's chunks of 64: gradients and predictions against the
+    oracle with its BF16 rounding points (tolerances of the tests above), then
+    one Adam step of the same batch: a first step moves every parameter with a
+    gradient by the rate, towards lower loss."""
+    import portal_gb300 as pg
+
+    shapes = om.layer_shapes(*shape)
+    p = _params(shapes, 3)
+    rng = np.random.default_rng(B)
+    X = rng.normal(size=(B, shape[0])).astype(np.float32)
+    T = rng.normal(size=(B, shape[3])).astype(np.float32)
+    with pg.MLP(*shape, seed=1) as m:
+        m.set_params(p)
+        loss, g = m.gradients(X, T)
+        Y = m.predict(X)
+    lref, gref = om.loss_and_grad(p, shapes, X, T, bf16=True)
+    assert abs(loss - lref) <= 1e-5 * lref
+    o = 0
+    for fo, fi in shapes:
+        for n in (fo * fi, fo):
+            a, r = g[o:o + n].astype(np.float64), gref[o:o + n]
+            assert np.abs(a - r).max() <= 2e-3 * np.abs(r).max(), (o, n)
+            o += n
+    Yo = om.predict(p, np.concatenate([np.zeros(shape[0]), np.ones(shape[0]), np.zeros(shape[3]), np.ones(shape[3])]),
+                    shapes, X, bf16=True)
+    assert np.abs(Y - Yo).max() <= 2e-3 * np.abs(Yo).max()
+    with pg.MLP(*shape, seed=1) as m:
+        m.set_params(p)
+        m.train(X, T, epochs=1, batch=B, lr=1e-3, seed=0)
+        q, st = m.get_params()
+    d = np.abs(q - p)
+    assert d.max() <= 1.01e-3 and (B == 1 or np.median(d) >= 0.9e-3)
