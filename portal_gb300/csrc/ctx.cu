@@ -15,8 +15,12 @@
 //                       coordinates
 //   levp   (nlev,N) FP64 level populations, plus the per-node scalars
 //                       (b, T_kin, T_dust, dust, n_H2, abundance) in FP64.
+#include <unistd.h>
+
+#include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <thread>
 
 #include "common.cuh"
 
@@ -116,6 +120,7 @@ extern "C" int portal_set_molecule(portal_ctx *c, int nlev, const int *j_lev, co
     c->col_temps.assign(col_temps, col_temps + c_temp);
     c->Cji.assign(t_Cji, t_Cji + (size_t)c_temp * c_num * c_par);
     c->have_mol = true;
+    c->lines_ready = false;
     c->se_kmax = -1;  // SE program must be rebuilt
     c->j_valid = false;
     c->ali_valid = false;
@@ -274,6 +279,7 @@ extern "C" int portal_set_star(portal_ctx *c, int star_mod, double T_star, doubl
     if (star_mod == 1 && (!X_star || !(R_star > 0.0) || !(T_star >= 0.0)))
         return set_err(c, PORTAL_ERR_ARG, "portal_set_star: R_star > 0, T_star >= 0 and X_star(3) needed");
     cudaSetDevice(c->device);
+    c->lines_ready = false;
     c->star_mode = star_mod;
     c->T_star = star_mod ? T_star : 0.0;
     c->R_star_m = star_mod ? R_star : 0.0;
@@ -331,6 +337,29 @@ extern "C" int portal_last_kernel_times(const portal_ctx *c, double *times_ms, i
 }
 
 namespace portal {
+
+void touch_pages(const HostSpan *spans, int n) {
+    const size_t page = (size_t)std::max<long>(4096, sysconf(_SC_PAGESIZE));
+    size_t pages = 0;
+    for (int i = 0; i < n; i++)
+        if (spans[i].p) pages += spans[i].bytes / page;
+    if (pages < 16) return;   // small results: the copy's own faults cost less than a thread
+    const int nt = pages < 64 ? 1 : 4;
+    auto work = [&](int t) {
+        for (int i = 0; i < n; i++) {
+            if (!spans[i].p) continue;
+            volatile char *b = static_cast<volatile char *>(spans[i].p);
+            for (size_t o = (size_t)t * page; o < spans[i].bytes; o += (size_t)nt * page) b[o] = 0;
+        }
+    };
+    std::vector<std::thread> th;
+    try {
+        for (int t = 1; t < nt; t++) th.emplace_back(work, t);
+    } catch (...) {   // no thread to be had: the pages not touched here fault in the copy
+    }
+    work(0);
+    for (auto &x : th) x.join();
+}
 
 void gauss_legendre(int n, double *x, double *w) {
     const long double pi = 3.141592653589793238462643383279502884L;

@@ -773,11 +773,18 @@ static int image_call(portal_ctx *c, const double *pol_pops, int nlines, const i
             na.R[i + 3 * j] = s;
         }
     // device buffers
-    DevBuf<double> xyz_r, pops_d, vel_d, nrm2, ibb;
-    DevBuf<int> jl;
-    DevBuf<float4> cellv, cellb, coef;
-    DevBuf<float> outd;
-    DevBuf<int> stat;
+    DevBuf<double> &xyz_r = c->im_xyz, &pops_d = c->im_pops, &nrm2 = c->im_nrm2, &ibb = c->im_ibb;
+    DevBuf<int> &jl = c->im_jl, &stat = c->im_stat, &cnt = c->im_cnt;
+    DevBuf<float4> &cellv = c->im_cellv, &cellb = c->im_cellb, &coef = c->im_coef;
+    DevBuf<float> &outd = c->im_out;
+    DevBuf<unsigned char> &on_star = c->im_star;
+    // the cubes are kept for the next call up to 1 GB
+    struct KeepSmall {
+        DevBuf<float> &b;
+        ~KeepSmall() {
+            if (b.n * sizeof(float) > (size_t)1 << 30) b.release();
+        }
+    } keep{outd};
     const size_t cube = (size_t)nrays * nch * nlines;
     if (xyz_r.reserve(3 * (size_t)N) || nrm2.reserve(N) || cellv.reserve(N) || cellb.reserve(N) ||
         coef.reserve((size_t)nlines * N) || jl.reserve(nlev) || stat.reserve((size_t)(nrays > 0 ? nrays : 1)))
@@ -839,8 +846,6 @@ static int image_call(portal_ctx *c, const double *pol_pops, int nlines, const i
         cudaGetLastError();
         if ((batches /= 2) < 1) return set_err(c, PORTAL_ERR_NOMEM, "image walk scratch");
     }
-    DevBuf<int> cnt;
-    DevBuf<unsigned char> on_star;
     if (cnt.reserve(32 * batches) || on_star.reserve(32 * batches))
         return set_err(c, PORTAL_ERR_NOMEM, "image walk scratch");
     ia.walk = c->walk.p;
@@ -871,6 +876,10 @@ static int image_call(portal_ctx *c, const double *pol_pops, int nlines, const i
     }
     timer_stop(c, T_IMWALK);
     PCHECK(c, cudaGetLastError());
+    HostSpan spans[9];
+    for (int q = 0; q < 8; q++) spans[q] = {dout[q], cube * sizeof(float)};
+    spans[8] = {xy, 2 * (size_t)nrays * sizeof(double)};
+    touch_pages(spans, 9);   // while the kernels run
     for (int q = 0; q < 8; q++)
         if (dout[q])
             PCHECK(c, cudaMemcpyAsync(dout[q], ia.out[q], cube * sizeof(float), cudaMemcpyDeviceToHost, c->stream));

@@ -34,8 +34,8 @@
 
 namespace portal {
 int run_radiation_field(portal_ctx *c, int nth, int nph, int nvel, const double *gvec, double dx,
-                        int n_depth, long long *n_segments, int *n_failed, bool split);
-int run_solve_se(portal_ctx *c, int kmax, int *n_singular, bool rates);
+                        int n_depth, long long *n_segments, int *n_failed, bool split, const HostSpan *out, int n_out);
+int run_solve_se(portal_ctx *c, int kmax, int *n_singular, bool rates, const HostSpan *out, int n_out);
 }  // namespace portal
 using namespace portal;
 
@@ -209,10 +209,11 @@ extern "C" int portal_lambda_iterate(portal_ctx *c, int nth, int nph, int nvel, 
         long long nseg = 0;
         int nfail = 0;
         const bool split = local_operator && !verify;
-        if ((rc = run_radiation_field(c, nth, nph, nvel, gvec, dx, n_depth, &nseg, &nfail, split))) return rc;
+        if ((rc = run_radiation_field(c, nth, nph, nvel, gvec, dx, n_depth, &nseg, &nfail, split, nullptr, 0)))
+            return rc;
         nseg_tot += nseg;
         int nsing = 0;
-        if ((rc = run_solve_se(c, kmax, &nsing, false))) return rc;
+        if ((rc = run_solve_se(c, kmax, &nsing, false, nullptr, 0))) return rc;
         if (nsing) return set_err(c, PORTAL_ERR_SINGULAR, std::to_string(nsing) + " singular SE systems");
         PCHECK(c, cudaMemsetAsync(c->counters.p + 3, 0, sizeof(unsigned long long), c->stream));
         k_update<<<nb, tb, 0, c->stream>>>(N, c->bulk, nlev, c->pops.p, c->nmol.p, c->active_ab(), jl.p, c->levp.p,

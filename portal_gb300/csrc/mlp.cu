@@ -906,6 +906,8 @@ struct portal_mlp {
     DevBuf<unsigned char> fbuf;          // buffers of a training batch (FusedBatch)
     FusedBatch fb;
     int fcap = 0;                        // rows fb holds
+    DevBuf<float> train_x, train_y;      // a training call's rows and
+    DevBuf<int> train_perm;              // their order, kept for the next call
     DevBuf<int> tc_err;  // set by a tensor-core GEMM whose completion wait timed out
     int cap_batch = 0;
     long long step = 0;
@@ -1293,20 +1295,26 @@ extern "C" int portal_mlp_train(portal_mlp *m, const float *X, const float *Y, i
     const int nin = m->n_in, nout = m->n_out;
     // statistics (FP64 on the host)
     std::vector<float> st(2 * (size_t)(nin + nout));
-    for (int k = 0; k < nin; k++) {
-        double s = 0, s2 = 0;
-        for (int i = 0; i < M; i++) { double v = X[(size_t)i * nin + k]; s += v; s2 += v * v; }
-        const double mu = s / M, sd = std::sqrt(std::max(s2 / M - mu * mu, 1e-12));
-        st[k] = (float)mu; st[nin + k] = (float)sd;
-    }
-    for (int k = 0; k < nout; k++) {
-        double s = 0, s2 = 0;
-        for (int i = 0; i < M; i++) { double v = Y[(size_t)i * nout + k]; s += v; s2 += v * v; }
-        const double mu = s / M, sd = std::sqrt(std::max(s2 / M - mu * mu, 1e-12));
-        st[2 * nin + k] = (float)mu; st[2 * nin + nout + k] = (float)sd;
-    }
+    // (row by row: a column's sums run over the rows in order, and the columns
+    // of a row are next to each other in memory)
+    auto column_stats = [M](const float *A, int n, float *mean, float *dev) {
+        std::vector<double> s(n, 0.0), s2(n, 0.0);
+        for (int i = 0; i < M; i++)
+            for (int k = 0; k < n; k++) {
+                const double v = A[(size_t)i * n + k];
+                s[k] += v;
+                s2[k] += v * v;
+            }
+        for (int k = 0; k < n; k++) {
+            const double mu = s[k] / M;
+            mean[k] = (float)mu;
+            dev[k] = (float)std::sqrt(std::max(s2[k] / M - mu * mu, 1e-12));
+        }
+    };
+    column_stats(X, nin, st.data(), st.data() + nin);
+    column_stats(Y, nout, st.data() + 2 * nin, st.data() + 2 * nin + nout);
     MCHECK(m, cudaMemcpyAsync(m->stats.p, st.data(), st.size() * sizeof(float), cudaMemcpyHostToDevice, m->stream));
-    DevBuf<float> dX, dY;
+    DevBuf<float> &dX = m->train_x, &dY = m->train_y;
     if (dX.reserve((size_t)M * nin) || dY.reserve((size_t)M * nout)) return mlp_fail(m, PORTAL_ERR_NOMEM, "MLP data");
     MCHECK(m, cudaMemcpyAsync(dX.p, X, (size_t)M * nin * sizeof(float), cudaMemcpyHostToDevice, m->stream));
     MCHECK(m, cudaMemcpyAsync(dY.p, Y, (size_t)M * nout * sizeof(float), cudaMemcpyHostToDevice, m->stream));
@@ -1319,10 +1327,10 @@ extern "C" int portal_mlp_train(portal_mlp *m, const float *X, const float *Y, i
     std::vector<int> perm(M);
     for (int i = 0; i < M; i++) perm[i] = i;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-    DevBuf<int> pidx;
+    DevBuf<int> &pidx = m->train_perm;
     if (pidx.reserve(M)) return mlp_fail(m, PORTAL_ERR_NOMEM, "MLP permutation");
+    std::shuffle(perm.begin(), perm.end(), rng);
     for (int ep = 0; ep < epochs; ep++) {
-        std::shuffle(perm.begin(), perm.end(), rng);
         int nbatch = 0;
         MCHECK(m, cudaMemcpyAsync(pidx.p, perm.data(), (size_t)M * sizeof(int), cudaMemcpyHostToDevice, m->stream));
         if (loss_per_epoch) {
@@ -1354,6 +1362,7 @@ extern "C" int portal_mlp_train(portal_mlp *m, const float *X, const float *Y, i
             nbatch++;
         }
         MCHECK(m, cudaGetLastError());
+        if (ep + 1 < epochs) std::shuffle(perm.begin(), perm.end(), rng);   // the next epoch's, while this one runs
         if (loss_per_epoch) {
             double eloss = 0.0;
             MCHECK(m, cudaMemcpyAsync(&eloss, m->lossacc.p, sizeof(double), cudaMemcpyDeviceToHost, m->stream));

@@ -279,46 +279,65 @@ int rf_prepare(portal_ctx *c, int nth, int nph, int nvel, const double *gvec, do
         return set_err(c, PORTAL_ERR_ARG, "portal_radiation_field: bad nth/nph/nvel/n_depth/dx "
                                           "(at most 288 channels)");
     cudaSetDevice(c->device);
-    int rc;
-    if ((rc = upload_lines(c))) return rc;
     const int L = c->r_num, N = c->N;
-    // direction table (legendre_all) and channel tables
-    std::vector<double> xth;
-    const int ndir = legendre_all(nth, nph, xth);
-    std::vector<double> dt(6 * (size_t)ndir);
-    for (int k = 0; k < ndir; k++) {
-        double mu = xth[3 * k], ph = xth[3 * k + 1], w = xth[3 * k + 2];
-        double th = std::acos(mu);
-        double c_in = (3.0 * mu * mu - 1.0) / 2.0;
-        dt[6 * k + 0] = std::cos(th);
-        dt[6 * k + 1] = std::sin(th);
-        dt[6 * k + 2] = std::cos(ph);
-        dt[6 * k + 3] = std::sin(ph);
-        dt[6 * k + 4] = w;
-        dt[6 * k + 5] = w * c_in / std::sqrt(2.0);
-    }
     const int nch = 2 * nvel + 1;
-    std::vector<float> ct(2 * (size_t)nch);
-    const double spi = std::sqrt(std::acos(-1.0));
-    for (int i = 0; i < nch; i++) {
-        int nv = i - nvel;
-        double q0 = 2.0 * nv / nvel;
-        ct[i] = (float)q0;
-        // phi_v0 * d_v = exp(-q0^2)/(sqrt(pi) b) * 2 b / nvel
-        ct[nch + i] = (float)(std::exp(-q0 * q0) * 2.0 / (spi * nvel));
+    // line constants, direction table (legendre_all) and channel tables: kept
+    // until the molecule, the star, the angles or the channels change (the
+    // quadrature's knots are found in long double, which this machine has in
+    // software: 0.1 ms of each call)
+    const bool new_lines = !c->lines_ready, new_dirs = nth != c->tab_nth || nph != c->tab_nph,
+               new_ch = nvel != c->tab_nvel;
+    if (new_lines) {
+        if (int rc = upload_lines(c)) return rc;
     }
-    if (c->dirtab.reserve(dt.size()) || c->chtab.reserve(ct.size()) ||
+    std::vector<double> dt;
+    std::vector<float> ct;
+    int ndir = c->tab_ndir;
+    if (new_dirs) {
+        std::vector<double> xth;
+        ndir = legendre_all(nth, nph, xth);
+        dt.resize(6 * (size_t)ndir);
+        for (int k = 0; k < ndir; k++) {
+            double mu = xth[3 * k], ph = xth[3 * k + 1], w = xth[3 * k + 2];
+            double th = std::acos(mu);
+            double c_in = (3.0 * mu * mu - 1.0) / 2.0;
+            dt[6 * k + 0] = std::cos(th);
+            dt[6 * k + 1] = std::sin(th);
+            dt[6 * k + 2] = std::cos(ph);
+            dt[6 * k + 3] = std::sin(ph);
+            dt[6 * k + 4] = w;
+            dt[6 * k + 5] = w * c_in / std::sqrt(2.0);
+        }
+    }
+    if (new_ch) {
+        ct.resize(2 * (size_t)nch);
+        const double spi = std::sqrt(std::acos(-1.0));
+        for (int i = 0; i < nch; i++) {
+            int nv = i - nvel;
+            double q0 = 2.0 * nv / nvel;
+            ct[i] = (float)q0;
+            // phi_v0 * d_v = exp(-q0^2)/(sqrt(pi) b) * 2 b / nvel
+            ct[nch + i] = (float)(std::exp(-q0 * q0) * 2.0 / (spi * nvel));
+        }
+    }
+    if (c->dirtab.reserve(6 * (size_t)ndir) || c->chtab.reserve(2 * (size_t)nch) ||
         c->ltab.reserve((size_t)L * N) || c->J0.reserve((size_t)L * N) || c->J2.reserve((size_t)L * N) ||
         c->nodeseg.reserve((size_t)N) || c->frames.reserve(FRAME_N * (size_t)N) || c->kmom.reserve((size_t)6 * N))
         return set_err(c, PORTAL_ERR_NOMEM, "radiation-field buffers");
     if (split && (c->JE.reserve((size_t)L * N) || c->LS.reserve((size_t)L * N)))
         return set_err(c, PORTAL_ERR_NOMEM, "split-field buffers");
-    PCHECK(c, cudaMemcpyAsync(c->dirtab.p, dt.data(), dt.size() * sizeof(double),
-                              cudaMemcpyHostToDevice, c->stream));
-    PCHECK(c, cudaMemcpyAsync(c->chtab.p, ct.data(), ct.size() * sizeof(float),
-                              cudaMemcpyHostToDevice, c->stream));
+    c->tab_nth = c->tab_nvel = 0;   // (until the copies below are made)
+    c->lines_ready = false;
+    if (new_dirs)
+        PCHECK(c, cudaMemcpyAsync(c->dirtab.p, dt.data(), dt.size() * sizeof(double), cudaMemcpyHostToDevice,
+                                  c->stream));
+    if (new_ch)
+        PCHECK(c, cudaMemcpyAsync(c->chtab.p, ct.data(), ct.size() * sizeof(float), cudaMemcpyHostToDevice,
+                                  c->stream));
     // the host vectors go out of scope: the copies must have happened
-    PCHECK(c, cudaStreamSynchronize(c->stream));
+    if (new_lines || new_dirs || new_ch) PCHECK(c, cudaStreamSynchronize(c->stream));
+    c->tab_nth = nth; c->tab_nph = nph; c->tab_ndir = ndir; c->tab_nvel = nvel;
+    c->lines_ready = true;
     RFArgs a;
     a.N = N; a.bulk = c->bulk; a.L = L; a.nvel = nvel; a.nch = nch; a.ndir = ndir; a.n_depth = n_depth;
     a.dx32 = (float)dx;
@@ -371,7 +390,8 @@ int rf_pass(portal_ctx *c, const RFArgs &a, cudaStream_t s) {
 // Runs the line table + radiation field on the device; J stays in c->J0/J2
 // (and the split field in c->JE/LS when `split`).
 int run_radiation_field(portal_ctx *c, int nth, int nph, int nvel, const double *gvec, double dx,
-                        int n_depth, long long *n_segments, int *n_failed, bool split) {
+                        int n_depth, long long *n_segments, int *n_failed, bool split, const HostSpan *out,
+                        int n_out) {
     RFArgs a;
     int rc = rf_prepare(c, nth, nph, nvel, gvec, dx, n_depth, split, &a);
     if (rc) return rc;
@@ -380,6 +400,7 @@ int run_radiation_field(portal_ctx *c, int nth, int nph, int nvel, const double 
     if ((rc = rf_pass(c, a, c->stream))) return rc;
     timer_stop(c, T_LINETAB);
     if ((rc = dispatch_rf(c, a, n_depth))) return rc;
+    touch_pages(out, n_out);   // the caller's result arrays, while the kernel runs
     unsigned long long cnt[8];
     PCHECK(c, cudaMemcpyAsync(cnt, c->counters.p, sizeof cnt, cudaMemcpyDeviceToHost, c->stream));
     PCHECK(c, cudaStreamSynchronize(c->stream));
@@ -421,9 +442,11 @@ int radiation_field_call(portal_ctx *c, int nth, int nph, int nvel, const double
                          long long *n_segments) {
     if (!c) return PORTAL_ERR_ARG;
     timers_reset(c);
-    int rc = portal::run_radiation_field(c, nth, nph, nvel, gvec, dx, n_depth, n_segments, nullptr, split);
-    if (rc) return rc;
     const size_t LN = (size_t)c->r_num * c->N;
+    const HostSpan out[4] = {{J0, LN * sizeof(double)}, {J2, LN * sizeof(double)}, {JE, LN * sizeof(double)},
+                             {LS, LN * sizeof(double)}};
+    int rc = portal::run_radiation_field(c, nth, nph, nvel, gvec, dx, n_depth, n_segments, nullptr, split, out, 4);
+    if (rc) return rc;
     if (J0) PCHECK(c, cudaMemcpyAsync(J0, c->J0.p, LN * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     if (J2) PCHECK(c, cudaMemcpyAsync(J2, c->J2.p, LN * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     if (split && JE) PCHECK(c, cudaMemcpyAsync(JE, c->JE.p, LN * sizeof(double), cudaMemcpyDeviceToHost, c->stream));

@@ -972,7 +972,7 @@ int launch_se(portal_ctx *c, SEArgs &a, size_t wb) {
     return PORTAL_OK;
 }
 
-int run_solve_se(portal_ctx *c, int kmax, int *n_singular, bool rates) {
+int run_solve_se(portal_ctx *c, int kmax, int *n_singular, bool rates, const HostSpan *out, int n_out) {
     SEArgs a;
     size_t wb = 0;
     int rc = se_prepare(c, kmax, &a, &wb);
@@ -991,6 +991,7 @@ int run_solve_se(portal_ctx *c, int kmax, int *n_singular, bool rates) {
     else
         rc = few_rows ? launch_se<1, 3>(c, a, wb) : launch_se<1, SE_MAX_ROWS>(c, a, wb);
     if (rc) return rc;
+    touch_pages(out, n_out);   // the caller's result arrays, while the kernel runs
     int nf = 0;
     PCHECK(c, cudaMemcpyAsync(&nf, c->counters.p + 2, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     PCHECK(c, cudaStreamSynchronize(c->stream));
@@ -1021,7 +1022,9 @@ extern "C" int portal_solve_se(portal_ctx *c, int kmax, const double *J0, const 
     }
     timers_reset(c);
     int nsing = 0;
-    int rc = portal::run_solve_se(c, kmax, &nsing, rates != nullptr);
+    const HostSpan out[3] = {{pol_pops, (size_t)c->N * 2 * c->nlev * sizeof(double)}, {JJ_20, LN * sizeof(double)},
+                             {rates, (size_t)c->N * 6 * c->nlev * sizeof(double)}};
+    int rc = portal::run_solve_se(c, kmax, &nsing, rates != nullptr, out, 3);
     if (rc) return rc;
     if (pol_pops)
         PCHECK(c, cudaMemcpyAsync(pol_pops, c->pops.p, (size_t)c->N * 2 * c->nlev * sizeof(double),
