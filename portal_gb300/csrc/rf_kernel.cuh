@@ -291,9 +291,8 @@ constexpr int RF_RAYS_BYTES = (sizeof(RayBatchStar) + 15) & ~15;   // at the sta
 // over the channels live in registers).  A pass covers two slots of 32
 // channels (the last one, when the slot count is odd, a single slot); the
 // intensities of the passes not running wait in shared memory between two
-// chunks of 32 cells.  Without dust, lines are handled in packs of two on the
-// packed FP32x2 pipe (the last line of an odd group packs its two channel
-// slots instead); with dust one by one.
+// chunks of 32 cells.  Lines are handled in packs of two on the packed FP32x2
+// pipe (the last line of an odd group packs its two channel slots instead).
 struct RFShape {
     int L, nlg, groups, npk, nslot, rt, split;
     int rec_ld, om_ld;                    // row strides: float4 per cell, float per cell
@@ -320,7 +319,7 @@ __host__ __device__ inline RFShape rf_shape(int L, int max_group, int nch, bool 
     s.rt = rt;
     s.split = split;
     s.nslot = (nch - rt + 31) / 32;
-    s.rec_ld = (dust ? s.nlg : s.npk) | 1;
+    s.rec_ld = (dust ? 2 * s.npk : s.npk) | 1;
     s.om_ld = s.nlg | 1;
     const int nq = split ? 3 : 1;
     int o = RF_RAYS_BYTES;
@@ -328,7 +327,7 @@ __host__ __device__ inline RFShape rf_shape(int L, int max_group, int nch, bool 
     s.o_qd = o; o += 32 * 16;
     s.o_I = o; o += ((s.nslot / 2) * s.nlg + (s.nslot & 1) * s.npk) * 32 * 8;
     s.o_part = o; o += nq * s.npk * 32 * 8;
-    s.o_row = o; o += s.groups * (dust ? s.nlg : s.npk) * 16;
+    s.o_row = o; o += s.groups * (dust ? 2 : 1) * s.npk * 16;
     s.o_bb = o; o += 2 * s.groups * 2 * s.npk * 4;
     s.o_om = o; o += rt ? 32 * s.om_ld * 4 : 0;
     s.o_v = o; o += nq * 32 * L * 4;
@@ -379,6 +378,48 @@ __device__ __forceinline__ void transfer1(bool thin, float &I, float A, float S,
     I = fmaf(om, S - I, I);
 }
 
+// With dust: tau = (kv phi + alpha) dx n, S = (ev phi + j) / (kv phi + alpha),
+// and ray_in's gate tau > 1e-30 (inverse_rt.f90:308).  fast: the quotient
+// without the division's slow path (quot_rn; the numerator scaled by 2^60, so
+// that nothing in it is subnormal), for chunks whose staged values are inside
+// its range -- a slow-path branch per division kept the updates from
+// overlapping.
+struct DustPack {
+    float2 A, E, Ad, Jd;
+};
+__device__ __forceinline__ void transfer2_dust(bool thin, bool fast, float2 &I, const DustPack &c, float2 g2) {
+    const float2 tau = __ffma2_rn(c.A, g2, c.Ad), num = __ffma2_rn(c.E, g2, c.Jd);
+    float2 S;
+    if (fast) {
+        const float2 n2 = __fmul2_rn(num, make_float2(0x1p60f, 0x1p60f)), m = __fmul2_rn(tau, make_float2(-1.f, -1.f));
+        const float2 r0 = make_float2(rcp_approx(tau.x), rcp_approx(tau.y));
+        const float2 r = __ffma2_rn(r0, __ffma2_rn(m, r0, make_float2(1.f, 1.f)), r0);
+        const float2 q = __fmul2_rn(n2, r);
+        S = __fmul2_rn(__ffma2_rn(r, __ffma2_rn(m, q, n2), q), make_float2(0x1p-60f, 0x1p-60f));
+    } else {
+        S = make_float2(num.x / tau.x, num.y / tau.y);
+    }
+    const float2 x = __fmul2_rn(tau, make_float2(LOG2E_F, LOG2E_F));
+    float2 om = om_taylor2(x);
+    if (!thin) {   // (x < 0 fails the gate below)
+        const float e0 = ex2(-x.x), e1 = ex2(-x.y);
+        asm("{\n .reg .pred p;\n setp.ge.f32 p, %1, %3;\n @p sub.rn.f32 %0, %4, %2;\n}"
+            : "+f"(om.x) : "f"(x.x), "f"(e0), "f"(OM_TAYLOR_X), "f"(1.f));
+        asm("{\n .reg .pred p;\n setp.ge.f32 p, %1, %3;\n @p sub.rn.f32 %0, %4, %2;\n}"
+            : "+f"(om.y) : "f"(x.y), "f"(e1), "f"(OM_TAYLOR_X), "f"(1.f));
+    }
+    const float2 d = __ffma2_rn(I, make_float2(-1.f, -1.f), S);
+    asm("{\n .reg .pred p;\n setp.gt.f32 p, %1, %4;\n @p fma.rn.f32 %0, %2, %3, %0;\n}"
+        : "+f"(I.x) : "f"(tau.x), "f"(om.x), "f"(d.x), "f"(1e-30f));
+    asm("{\n .reg .pred p;\n setp.gt.f32 p, %1, %4;\n @p fma.rn.f32 %0, %2, %3, %0;\n}"
+        : "+f"(I.y) : "f"(tau.y), "f"(om.y), "f"(d.y), "f"(1e-30f));
+}
+// the staged values of a cell and line inside the range of the fast quotient
+// (|tau| <= |A| + |Ad|, |numerator| <= |E| + |Jd|; a NaN fails)
+__device__ __forceinline__ bool dust_in_range(float4 v) {
+    return fabsf(v.x) + fabsf(v.z) < 0x1p90f && fabsf(v.y) + fabsf(v.w) < 0x1p-34f;
+}
+
 // Sums of N per-lane values over the warp, value l's sum on every lane whose
 // low bits name it (sum_line).  Each butterfly step halves the values a lane
 // carries while there are two or more left; every sum adds the same partners
@@ -425,13 +466,13 @@ struct WarpMem {
 };
 
 // One pass over NSL channel slots (from slot s0) of a chunk of nc cells for
-// the line group g without dust: tk of the group's trailing packs take the
-// Taylor form alone.  first: the intensities start from the background bb;
+// the line group g: tk of the group's trailing packs take the Taylor form
+// alone (with dust: all or none), fast: transfer2_dust's.  first: the intensities start from the background bb;
 // last: the central cell and the weighted channel sums follow, else the
 // intensities go back to shared memory.
-template <int NLG, int NSL>
+template <int NLG, int NSL, bool DUST>
 __device__ __forceinline__ void channel_pass(const RFShape &sh, const WarpMem &m, const float2 *chtab, int nch,
-                                             int nvel, int lane, int g, int s0, int nc, int tk, bool first,
+                                             int nvel, int lane, int g, int s0, int nc, int tk, bool fast, bool first,
                                              bool last, const float *bb, float fst0) {
     constexpr int NP = NLG / 2, ODD = NLG & 1, NPK = NP + ODD;
     float2 I[NSL][NP > 0 ? NP : 1], Io;   // Io: the odd line's slots
@@ -451,8 +492,9 @@ __device__ __forceinline__ void channel_pass(const RFShape &sh, const WarpMem &m
     }
     const float4 *rec = m.rec(sh), *qd = m.qd(sh);
     const float2 ch2 = make_float2((float)(lane + 32 * s0 - nvel), (float)(lane + 32 * (s0 + 1) - nvel));
-    auto run = [&](auto tag) {
+    auto run = [&](auto tag, auto fast_tag) {
         constexpr int TK = decltype(tag)::value;
+        constexpr bool FAST = decltype(fast_tag)::value;
         auto cell = [&](int u) {
             const float4 q4 = qd[u];
             // Gaussian profile of the cell at the lane's channels, exp(-q^2) =
@@ -470,13 +512,27 @@ __device__ __forceinline__ void channel_pass(const RFShape &sh, const WarpMem &m
             const float4 *r = rec + u * sh.rec_ld;
 #pragma unroll
             for (int k = 0; k < NP; k++) {
+                if constexpr (DUST) {
+                    const float4 v = r[2 * k], w = r[2 * k + 1];
+                    const DustPack c{make_float2(v.x, v.y), make_float2(v.z, v.w), make_float2(w.x, w.y),
+                                     make_float2(w.z, w.w)};
+#pragma unroll
+                    for (int s = 0; s < NSL; s++)
+                        transfer2_dust(TK > 0, FAST, I[s][k], c, make_float2(gs[s], gs[s]));
+                    continue;
+                }
                 const float4 v = r[k];
 #pragma unroll
                 for (int s = 0; s < NSL; s++)
                     transfer2(k >= NPK - TK, I[s][k], make_float2(v.x, v.y), make_float2(v.z, v.w),
                               make_float2(gs[s], gs[s]));
             }
-            if (ODD) {
+            if (ODD && DUST) {
+                const float4 v = r[2 * NP], w = r[2 * NP + 1];
+                const DustPack c{make_float2(v.x, v.y), make_float2(v.z, v.w), make_float2(w.x, w.y),
+                                 make_float2(w.z, w.w)};
+                transfer2_dust(TK > 0, FAST, Io, c, make_float2(gs[0], gs[1]));
+            } else if (ODD) {
                 const float4 v = r[NP];
                 if (NSL == 2)
                     transfer2(TK >= 1, Io, make_float2(v.x, v.y), make_float2(v.z, v.w), make_float2(gs[0], gs[1]));
@@ -486,11 +542,18 @@ __device__ __forceinline__ void channel_pass(const RFShape &sh, const WarpMem &m
         };
         // enough independent updates in flight per iteration: narrow groups
         // run several cells at once (their weights do not depend on each other)
-        constexpr int U = NSL * NLG >= 10 ? 1 : NSL * NLG >= 5 ? 2 : 4;
+        constexpr int U = DUST ? 1 : NSL * NLG >= 10 ? 1 : NSL * NLG >= 5 ? 2 : 4;
 #pragma unroll U
         for (int u = 0; u < nc; u++) cell(u);
     };
-    with_thin_packs<NPK>(tk, run);
+    if constexpr (DUST) {
+        if (!fast) run(std::integral_constant<int, 0>{}, std::false_type{});
+        else if (tk == NPK) run(std::integral_constant<int, 1>{}, std::true_type{});
+        else run(std::integral_constant<int, 0>{}, std::true_type{});
+    } else {
+        auto plain = [&](auto tag) { run(tag, std::false_type{}); };
+        with_thin_packs<NPK>(tk, plain);
+    }
     if (!last) {
 #pragma unroll
         for (int s = 0; s < NSL; s++)
@@ -502,9 +565,36 @@ __device__ __forceinline__ void channel_pass(const RFShape &sh, const WarpMem &m
     // central cell (inverse_rt.f90:320-339): no gate, profile at the node's own
     // b, then the weighted channel sum, slot by slot
     float2 *part = m.part(sh) + lane;
-    const float4 *row = m.row(sh) + g * NPK;
+    const float4 *row = m.row(sh) + g * (DUST ? 2 : 1) * NPK;
     const int np32 = sh.npk * 32;
-    auto weigh = [&](float2 &I2, float4 v, float2 g0, float2 &om, float2 &Ie) {
+    // the intensity after the cell; om and Ie: what L* and J_eff sum
+    auto weigh = [&](float2 &I2, int k, float2 g0, float2 &om, float2 &Ie) {
+        if constexpr (DUST) {
+            const float4 v = row[2 * k], w = row[2 * k + 1];
+            const float A[2] = {v.x, v.y}, Sl[2] = {v.z, v.w}, al[2] = {w.x, w.y}, Jd[2] = {w.z, w.w};
+            const float gg[2] = {g0.x, g0.y}, Iv[2] = {I2.x, I2.y};
+            float o[2], omv[2], Iev[2];
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                const float kap = fmaf(A[q], gg[q], al[q]);
+                const float tau = kap * fst0;
+                const float Sv = fmaf(Sl[q] * A[q], gg[q], Jd[q]) / kap;
+                const float x = tau * LOG2E_F;
+                const float w1 = one_minus_exp(x, ex2(-x));
+                o[q] = fmaf(w1, Sv - Iv[q], Iv[q]);
+                omv[q] = Iev[q] = 0.f;
+                if (sh.split) {
+                    const float lf = A[q] * gg[q] / kap;   // line share of the opacity
+                    const float Sd = Jd[q] / kap;          // dust emission share of S
+                    Iev[q] = fmaf(w1, Sd - Iv[q], Iv[q]);
+                    omv[q] = lf * w1;
+                }
+            }
+            om = make_float2(omv[0], omv[1]);
+            Ie = make_float2(Iev[0], Iev[1]);
+            return make_float2(o[0], o[1]);
+        }
+        const float4 v = row[k];
         const float2 x = __fmul2_rn(__fmul2_rn(__fmul2_rn(make_float2(v.x, v.y), g0), make_float2(fst0, fst0)),
                                     make_float2(LOG2E_F, LOG2E_F));
         om = one_minus_exp2(x, ex2(-x.x), ex2(-x.y));
@@ -521,7 +611,7 @@ __device__ __forceinline__ void channel_pass(const RFShape &sh, const WarpMem &m
 #pragma unroll
         for (int k = 0; k < NP; k++) {
             float2 om, Ie;
-            const float2 o = weigh(I[s][k], row[k], g0, om, Ie);
+            const float2 o = weigh(I[s][k], k, g0, om, Ie);
             if (valid) part[k * 32] = __ffma2_rn(w2, o, part[k * 32]);
             if (sh.split && valid) {
                 part[np32 + k * 32] = __ffma2_rn(w2, Ie, part[np32 + k * 32]);
@@ -534,7 +624,7 @@ __device__ __forceinline__ void channel_pass(const RFShape &sh, const WarpMem &m
         const bool v0 = ch < nch - sh.rt, v1 = NSL == 2 && ch + 32 < nch - sh.rt;
         const float2 c0 = chtab[v0 ? ch : 0], c1 = chtab[v1 ? ch + 32 : 0];
         float2 om, Ie;
-        const float2 o = weigh(Io, row[NP], make_float2(c0.x, c1.x), om, Ie);
+        const float2 o = weigh(Io, NP, make_float2(c0.x, c1.x), om, Ie);
         auto add = [&](float2 *q, float2 y) {
             if (v0) q->x = fmaf(c0.y, y.x, q->x);
             if (v1) q->x = fmaf(c1.y, y.y, q->x);
@@ -543,84 +633,6 @@ __device__ __forceinline__ void channel_pass(const RFShape &sh, const WarpMem &m
         if (sh.split) {
             add(part + np32 + NP * 32, Ie);
             add(part + 2 * np32 + NP * 32, om);
-        }
-    }
-}
-
-// The same with dust: line by line, tau = (kv phi + alpha) dx n, S = (ev phi
-// + j) / (kv phi + alpha), with ray_in's gate tau > 1e-30
-// (inverse_rt.f90:308).
-template <int NLG, int NSL>
-__device__ __forceinline__ void channel_pass_dust(const RFShape &sh, const WarpMem &m, const float2 *chtab, int nch,
-                                                  int nvel, int lane, int g, int s0, int nc, bool first, bool last,
-                                                  const float *bb, float fst0) {
-    float I[NSL][NLG];
-    float *sv = (float *)m.I(sh) + (size_t)s0 * NLG * 32 + lane;
-#pragma unroll
-    for (int s = 0; s < NSL; s++)
-#pragma unroll
-        for (int l = 0; l < NLG; l++) I[s][l] = first ? bb[l] : sv[(s * NLG + l) * 32];
-    const float4 *rec = m.rec(sh), *qd = m.qd(sh);
-    const float ch0 = (float)(lane + 32 * s0 - nvel), ch1 = (float)(lane + 32 * (s0 + 1) - nvel);
-#pragma unroll 1
-    for (int u = 0; u < nc; u++) {
-        const float4 q4 = qd[u];
-        float gs[2];
-        {
-            const float q = fmaf(q4.z, ch0, q4.x);
-            gs[0] = ex2(-(q * q));
-            gs[1] = 0.f;
-        }
-        if (NSL == 2) {
-            const float q = fmaf(q4.z, ch1, q4.x);
-            gs[1] = ex2(-(q * q));
-        }
-        const float4 *r = rec + u * sh.rec_ld;
-#pragma unroll
-        for (int l = 0; l < NLG; l++) {
-            const float4 v = r[l];
-#pragma unroll
-            for (int s = 0; s < NSL; s++) {
-                const float tau = fmaf(v.x, gs[s], v.z);
-                const float Sv = fmaf(v.y, gs[s], v.w) / tau;
-                const float x = tau * LOG2E_F;
-                const float om = one_minus_exp(x, ex2(-x));
-                const float In = fmaf(om, Sv - I[s][l], I[s][l]);
-                I[s][l] = (tau > 1e-30f) ? In : I[s][l];
-            }
-        }
-    }
-    if (!last) {
-#pragma unroll
-        for (int s = 0; s < NSL; s++)
-#pragma unroll
-            for (int l = 0; l < NLG; l++) sv[(s * NLG + l) * 32] = I[s][l];
-        return;
-    }
-    float *part = (float *)m.part(sh) + lane;     // [line][lane]
-    const float4 *row = m.row(sh) + g * NLG;
-    const int np32 = 2 * sh.npk * 32;
-#pragma unroll
-    for (int s = 0; s < NSL; s++) {
-        const int ch = lane + 32 * (s0 + s);
-        if (ch >= nch) continue;
-        const float2 ct = chtab[ch];
-#pragma unroll
-        for (int l = 0; l < NLG; l++) {
-            const float4 v = row[l];
-            const float kap = fmaf(v.x, ct.x, v.z);
-            const float tau = kap * fst0;
-            const float Sv = fmaf(v.y * v.x, ct.x, v.w) / kap;
-            const float x = tau * LOG2E_F;
-            const float om = one_minus_exp(x, ex2(-x));
-            const float Io = fmaf(om, Sv - I[s][l], I[s][l]);
-            part[l * 32] = fmaf(ct.y, Io, part[l * 32]);
-            if (sh.split) {
-                const float lf = v.x * ct.x / kap;   // line share of the opacity
-                const float Sd = v.w / kap;          // dust emission share of S
-                part[np32 + l * 32] = fmaf(ct.y, fmaf(om, Sd - I[s][l], I[s][l]), part[np32 + l * 32]);
-                part[2 * np32 + l * 32] = fmaf(ct.y, lf * om, part[2 * np32 + l * 32]);
-            }
         }
     }
 }
@@ -672,6 +684,7 @@ __device__ __forceinline__ void integrate_batch(const RFArgs &a, const RFShape &
                 }
                 __syncwarp();
                 unsigned thin = (1u << NPK) - 1u;   // the packs thin in this cell
+                bool in_range = true;               // dust: the fast quotient serves this cell
                 if (lane < nc) {
                     const float4 cv = a.cellv[wc.x];
                     const float4 *lt = a.ltab + (size_t)wc.x * L;
@@ -681,10 +694,23 @@ __device__ __forceinline__ void integrate_batch(const RFArgs &a, const RFShape &
                     const float2 qdl = make_float2((d4.w - vp) * ib, dqfac * ib);
                     m.qd(sh)[lane] = make_float4(qdl.x, qdl.x, qdl.y, qdl.y);
                     if constexpr (DUST) {
+                        float4 v[2 * NPK];
+#pragma unroll
+                        for (int l = 0; l < NLG; l++) v[l] = lt[min(l0 + l, L - 1)];
 #pragma unroll
                         for (int l = 0; l < NLG; l++) {
-                            const float4 v = lt[min(l0 + l, L - 1)];
-                            rec[l] = make_float4(v.x * fst, v.y * v.x * fst, v.z * fst, v.w * fst);
+                            const float4 t = v[l];
+                            v[l] = make_float4(t.x * fst, t.y * t.x * fst, t.z * fst, t.w * fst);
+                            in_range = in_range && dust_in_range(v[l]);
+                            // |tau| <= |A| + |Ad|: the Taylor form in every channel
+                            if (!((fabsf(v[l].x) + fabsf(v[l].z)) * LOG2E_F < OM_THIN_A)) thin &= ~(1u << (l / 2));
+                        }
+                        if (ODD) v[NLG] = v[NLG - 1];
+#pragma unroll
+                        for (int k = 0; k < NPK; k++) {
+                            const float4 t = v[2 * k], w = v[2 * k + 1];
+                            rec[2 * k] = make_float4(t.x, w.x, t.y, w.y);
+                            rec[2 * k + 1] = make_float4(t.z, w.z, t.w, w.w);
                         }
                     } else {
                         // optical depth at unit profile in log2 units (ex2 takes
@@ -728,7 +754,8 @@ __device__ __forceinline__ void integrate_batch(const RFArgs &a, const RFShape &
                 // alone in every channel: the full update would pick exactly that
                 // value.  Decided per chunk, uniform over the warp, for the
                 // group's trailing packs (a rotor's higher lines are the thinner).
-                const int tk = DUST ? 0 : __clz(~(__reduce_and_sync(FULL, thin) << (32 - NPK)));
+                const int tk = __clz(~(__reduce_and_sync(FULL, thin) << (32 - NPK)));
+                const bool fast = DUST && __all_sync(FULL, in_range);
                 __syncwarp();
                 if (!DUST && sh.rt && lane < NLG) {
                     const float *om = m.om(sh) + lane;
@@ -737,18 +764,12 @@ __device__ __forceinline__ void integrate_batch(const RFArgs &a, const RFShape &
                     for (int u = 0; u < nc; u++) Irem = fmaf(om[u * sh.om_ld], S[u * sh.rec_ld * 4] - Irem, Irem);
                 }
                 int s0 = 0;
-                for (; s0 + 1 < sh.nslot; s0 += 2) {
-                    if constexpr (DUST)
-                        channel_pass_dust<NLG, 2>(sh, m, chtab, nch, nvel, lane, g, s0, nc, first, last, bb, fst0);
-                    else
-                        channel_pass<NLG, 2>(sh, m, chtab, nch, nvel, lane, g, s0, nc, tk, first, last, bb, fst0);
-                }
-                if (s0 < sh.nslot) {
-                    if constexpr (DUST)
-                        channel_pass_dust<NLG, 1>(sh, m, chtab, nch, nvel, lane, g, s0, nc, first, last, bb, fst0);
-                    else
-                        channel_pass<NLG, 1>(sh, m, chtab, nch, nvel, lane, g, s0, nc, tk, first, last, bb, fst0);
-                }
+                for (; s0 + 1 < sh.nslot; s0 += 2)
+                    channel_pass<NLG, 2, DUST>(sh, m, chtab, nch, nvel, lane, g, s0, nc, tk, fast, first, last, bb,
+                                               fst0);
+                if (s0 < sh.nslot)
+                    channel_pass<NLG, 1, DUST>(sh, m, chtab, nch, nvel, lane, g, s0, nc, tk, fast, first, last, bb,
+                                               fst0);
                 if (last) break;
             }
             // the channel sums over the lanes, the remainder channel's share
@@ -757,18 +778,13 @@ __device__ __forceinline__ void integrate_batch(const RFArgs &a, const RFShape &
             for (int q = 0; q < (sh.split ? 3 : 1); q++) {
                 const float2 *part = m.part(sh) + q * NPK * 32 + lane;
                 float v[NLG];
-                if constexpr (DUST) {
-#pragma unroll
-                    for (int l = 0; l < NLG; l++) v[l] = reinterpret_cast<const float *>(part - lane)[l * 32 + lane];
-                } else {
 #pragma unroll
                     for (int k = 0; k < NP; k++) {
                         const float2 p = part[k * 32];
                         v[2 * k] = p.x;
                         v[2 * k + 1] = p.y;
                     }
-                    if (ODD) v[NLG - 1] = part[NP * 32].x;
-                }
+                if (ODD) v[NLG - 1] = part[NP * 32].x;
                 const float t = sum_lines<NLG>(v, 16, lane);
                 float *dst = m.v(sh) + (q * 32 + rr) * L;
                 if (line < min(l0 + NLG, L)) dst[line] = t;
@@ -918,16 +934,12 @@ __global__ void __launch_bounds__(256, (NLG >= 1 && NLG <= 4) ? 3 : 2) k_radiati
             {
                 const float4 *lt = a.ltab + (size_t)node * sh.L;
                 float4 *row = m.row(sh);
-                const int per = DUST ? sh.nlg : sh.npk;
-                for (int i = lane; i < sh.groups * per; i += 32) {
-                    const int l0 = (i / per) * sh.nlg, k = i % per;
-                    if (DUST) {
-                        row[i] = lt[min(l0 + k, sh.L - 1)];
-                    } else {
-                        const float4 v = lt[min(l0 + 2 * k, sh.L - 1)];
-                        const float4 w = lt[min(l0 + min(2 * k + 1, sh.nlg - 1), sh.L - 1)];
-                        row[i] = make_float4(v.x, w.x, v.y, w.y);
-                    }
+                for (int i = lane; i < sh.groups * sh.npk; i += 32) {
+                    const int l0 = (i / sh.npk) * sh.nlg, k = i % sh.npk;
+                    const float4 v = lt[min(l0 + 2 * k, sh.L - 1)];
+                    const float4 w = lt[min(l0 + min(2 * k + 1, sh.nlg - 1), sh.L - 1)];
+                    row[DUST ? 2 * i : i] = make_float4(v.x, w.x, v.y, w.y);
+                    if (DUST) row[2 * i + 1] = make_float4(v.z, w.z, v.w, w.w);
                 }
                 for (int i = lane; i < (sh.split ? 8 : 4) * sh.L; i += 32) m.acc(sh)[i] = 0.f;
             }
@@ -983,6 +995,7 @@ __global__ void __launch_bounds__(256, (NLG >= 1 && NLG <= 4) ? 3 : 2) k_radiati
                     float rh = (float)sexit, rl = (float)(sexit - (double)rh);
                     float rx = 0.f, ry = 0.f, rz = 0.f;
                     int c = node;
+                    const bool step_ok = a.dx32 > 1e-20f && a.dx32 < 1e20f;   // quot_rn's range
                     for (;;) {
                         const float tsph = rh + rl;
                         const int o = a.off[c], deg = a.off[c + 1] - o;
@@ -1009,9 +1022,10 @@ __global__ void __launch_bounds__(256, (NLG >= 1 && NLG <= 4) ? 3 : 2) k_radiati
                                 }
                             }
                         }
-                        const float delta = (bj < 0) ? tsph : bnum / bden;
+                        // (0 < bnum <= 2 bden, both lengths of the cloud's geometry)
+                        const float delta = (bj < 0) ? tsph : quot_rn(bnum, bden);
                         if (K >= n_depth) { over = true; break; }
-                        const int steps = (int)roundf(delta / a.dx32);   // nint(delta_x/dx)
+                        const int steps = (int)roundf(step_ok ? quot_rn(delta, a.dx32) : delta / a.dx32);   // nint(delta_x/dx)
                         walk[walk_at(K, lane)] = make_int2(c, steps);
                         if (K == 0) B.st0[lane] = steps;
                         K++;
