@@ -13,6 +13,8 @@
 //                       its photon position relative to the current node
 //                       finds every face crossing in FP32 without absolute
 //                       coordinates
+//   wstart, whead, wedge, wnext   the same edges in blocks of slots for the
+//                       radiation field's walk
 //   levp   (nlev,N) FP64 level populations, plus the per-node scalars
 //                       (b, T_kin, T_dust, dust, n_H2, abundance) in FP64.
 #include <unistd.h>
@@ -130,13 +132,16 @@ extern "C" int portal_set_molecule(portal_ctx *c, int nlev, const int *j_lev, co
 // Edge geometry from the FP64 positions; one thread per (node, slot).
 __global__ void k_build_edges(int N, int maxne, const int *__restrict__ del_ne,
                               const int *__restrict__ off, const double *__restrict__ pos,
-                              int *__restrict__ nb_idx, float4 *__restrict__ edge) {
+                              int *__restrict__ nb_idx, float4 *__restrict__ edge, const int *__restrict__ wstart,
+                              int2 *__restrict__ whead, float4 *__restrict__ wedge, int *__restrict__ wnext) {
     long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     long long tot = (long long)N * maxne;
     if (tid >= tot) return;
     int s = (int)(tid / N);
     int i = (int)(tid - (long long)s * N);
     int o = off[i], deg = off[i + 1] - o;
+    const size_t w = 4 * (size_t)wstart[i];
+    if (s == 0) whead[wstart[i]] = make_int2(deg, i);
     if (s >= deg) return;
     int nb = del_ne[(size_t)i + (size_t)N * s] - 1;
     double ex = pos[3 * (size_t)nb] - pos[3 * (size_t)i];
@@ -144,7 +149,10 @@ __global__ void k_build_edges(int N, int maxne, const int *__restrict__ del_ne,
     double ez = pos[3 * (size_t)nb + 2] - pos[3 * (size_t)i + 2];
     double h = 0.5 * (ex * ex + ey * ey + ez * ez);
     nb_idx[o + s] = nb;
-    edge[o + s] = make_float4((float)ex, (float)ey, (float)ez, (float)h);
+    const float4 e = make_float4((float)ex, (float)ey, (float)ez, (float)h);
+    edge[o + s] = e;
+    wedge[w + s] = e;
+    wnext[w + s] = wstart[nb];
 }
 
 __global__ void k_cellv(int N, const double *__restrict__ vel, const double *__restrict__ b,
@@ -195,6 +203,17 @@ extern "C" int portal_set_cloud(portal_ctx *c, int N, int bulk, int nlev, const 
         }
     }
     int nnz = off[N];
+    // the walk tables' blocks: degrees rounded up to groups of 4 slots, at least
+    // one (an isolated node has a header too), and a tail that the first
+    // loads of the last blocks may run into
+    std::vector<int> ws(N);
+    size_t groups = 0;
+    for (int i = 0; i < N; i++) {
+        ws[i] = (int)groups;
+        groups += std::max(1, (off[i + 1] - off[i] + 3) / 4);
+    }
+    groups += 4;
+    const size_t slots = 4 * groups;
     c->have_cloud = false;
     c->j_valid = false;
     c->ali_valid = false;
@@ -202,7 +221,8 @@ extern "C" int portal_set_cloud(portal_ctx *c, int N, int bulk, int nlev, const 
         c->cellv.reserve(N) || c->nb_off.reserve(N + 1) || c->nb_idx.reserve(nnz) ||
         c->edge.reserve(nnz) || c->levp.reserve((size_t)nlev * N) || c->b64.reserve(N) ||
         c->tkin.reserve(N) || c->tdust.reserve(N) || c->dustp.reserve(N) || c->h2.reserve(N) ||
-        c->ab.reserve(N) || c->status.reserve(N) || c->nmol.reserve(N))
+        c->ab.reserve(N) || c->status.reserve(N) || c->nmol.reserve(N) || c->wstart.reserve(N) ||
+        c->whead.reserve(groups) || c->wedge.reserve(slots) || c->wnext.reserve(slots))
         return set_err(c, PORTAL_ERR_NOMEM, "portal_set_cloud: device allocation failed");
     std::vector<double> tk(N), td(N), nm(N);
     bool dust = false;
@@ -227,6 +247,10 @@ extern "C" int portal_set_cloud(portal_ctx *c, int N, int bulk, int nlev, const 
     if ((rc = upload(c, c->nmol.p, nm.data(), N))) return rc;
     PCHECK(c, cudaMemcpyAsync(c->nb_off.p, off.data(), (N + 1) * sizeof(int),
                               cudaMemcpyHostToDevice, c->stream));
+    PCHECK(c, cudaMemcpyAsync(c->wstart.p, ws.data(), N * sizeof(int), cudaMemcpyHostToDevice, c->stream));
+    // (slots past a node's degree are loaded, never used)
+    PCHECK(c, cudaMemsetAsync(c->wedge.p, 0, slots * sizeof(float4), c->stream));
+    PCHECK(c, cudaMemsetAsync(c->wnext.p, 0, slots * sizeof(int), c->stream));
     DevBuf<int> dne;
     if (dne.reserve((size_t)N * maxne) || c->vel64.reserve(3 * (size_t)N))
         return set_err(c, PORTAL_ERR_NOMEM, "portal_set_cloud: staging allocation failed");
@@ -237,7 +261,8 @@ extern "C" int portal_set_cloud(portal_ctx *c, int N, int bulk, int nlev, const 
     long long tot = (long long)N * maxne;
     k_build_edges<<<(unsigned)((tot + 255) / 256), 256, 0, c->stream>>>(N, maxne, dne.p, c->nb_off.p,
                                                                       c->pos64.p, c->nb_idx.p,
-                                                                      c->edge.p);
+                                                                      c->edge.p, c->wstart.p, c->whead.p,
+                                                                      c->wedge.p, c->wnext.p);
     PCHECK(c, cudaGetLastError());
     k_cellv<<<(N + 255) / 256, 256, 0, c->stream>>>(N, c->vel64.p, c->b64.p, c->cellv.p);
     PCHECK(c, cudaGetLastError());

@@ -15,9 +15,11 @@ struct RFArgs {
     double *frames;                   // (N, 13) node frames (k_line_table)
     const double *__restrict__ ab;
     const float4 *__restrict__ cellv;
-    const int *__restrict__ off;
-    const int *__restrict__ idx;
-    const float4 *__restrict__ edge;
+    // the walk's tables (ctx.cu): a block of slots per node, in groups of 4
+    const int *__restrict__ wstart;     // (N) first group of each node's block
+    const int2 *__restrict__ whead;     // per group; a block's first: (degree, node)
+    const float4 *__restrict__ wedge;   // per slot: the edge record
+    const int *__restrict__ wnext;      // per slot: the neighbour's first group
     const float4 *__restrict__ ltab;
     const double *__restrict__ dirs;  // (ndir, 6): mu, sin th, cos ph, sin ph, w, w*c_in/sqrt2
     const float *__restrict__ chq;    // (nch) 2 nv / nvel

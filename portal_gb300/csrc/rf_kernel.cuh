@@ -495,11 +495,10 @@ __device__ __forceinline__ void channel_pass(const RFShape &sh, const WarpMem &m
     auto run = [&](auto tag, auto fast_tag) {
         constexpr int TK = decltype(tag)::value;
         constexpr bool FAST = decltype(fast_tag)::value;
-        auto cell = [&](int u) {
+        // Gaussian profile of a cell at the lane's channels, exp(-q^2) = 2^(-q'^2)
+        // with q' = q sqrt(log2 e) (staged scaled)
+        auto profile = [&](int u, float (&gs)[2]) {
             const float4 q4 = qd[u];
-            // Gaussian profile of the cell at the lane's channels, exp(-q^2) =
-            // 2^(-q'^2) with q' = q sqrt(log2 e) (staged scaled)
-            float gs[2];
             if (NSL == 2) {
                 const float2 q = __ffma2_rn(make_float2(q4.z, q4.w), ch2, make_float2(q4.x, q4.y));
                 const float2 t = __fmul2_rn(q, q);
@@ -509,6 +508,8 @@ __device__ __forceinline__ void channel_pass(const RFShape &sh, const WarpMem &m
                 const float q = fmaf(q4.z, ch2.x, q4.x);
                 gs[0] = gs[1] = ex2(-(q * q));
             }
+        };
+        auto cell = [&](int u, const float (&gs)[2]) {
             const float4 *r = rec + u * sh.rec_ld;
 #pragma unroll
             for (int k = 0; k < NP; k++) {
@@ -544,7 +545,11 @@ __device__ __forceinline__ void channel_pass(const RFShape &sh, const WarpMem &m
         // run several cells at once (their weights do not depend on each other)
         constexpr int U = DUST ? 1 : NSL * NLG >= 10 ? 1 : NSL * NLG >= 5 ? 2 : 4;
 #pragma unroll U
-        for (int u = 0; u < nc; u++) cell(u);
+        for (int u = 0; u < nc; u++) {
+            float gs[2];
+            profile(u, gs);
+            cell(u, gs);
+        }
     };
     if constexpr (DUST) {
         if (!fast) run(std::integral_constant<int, 0>{}, std::false_type{});
@@ -994,43 +999,64 @@ __global__ void __launch_bounds__(256, (NLG >= 1 && NLG <= 4) ? 3 : 2) k_radiati
                     // (rh + rl), decremented exactly by each step
                     float rh = (float)sexit, rl = (float)(sexit - (double)rh);
                     float rx = 0.f, ry = 0.f, rz = 0.f;
-                    int c = node;
                     const bool step_ok = a.dx32 > 1e-20f && a.dx32 < 1e20f;   // quot_rn's range
+                    int wg = a.wstart[node];
                     for (;;) {
+                        // the cell's block of the walk tables: its header, the first 12
+                        // edges and where their neighbours' blocks start, all in
+                        // flight at once (scattered L2 reads: the walk is their
+                        // latency, one round trip per step this way, five or six
+                        // when offsets, edges and ids were read one after the other)
+                        const int2 hd = a.whead[wg];   // (degree, node)
+                        const float4 *we = a.wedge + 4 * (size_t)wg;
+                        const int4 *wn = reinterpret_cast<const int4 *>(a.wnext) + wg;
+                        float4 e[12];
+                        int4 t[3];
+#pragma unroll
+                        for (int i = 0; i < 12; i++) e[i] = we[i];
+#pragma unroll
+                        for (int i = 0; i < 3; i++) t[i] = wn[i];
                         const float tsph = rh + rl;
-                        const int o = a.off[c], deg = a.off[c + 1] - o;
                         // check_neigh_fast's scan: best starts at the sphere exit, a
                         // neighbour replaces it when FACE_EPS < t <= best (so among equal
                         // t the later neighbour wins).  t = num/den compared by cross
-                        // multiplication (den > 0).  Eight neighbours' records are loaded
-                        // before they are compared: the loads are scattered L2 reads.
+                        // multiplication (den > 0).
                         float bnum = tsph, bden = 1.f;
-                        int bj = -1;
-                        for (int j0 = 0; j0 < deg; j0 += 8) {
-                            float4 e8[8];
-#pragma unroll
-                            for (int i = 0; i < 8; i++) e8[i] = a.edge[o + min(j0 + i, deg - 1)];
-#pragma unroll
-                            for (int i = 0; i < 8; i++) {
-                                const float4 e = e8[i];
-                                const float den = e.x * fdx + e.y * fdy + e.z * fdz;
-                                const float num = e.w - (e.x * rx + e.y * ry + e.z * rz);
-                                if (j0 + i < deg && den > 0.f && num > FACE_EPS * den && num * bden <= bnum * den) {
-                                    bnum = num;
-                                    bden = den;
-                                    bj = j0 + i;
-                                }
+                        int bj = -1, bw = 0;
+                        auto face = [&](int j, float4 e, int next) {
+                            const float den = e.x * fdx + e.y * fdy + e.z * fdz;
+                            const float num = e.w - (e.x * rx + e.y * ry + e.z * rz);
+                            if (j < hd.x && den > 0.f && num > FACE_EPS * den && num * bden <= bnum * den) {
+                                bnum = num;
+                                bden = den;
+                                bj = j;
+                                bw = next;
                             }
+                        };
+#pragma unroll
+                        for (int i = 0; i < 12; i++) {
+                            const int4 q = t[i / 4];
+                            face(i, e[i], (i & 3) == 0 ? q.x : (i & 3) == 1 ? q.y : (i & 3) == 2 ? q.z : q.w);
+                        }
+                        for (int j = 12; j < hd.x; j += 4) {
+                            float4 e4[4];
+#pragma unroll
+                            for (int i = 0; i < 4; i++) e4[i] = we[j + i];
+                            const int4 q = wn[j >> 2];
+                            face(j, e4[0], q.x);
+                            face(j + 1, e4[1], q.y);
+                            face(j + 2, e4[2], q.z);
+                            face(j + 3, e4[3], q.w);
                         }
                         // (0 < bnum <= 2 bden, both lengths of the cloud's geometry)
                         const float delta = (bj < 0) ? tsph : quot_rn(bnum, bden);
                         if (K >= n_depth) { over = true; break; }
                         const int steps = (int)roundf(step_ok ? quot_rn(delta, a.dx32) : delta / a.dx32);   // nint(delta_x/dx)
-                        walk[walk_at(K, lane)] = make_int2(c, steps);
+                        walk[walk_at(K, lane)] = make_int2(hd.y, steps);
                         if (K == 0) B.st0[lane] = steps;
                         K++;
                         if (bj < 0) break;
-                        const float4 e = a.edge[o + bj];
+                        const float4 eb = we[bj];
                         {   // (rh, rl) -= delta: two-sum, then renormalise
                             const float t = rh - delta;
                             const float bv = t - rh;
@@ -1039,10 +1065,10 @@ __global__ void __launch_bounds__(256, (NLG >= 1 && NLG <= 4) ? 3 : 2) k_radiati
                             rh = t + lo;
                             rl = lo - (rh - t);
                         }
-                        rx = fmaf(delta, fdx, rx) - e.x;
-                        ry = fmaf(delta, fdy, ry) - e.y;
-                        rz = fmaf(delta, fdz, rz) - e.z;
-                        c = a.idx[o + bj];
+                        rx = fmaf(delta, fdx, rx) - eb.x;
+                        ry = fmaf(delta, fdy, ry) - eb.y;
+                        rz = fmaf(delta, fdz, rz) - eb.z;
+                        wg = bw;
                     }
                     B.K[lane] = K;
                 }
