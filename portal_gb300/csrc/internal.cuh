@@ -124,9 +124,12 @@ struct SEBatch {
 int rf_prepare(portal_ctx *c, int nth, int nph, int nvel, const double *gvec, double dx, int n_depth,
                bool split, RFArgs *a);
 int rf_pass(portal_ctx *c, const RFArgs &a, cudaStream_t s);
-const void *rf_kernel_narrow(int nlg);   // the single-model kernel for groups of nlg lines: 1..5,
-const void *rf_kernel_wide(int nlg);     // 6..10,
-const void *rf_kernel_dust(int nlg);     // with dust, 1..5
+// the single-model kernel for groups of nlg lines (1..10, with dust 1..5):
+const void *rf_kernel_one(int nlg, bool split);    // one slot of channels
+const void *rf_kernel_even(int nlg);               // an even number of slots
+const void *rf_kernel_even_split(int nlg);
+const void *rf_kernel_any(int nlg);                // any, split or not
+const void *rf_kernel_dust(int nlg, int slots);    // slots 1: one, 2: an even number, 0: any
 size_t rf_walk_records(int n_depth);     // walk scratch per warp, int2 records
 // the batched launch: its shape for these models (max_group: the widest line
 // group wanted), and the blocks per SM the kernel reaches with it

@@ -176,7 +176,12 @@ int launch_rf(portal_ctx *c, RFArgs &a, int n_depth) {
     const bool dust = c->has_dust, split = a.JE != nullptr;
     const int rt = rf_remainder(a.nch, dust, a.L);
     RFShape sh = rf_shape(a.L, max_line_group(), a.nch, dust, rt, split);
-    const void *kern = dust ? rf_kernel_dust(sh.nlg) : sh.nlg <= 5 ? rf_kernel_narrow(sh.nlg) : rf_kernel_wide(sh.nlg);
+    const int slots = sh.nslot == 1 ? 1 : sh.nslot % 2 == 0 ? 2 : 0;
+    const void *kern = dust         ? rf_kernel_dust(sh.nlg, slots)
+                       : slots == 1 ? rf_kernel_one(sh.nlg, split)
+                       : slots == 0 ? rf_kernel_any(sh.nlg)
+                       : split      ? rf_kernel_even_split(sh.nlg)
+                                    : rf_kernel_even(sh.nlg);
     const size_t table = (a.nch * sizeof(float2) + 15) & ~(size_t)15;
     int wpb = rf_warps();
     while (wpb > 1 && table + (size_t)wpb * sh.bytes > 200 * 1024) wpb--;   // many lines and channels

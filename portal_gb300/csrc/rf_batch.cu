@@ -7,7 +7,8 @@
 namespace {
 
 const void *batch_kernel(bool dust) {
-    return dust ? (const void *)k_radiation_field<0, true, true> : (const void *)k_radiation_field<0, false, true>;
+    return dust ? (const void *)k_radiation_field<0, true, true, 0, true>
+                : (const void *)k_radiation_field<0, false, true, 0, true>;
 }
 
 size_t batch_dyn_smem(const RFBatch &bw) {

@@ -1,14 +1,25 @@
-// The single-model radiation-field kernel with dust, groups of 1 to 5 lines.
+// The single-model radiation-field kernel: with dust, groups of 1 to 5 lines
+// (compiled apart so that the instantiations build in parallel).
 #include "rf_kernel.cuh"
 
 namespace portal {
-const void *rf_kernel_dust(int nlg) {
+const void *rf_kernel_dust(int nlg, int slots) {
     switch (nlg) {
-    case 1: return (const void *)k_radiation_field<1, true, false>;
-    case 2: return (const void *)k_radiation_field<2, true, false>;
-    case 3: return (const void *)k_radiation_field<3, true, false>;
-    case 4: return (const void *)k_radiation_field<4, true, false>;
-    default: return (const void *)k_radiation_field<5, true, false>;
+    case 1: return slots == 1   ? (const void *)k_radiation_field<1, true, false, 1, true>
+                   : slots == 2 ? (const void *)k_radiation_field<1, true, false, 2, true>
+                                : (const void *)k_radiation_field<1, true, false, 0, true>;
+    case 2: return slots == 1   ? (const void *)k_radiation_field<2, true, false, 1, true>
+                   : slots == 2 ? (const void *)k_radiation_field<2, true, false, 2, true>
+                                : (const void *)k_radiation_field<2, true, false, 0, true>;
+    case 3: return slots == 1   ? (const void *)k_radiation_field<3, true, false, 1, true>
+                   : slots == 2 ? (const void *)k_radiation_field<3, true, false, 2, true>
+                                : (const void *)k_radiation_field<3, true, false, 0, true>;
+    case 4: return slots == 1   ? (const void *)k_radiation_field<4, true, false, 1, true>
+                   : slots == 2 ? (const void *)k_radiation_field<4, true, false, 2, true>
+                                : (const void *)k_radiation_field<4, true, false, 0, true>;
+    default: return slots == 1   ? (const void *)k_radiation_field<5, true, false, 1, true>
+                   : slots == 2 ? (const void *)k_radiation_field<5, true, false, 2, true>
+                                : (const void *)k_radiation_field<5, true, false, 0, true>;
     }
 }
 }  // namespace portal

@@ -470,11 +470,12 @@ struct WarpMem {
 // alone (with dust: all or none), fast: transfer2_dust's.  first: the intensities start from the background bb;
 // last: the central cell and the weighted channel sums follow, else the
 // intensities go back to shared memory.
-template <int NLG, int NSL, bool DUST>
+template <int NLG, int NSL, bool DUST, bool SPLIT>
 __device__ __forceinline__ void channel_pass(const RFShape &sh, const WarpMem &m, const float2 *chtab, int nch,
                                              int nvel, int lane, int g, int s0, int nc, int tk, bool fast, bool first,
                                              bool last, const float *bb, float fst0) {
     constexpr int NP = NLG / 2, ODD = NLG & 1, NPK = NP + ODD;
+    const bool split = SPLIT && sh.split;
     float2 I[NSL][NP > 0 ? NP : 1], Io;   // Io: the odd line's slots
     float2 *sv = m.I(sh) + (size_t)(s0 / 2) * NLG * 32 + lane;
     if (first) {
@@ -557,7 +558,11 @@ __device__ __forceinline__ void channel_pass(const RFShape &sh, const WarpMem &m
         else run(std::integral_constant<int, 0>{}, std::true_type{});
     } else {
         auto plain = [&](auto tag) { run(tag, std::false_type{}); };
-        with_thin_packs<NPK>(tk, plain);
+        // (a pass of one slot is a small part of its cell's work: two classes,
+        // as every further body costs instruction fetch)
+        if constexpr (NSL == 2) with_thin_packs<NPK>(tk, plain);
+        else if (tk == NPK) plain(std::integral_constant<int, NPK>{});
+        else plain(std::integral_constant<int, 0>{});
     }
     if (!last) {
 #pragma unroll
@@ -588,7 +593,7 @@ __device__ __forceinline__ void channel_pass(const RFShape &sh, const WarpMem &m
                 const float w1 = one_minus_exp(x, ex2(-x));
                 o[q] = fmaf(w1, Sv - Iv[q], Iv[q]);
                 omv[q] = Iev[q] = 0.f;
-                if (sh.split) {
+                if (split) {
                     const float lf = A[q] * gg[q] / kap;   // line share of the opacity
                     const float Sd = Jd[q] / kap;          // dust emission share of S
                     Iev[q] = fmaf(w1, Sd - Iv[q], Iv[q]);
@@ -618,7 +623,7 @@ __device__ __forceinline__ void channel_pass(const RFShape &sh, const WarpMem &m
             float2 om, Ie;
             const float2 o = weigh(I[s][k], k, g0, om, Ie);
             if (valid) part[k * 32] = __ffma2_rn(w2, o, part[k * 32]);
-            if (sh.split && valid) {
+            if (split && valid) {
                 part[np32 + k * 32] = __ffma2_rn(w2, Ie, part[np32 + k * 32]);
                 part[2 * np32 + k * 32] = __ffma2_rn(w2, om, part[2 * np32 + k * 32]);
             }
@@ -635,7 +640,7 @@ __device__ __forceinline__ void channel_pass(const RFShape &sh, const WarpMem &m
             if (v1) q->x = fmaf(c1.y, y.y, q->x);
         };
         add(part + NP * 32, o);
-        if (sh.split) {
+        if (split) {
             add(part + np32 + NP * 32, Ie);
             add(part + 2 * np32 + NP * 32, om);
         }
@@ -646,11 +651,12 @@ __device__ __forceinline__ void channel_pass(const RFShape &sh, const WarpMem &m
 // line the weighted channel sum at the node (v), with split also those of
 // J_eff and L*.  One chunk of up to 32 cells at a time is staged in shared
 // memory (lane = cell); then lanes run over channels, pass by pass.
-template <int NLG, bool DUST, bool STAR>
+template <int NLG, bool DUST, bool STAR, int SLOTS, bool SPLIT>
 __device__ __forceinline__ void integrate_batch(const RFArgs &a, const RFShape &sh, const WarpMem &m,
                                                 const RayBatch &B, unsigned smask, const float2 *chtab,
                                                 const int2 *walk, int nr, float dqfac, int lane) {
     const unsigned FULL = 0xffffffffu;
+    const bool split = SPLIT && sh.split;
     constexpr int NP = NLG / 2, ODD = NLG & 1, NPK = NP + ODD;
     const int L = a.L, nch = a.nch, nvel = a.nvel;
     float4 *rec = m.rec(sh) + lane * sh.rec_ld;
@@ -673,7 +679,7 @@ __device__ __forceinline__ void integrate_batch(const RFArgs &a, const RFShape &
             float Irem = (sh.rt && lane < NLG) ? bb[lane] : 0.f;
             {
                 float2 *part = m.part(sh) + lane;
-                for (int k = 0; k < (sh.split ? 3 : 1) * NPK; k++) part[k * 32] = make_float2(0.f, 0.f);
+                for (int k = 0; k < (split ? 3 : 1) * NPK; k++) part[k * 32] = make_float2(0.f, 0.f);
             }
             for (int hi = Kr - 1, first = 1;; hi -= 32, first = 0) {
                 const int nc = max(0, min(32, hi));
@@ -721,17 +727,17 @@ __device__ __forceinline__ void integrate_batch(const RFArgs &a, const RFShape &
                         // optical depth at unit profile in log2 units (ex2 takes
                         // it as is) and the source function.  A cell line with kv
                         // <= 0 fails ray_in's gate tau > 1e-30 in every channel
-                        // (inverse_rt.f90:308), and so does a padding line of the
-                        // last group: both get A = S = 0, which leaves I unchanged
-                        // exactly; 0 < tau < 2^-54 rounds to a zero weight as in
-                        // FP64, so the gate needs no test.
+                        // (inverse_rt.f90:308): A = S = 0 leaves I unchanged exactly;
+                        // 0 < tau < 2^-54 rounds to a zero weight as in FP64, so
+                        // the gate needs no test.  (The padding lines of a last group
+                        // repeat its last line; nothing reads their sums.)
                         float2 v[NLG];
 #pragma unroll
                         for (int l = 0; l < NLG; l++)
                             v[l] = *reinterpret_cast<const float2 *>(lt + min(l0 + l, L - 1));
 #pragma unroll
                         for (int l = 0; l < NLG; l++) {
-                            const bool on = v[l].x > 0.f && l0 + l < L;
+                            const bool on = v[l].x > 0.f;
                             v[l].x = on ? v[l].x * fst * LOG2E_F : 0.f;
                             v[l].y = on ? v[l].y : 0.f;
                             if (!(v[l].x < OM_THIN_A)) thin &= ~(1u << (l / 2));
@@ -747,9 +753,15 @@ __device__ __forceinline__ void integrate_batch(const RFArgs &a, const RFShape &
                             const float gr = ex2(-(q * q));
                             float *om = m.om(sh) + lane * sh.om_ld;
 #pragma unroll
-                            for (int l = 0; l < NLG; l++) {
-                                const float x = v[l].x * gr;
-                                om[l] = one_minus_exp(x, ex2(-x));
+                            for (int k = 0; k < NP; k++) {
+                                const float2 x = __fmul2_rn(make_float2(v[2 * k].x, v[2 * k + 1].x), make_float2(gr, gr));
+                                const float2 w = one_minus_exp2(x, ex2(-x.x), ex2(-x.y));
+                                om[2 * k] = w.x;
+                                om[2 * k + 1] = w.y;
+                            }
+                            if (ODD) {
+                                const float x = v[NLG - 1].x * gr;
+                                om[NLG - 1] = one_minus_exp(x, ex2(-x));
                             }
                         }
                     }
@@ -769,18 +781,20 @@ __device__ __forceinline__ void integrate_batch(const RFArgs &a, const RFShape &
                     for (int u = 0; u < nc; u++) Irem = fmaf(om[u * sh.om_ld], S[u * sh.rec_ld * 4] - Irem, Irem);
                 }
                 int s0 = 0;
-                for (; s0 + 1 < sh.nslot; s0 += 2)
-                    channel_pass<NLG, 2, DUST>(sh, m, chtab, nch, nvel, lane, g, s0, nc, tk, fast, first, last, bb,
-                                               fst0);
-                if (s0 < sh.nslot)
-                    channel_pass<NLG, 1, DUST>(sh, m, chtab, nch, nvel, lane, g, s0, nc, tk, fast, first, last, bb,
-                                               fst0);
+                if constexpr (SLOTS != 1)
+                    for (; s0 + 1 < sh.nslot; s0 += 2)
+                        channel_pass<NLG, 2, DUST, SPLIT>(sh, m, chtab, nch, nvel, lane, g, s0, nc, tk, fast, first,
+                                                          last, bb, fst0);
+                if constexpr (SLOTS != 2)
+                    if (s0 < sh.nslot)
+                        channel_pass<NLG, 1, DUST, SPLIT>(sh, m, chtab, nch, nvel, lane, g, s0, nc, tk, fast, first,
+                                                          last, bb, fst0);
                 if (last) break;
             }
             // the channel sums over the lanes, the remainder channel's share
             // added last
             const int line = l0 + sum_line<NLG>(lane);
-            for (int q = 0; q < (sh.split ? 3 : 1); q++) {
+            for (int q = 0; q < (split ? 3 : 1); q++) {
                 const float2 *part = m.part(sh) + q * NPK * 32 + lane;
                 float v[NLG];
 #pragma unroll
@@ -816,7 +830,7 @@ template <int NLG, bool DUST>
 __device__ __noinline__ void integrate_any_width(const RFArgs &a, const RFShape &sh, const WarpMem &m, const RayBatch &B,
                                         unsigned smask, const float2 *chtab, const int2 *walk, int nr, float dqfac,
                                         int lane) {
-    integrate_batch<NLG, DUST, true>(a, sh, m, B, smask, chtab, walk, nr, dqfac, lane);
+    integrate_batch<NLG, DUST, true, 0, true>(a, sh, m, B, smask, chtab, walk, nr, dqfac, lane);
 }
 
 // FP32 sums over rays, in ray order.
@@ -841,6 +855,12 @@ __device__ __forceinline__ float moment_add(float km, int k, float w, float v, f
 }
 
 // NLG: lines per group (0: the model's own, BATCH only).
+// SLOTS: 1 for layouts of one slot, 2 for an even number, 0 for any; SPLIT:
+// with the split field (when the launch asks for it).  What a layout cannot
+// need is left out: the size of the cell loops' code decides how well they
+// fetch (65,536 points x 129 channels without the one-slot pass and the split
+// sums: 318 -> 310 ms; 2,500 points x 33 channels without the two-slot pass:
+// 0.498 -> 0.455).
 // BATCH: the work items are (model, node) pairs of many models (RFBatch);
 // each warp copies the argument block of its current model into shared
 // memory.  Otherwise the nodes of the one model a0, or -- a0.rays_per_item >
@@ -848,7 +868,7 @@ __device__ __forceinline__ float moment_add(float km, int k, float w, float v, f
 // a warp per node, so each item is a part of a node's rays and stores their
 // per-line channel sums, which k_rf_finish adds up in ray order afterwards
 // (the same sums in the same order).
-template <int NLG, bool DUST, bool BATCH>
+template <int NLG, bool DUST, bool BATCH, int SLOTS, bool SPLIT>
 __global__ void __launch_bounds__(256, (NLG >= 1 && NLG <= 4) ? 3 : 2) k_radiation_field(RFArgs a0, RFBatch bw, RFShape sh0) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -946,7 +966,7 @@ __global__ void __launch_bounds__(256, (NLG >= 1 && NLG <= 4) ? 3 : 2) k_radiati
                     row[DUST ? 2 * i : i] = make_float4(v.x, w.x, v.y, w.y);
                     if (DUST) row[2 * i + 1] = make_float4(v.z, w.z, v.w, w.w);
                 }
-                for (int i = lane; i < (sh.split ? 8 : 4) * sh.L; i += 32) m.acc(sh)[i] = 0.f;
+                for (int i = lane; i < ((SPLIT && sh.split) ? 8 : 4) * sh.L; i += 32) m.acc(sh)[i] = 0.f;
             }
             __syncwarp();
             int n_rays = a.ndir;
@@ -1078,7 +1098,7 @@ __global__ void __launch_bounds__(256, (NLG >= 1 && NLG <= 4) ? 3 : 2) k_radiati
 
                 // ---- (3)+(4) channel integration of the batch's rays ----
                 if constexpr (NLG > 0) {
-                    integrate_batch<NLG, DUST, BATCH>(a, sh, m, B, smask, chtab, walk, nr, dqfac, lane);
+                    integrate_batch<NLG, DUST, BATCH, SLOTS, SPLIT>(a, sh, m, B, smask, chtab, walk, nr, dqfac, lane);
                 } else {
                     switch (sh.nlg) {
 #define RF_WIDTH(n)                                                                                        \
@@ -1100,7 +1120,7 @@ __global__ void __launch_bounds__(256, (NLG >= 1 && NLG <= 4) ? 3 : 2) k_radiati
                 const int L = sh.L;
                 if (rpi) {   // the rays' channel sums and directions for k_rf_finish
                     const size_t ray0 = (size_t)node * a.ndir + k0, plane = (size_t)a.bulk * a.ndir * L;
-                    for (int q = 0; q < (sh.split ? 3 : 1); q++)
+                    for (int q = 0; q < ((SPLIT && sh.split) ? 3 : 1); q++)
                         for (int i = lane; i < nr * L; i += 32) a.vray[q * plane + ray0 * L + i] = v[q * 32 * L + i];
                     if (lane < nr) a.dray[ray0 + lane] = B.dir[lane];
                 } else {
@@ -1110,7 +1130,7 @@ __global__ void __launch_bounds__(256, (NLG >= 1 && NLG <= 4) ? 3 : 2) k_radiati
                         s.j0.s = acc[0]; s.j0.c = acc[L]; s.j2.s = acc[2 * L]; s.j2.c = acc[3 * L];
                         for (int r = 0; r < nr; r++) s.add(B.wts[r], v[r * L + l]);
                         acc[0] = s.j0.s; acc[L] = s.j0.c; acc[2 * L] = s.j2.s; acc[3 * L] = s.j2.c;
-                        if (sh.split) {
+                        if ((SPLIT && sh.split)) {
                             s.je.s = acc[4 * L]; s.je.c = acc[5 * L]; s.ls.s = acc[6 * L]; s.ls.c = acc[7 * L];
                             for (int r = 0; r < nr; r++)
                                 s.add_split(B.wts[r].x, v[(32 + r) * L + l], v[(64 + r) * L + l]);
@@ -1139,7 +1159,7 @@ __global__ void __launch_bounds__(256, (NLG >= 1 && NLG <= 4) ? 3 : 2) k_radiati
             for (int l = lane; l < L; l += 32) {
                 a.J0[(size_t)node * L + l] = value(0, l);
                 a.J2[(size_t)node * L + l] = value(1, l);
-                if (sh.split) {
+                if ((SPLIT && sh.split)) {
                     a.JE[(size_t)node * L + l] = value(2, l);
                     a.LS[(size_t)node * L + l] = value(3, l);
                 }
