@@ -130,6 +130,8 @@ const void *rf_kernel_even(int nlg);               // an even number of slots
 const void *rf_kernel_even_split(int nlg);
 const void *rf_kernel_any(int nlg);                // any, split or not
 const void *rf_kernel_dust(int nlg, int slots);    // slots 1: one, 2: an even number, 0: any
+const void *rf_batch_even();                       // the batched kernel's instantiations
+const void *rf_batch_any(bool dust, bool one_slot, bool split);
 size_t rf_walk_records(int n_depth);     // walk scratch per warp, int2 records
 // the batched launch: its shape for these models (max_group: the widest line
 // group wanted), and the blocks per SM the kernel reaches with it

@@ -6,9 +6,11 @@
 
 namespace {
 
-const void *batch_kernel(bool dust) {
-    return dust ? (const void *)k_radiation_field<0, true, true, 0, true>
-                : (const void *)k_radiation_field<0, false, true, 0, true>;
+// (instantiations in rf_batch_even.cu and rf_batch_any.cu)
+const void *batch_kernel(const RFBatch &bw, bool dust) {
+    const int nslot = (bw.nch - bw.rt + 31) / 32;
+    if (!dust && !bw.split && nslot % 2 == 0) return rf_batch_even();
+    return rf_batch_any(dust, nslot == 1, bw.split);
 }
 
 size_t batch_dyn_smem(const RFBatch &bw) {
@@ -35,7 +37,7 @@ void rf_batch_shape(RFBatch *bw, const int *lines, int n_models, int nch, bool d
 // Also raises the kernel's dynamic shared-memory limit: called for every
 // candidate before the pass is captured.
 int rf_batch_blocks_per_sm(const RFBatch &bw, bool dust, int *blocks) {
-    const void *k = batch_kernel(dust);
+    const void *k = batch_kernel(bw, dust);
     const size_t dyn = batch_dyn_smem(bw);
     *blocks = 0;
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn) != cudaSuccess)
@@ -49,7 +51,7 @@ int rf_batch_launch(cudaStream_t s, int grid, bool dust, const RFBatch &bw) {
     RFBatch b = bw;
     RFShape sh{};
     void *args[] = {&a0, &b, &sh};
-    cudaError_t e = cudaLaunchKernel(batch_kernel(dust), dim3(grid), dim3(32 * RF_BATCH_WARPS), args,
+    cudaError_t e = cudaLaunchKernel(batch_kernel(bw, dust), dim3(grid), dim3(32 * RF_BATCH_WARPS), args,
                                      batch_dyn_smem(bw), s);
     return e == cudaSuccess ? PORTAL_OK : PORTAL_ERR_CUDA;
 }

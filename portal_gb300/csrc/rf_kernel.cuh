@@ -826,11 +826,11 @@ __device__ __forceinline__ void integrate_batch(const RFArgs &a, const RFShape &
 
 // integrate_batch for a run-time group width (the batched kernel: models of
 // any line count in one launch)
-template <int NLG, bool DUST>
+template <int NLG, bool DUST, int SLOTS, bool SPLIT>
 __device__ __noinline__ void integrate_any_width(const RFArgs &a, const RFShape &sh, const WarpMem &m, const RayBatch &B,
                                         unsigned smask, const float2 *chtab, const int2 *walk, int nr, float dqfac,
                                         int lane) {
-    integrate_batch<NLG, DUST, true, 0, true>(a, sh, m, B, smask, chtab, walk, nr, dqfac, lane);
+    integrate_batch<NLG, DUST, true, SLOTS, SPLIT>(a, sh, m, B, smask, chtab, walk, nr, dqfac, lane);
 }
 
 // FP32 sums over rays, in ray order.
@@ -1102,15 +1102,15 @@ __global__ void __launch_bounds__(256, (NLG >= 1 && NLG <= 4) ? 3 : 2) k_radiati
                 } else {
                     switch (sh.nlg) {
 #define RF_WIDTH(n)                                                                                        \
-    case n: integrate_any_width<n, DUST>(a, sh, m, B, smask, chtab, walk, nr, dqfac, lane); break;
+    case n: integrate_any_width<n, DUST, SLOTS, SPLIT>(a, sh, m, B, smask, chtab, walk, nr, dqfac, lane); break;
                         RF_WIDTH(1) RF_WIDTH(2) RF_WIDTH(3) RF_WIDTH(4)
                     default:
                         if constexpr (DUST) {
-                            integrate_any_width<5, DUST>(a, sh, m, B, smask, chtab, walk, nr, dqfac, lane);
+                            integrate_any_width<5, DUST, SLOTS, SPLIT>(a, sh, m, B, smask, chtab, walk, nr, dqfac, lane);
                         } else {
                             switch (sh.nlg) {
                                 RF_WIDTH(5) RF_WIDTH(6) RF_WIDTH(7) RF_WIDTH(8) RF_WIDTH(9)
-                            default: integrate_any_width<10, DUST>(a, sh, m, B, smask, chtab, walk, nr, dqfac, lane);
+                            default: integrate_any_width<10, DUST, SLOTS, SPLIT>(a, sh, m, B, smask, chtab, walk, nr, dqfac, lane);
                             }
                         }
                     }
