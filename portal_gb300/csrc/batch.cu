@@ -38,6 +38,7 @@ struct portal_batch {
     size_t se_wb = 0;
     size_t se_a64_stride = 0;           // largest model's matrix slot
     int se_max_dim = 0;                 // largest model's c_dim
+    bool se_gauss = true;               // every model's SE system is inverted
     DevBuf<double> se_a64;              // FP64 SE matrices, one per resident warp
     DevBuf<int2> walk;
     DevBuf<unsigned long long> queue;   // [0] next item, [1] segments
@@ -98,9 +99,9 @@ int enqueue_pass(portal_batch *b, const int2 *items, long long n_items) {
     if ((rc = rf_batch_launch(b->stream, b->rf_bps * b->sm_count, b->dust, rb)))
         return bfail(b, rc, "radiation-field launch failed");
     for (size_t m = 0; m < b->models.size(); m++)
-        if ((rc = se_pass(b->models[m], b->stream)))
+        if ((rc = se_batch_pass(b->models[m], b->stream)))
             return bfail(b, rc, "model " + std::to_string(m) + ": " + b->models[m]->err);
-    SEBatch sb{b->d_se.p, items, n_items, b->se_wb, b->se_a64.p, b->se_a64_stride, b->se_max_dim};
+    SEBatch sb{b->d_se.p, items, n_items, b->se_wb, b->se_a64.p, b->se_a64_stride, b->se_max_dim, b->se_gauss};
     if ((rc = se_batch_launch(b->stream, b->se_bps * b->sm_count, b->se_warps, sb)))
         return bfail(b, rc, "SE launch failed");
     return PORTAL_OK;
@@ -203,6 +204,17 @@ extern "C" int portal_batch_prepare(portal_batch *b, int nth, int nph, int nvel,
     b->nch = 2 * nvel + 1;
     b->n_depth = n_depth;
     b->kmax = kmax;
+    if (2 * wb > 200 * 1024) return bfail(b, PORTAL_ERR_ARG, "SE system too large for shared memory");
+    // every model's system inverted, where all can be at two warps a block
+    size_t gwb = 0;
+    b->se_gauss = true;
+    for (portal_ctx *c : b->models) {
+        b->se_gauss = b->se_gauss && se_gauss(c);
+        gwb = std::max(gwb, se_gauss_team_bytes(c));
+    }
+    b->se_gauss = b->se_gauss && 2 * gwb <= 200 * 1024;
+    const int team = se_batch_team(b->se_max_dim, b->se_gauss);
+    if (b->se_gauss) wb = gwb;
     b->se_wb = wb;
     // work items, models by descending cost per node
     std::vector<int> ord(M);
@@ -249,20 +261,19 @@ extern "C" int portal_batch_prepare(portal_batch *b, int nth, int nph, int nvel,
     if (raise_rf_limit()) return bfail(b, PORTAL_ERR_CUDA, "occupancy query");
     std::vector<int> sec;
     for (int w : {2, 4, 8})
-        if (wb * w <= 200 * 1024) sec.push_back(w);
-    if (sec.empty()) return bfail(b, PORTAL_ERR_ARG, "SE system too large for shared memory");
+        if (team > 1 ? w == team : wb * w <= 200 * 1024) sec.push_back(w);
     int dummy = 0;
-    if (se_batch_blocks_per_sm(sec.back(), wb, b->se_max_dim, &dummy))  // raises the smem limit to the largest candidate
+    if (se_batch_blocks_per_sm(sec.back(), wb, b->se_max_dim, b->se_gauss, &dummy))  // raises the smem limit to the largest candidate
         return bfail(b, PORTAL_ERR_CUDA, "SE occupancy query");
     // FP64 matrix slots for the largest SE grid among the candidates
     {
         size_t most = 0;
         for (int w : sec) {
             int bps = 0;
-            if (se_batch_blocks_per_sm(w, wb, b->se_max_dim, &bps)) return bfail(b, PORTAL_ERR_CUDA, "SE occupancy query");
+            if (se_batch_blocks_per_sm(w, wb, b->se_max_dim, b->se_gauss, &bps)) return bfail(b, PORTAL_ERR_CUDA, "SE occupancy query");
             most = std::max(most, (size_t)std::max(1, bps) * b->sm_count * w);
         }
-        se_batch_blocks_per_sm(sec.back(), wb, b->se_max_dim, &dummy);
+        se_batch_blocks_per_sm(sec.back(), wb, b->se_max_dim, b->se_gauss, &dummy);
         if (b->se_a64.reserve(most * b->se_a64_stride)) return bfail(b, PORTAL_ERR_NOMEM, "SE matrix scratch");
     }
     // walk scratch for the largest grid
@@ -286,22 +297,22 @@ extern "C" int portal_batch_prepare(portal_batch *b, int nth, int nph, int nvel,
         best = 1e300;
         for (int w : sec) {
             int bps = 0;
-            if (se_batch_blocks_per_sm(w, wb, b->se_max_dim, &bps)) return bfail(b, PORTAL_ERR_CUDA, "SE occupancy query");
+            if (se_batch_blocks_per_sm(w, wb, b->se_max_dim, b->se_gauss, &bps)) return bfail(b, PORTAL_ERR_CUDA, "SE occupancy query");
             bps = std::max(1, bps);
-            SEBatch sb{b->d_se.p, b->sample.p, b->n_sample, wb, b->se_a64.p, b->se_a64_stride, b->se_max_dim};
+            SEBatch sb{b->d_se.p, b->sample.p, b->n_sample, wb, b->se_a64.p, b->se_a64_stride, b->se_max_dim, b->se_gauss};
             double ms = 0.0;
             int rc = time_launch(b, [&]() { return se_batch_launch(b->stream, bps * b->sm_count, w, sb); }, &ms);
             if (rc) return rc;
             b->tune.insert(b->tune.end(), {(double)w, (double)bps, ms});
             if (ms < best) { best = ms; b->se_warps = w; b->se_bps = bps; }
         }
-        se_batch_blocks_per_sm(sec.back(), wb, b->se_max_dim, &dummy);
+        se_batch_blocks_per_sm(sec.back(), wb, b->se_max_dim, b->se_gauss, &dummy);
     } else {
         b->nlg = rfc[0].nlg;
         b->rf_bps = rfc[0].bps;
         b->se_warps = sec.back();
         int bps = 0;
-        se_batch_blocks_per_sm(b->se_warps, wb, b->se_max_dim, &bps);
+        se_batch_blocks_per_sm(b->se_warps, wb, b->se_max_dim, b->se_gauss, &bps);
         b->se_bps = std::max(1, bps);
     }
 

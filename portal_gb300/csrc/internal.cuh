@@ -79,10 +79,11 @@ struct SEArgs {
     const int *__restrict__ pack;       // (2 nlev) rho index or -1
     const int *__restrict__ row_off;    // (c_dim + 1) entries of each matrix row,
     const int *__restrict__ row_ent;    // ascending column (the rates' summation order)
-    const int4 *__restrict__ sp_rec;    // the matrix's entries row by row: (pos, first term, end, -1), row 1
-                                        // the normalisation's (pos, 0, 0, level)
-    const int *__restrict__ sp_off;     // (c_dim + 1) their row offsets,
+    const int4 *__restrict__ sp_rec;    // the matrix's entries, most terms first: (row | column << 16, first term,
+                                        // terms << 16 | entry, -1), row 1 the normalisation's (.., 0, entry, level)
+    const int *__restrict__ sp_off;     // (c_dim + 1) the entries' row offsets,
     const int *__restrict__ sp_col;     // columns
+    const unsigned short *__restrict__ sp_map;  // entry at each place, nnz: none (c_dim <= 96)
     int nnz;
     double *pops;                       // (N, 2 nlev) column-major
     double *jj20;                       // (N, L) or null
@@ -114,10 +115,11 @@ struct SEBatch {
     const SEArgs *models;
     const int2 *items;
     long long n_items;
-    size_t warp_bytes;           // dynamic shared memory per warp (largest model)
-    double *a64;                 // FP64 matrices, one slot of a64_stride doubles per warp
+    size_t team_bytes;           // dynamic shared memory per node solved (largest model)
+    double *a64;                 // FP64 matrices, one slot of a64_stride doubles per node solved
     size_t a64_stride;           // largest model's nnz + c_dim^2
     int max_dim;                 // largest model's c_dim
+    bool gauss;                  // every model's system is inverted
 };
 
 // rf.cu
@@ -141,9 +143,12 @@ int rf_batch_launch(cudaStream_t s, int grid, bool dust, const RFBatch &bw);
 constexpr int RF_BATCH_WARPS = 4;        // warps per block of the batched launch
 // se.cu
 int se_prepare(portal_ctx *c, int kmax, SEArgs *a, size_t *warp_bytes);
-int se_pass(portal_ctx *c, cudaStream_t s);
+int se_batch_pass(portal_ctx *c, cudaStream_t s);
 int se_batch_launch(cudaStream_t s, int grid, int warps_per_block, const SEBatch &bw);
-int se_batch_blocks_per_sm(int warps_per_block, size_t warp_bytes, int max_dim, int *blocks);
+int se_batch_blocks_per_sm(int warps_per_block, size_t team_bytes, int max_dim, bool gauss, int *blocks);
+bool se_gauss(const portal_ctx *c);            // the prepared system is inverted,
+size_t se_gauss_team_bytes(const portal_ctx *c);   // and its shared memory per node
+int se_batch_team(int max_dim, bool gauss);        // warps per node of the batched solve
 size_t se_matrix_doubles(const portal_ctx *c);  // matrix slot of the prepared SE program
 
 }  // namespace portal

@@ -22,13 +22,14 @@
 // rate equations), still linear in the populations.  At the fixed point
 // (S unchanged) both forms are the same equations.  The host turns setup_stateq's loops into that program once per
 // (molecule, kmax): a CSR list over matrix entries of (feature, coefficient)
-// terms.  The kernel (one warp per node, or a team of four warps for
-// systems of 48 or more unknowns) evaluates the features, assembles the
-// matrix (FP64, in an L2-resident slot per team), replaces row 1 by the normalisation
-// sum sqrt(2J+1) rho^0_0 = 1, factorises a row-scaled FP32 copy with partial
-// pivoting and refines the solution of A rho = e_1 with FP64 residuals.
-// Should the refinement stall (FP32 LU too inaccurate for the matrix's
-// condition) the node is refactorised in FP64 on the device and flagged.
+// terms.  The kernel (one warp per node or a team of four) evaluates the
+// features, assembles the matrix's entries (FP64), replaces row 1 by the
+// normalisation sum sqrt(2J+1) rho^0_0 = 1, inverts a row-scaled FP32 copy by
+// Gauss-Jordan elimination with partial pivoting (up to 96 unknowns; above,
+// FP32 LU factors) and refines the solution of A rho = e_1 with FP64
+// residuals.  Should the refinement stall (FP32 too inaccurate for the
+// matrix's condition) the node is factorised in FP64 on the device and
+// flagged.
 //
 // Depolarising collisions (portal_set_depolarization; off by default, as
 // main_sub.f90:96 passes D0 = 0): setup_stateq's col_dep slot
@@ -42,6 +43,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
+#include <cstring>
 #include <map>
 
 #include "internal.cuh"
@@ -57,11 +59,6 @@ namespace {
 
 constexpr double A_TO_B = 6.781962e49;  // pop_eqs.f90:419
 constexpr double HK = 4.79924e-11;      // pop_eqs.f90:535
-
-__device__ __forceinline__ double warp_max(double v) {
-    for (int o = 16; o >= 1; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
 
 // In-place LU with partial pivoting of the n x n column-major matrix M
 // (pivot: the first row of largest modulus, as LAPACK's IDAMAX picks).
@@ -242,6 +239,8 @@ __device__ bool team_lu(int n, T *M, int *piv, int tid, double *red_v, int *red_
 // per-team slot of global memory, followed by the dense matrix of the FP64
 // fallback: kept out of shared memory they let 3x more warps share an SM.
 constexpr int NF = 7;  // features per transition
+constexpr int SE_GAUSS_DIM = 96;   // largest system inverted,
+constexpr int SE_WARP_DIM = 32;    // and by one warp in registers
 
 __host__ __device__ inline size_t se_warp_bytes(int n, int n_feat) {
     size_t b = 0;
@@ -251,26 +250,330 @@ __host__ __device__ inline size_t se_warp_bytes(int n, int n_feat) {
     return (b + 15) & ~(size_t)15;
 }
 
-// A team of TW warps per node.  TW = 1: every warp of the block is a team
-// (the systems of up to ~50 unknowns); TW > 1: the block is one team, whose
-// warps share the factorisation's pivot search, row operations and trailing
-// updates, the FP64 residuals, the assembly and the packing (larger
-// systems, whose one-warp solve is latency-bound at a few warps per SM).
-// The triangular solves of the refinement run on the team's first warp.
-// BATCH (TW = 1 only): the work items are (model, node) pairs of many models
-// (SEBatch); each warp copies its current model's argument block into shared
-// memory, and the dynamic shared memory per warp fits the largest model.
+// ---- FP32 inverse by Gauss-Jordan elimination ------------------------------
+//
+// Step k turns column k of the remaining system into the inverse's: with p the
+// pivot row (of largest modulus to 16 bits among the rows not yet used, the
+// first of those; rows stay where they are), d = 1 / a_pk and s_j = a_pj d
+// (s_k = d),
+//     a_ij <- a_ij - a_ik s_j  (a_ik <- -a_ik d),   a_pj <- s_j.
+// After the n steps row p_k of a yields x_k from z_j = r_(p_j): a correction of
+// the refinement is one product with a, of independent fused multiply-adds,
+// where triangular solves are two chains of n dependent steps (they were 43 %
+// of the 74 x 74 systems' time, at 320 cycles a step).
+//
+// The matrix lives in registers: row i in lane i % 32 (register m = i / 32),
+// column j in warp j % TW (slot c = j / TW).  The pivot column's slot must be
+// a compile-time register, so the slots turn: after every ROT columns of this
+// warp the array moves down by ROT, the used columns going to the end of the
+// slots in use.  The pivot row goes through shared memory once a step.  A step
+// is a chain (search, reciprocal, row, update) of a few hundred cycles: every
+// slot is worked on without a test (branches a group of slots made it twice as
+// long), so the instances hold the next larger number of slots.
+// Measured, LU -> this (with the assembly in order of terms and the work of
+// the temperature once a node): 8,192 systems of 74 unknowns 2.29 -> 0.95 ms,
+// 8,192 of 39 1.51 -> 0.44 ms, 1,024 of 14 72 -> 29 us.  Of the 74 x 74
+// systems' time two thirds are the elimination (issue slots: 60 multiply-adds
+// in some 200 instructions a warp and step), the rest FP64 work.
+//
+// Every form below (one warp or four, registers or shared memory) does the
+// same operations per element, so that their inverses are the same.
+
+// The pivot row of a column over the rows not done (warp-wide), and the
+// reciprocal of its element (0, and not ok, where it is 0, denormal or NaN).
+template <int MR>
+__device__ __forceinline__ int pivot_row(const float (&col)[MR], unsigned done, int lane, float *recip, bool *ok) {
+    unsigned key = 0;
+    float v = 0.f;
+#pragma unroll
+    for (int m = 0; m < MR; m++) {
+        const unsigned bits = __float_as_uint(col[m]) & 0x7fffffffu;
+        // ordered by modulus, then the first row; a NaN below every number
+        const unsigned q = (bits > 0x7f800000u ? 0u : bits & ~127u) | (127u - (unsigned)(lane + 32 * m));
+        if (!(done >> m & 1) && q > key) { key = q; v = col[m]; }
+    }
+    const unsigned top = __reduce_max_sync(0xffffffffu, key);
+    const bool good = (key & ~127u) >= 0x00800000u;
+    const float d = __shfl_sync(0xffffffffu, good ? rcp_approx(v) : 0.f, (127 - (int)(top & 127u)) & 31);
+    if (top < 0x00800000u) *ok = false;
+    *recip = d;
+    return 127 - (int)(top & 127u);
+}
+
+// One step's work of a warp on its slots: the pivot row's lane stages the
+// scaled row and clears it (its update, with the multiplier -1, leaves the
+// scaled row), then every lane updates its rows.  own_slot holds the pivot
+// column, if this warp does (zero by then).
+// The row's register is chosen by a branch per register; the markers keep the
+// compiler from merging the branches into one that indexes the registers at
+// run time, which would put the matrix into local memory.
+template <int M, int MR, int NC>
+__device__ __forceinline__ void stage_row_of(float (&a)[NC][MR], float (&l)[MR], int pm, float d, int own_slot,
+                                             float *row, unsigned &done) {
+    if (pm == M) {
+        asm volatile("// pivot row in register %0" ::"n"(M));
+#pragma unroll
+        for (int g = 0; g < NC; g += 4) {
+            float4 s = make_float4(a[g][M] * d, a[g + 1][M] * d, a[g + 2][M] * d, a[g + 3][M] * d);
+            if (g == 0) {
+                if (own_slot == 0) s.x = d;
+                if (own_slot == 1) s.y = d;
+                if (own_slot == 2) s.z = d;
+                if (own_slot == 3) s.w = d;
+            }
+            *reinterpret_cast<float4 *>(row + g) = s;
+            a[g][M] = a[g + 1][M] = a[g + 2][M] = a[g + 3][M] = 0.f;
+        }
+        l[M] = -1.f;
+        done |= 1u << M;
+        asm volatile("// staged %0" ::"n"(M));
+    }
+}
+template <int MR, int NC>
+__device__ __forceinline__ void stage_row(float (&a)[NC][MR], float (&l)[MR], int p, float d, int own_slot,
+                                          float *row, int lane, unsigned &done) {
+    if (lane != (p & 31)) return;
+    stage_row_of<0, MR, NC>(a, l, p >> 5, d, own_slot, row, done);
+    if constexpr (MR > 1) stage_row_of<1, MR, NC>(a, l, p >> 5, d, own_slot, row, done);
+    if constexpr (MR > 2) stage_row_of<2, MR, NC>(a, l, p >> 5, d, own_slot, row, done);
+}
+template <int MR, int NC>
+__device__ __forceinline__ void update_group(float (&a)[NC][MR], const float (&l)[MR], const float *row, int g) {
+    const float4 s = *reinterpret_cast<const float4 *>(row + g);
+#pragma unroll
+    for (int m = 0; m < MR; m++) {
+        a[g][m] = fmaf(-l[m], s.x, a[g][m]);
+        a[g + 1][m] = fmaf(-l[m], s.y, a[g + 1][m]);
+        a[g + 2][m] = fmaf(-l[m], s.z, a[g + 2][m]);
+        a[g + 3][m] = fmaf(-l[m], s.w, a[g + 3][m]);
+    }
+}
+// slots [0, na) turn by R (na a multiple of R)
+template <int MR, int NC, int R>
+__device__ __forceinline__ void turn_slots(float (&a)[NC][MR], int na) {
+    float t[R][MR];
+#pragma unroll
+    for (int q = 0; q < R; q++)
+#pragma unroll
+        for (int m = 0; m < MR; m++) t[q][m] = a[q][m];
+#pragma unroll
+    for (int c = 0; c < NC; c += R)
+#pragma unroll
+        for (int q = 0; q < R; q++)
+#pragma unroll
+            for (int m = 0; m < MR; m++) {
+                const float next = c + R + q < NC ? a[(c + R + q) % NC][m] : 0.f;
+                a[c + q][m] = c + R == na ? t[q][m] : next;
+            }
+}
+
+// Shared memory of a team (see se_gauss_bytes).
+struct GaussMem {
+    float *row;    // [8 nq] staged pivot rows, two per warp
+    float *z;      // [4 nq] permuted residual
+    double *feat, *x, *r, *val;
+    float *valf;   // [nnz + 1] scaled entries, 0
+    float *scl;    // [n]
+    float *part;   // [4 n] partial products
+    float *lcol;   // [2][n32] published pivot columns
+    float *pd;     // [2][4] pivot row, 1 / pivot, ok
+    int *rmax, *kof;
+    float *dense;  // [n n] the inverse of the shared-memory form
+};
+// columns a warp of four holds in an instance (a quarter of them all), which
+// sizes its staged rows
+template <int TW, int NC>
+constexpr int gauss_quads = NC == 0 ? SE_GAUSS_DIM / 4 : NC * TW / 4;
+__host__ __device__ inline size_t se_gauss_bytes(int n, int n_feat, int nnz, int nq, bool dense) {
+    size_t b = sizeof(float) * 12 * (size_t)nq;
+    b += sizeof(double) * ((size_t)n_feat + 2 * (size_t)n + (size_t)nnz);
+    b += sizeof(float) * ((size_t)nnz + 1 + 7 * (size_t)n + 2 * (size_t)((n + 31) & ~31) + 8);
+    if (dense) b += sizeof(float) * (size_t)n * n;
+    return (b + 15) & ~(size_t)15;
+}
+__device__ __forceinline__ GaussMem gauss_mem(unsigned char *base, int n, int n_feat, int nnz, int nq) {
+    GaussMem g;
+    g.row = (float *)base;
+    g.z = g.row + 8 * nq;
+    g.feat = (double *)(g.z + 4 * nq);
+    g.x = g.feat + n_feat;
+    g.r = g.x + n;
+    g.val = g.r + n;
+    g.valf = (float *)(g.val + nnz);
+    g.scl = g.valf + nnz + 1;
+    g.part = g.scl + n;
+    g.lcol = g.part + 4 * n;
+    g.pd = g.lcol + 2 * ((n + 31) & ~31);
+    g.rmax = (int *)(g.pd + 8);
+    g.kof = g.rmax + n;
+    g.dense = (float *)(g.kof + n);
+    return g;
+}
+
+// The elimination in registers; kof[p] = k.  False where a pivot was 0 or NaN.
+template <int TW, int MR, int NC>
+__device__ __forceinline__ bool gauss_registers(int n, float (&a)[NC][MR], const GaussMem &g, int lane, int w) {
+    constexpr int nq = gauss_quads<TW, NC>;
+    unsigned done = 0;
+#pragma unroll
+    for (int m = 0; m < MR; m++)
+        if (lane + 32 * m >= n) done |= 1u << m;
+    bool ok = true;
+    if constexpr (TW == 1) {
+        const int na = (n + 3) & ~3;
+        float *buf = g.row;
+        for (int k0 = 0; k0 < n; k0 += 4) {
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const int k = k0 + q;
+                if (k < n) {
+                    float l[MR], d;
+                    const int p = pivot_row<MR>(a[q], done, lane, &d, &ok);
+#pragma unroll
+                    for (int m = 0; m < MR; m++) { l[m] = a[q][m]; a[q][m] = 0.f; }
+                    float *row = buf + (k & 1) * 4 * nq;
+                    if (lane == (p & 31)) g.kof[p] = k;
+                    stage_row<MR, NC>(a, l, p, d, q, row, lane, done);
+                    __syncwarp();
+#pragma unroll
+                    for (int c = 0; c < NC; c += 4) update_group<MR, NC>(a, l, row, c);
+                }
+            }
+            turn_slots<MR, NC, 4>(a, na);
+        }
+        __syncwarp();
+    } else {
+        const int na = (n + TW - 1) / TW, n32 = (n + 31) & ~31;
+        auto publish = [&](const float (&col)[MR], int b) {
+            float d;
+            bool good = true;
+            const int p = pivot_row<MR>(col, done, lane, &d, &good);
+#pragma unroll
+            for (int m = 0; m < MR; m++)
+                if (32 * m < n32) g.lcol[b * n32 + lane + 32 * m] = col[m];
+            if (lane == 0) {
+                g.pd[4 * b] = __int_as_float(p);
+                g.pd[4 * b + 1] = d;
+                g.pd[4 * b + 2] = good ? 1.f : 0.f;
+            }
+        };
+        if (w == 0) publish(a[0], 0);
+        for (int c0 = 0; c0 < na; c0++) {
+            for (int q = 0; q < TW; q++) {
+                const int k = TW * c0 + q;
+                if (k >= n) break;
+                // the pivot column of step k is published; the other buffer's
+                // readers (step k - 1) are done
+                __syncthreads();
+                const int b = k & 1;
+                const int p = __float_as_int(g.pd[4 * b]);
+                const float d = g.pd[4 * b + 1];
+                if (g.pd[4 * b + 2] == 0.f) ok = false;
+                float l[MR];
+#pragma unroll
+                for (int m = 0; m < MR; m++) l[m] = (32 * m < n32) ? g.lcol[b * n32 + lane + 32 * m] : 0.f;
+                if (w == q)
+#pragma unroll
+                    for (int m = 0; m < MR; m++) a[0][m] = 0.f;
+                float *row = g.row + (2 * w + b) * nq;
+                if (w == 0 && lane == 0) g.kof[p] = k;
+                stage_row<MR, NC>(a, l, p, d, w == q ? 0 : -1, row, lane, done);
+                __syncwarp();
+                update_group<MR, NC>(a, l, row, 0);
+                // the next pivot column first, so that its search overlaps the
+                // other warps' updates
+                if (k + 1 < n && w == (q + 1) % TW) {
+                    float col[MR];
+#pragma unroll
+                    for (int m = 0; m < MR; m++) col[m] = (q == TW - 1) ? a[1][m] : a[0][m];
+                    publish(col, b ^ 1);
+                }
+#pragma unroll
+                for (int c = 4; c < NC; c += 4) update_group<MR, NC>(a, l, row, c);
+            }
+            turn_slots<MR, NC, 1>(a, na);
+        }
+        __syncthreads();
+    }
+    return ok;
+}
+
+// The elimination in shared memory, one warp (systems its registers cannot
+// hold).  a is column-major; row [4 quads] stages the pivot row.
+template <int MR>
+__device__ bool gauss_shared(int n, float *a, float *row, int *kof, int lane) {
+    unsigned done = 0;
+#pragma unroll
+    for (int m = 0; m < MR; m++)
+        if (lane + 32 * m >= n) done |= 1u << m;
+    bool ok = true;
+    for (int k = 0; k < n; k++) {
+        float l[MR], d;
+#pragma unroll
+        for (int m = 0; m < MR; m++) {
+            const int i = lane + 32 * m;
+            l[m] = (i < n) ? a[i + n * k] : 0.f;
+            if (i < n) a[i + n * k] = 0.f;
+        }
+        const int p = pivot_row<MR>(l, done, lane, &d, &ok);
+        if (lane == (p & 31)) {
+            kof[p] = k;
+            done |= 1u << (p >> 5);
+        }
+        __syncwarp();
+        for (int j = lane; j < n; j += 32) {
+            row[j] = (j == k) ? d : a[p + n * j] * d;
+            a[p + n * j] = 0.f;
+        }
+#pragma unroll
+        for (int m = 0; m < MR; m++)
+            if (lane + 32 * m == p) l[m] = -1.f;
+        __syncwarp();
+#pragma unroll
+        for (int m = 0; m < MR; m++) {
+            float *ai = a + lane + 32 * m;
+            if (lane + 32 * m >= n) break;
+            int j = 0;
+            for (; j + 3 < n; j += 4) {
+                const float a0 = ai[n * j], a1 = ai[n * (j + 1)], a2 = ai[n * (j + 2)], a3 = ai[n * (j + 3)];
+                const float4 s = *reinterpret_cast<const float4 *>(row + j);
+                ai[n * j] = fmaf(-l[m], s.x, a0);
+                ai[n * (j + 1)] = fmaf(-l[m], s.y, a1);
+                ai[n * (j + 2)] = fmaf(-l[m], s.z, a2);
+                ai[n * (j + 3)] = fmaf(-l[m], s.w, a3);
+            }
+            for (; j < n; j++) ai[n * j] = fmaf(-l[m], row[j], ai[n * j]);
+        }
+        __syncwarp();
+    }
+    return ok;
+}
+
+// A team of TW warps per node.  TW = 1: every warp of the block is a team;
+// TW > 1: the block is one team.
+// BATCH: the work items are (model, node) pairs of many models (SEBatch); each
+// team copies its current model's argument block into shared memory, and the
+// dynamic shared memory per team fits the largest model.
 // Otherwise the nodes of the one model a0.
-// MR: rows per lane of the triangular solves and the team factorisation
-// (c_dim <= 32 MR).
-template <int TW, bool BATCH, int MR>
-__global__ void __launch_bounds__(TW == 1 ? 256 : 32 * TW, TW == 1 ? 3 : 24 / TW) k_solve_se(SEArgs a0, SEBatch bw) {
-    static_assert(TW == 1 || !BATCH, "teams of several warps run the single-model kernel");
+// NC >= 0: the inverse by Gauss-Jordan elimination, in registers (NC slots of
+// MR rows a lane) or, NC = 0, in shared memory.  NC = -1: LU factors of up to
+// 32 MR rows in shared memory, the triangular solves on the team's first warp.
+// Blocks per SM: what the matrix's registers leave room for.
+template <int TW, int MR, int NC>
+constexpr int se_min_blocks() {
+    return NC < 0 ? (TW == 1 ? 3 : 24 / TW) : TW == 1 ? 3 : MR * NC > 64 ? 4 : MR * NC > 32 ? 5 : 8;
+}
+template <int TW, bool BATCH, int MR, int NC>
+__global__ void __launch_bounds__(TW == 1 ? 256 : 32 * TW, se_min_blocks<TW, MR, NC>()) k_solve_se(SEArgs a0, SEBatch bw) {
+    static_assert(TW == 1 || NC != 0, "the shared-memory elimination is one warp's");
+    constexpr bool GAUSS = NC >= 0;
+    constexpr int nq = GAUSS ? gauss_quads<TW, NC> : 0;
     constexpr int TS = 32 * TW;   // threads per team
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ SEArgs margs[BATCH ? 8 : 1];
+    __shared__ SEArgs margs[BATCH && TW == 1 ? 8 : 1];
     __shared__ double red_v[TW];  // cross-warp reductions of a team
     __shared__ int red_i[TW];
+    __shared__ unsigned red_k[2 * TW];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int tid = (TW == 1) ? lane : (int)threadIdx.x;    // thread within the team
     const int teams = (TW == 1) ? (int)(blockDim.x >> 5) : 1;
@@ -279,32 +582,38 @@ __global__ void __launch_bounds__(TW == 1 ? 256 : 32 * TW, TW == 1 ? 3 : 24 / TW
         if constexpr (TW == 1) __syncwarp();
         else __syncthreads();
     };
-    auto team_max = [&](double v) {
-        v = warp_max(v);
+    // the largest of two keys each over the team
+    auto team_max2 = [&](unsigned &k0, unsigned &k1) {
+        k0 = __reduce_max_sync(0xffffffffu, k0);
+        k1 = __reduce_max_sync(0xffffffffu, k1);
         if constexpr (TW > 1) {
-            if (lane == 0) red_v[wib] = v;
+            if (lane == 0) { red_k[2 * wib] = k0; red_k[2 * wib + 1] = k1; }
             __syncthreads();
-            v = red_v[0];
-            for (int q = 1; q < TW; q++) v = fmax(v, red_v[q]);
-            __syncthreads();
+#pragma unroll
+            for (int q = 0; q < TW; q++) {
+                k0 = max(k0, red_k[2 * q]);
+                k1 = max(k1, red_k[2 * q + 1]);
+            }
         }
-        return v;
     };
     const long long n_items = BATCH ? bw.n_items : (long long)a0.bulk;
-    const size_t wbytes = BATCH ? bw.warp_bytes : se_warp_bytes(a0.c_dim, a0.n_feat);
+    const size_t wbytes = BATCH   ? bw.team_bytes
+                          : GAUSS ? se_gauss_bytes(a0.c_dim, a0.n_feat, a0.nnz, nq, NC == 0)
+                                  : se_warp_bytes(a0.c_dim, a0.n_feat);
     unsigned char *base = smem + wbytes * team;
-    double *const val = (BATCH ? bw.a64 : a0.a64) +
-                        (size_t)((long long)blockIdx.x * teams + team) * (BATCH ? bw.a64_stride : a0.a64_stride);
+    double *const slot = (BATCH ? bw.a64 : a0.a64) +
+                         (size_t)((long long)blockIdx.x * teams + team) * (BATCH ? bw.a64_stride : a0.a64_stride);
     int cur_model = -1;
 
-    for (long long item = (long long)blockIdx.x * teams + team; item < n_items; item += (long long)gridDim.x * teams) {
+    // (nodes go to the blocks in turn, so that few nodes spread over the SMs)
+    for (long long item = (long long)team * gridDim.x + blockIdx.x; item < n_items; item += (long long)gridDim.x * teams) {
         int node;
         if (BATCH) {
             const int2 wi = bw.items[item];
             if (wi.x != cur_model) {
                 tsync();
                 const int *src = reinterpret_cast<const int *>(bw.models + wi.x);
-                int *dst = reinterpret_cast<int *>(&margs[wib]);
+                int *dst = reinterpret_cast<int *>(&margs[team]);
                 for (int k = tid; k < (int)(sizeof(SEArgs) / sizeof(int)); k += TS) dst[k] = src[k];
                 tsync();
                 cur_model = wi.x;
@@ -313,54 +622,75 @@ __global__ void __launch_bounds__(TW == 1 ? 256 : 32 * TW, TW == 1 ? 3 : 24 / TW
         } else {
             node = (int)item;
         }
-        const SEArgs &a = BATCH ? margs[wib] : a0;
+        const SEArgs &a = BATCH ? margs[team] : a0;
         const int n = a.c_dim;
-        double *feat = (double *)base;
-        double *x = feat + (size_t)a.n_feat;
+        const GaussMem gm = GAUSS ? gauss_mem(base, n, a.n_feat, a.nnz, nq) : GaussMem{};
+        double *feat = GAUSS ? gm.feat : (double *)base;
+        double *x = GAUSS ? gm.x : feat + (size_t)a.n_feat;
         double *r = x + n;   // scratch (the rates)
+        double *val = GAUSS ? gm.val : slot;
         float *LU = (float *)(r + n);
         float *d32 = LU + (size_t)n * n;
-        float *scl = d32 + n;
-        int *piv = (int *)(scl + n);
-        if (!(a.ab[node] > 0.0)) continue;  // main_para.f90:213 (pops stay 0)
+        float *scl = GAUSS ? gm.scl : d32 + n;
+        int *piv = GAUSS ? gm.kof : (int *)(scl + n);
+        if (!(a.ab[node] > 0.0)) {  // main_para.f90:213 (pops and alignments stay 0)
+            if (!BATCH) {
+                for (int c2 = tid; c2 < 2 * a.nlev; c2 += TS) a.pops[(size_t)node + (size_t)a.N * c2] = 0.0;
+                for (int l = tid; l < a.L; l += TS) a.jj20[(size_t)node + (size_t)a.N * l] = 0.0;
+            }
+            continue;
+        }
         const double T = a.tkin[node], nH2 = a.h2[node];
         // ---- features (make_AC miscellaneous.f90:331-390) ----
+        // What depends on the temperature alone once per node: an FP64
+        // instruction of a warp takes the SM 16 cycles.
+        // Temperature interpolation (first bracket; below the table the first
+        // bracket extrapolates, as the reference's loop does)
+        int ib = 0;   // the first i >= 1 with col_temps[i] > T, 0: none
+        for (int i0 = 1; i0 < a.c_temp && !ib; i0 += 32) {
+            const unsigned above = __ballot_sync(0xffffffffu, i0 + lane < a.c_temp && a.col_temps[i0 + lane] > T);
+            if (above) ib = i0 + __ffs(above) - 1;
+        }
+        double ddT = 0.0;
+        if (ib) ddT = (T - a.col_temps[ib - 1]) / (a.col_temps[ib] - a.col_temps[ib - 1]);
+        const bool below = a.c_temp > 0 && T <= a.col_temps[0];
+        const double rT = 1.0 / T;
+        if constexpr (GAUSS)
+            for (int i = tid; i < n; i += TS) gm.rmax[i] = 0;
         for (int t = tid; t < a.n_trans; t += TS) {
             const int rr = a.tr_rad[t], cc = a.tr_col[t];
-            const double B21 = a.tr_B21[t];
-            double j0 = 0.0, j2 = 0.0, je = 0.0, ls = 0.0, C21 = 0.0;
+            const double B21 = a.tr_B21[t], A21 = a.tr_A[t];
+            double f0 = 0.0, f1 = 0.0, f5 = 0.0, f6 = A21, C21 = 0.0;
             if (rr >= 0) {
-                j0 = a.J0[(size_t)node * a.L + rr];
-                j2 = a.J2[(size_t)node * a.L + rr];
-                je = a.JE ? a.JE[(size_t)node * a.L + rr] : j0;
-                ls = a.LS ? a.LS[(size_t)node * a.L + rr] : 0.0;
+                f0 = B21 * a.J0[(size_t)node * a.L + rr];
+                f1 = B21 * a.J2[(size_t)node * a.L + rr];
+                f5 = a.JE ? B21 * a.JE[(size_t)node * a.L + rr] : f0;
+                if (a.LS) f6 = A21 * (1.0 - a.LS[(size_t)node * a.L + rr]);
             }
             if (cc >= 0) {
-                // temperature interpolation (first bracket; below the table the
-                // first bracket extrapolates, as the reference's loop does)
                 const int nT = a.c_temp;
                 double cr = 0.0;
                 for (int p = 0; p < a.c_par; p++) {
                     const double *Ct = a.Cji + (size_t)nT * (cc + (size_t)a.c_num * p);
-                    double v = (T <= a.col_temps[0]) ? Ct[0] : 0.0;
-                    for (int i = 1; i < nT; i++)
-                        if (a.col_temps[i] > T) {
-                            const double ddT = (T - a.col_temps[i - 1]) / (a.col_temps[i] - a.col_temps[i - 1]);
-                            v = Ct[i - 1] + ddT * (Ct[i] - Ct[i - 1]);
-                            break;
-                        }
+                    double v = below ? Ct[0] : 0.0;
+                    if (ib) v = Ct[ib - 1] + ddT * (Ct[ib] - Ct[ib - 1]);
                     cr += (a.c_par == 2 ? (p == 0 ? 0.25 : 0.75) : 1.0) * v;
                 }
                 C21 = cr * nH2 * 1e-6;
             }
+            // -h nu / k T: the product with 1 / T, one step of the remainder
+            const double hn = -HK * a.tr_nu[t];
+            double e = hn * rT;
+            const double rem = fma(-e, T, hn);
+            if (rem - rem == 0.0) e = fma(rem, rT, e);
             double *f = feat + NF * (size_t)t;
-            f[0] = B21 * j0;
-            f[1] = B21 * j2;
-            f[2] = a.tr_A[t];
+            f[0] = f0;
+            f[1] = f1;
+            f[2] = A21;
             f[3] = C21;
-            f[4] = C21 * exp(-HK * a.tr_nu[t] / T);
-            f[5] = B21 * je;
-            f[6] = a.tr_A[t] * (1.0 - ls);
+            f[4] = C21 * exp(e);
+            f[5] = f5;
+            f[6] = f6;
         }
         if (a.depol) {
             // make_depolarization_temp: every bracket with col_temps(i) > T
@@ -382,12 +712,14 @@ __global__ void __launch_bounds__(TW == 1 ? 256 : 32 * TW, TW == 1 ? 3 : 24 / TW
                 if (a.depol == 2) feat[NF * (size_t)a.n_trans + a.n_dep + d] = v;
             }
         }
-        if (!a.fp64_only)
-            for (int i = tid; i < n * n; i += TS) LU[i] = 0.f;
+        if constexpr (!GAUSS)
+            if (!a.fp64_only)
+                for (int i = tid; i < n * n; i += TS) LU[i] = 0.f;
         tsync();
         // ---- assembly (setup_stateq), row 1 replaced by the normalisation
-        // (em_coefs.f90:158-164): four records per thread in flight; each
-        // entry's terms summed in program order
+        // (em_coefs.f90:158-164): the entries with the most terms first, so
+        // that the lanes of a warp have equally many; four records per thread
+        // in flight; each entry's terms summed in program order
         for (int e0 = tid; e0 < a.nnz; e0 += 4 * TS) {
             int4 rec[4];
 #pragma unroll
@@ -400,71 +732,233 @@ __global__ void __launch_bounds__(TW == 1 ? 256 : 32 * TW, TW == 1 ? 3 : 24 / TW
                 if (rec[u].x < 0) continue;
                 double v = 0.0;
                 if (rec[u].w >= 0) v = a.norm_val[rec[u].w];
-                else
-                    for (int q = rec[u].y; q < rec[u].z; q++) v = fma(a.term_c[q], feat[a.term_f[q]], v);
-                val[e0 + u * TS] = v;
+                else {
+                    const int q1 = rec[u].y + (int)((unsigned)rec[u].z >> 16);
+                    int q = rec[u].y;
+                    for (; q + 3 < q1; q += 4) {
+                        const double c0 = a.term_c[q], c1 = a.term_c[q + 1], c2 = a.term_c[q + 2], c3 = a.term_c[q + 3];
+                        const int f0 = a.term_f[q], f1 = a.term_f[q + 1], f2 = a.term_f[q + 2], f3 = a.term_f[q + 3];
+                        v = fma(c0, feat[f0], v);
+                        v = fma(c1, feat[f1], v);
+                        v = fma(c2, feat[f2], v);
+                        v = fma(c3, feat[f3], v);
+                    }
+                    for (; q < q1; q++) v = fma(a.term_c[q], feat[a.term_f[q]], v);
+                }
+                val[rec[u].z & 0xffff] = v;
+                if constexpr (GAUSS)
+                    if (v == v) atomicMax(&gm.rmax[rec[u].x & 0xffff], __double2hiint(v) & 0x7fffffff);
             }
         }
         tsync();
-        // ---- FP32 LU of the row-scaled matrix (skipped in FP64 mode) ----
         int st = 0;
         bool ok = false, conv = false;
-        if (!a.fp64_only) {
-            for (int i = tid; i < n; i += TS) {
-                double m = 0.0;
-                for (int q = a.sp_off[i]; q < a.sp_off[i + 1]; q++) m = fmax(m, fabs(val[q]));
-                const float sc = (m > 0.0) ? (float)(1.0 / m) : 1.f;
-                scl[i] = sc;
-                for (int q = a.sp_off[i]; q < a.sp_off[i + 1]; q++)
-                    LU[i + (size_t)n * a.sp_col[q]] = (float)(val[q] * (double)sc);
-            }
-            tsync();
-            ok = team_lu<float, TW, MR>(n, LU, piv, tid, red_v, red_i);
-        }
-        if (ok) {
-            for (int i = tid; i < n; i += TS) x[i] = 0.0;
-            tsync();
-            double xmax = 0.0, dprev = 1e300;
-            for (int it = 0; it < 10; it++) {
-                // r = e_1 - A x (FP64)
+        if constexpr (GAUSS) {
+            // ---- FP32 inverse of the matrix, its rows scaled by powers of two
+            // to a largest modulus in [1, 2) ----
+            float m[NC > 0 ? NC : 1][MR];
+            if (!a.fp64_only) {
                 for (int i = tid; i < n; i += TS) {
-                    double s = (i == 0) ? 1.0 : 0.0, s1 = 0.0;   // two chains of dependent FP64 sums
-                    int q = a.sp_off[i];
-                    const int q1 = a.sp_off[i + 1];
-                    for (; q + 1 < q1; q += 2) {
-                        s -= val[q] * x[a.sp_col[q]];
-                        s1 -= val[q + 1] * x[a.sp_col[q + 1]];
+                    const int e = gm.rmax[i] >> 20;
+                    scl[i] = e == 0 ? 1.f : e >= 2046 ? 0.f : (float)__hiloint2double((2046 - e) << 20, 0);
+                }
+                for (int q = tid; q < a.nnz; q += TS) {
+                    const int4 rec = a.sp_rec[q];
+                    const int e = gm.rmax[rec.x & 0xffff] >> 20, dst = rec.z & 0xffff;
+                    const double sc = e == 0 ? 1.0 : e >= 2046 ? 0.0 : __hiloint2double((2046 - e) << 20, 0);
+                    gm.valf[dst] = (float)(val[dst] * sc);
+                }
+                if (tid == 0) gm.valf[a.nnz] = 0.f;
+                for (int i = tid; i < 4 * nq; i += TS) gm.z[i] = 0.f;
+                tsync();
+                if constexpr (NC > 0) {
+#pragma unroll
+                    for (int c = 0; c < NC; c++) {
+                        const int j = (TW == 1 ? 0 : wib) + TW * c;
+#pragma unroll
+                        for (int u = 0; u < MR; u++) {
+                            const int i = lane + 32 * u;
+                            m[c][u] = (i < n && j < n) ? gm.valf[a.sp_map[i + n * j]] : 0.f;
+                        }
                     }
-                    if (q < q1) s -= val[q] * x[a.sp_col[q]];
-                    d32[i] = (float)((s + s1) * (double)scl[i]);
+                    ok = gauss_registers<TW, MR, NC>(n, m, gm, lane, TW == 1 ? 0 : wib);
+                } else {
+                    for (int i = lane; i < n * n; i += 32) gm.dense[i] = gm.valf[a.sp_map[i]];
+                    __syncwarp();
+                    ok = gauss_shared<MR>(n, gm.dense, gm.row, gm.kof, lane);
                 }
-                tsync();
-                if (TW == 1 || wib == 0) warp_lu_solve<float, float, MR>(n, LU, piv, d32, lane);
-                tsync();
-                double dm = 0.0;
+            }
+            if (ok) {
+                for (int i = tid; i < n; i += TS) x[i] = 0.0;
+                double dprev = 1e300;
+                for (int it = 0; it < 10; it++) {
+                    // r = e_1 - A x (FP64; x = 0 at first), at its pivot's place
+                    for (int i = tid; i < n; i += TS) {
+                        double s = (i == 0) ? 1.0 : 0.0;
+                        if (it) {
+                            double s1 = 0.0;   // two chains of dependent FP64 sums
+                            int q = a.sp_off[i];
+                            const int q1 = a.sp_off[i + 1];
+                            for (; q + 1 < q1; q += 2) {
+                                s -= val[q] * x[a.sp_col[q]];
+                                s1 -= val[q + 1] * x[a.sp_col[q + 1]];
+                            }
+                            if (q < q1) s -= val[q] * x[a.sp_col[q]];
+                            s += s1;
+                        }
+                        const int k = gm.kof[i];
+                        const int zi = (NC > 0 && TW > 1) ? (k % TW) * nq + k / TW : k;
+                        gm.z[zi] = (float)(s * (double)scl[i]);
+                    }
+                    tsync();
+                    // the correction: row i of the inverse gives x[kof[i]]; its
+                    // terms in four sums, by column j % 4
+                    float cor[MR];
+                    if constexpr (NC > 0 && TW == 1) {
+#pragma unroll
+                        for (int u = 0; u < MR; u++) cor[u] = 0.f;
+                        float p4[MR][4] = {};
+#pragma unroll
+                        for (int c = 0; c < NC; c += 4) {
+                            const float4 zz = *reinterpret_cast<const float4 *>(gm.z + c);
+#pragma unroll
+                            for (int u = 0; u < MR; u++) {
+                                p4[u][0] = fmaf(m[c][u], zz.x, p4[u][0]);
+                                p4[u][1] = fmaf(m[c + 1][u], zz.y, p4[u][1]);
+                                p4[u][2] = fmaf(m[c + 2][u], zz.z, p4[u][2]);
+                                p4[u][3] = fmaf(m[c + 3][u], zz.w, p4[u][3]);
+                            }
+                        }
+#pragma unroll
+                        for (int u = 0; u < MR; u++) cor[u] = (p4[u][0] + p4[u][1]) + (p4[u][2] + p4[u][3]);
+                    } else if constexpr (NC > 0) {
+                        float acc[MR] = {};
+                        const float *zw = gm.z + wib * nq;
+#pragma unroll
+                        for (int c = 0; c < NC; c += 4) {
+                            const float4 zz = *reinterpret_cast<const float4 *>(zw + c);
+#pragma unroll
+                            for (int u = 0; u < MR; u++) {
+                                acc[u] = fmaf(m[c][u], zz.x, acc[u]);
+                                acc[u] = fmaf(m[c + 1][u], zz.y, acc[u]);
+                                acc[u] = fmaf(m[c + 2][u], zz.z, acc[u]);
+                                acc[u] = fmaf(m[c + 3][u], zz.w, acc[u]);
+                            }
+                        }
+#pragma unroll
+                        for (int u = 0; u < MR; u++)
+                            if (lane + 32 * u < n) gm.part[wib * n + lane + 32 * u] = acc[u];
+                        __syncthreads();
+                    } else {
+#pragma unroll
+                        for (int u = 0; u < MR; u++) {
+                            const int i = lane + 32 * u;
+                            float p0 = 0.f, p1 = 0.f, p2 = 0.f, p3 = 0.f;
+                            if (i < n) {
+                                int j = 0;
+                                for (; j + 3 < n; j += 4) {
+                                    p0 = fmaf(gm.dense[i + n * j], gm.z[j], p0);
+                                    p1 = fmaf(gm.dense[i + n * (j + 1)], gm.z[j + 1], p1);
+                                    p2 = fmaf(gm.dense[i + n * (j + 2)], gm.z[j + 2], p2);
+                                    p3 = fmaf(gm.dense[i + n * (j + 3)], gm.z[j + 3], p3);
+                                }
+                                if (j < n) p0 = fmaf(gm.dense[i + n * j], gm.z[j], p0);
+                                if (j + 1 < n) p1 = fmaf(gm.dense[i + n * (j + 1)], gm.z[j + 1], p1);
+                                if (j + 2 < n) p2 = fmaf(gm.dense[i + n * (j + 2)], gm.z[j + 2], p2);
+                            }
+                            cor[u] = (p0 + p1) + (p2 + p3);
+                        }
+                    }
+                    unsigned kd = 0, kx = 0;   // largest |correction| (FP32) and |x| (upper word)
+                    auto apply = [&](int i, float d) {
+                        const int k = gm.kof[i];
+                        const double xv = x[k] + (double)d;
+                        x[k] = xv;
+                        kd = max(kd, __float_as_uint(fabsf(d)));
+                        kx = max(kx, (unsigned)__double2hiint(xv) & 0x7fffffffu);
+                    };
+                    if constexpr (TW == 1) {
+#pragma unroll
+                        for (int u = 0; u < MR; u++)
+                            if (lane + 32 * u < n) apply(lane + 32 * u, cor[u]);
+                    } else {
+                        for (int i = tid; i < n; i += TS)
+                            apply(i, (gm.part[i] + gm.part[n + i]) + (gm.part[2 * n + i] + gm.part[3 * n + i]));
+                    }
+                    team_max2(kd, kx);
+                    if (TW == 1) __syncwarp();
+                    if (kd >= 0x7f800000u || kx >= 0x7ff00000u) break;  // infinite or NaN
+                    const double dm = (double)__uint_as_float(kd), xmax = __hiloint2double((int)kx, 0);
+                    // converged: the correction is at the level FP64 residuals can
+                    // resolve (~cond(SA) * eps), or it stopped shrinking there, or
+                    // the next one, dm / dprev of this one's size, would be below
+                    // half a unit in the last place
+                    if (dm <= 2e-14 * xmax) { conv = true; break; }
+                    if (it >= 2 && dm <= 1e-12 * xmax && dm > 0.5 * dprev) { conv = true; break; }
+                    if (it >= 2 && dm <= 1e-3 * dprev && dm * dm <= 1e-16 * xmax * dprev) { conv = true; break; }
+                    dprev = dm;
+                }
+            }
+        } else {
+            // ---- FP32 LU of the row-scaled matrix (skipped in FP64 mode) ----
+            if (!a.fp64_only) {
                 for (int i = tid; i < n; i += TS) {
-                    x[i] += (double)d32[i];
-                    dm = fmax(dm, fabs((double)d32[i]));
+                    double m = 0.0;
+                    for (int q = a.sp_off[i]; q < a.sp_off[i + 1]; q++) m = fmax(m, fabs(val[q]));
+                    const float sc = (m > 0.0) ? (float)(1.0 / m) : 1.f;
+                    scl[i] = sc;
+                    for (int q = a.sp_off[i]; q < a.sp_off[i + 1]; q++)
+                        LU[i + (size_t)n * a.sp_col[q]] = (float)(val[q] * (double)sc);
                 }
                 tsync();
-                double xm = 0.0;
-                for (int i = tid; i < n; i += TS) xm = fmax(xm, fabs(x[i]));
-                dm = team_max(dm);
-                xmax = team_max(xm);
-                if (!(dm == dm) || !(xmax == xmax)) break;  // NaN
-                // converged: the correction is at the level FP64 residuals can
-                // resolve (~cond(SA) * eps), or it stopped shrinking there
-                if (dm <= 2e-14 * xmax) { conv = true; break; }
-                if (it >= 2 && dm <= 1e-12 * xmax && dm > 0.5 * dprev) { conv = true; break; }
-                dprev = dm;
+                ok = team_lu<float, TW, MR>(n, LU, piv, tid, red_v, red_i);
+            }
+            if (ok) {
+                for (int i = tid; i < n; i += TS) x[i] = 0.0;
+                tsync();
+                double dprev = 1e300;
+                for (int it = 0; it < 10; it++) {
+                    // r = e_1 - A x (FP64)
+                    for (int i = tid; i < n; i += TS) {
+                        double s = (i == 0) ? 1.0 : 0.0, s1 = 0.0;   // two chains of dependent FP64 sums
+                        int q = a.sp_off[i];
+                        const int q1 = a.sp_off[i + 1];
+                        for (; q + 1 < q1; q += 2) {
+                            s -= val[q] * x[a.sp_col[q]];
+                            s1 -= val[q + 1] * x[a.sp_col[q + 1]];
+                        }
+                        if (q < q1) s -= val[q] * x[a.sp_col[q]];
+                        d32[i] = (float)((s + s1) * (double)scl[i]);
+                    }
+                    tsync();
+                    if (TW == 1 || wib == 0) warp_lu_solve<float, float, MR>(n, LU, piv, d32, lane);
+                    tsync();
+                    unsigned kd = 0, kx = 0;   // largest |correction| (FP32) and |x| (upper word)
+                    for (int i = tid; i < n; i += TS) {
+                        const double xv = x[i] + (double)d32[i];
+                        x[i] = xv;
+                        kd = max(kd, __float_as_uint(fabsf(d32[i])));
+                        kx = max(kx, (unsigned)__double2hiint(xv) & 0x7fffffffu);
+                    }
+                    team_max2(kd, kx);
+                    if (TW == 1) __syncwarp();
+                    if (kd >= 0x7f800000u || kx >= 0x7ff00000u) break;  // infinite or NaN
+                    const double dm = (double)__uint_as_float(kd), xmax = __hiloint2double((int)kx, 0);
+                    if (dm <= 2e-14 * xmax) { conv = true; break; }
+                    if (it >= 2 && dm <= 1e-12 * xmax && dm > 0.5 * dprev) { conv = true; break; }
+                    dprev = dm;
+                }
             }
         }
         if (!conv) {
             // FP64 LU on the device, dense
-            double *M = val + a.nnz;
+            double *M = slot + a.nnz;
             for (int i = tid; i < n * n; i += TS) M[i] = 0.0;
             tsync();
-            for (int q = tid; q < a.nnz; q += TS) M[a.sp_rec[q].x] = val[q];
+            for (int q = tid; q < a.nnz; q += TS) {
+                const int4 rec = a.sp_rec[q];
+                M[(rec.x & 0xffff) + (size_t)n * (rec.x >> 16)] = val[rec.z & 0xffff];
+            }
             tsync();
             st |= ok ? PORTAL_NODE_REFINE : 0;
             bool ok64 = team_lu<double, TW, MR>(n, M, piv, tid, red_v, red_i);
@@ -479,20 +973,14 @@ __global__ void __launch_bounds__(TW == 1 ? 256 : 32 * TW, TW == 1 ? 3 : 24 / TW
             }
         }
         tsync();
-        // ---- packing (main_sub.f90:112-137) ----
-        for (int c2 = tid; c2 < 2 * a.nlev; c2 += TS) {
-            const int p = a.pack[c2];
-            double v = (p >= 0 && !(st & PORTAL_NODE_SINGULAR)) ? x[p] : 0.0;
-            if (st & PORTAL_NODE_SINGULAR) v = 0.0;
-            a.pops[(size_t)node + (size_t)a.N * c2] = v;
-        }
-        tsync();
+        // ---- packing (main_sub.f90:112-137): a NaN population zeroes both ----
         for (int l = tid; l < a.nlev; l += TS) {
-            const double v0 = a.pops[(size_t)node + (size_t)a.N * (2 * l)];
-            if (v0 != v0) {
-                a.pops[(size_t)node + (size_t)a.N * (2 * l)] = 0.0;
-                a.pops[(size_t)node + (size_t)a.N * (2 * l + 1)] = 0.0;
-            }
+            const int p0 = a.pack[2 * l], p1 = a.pack[2 * l + 1];
+            const bool solved = !(st & PORTAL_NODE_SINGULAR);
+            double v0 = (p0 >= 0 && solved) ? x[p0] : 0.0, v1 = (p1 >= 0 && solved) ? x[p1] : 0.0;
+            if (v0 != v0) v0 = v1 = 0.0;
+            a.pops[(size_t)node + (size_t)a.N * (2 * l)] = v0;
+            a.pops[(size_t)node + (size_t)a.N * (2 * l + 1)] = v1;
         }
         if (a.rates) {
             // extra_info rates (em_coefs.f90:188-198): per component i and kind
@@ -551,6 +1039,17 @@ __global__ void __launch_bounds__(TW == 1 ? 256 : 32 * TW, TW == 1 ? 3 : 24 / TW
             if (st & PORTAL_NODE_SINGULAR) atomicAdd(a.nfail, 1);
         }
         tsync();
+    }
+    if (!BATCH) {
+        // the boundary nodes' rows are 0
+        const int nb = a0.N - a0.bulk, cols = 2 * a0.nlev + a0.L;
+        const long long total = (long long)nb * cols;
+        for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < total;
+             q += (long long)gridDim.x * blockDim.x) {
+            const int col = (int)(q / nb), i = a0.bulk + (int)(q % nb);
+            if (col < 2 * a0.nlev) a0.pops[(size_t)i + (size_t)a0.N * col] = 0.0;
+            else a0.jj20[(size_t)i + (size_t)a0.N * (col - 2 * a0.nlev)] = 0.0;
+        }
     }
 }
 
@@ -801,27 +1300,46 @@ int prepare_se(portal_ctx *c, int kmax) {
     size_t o_rad = putI(P.tr_rad), o_col = putI(P.tr_col), o_eoff = putI(P.ent_off),
            o_epos = putI(P.ent_pos), o_tf = putI(P.term_f), o_nc = putI(P.count_array),
            o_pack = putI(P.pack), o_roff = putI(P.row_off), o_rent = putI(P.row_ent);
-    // the matrix's entries row by row in ascending column order: records (pos,
-    // first term, end, -1), row 1 replaced by the normalisation's (pos, 0, 0,
-    // level); 16-byte aligned for one load each
-    std::vector<int> sp_rec, sp_off(1, 0), sp_col;
+    // the matrix's entries row by row in ascending column order: row offsets
+    // and columns; row 1 is the normalisation's
+    struct Rec { int pos, first, count, norm; };
+    std::vector<Rec> recs;
+    std::vector<int> sp_off(1, 0), sp_col;
     for (int i = 0; i < P.c_dim; i++) {
         if (i == 0) {
             for (int l = 0; l < c->nlev; l++) {
-                sp_rec.insert(sp_rec.end(), {P.c_dim * P.count_array[l], 0, 0, l});
+                recs.push_back({P.count_array[l] << 16, 0, 0, l});
                 sp_col.push_back(P.count_array[l]);
             }
         } else {
             for (int q = P.row_off[i]; q < P.row_off[i + 1]; q++) {
                 const int e = P.row_ent[q];
                 if (P.ent_off[e + 1] == P.ent_off[e]) continue;
-                sp_rec.insert(sp_rec.end(), {P.ent_pos[e], P.ent_off[e], P.ent_off[e + 1], -1});
-                sp_col.push_back(P.ent_pos[e] / P.c_dim);
+                const int col = P.ent_pos[e] / P.c_dim;
+                recs.push_back({i | col << 16, P.ent_off[e], P.ent_off[e + 1] - P.ent_off[e], -1});
+                sp_col.push_back(col);
             }
         }
         sp_off.push_back((int)sp_col.size());
     }
-    const size_t o_soff = putI(sp_off), o_scol = putI(sp_col);
+    // the assembly's records (row | column << 16, first term, terms << 16 |
+    // entry, -1 or the normalisation's level), most terms first; 16-byte
+    // aligned for one load each
+    std::vector<int> ord(recs.size()), sp_rec;
+    for (size_t e = 0; e < ord.size(); e++) ord[e] = (int)e;
+    std::stable_sort(ord.begin(), ord.end(), [&](int p, int q) { return recs[p].count > recs[q].count; });
+    for (int e : ord)
+        sp_rec.insert(sp_rec.end(), {recs[e].pos, recs[e].first, (int)((unsigned)recs[e].count << 16 | (unsigned)e), recs[e].norm});
+    // the entry at every place of the matrix (column-major; the one past the
+    // last where there is none), for the systems inverted
+    std::vector<int> sp_map;
+    if (P.c_dim <= SE_GAUSS_DIM) {
+        std::vector<unsigned short> at(((size_t)P.c_dim * P.c_dim + 1) & ~(size_t)1, (unsigned short)recs.size());
+        for (size_t e = 0; e < recs.size(); e++) at[(recs[e].pos & 0xffff) + (size_t)P.c_dim * (recs[e].pos >> 16)] = (unsigned short)e;
+        sp_map.resize(at.size() / 2);
+        std::memcpy(sp_map.data(), at.data(), at.size() * sizeof(unsigned short));
+    }
+    const size_t o_soff = putI(sp_off), o_scol = putI(sp_col), o_map = putI(sp_map);
     while (I.size() % 4) I.push_back(0);
     const size_t o_asm = putI(sp_rec);
     size_t o_nu = putD(P.tr_nu), o_A = putD(P.tr_A), o_B = putD(P.tr_B21), o_tc = putD(P.term_c),
@@ -842,7 +1360,7 @@ int prepare_se(portal_ctx *c, int kmax) {
     c->se_offs[7] = o_nu; c->se_offs[8] = o_A; c->se_offs[9] = o_B; c->se_offs[10] = o_tc;
     c->se_offs[11] = o_nv; c->se_offs[12] = o_ct; c->se_offs[13] = o_C;
     c->se_offs[14] = o_roff; c->se_offs[15] = o_rent; c->se_offs[16] = o_dep; c->se_offs[17] = o_asm;
-    c->se_offs[18] = o_soff; c->se_offs[19] = o_scol;
+    c->se_offs[18] = o_soff; c->se_offs[19] = o_scol; c->se_offs[20] = o_map;
     c->se_nnz = (int)sp_col.size();
     c->n_dep = P.n_dep;
     c->n_feat = NF * P.n_trans + (c->depol == 2 ? 2 : 1) * P.n_dep;
@@ -881,6 +1399,7 @@ int se_prepare(portal_ctx *c, int kmax, SEArgs *out, size_t *warp_bytes) {
     a.row_off = I + c->se_offs[14]; a.row_ent = I + c->se_offs[15];
     a.sp_rec = reinterpret_cast<const int4 *>(I + c->se_offs[17]);
     a.sp_off = I + c->se_offs[18]; a.sp_col = I + c->se_offs[19];
+    a.sp_map = reinterpret_cast<const unsigned short *>(I + c->se_offs[20]);
     a.nnz = c->se_nnz;
     a.dep_tab = c->n_dep ? D + c->se_offs[16] : nullptr;
     a.pops = c->pops.p; a.jj20 = c->jj20.p; a.status = c->status.p;
@@ -897,26 +1416,44 @@ int se_prepare(portal_ctx *c, int kmax, SEArgs *out, size_t *warp_bytes) {
     return PORTAL_OK;
 }
 
-// The per-pass device work before the solve: zeroed outputs and failure
-// count.  Stream-ordered only (capturable).
+// The per-pass device work before the solve: the failure count.
+// Stream-ordered only (capturable).
 int se_pass(portal_ctx *c, cudaStream_t s) {
-    PCHECK(c, cudaMemsetAsync(c->pops.p, 0, (size_t)c->N * 2 * c->nlev * sizeof(double), s));
-    PCHECK(c, cudaMemsetAsync(c->jj20.p, 0, (size_t)c->N * c->r_num * sizeof(double), s));
     PCHECK(c, cudaMemsetAsync(c->counters.p + 2, 0, sizeof(unsigned long long), s));
     return PORTAL_OK;
+}
+// ... and, before a batched solve, zeroed outputs (its items are the bulk
+// nodes; the single-model kernel writes the other rows itself)
+int se_batch_pass(portal_ctx *c, cudaStream_t s) {
+    PCHECK(c, cudaMemsetAsync(c->pops.p, 0, (size_t)c->N * 2 * c->nlev * sizeof(double), s));
+    PCHECK(c, cudaMemsetAsync(c->jj20.p, 0, (size_t)c->N * c->r_num * sizeof(double), s));
+    return se_pass(c, s);
 }
 
 size_t se_matrix_doubles(const portal_ctx *c) { return (size_t)c->se_nnz + (size_t)c->c_dim * c->c_dim; }
 
-// The batched kernel's instance for the batch's largest system: 3 rows per
-// lane up to 96 unknowns, SE_MAX_ROWS above.
-static const void *se_batch_kernel(int max_dim) {
-    return max_dim <= 96 ? (const void *)k_solve_se<1, true, 3> : (const void *)k_solve_se<1, true, SE_MAX_ROWS>;
+// Whether the prepared system is inverted, and the inversion's shared memory
+// per warp.  The limit is on the largest form, the same for every launch.
+bool se_gauss(const portal_ctx *c) {
+    return c->c_dim <= SE_GAUSS_DIM && se_gauss_bytes(c->c_dim, c->n_feat, c->se_nnz, SE_GAUSS_DIM / 4, true) <= 200 * 1024;
+}
+size_t se_gauss_team_bytes(const portal_ctx *c) {
+    return se_gauss_bytes(c->c_dim, c->n_feat, c->se_nnz, SE_GAUSS_DIM / 4, false);
 }
 
-int se_batch_blocks_per_sm(int warps_per_block, size_t warp_bytes, int max_dim, int *blocks) {
-    const size_t smem = warp_bytes * warps_per_block;
-    const void *k = se_batch_kernel(max_dim);
+// The batched kernel's instance for the batch's largest system, and its warps
+// per node.
+static const void *se_batch_kernel(int max_dim, bool gauss) {
+    return !gauss                   ? (const void *)k_solve_se<1, true, SE_MAX_ROWS, -1>
+           : max_dim <= SE_WARP_DIM ? (const void *)k_solve_se<1, true, 1, SE_WARP_DIM>
+           : max_dim <= 48          ? (const void *)k_solve_se<4, true, 2, 12>
+                                    : (const void *)k_solve_se<4, true, 3, 24>;
+}
+int se_batch_team(int max_dim, bool gauss) { return gauss && max_dim > SE_WARP_DIM ? 4 : 1; }
+
+int se_batch_blocks_per_sm(int warps_per_block, size_t team_bytes, int max_dim, bool gauss, int *blocks) {
+    const size_t smem = team_bytes * (warps_per_block / se_batch_team(max_dim, gauss));
+    const void *k = se_batch_kernel(max_dim, gauss);
     *blocks = 0;
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return PORTAL_ERR_CUDA;
@@ -928,34 +1465,37 @@ int se_batch_blocks_per_sm(int warps_per_block, size_t warp_bytes, int max_dim, 
 // (the kernel's dynamic shared memory limit must have been raised by
 // se_batch_blocks_per_sm for at least this many warps)
 int se_batch_launch(cudaStream_t s, int grid, int warps_per_block, const SEBatch &bw) {
-    const size_t smem = bw.warp_bytes * warps_per_block;
+    const size_t smem = bw.team_bytes * (warps_per_block / se_batch_team(bw.max_dim, bw.gauss));
     SEArgs a0{};
     SEBatch b = bw;
     void *args[] = {&a0, &b};
-    if (cudaLaunchKernel(se_batch_kernel(bw.max_dim), dim3(grid), dim3(32 * warps_per_block), args, smem, s) !=
-        cudaSuccess)
+    if (cudaLaunchKernel(se_batch_kernel(bw.max_dim, bw.gauss), dim3(grid), dim3(32 * warps_per_block), args, smem,
+                         s) != cudaSuccess)
         return PORTAL_ERR_CUDA;
     return cudaGetLastError() == cudaSuccess ? PORTAL_OK : PORTAL_ERR_CUDA;
 }
 
-// Warps per node: one up to SE_TEAM_MIN_N unknowns, a team of four above
-// (PORTAL_SE_TEAM=1|4 overrides).  Teams of two measured slower than either
-// on 34 x 34 and 74 x 74 systems.
-constexpr int SE_TEAM_MIN_N = 48;
+// Warps per node: one up to SE_WARP_DIM unknowns, a team of four above
+// (PORTAL_SE_TEAM=1|4 overrides).  The barrier a step costs a team more than
+// the columns save it while one warp's registers hold them: 1,024 systems of
+// 14 unknowns 29 us by one warp, 41 by a team; 1,700 of 19 49 and 98 us.
+// Beyond its registers one warp works in shared memory: 8,192 of 39 0.86 ms,
+// a team 0.44; of 74 3.4 and 0.95.
 inline int se_team_warps(int n) {
     const char *e = getenv("PORTAL_SE_TEAM");
     if (e) {
         const int v = atoi(e);
         if (v == 1 || v == 4) return v;
     }
-    return n >= SE_TEAM_MIN_N ? 4 : 1;
+    return n > SE_WARP_DIM ? 4 : 1;
 }
 
 // TW = 1: blocks of up to 8 independent warps; TW > 1: one team per block.
 // One FP64 matrix slot per team of the grid.
-template <int TW, int MR>
-int launch_se(portal_ctx *c, SEArgs &a, size_t wb) {
-    auto kern = k_solve_se<TW, false, MR>;
+template <int TW, int MR, int NC>
+int launch_se(portal_ctx *c, SEArgs &a) {
+    auto kern = k_solve_se<TW, false, MR, NC>;
+    const size_t wb = NC >= 0 ? se_gauss_bytes(a.c_dim, a.n_feat, a.nnz, gauss_quads<TW, NC>, NC == 0) : se_warp_bytes(a.c_dim, a.n_feat);
     const int teams = (TW == 1) ? (int)std::min<size_t>(8, (200 * 1024) / wb) : 1;
     const size_t smem = wb * teams;
     PCHECK(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -974,8 +1514,7 @@ int launch_se(portal_ctx *c, SEArgs &a, size_t wb) {
 
 int run_solve_se(portal_ctx *c, int kmax, int *n_singular, bool rates, const HostSpan *out, int n_out) {
     SEArgs a;
-    size_t wb = 0;
-    int rc = se_prepare(c, kmax, &a, &wb);
+    int rc = se_prepare(c, kmax, &a, nullptr);
     if (rc) return rc;
     if (rates) {
         const size_t nr = (size_t)c->N * 3 * 2 * c->nlev;
@@ -985,11 +1524,18 @@ int run_solve_se(portal_ctx *c, int kmax, int *n_singular, bool rates, const Hos
     }
     if ((rc = se_pass(c, c->stream))) return rc;
     a.a64_stride = se_matrix_doubles(c);
-    const bool few_rows = c->c_dim <= 96;
-    if (se_team_warps(c->c_dim) == 4)
-        rc = few_rows ? launch_se<4, 3>(c, a, wb) : launch_se<4, SE_MAX_ROWS>(c, a, wb);
+    const int n = c->c_dim;
+    if (se_team_warps(n) == 4)
+        rc = !se_gauss(c) ? launch_se<4, SE_MAX_ROWS, -1>(c, a)
+             : n <= 48    ? launch_se<4, 2, 12>(c, a)
+             : n <= 80    ? launch_se<4, 3, 20>(c, a)
+                          : launch_se<4, 3, 24>(c, a);
     else
-        rc = few_rows ? launch_se<1, 3>(c, a, wb) : launch_se<1, SE_MAX_ROWS>(c, a, wb);
+        rc = !se_gauss(c)       ? launch_se<1, SE_MAX_ROWS, -1>(c, a)
+             : n <= 16          ? launch_se<1, 1, 16>(c, a)
+             : n <= 24          ? launch_se<1, 1, 24>(c, a)
+             : n <= SE_WARP_DIM ? launch_se<1, 1, SE_WARP_DIM>(c, a)
+                                : launch_se<1, 3, 0>(c, a);
     if (rc) return rc;
     touch_pages(out, n_out);   // the caller's result arrays, while the kernel runs
     int nf = 0;
