@@ -33,9 +33,10 @@
 #include "common.cuh"
 
 namespace portal {
-int run_radiation_field(portal_ctx *c, int nth, int nph, int nvel, const double *gvec, double dx,
-                        int n_depth, long long *n_segments, int *n_failed, bool split, const HostSpan *out, int n_out);
-int run_solve_se(portal_ctx *c, int kmax, int *n_singular, bool rates, const HostSpan *out, int n_out);
+int enqueue_radiation_field(portal_ctx *c, int nth, int nph, int nvel, const double *gvec, double dx, int n_depth,
+                            bool split);
+int failed_nodes(portal_ctx *c);
+int enqueue_solve_se(portal_ctx *c, int kmax, bool rates, bool fresh);
 }  // namespace portal
 using namespace portal;
 
@@ -62,11 +63,14 @@ __global__ void k_rho_to_pops(int N, int bulk, int nlev, const double *__restric
         levp[(size_t)nlev * n + l] = nmol[n] * sqrt(2.0 * jl[l] + 1.0) * pp[(size_t)n + (size_t)N * (2 * l)];
 }
 
-// populations from the SE solution, and the residual (max relative change)
+// populations from the SE solution, and the residual (max relative change);
+// nothing where the pass failed (fail: singular systems, failed walks)
 __global__ void k_update(int N, int bulk, int nlev, const double *__restrict__ pops,
                          const double *__restrict__ nmol, const double *__restrict__ ab,
                          const int *__restrict__ jl, double *__restrict__ levp,
-                         double *__restrict__ rho_prev, unsigned long long *__restrict__ resid) {
+                         double *__restrict__ rho_prev, const unsigned long long *__restrict__ fail,
+                         unsigned long long *__restrict__ resid) {
+    if (*fail) return;
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     double r = 0.0;
     if (n < bulk && ab[n] > 0.0) {
@@ -206,22 +210,30 @@ extern "C" int portal_lambda_iterate(portal_ctx *c, int nth, int nph, int nvel, 
     double r = 1e300;
     bool verify = false;  // this pass is the plain pass that decides convergence
     while (it < max_iter) {
-        long long nseg = 0;
-        int nfail = 0;
         const bool split = local_operator && !verify;
-        if ((rc = run_radiation_field(c, nth, nph, nvel, gvec, dx, n_depth, &nseg, &nfail, split, nullptr, 0)))
-            return rc;
-        nseg_tot += nseg;
-        int nsing = 0;
-        if ((rc = run_solve_se(c, kmax, &nsing, false, nullptr, 0))) return rc;
-        if (nsing) return set_err(c, PORTAL_ERR_SINGULAR, std::to_string(nsing) + " singular SE systems");
-        PCHECK(c, cudaMemsetAsync(c->counters.p + 3, 0, sizeof(unsigned long long), c->stream));
+        // the pass enqueued as a whole, one wait (on its counters) at its end
+        if ((rc = enqueue_radiation_field(c, nth, nph, nvel, gvec, dx, n_depth, split))) return rc;
+        const bool j_before = c->j_valid;
+        c->j_valid = true;
+        c->ali_valid = split;
+        if ((rc = enqueue_solve_se(c, kmax, false, true))) return rc;
         k_update<<<nb, tb, 0, c->stream>>>(N, c->bulk, nlev, c->pops.p, c->nmol.p, c->active_ab(), jl.p, c->levp.p,
-                                           rho_prev.p, c->counters.p + 3);
+                                           rho_prev.p, c->counters.p + 2, c->counters.p + 3);
         PCHECK(c, cudaGetLastError());
-        unsigned long long rb = 0;
-        PCHECK(c, cudaMemcpyAsync(&rb, c->counters.p + 3, sizeof rb, cudaMemcpyDeviceToHost, c->stream));
+        unsigned long long cnt[4];
+        PCHECK(c, cudaMemcpyAsync(cnt, c->counters.p, sizeof cnt, cudaMemcpyDeviceToHost, c->stream));
         PCHECK(c, cudaStreamSynchronize(c->stream));
+        timer_collect(c, T_LINETAB);
+        timer_collect(c, T_RF);
+        timer_collect(c, T_SE);
+        nseg_tot += (long long)cnt[1];
+        if (cnt[2] >> 32) {
+            c->j_valid = j_before;
+            c->ali_valid = false;
+            return failed_nodes(c);
+        }
+        if (cnt[2]) return set_err(c, PORTAL_ERR_SINGULAR, std::to_string(cnt[2]) + " singular SE systems");
+        const unsigned long long rb = cnt[3];
         double rv;
         memcpy(&rv, &rb, sizeof rv);
         r = rv;

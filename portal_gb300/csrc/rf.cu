@@ -207,7 +207,6 @@ int launch_rf(portal_ctx *c, RFArgs &a, int n_depth) {
             return set_err(c, PORTAL_ERR_NOMEM, "ray sums");
         a.vray = c->vray.p; a.dray = c->dray.p; a.iseg = c->iseg.p;
     }
-    PCHECK(c, cudaMemsetAsync(c->counters.p, 0, 8 * sizeof(unsigned long long), c->stream));
     timer_start(c, T_RF);
     RFBatch none{};
     void *args[] = {&a, &none, &sh};
@@ -244,7 +243,6 @@ int launch_rf_star(portal_ctx *c, RFArgs &a, int n_depth) {
     }
     a.walk = c->walk.p;
     PCHECK(c, cudaMemcpyAsync(c->star_model.p, &a, sizeof(RFArgs), cudaMemcpyHostToDevice, c->stream));
-    PCHECK(c, cudaMemsetAsync(c->counters.p, 0, 8 * sizeof(unsigned long long), c->stream));
     bw.models = reinterpret_cast<const RFArgs *>(c->star_model.p);
     bw.items = c->star_items.p;
     bw.n_items = c->bulk;
@@ -370,33 +368,24 @@ int rf_prepare(portal_ctx *c, int nth, int nph, int nvel, const double *gvec, do
     return PORTAL_OK;
 }
 
-// The per-pass device work before the walk: zeroed outputs and the line
-// table from the current populations.  Stream-ordered only (capturable).
+// The per-pass device work before the walk: zeroed outputs and counters, node
+// frames and the line table from the current populations.  Stream-ordered only (capturable).
 int rf_pass(portal_ctx *c, const RFArgs &a, cudaStream_t s) {
     const int L = c->r_num, N = c->N;
-    PCHECK(c, cudaMemsetAsync(c->J0.p, 0, (size_t)L * N * sizeof(double), s));
-    PCHECK(c, cudaMemsetAsync(c->J2.p, 0, (size_t)L * N * sizeof(double), s));
-    PCHECK(c, cudaMemsetAsync(c->status.p, 0, (size_t)N * sizeof(int), s));
-    if (a.segs) PCHECK(c, cudaMemsetAsync(a.segs, 0, (size_t)N * sizeof(int), s));
-    if (a.kmom) PCHECK(c, cudaMemsetAsync(a.kmom, 0, (size_t)6 * N * sizeof(float), s));
-    if (a.JE) {
-        PCHECK(c, cudaMemsetAsync(c->JE.p, 0, (size_t)L * N * sizeof(double), s));
-        PCHECK(c, cudaMemsetAsync(c->LS.p, 0, (size_t)L * N * sizeof(double), s));
-    }
     const long long tot = (long long)N * L;
     const int table_blocks = (int)((tot + 255) / 256);
-    k_line_table<<<table_blocks + (a.bulk + 255) / 256, 256, 0, s>>>(
+    k_line_table<<<table_blocks + (std::max(N, 8) + 255) / 256, 256, 0, s>>>(
         N, L, c->rf_dxp, reinterpret_cast<const LineConst *>(c->linebuf.p), c->levp.p, c->nlev, c->b64.p,
         c->dustp.p, c->tdust.p, c->ltab.p, a, table_blocks);
     PCHECK(c, cudaGetLastError());
     return PORTAL_OK;
 }
 
-// Runs the line table + radiation field on the device; J stays in c->J0/J2
-// (and the split field in c->JE/LS when `split`).
-int run_radiation_field(portal_ctx *c, int nth, int nph, int nvel, const double *gvec, double dx,
-                        int n_depth, long long *n_segments, int *n_failed, bool split, const HostSpan *out,
-                        int n_out) {
+// Enqueues the line table and the radiation field; J stays in c->J0/J2 (and
+// the split field in c->JE/LS when `split`), the pass's counters in
+// c->counters ([1] segments).
+int enqueue_radiation_field(portal_ctx *c, int nth, int nph, int nvel, const double *gvec, double dx, int n_depth,
+                            bool split) {
     RFArgs a;
     int rc = rf_prepare(c, nth, nph, nvel, gvec, dx, n_depth, split, &a);
     if (rc) return rc;
@@ -404,38 +393,26 @@ int run_radiation_field(portal_ctx *c, int nth, int nph, int nvel, const double 
     timer_start(c, T_LINETAB);
     if ((rc = rf_pass(c, a, c->stream))) return rc;
     timer_stop(c, T_LINETAB);
-    if ((rc = dispatch_rf(c, a, n_depth))) return rc;
-    touch_pages(out, n_out);   // the caller's result arrays, while the kernel runs
-    unsigned long long cnt[8];
-    PCHECK(c, cudaMemcpyAsync(cnt, c->counters.p, sizeof cnt, cudaMemcpyDeviceToHost, c->stream));
+    return dispatch_rf(c, a, n_depth);
+}
+
+// The error of a pass with failed nodes: a walk past n_depth or a star ray set
+// past nth*nph is an error, as the reference stops there.
+int failed_nodes(portal_ctx *c) {
+    std::vector<int> st((size_t)c->N);
+    PCHECK(c, cudaMemcpyAsync(st.data(), c->status.p, st.size() * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     PCHECK(c, cudaStreamSynchronize(c->stream));
-    timer_collect(c, T_LINETAB);
-    timer_collect(c, T_RF);
-    if (n_segments) *n_segments = (long long)cnt[1];
-    // failed nodes, counted on the host from the status array when asked (the
-    // iterated node loop): a walk past n_depth or a star ray set past nth*nph
-    // is an error, as the reference stops there
-    if (n_failed) {
-        std::vector<int> st((size_t)c->N);
-        PCHECK(c, cudaMemcpyAsync(st.data(), c->status.p, st.size() * sizeof(int), cudaMemcpyDeviceToHost,
-                                  c->stream));
-        PCHECK(c, cudaStreamSynchronize(c->stream));
-        int nf = 0, first = -1, bits = 0;
-        for (int i = 0; i < c->N; i++)
-            if (st[i] & (PORTAL_NODE_DEPTH | PORTAL_NODE_STAR)) {
-                if (first < 0) first = i;
-                bits |= st[i];
-                nf++;
-            }
-        *n_failed = nf;
-        if (nf)
-            return set_err(c, (bits & PORTAL_NODE_DEPTH) ? PORTAL_ERR_DEPTH : PORTAL_ERR_ARG,
-                           std::string((bits & PORTAL_NODE_DEPTH) ? "node_count > n_depth" : "star rays > nth*nph") +
-                               " for " + std::to_string(nf) + " node(s), the first node " + std::to_string(first + 1));
-    }
-    c->j_valid = true;
-    c->ali_valid = split;
-    return PORTAL_OK;
+    int nf = 0, first = -1, bits = 0;
+    for (int i = 0; i < c->N; i++)
+        if (st[i] & (PORTAL_NODE_DEPTH | PORTAL_NODE_STAR)) {
+            if (first < 0) first = i;
+            bits |= st[i];
+            nf++;
+        }
+    if (!nf) return PORTAL_OK;
+    return set_err(c, (bits & PORTAL_NODE_DEPTH) ? PORTAL_ERR_DEPTH : PORTAL_ERR_ARG,
+                   std::string((bits & PORTAL_NODE_DEPTH) ? "node_count > n_depth" : "star rays > nth*nph") + " for " +
+                       std::to_string(nf) + " node(s), the first node " + std::to_string(first + 1));
 }
 
 }  // namespace portal
@@ -448,10 +425,11 @@ int radiation_field_call(portal_ctx *c, int nth, int nph, int nvel, const double
     if (!c) return PORTAL_ERR_ARG;
     timers_reset(c);
     const size_t LN = (size_t)c->r_num * c->N;
+    if (int rc = portal::enqueue_radiation_field(c, nth, nph, nvel, gvec, dx, n_depth, split)) return rc;
     const HostSpan out[4] = {{J0, LN * sizeof(double)}, {J2, LN * sizeof(double)}, {JE, LN * sizeof(double)},
                              {LS, LN * sizeof(double)}};
-    int rc = portal::run_radiation_field(c, nth, nph, nvel, gvec, dx, n_depth, n_segments, nullptr, split, out, 4);
-    if (rc) return rc;
+    touch_pages(out, 4);   // the caller's result arrays, while the kernel runs
+    // every copy behind the kernels, one wait for all
     if (J0) PCHECK(c, cudaMemcpyAsync(J0, c->J0.p, LN * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     if (J2) PCHECK(c, cudaMemcpyAsync(J2, c->J2.p, LN * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     if (split && JE) PCHECK(c, cudaMemcpyAsync(JE, c->JE.p, LN * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
@@ -460,7 +438,14 @@ int radiation_field_call(portal_ctx *c, int nth, int nph, int nvel, const double
     int *st = status;
     if (!st) { st_host.resize(c->N); st = st_host.data(); }
     PCHECK(c, cudaMemcpyAsync(st, c->status.p, (size_t)c->N * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    unsigned long long cnt[2];
+    PCHECK(c, cudaMemcpyAsync(cnt, c->counters.p, sizeof cnt, cudaMemcpyDeviceToHost, c->stream));
     PCHECK(c, cudaStreamSynchronize(c->stream));
+    timer_collect(c, T_LINETAB);
+    timer_collect(c, T_RF);
+    if (n_segments) *n_segments = (long long)cnt[1];
+    c->j_valid = true;
+    c->ali_valid = split;
     for (int i = 0; i < c->N; i++) {
         if (st[i] & PORTAL_NODE_DEPTH)
             return set_err(c, PORTAL_ERR_DEPTH, "node_count > n_depth for node " + std::to_string(i + 1));

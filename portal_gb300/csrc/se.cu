@@ -633,6 +633,8 @@ __global__ void __launch_bounds__(TW == 1 ? 256 : 32 * TW, se_min_blocks<TW, MR,
         float *d32 = LU + (size_t)n * n;
         float *scl = GAUSS ? gm.scl : d32 + n;
         int *piv = GAUSS ? gm.kof : (int *)(scl + n);
+        // (a failed walk of the iterated node loop: counted, its update stops)
+        if (!BATCH && tid == 0 && (a.status[node] & (PORTAL_NODE_DEPTH | PORTAL_NODE_STAR))) atomicAdd(a.nfail + 1, 1);
         if (!(a.ab[node] > 0.0)) {  // main_para.f90:213 (pops and alignments stay 0)
             if (!BATCH) {
                 for (int c2 = tid; c2 < 2 * a.nlev; c2 += TS) a.pops[(size_t)node + (size_t)a.N * c2] = 0.0;
@@ -1512,7 +1514,11 @@ int launch_se(portal_ctx *c, SEArgs &a) {
     return PORTAL_OK;
 }
 
-int run_solve_se(portal_ctx *c, int kmax, int *n_singular, bool rates, const HostSpan *out, int n_out) {
+// Enqueues the solve: results in c->pops, c->jj20, c->rates, c->status; the
+// numbers of singular systems and of nodes with failed walks in c->counters[2]
+// (its lower and upper half), zeroed here or, after a radiation field
+// enqueued before (fresh), with its counters.
+int enqueue_solve_se(portal_ctx *c, int kmax, bool rates, bool fresh) {
     SEArgs a;
     int rc = se_prepare(c, kmax, &a, nullptr);
     if (rc) return rc;
@@ -1522,7 +1528,7 @@ int run_solve_se(portal_ctx *c, int kmax, int *n_singular, bool rates, const Hos
         PCHECK(c, cudaMemsetAsync(c->rates.p, 0, nr * sizeof(double), c->stream));
         a.rates = c->rates.p;
     }
-    if ((rc = se_pass(c, c->stream))) return rc;
+    if (!fresh && (rc = se_pass(c, c->stream))) return rc;
     a.a64_stride = se_matrix_doubles(c);
     const int n = c->c_dim;
     if (se_team_warps(n) == 4)
@@ -1536,14 +1542,7 @@ int run_solve_se(portal_ctx *c, int kmax, int *n_singular, bool rates, const Hos
              : n <= 24          ? launch_se<1, 1, 24>(c, a)
              : n <= SE_WARP_DIM ? launch_se<1, 1, SE_WARP_DIM>(c, a)
                                 : launch_se<1, 3, 0>(c, a);
-    if (rc) return rc;
-    touch_pages(out, n_out);   // the caller's result arrays, while the kernel runs
-    int nf = 0;
-    PCHECK(c, cudaMemcpyAsync(&nf, c->counters.p + 2, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    PCHECK(c, cudaStreamSynchronize(c->stream));
-    timer_collect(c, T_SE);
-    if (n_singular) *n_singular = nf;
-    return PORTAL_OK;
+    return rc;
 }
 
 }  // namespace portal
@@ -1567,11 +1566,11 @@ extern "C" int portal_solve_se(portal_ctx *c, int kmax, const double *J0, const 
         return set_err(c, PORTAL_ERR_STATE, "portal_solve_se: no device-resident radiation field");
     }
     timers_reset(c);
-    int nsing = 0;
     const HostSpan out[3] = {{pol_pops, (size_t)c->N * 2 * c->nlev * sizeof(double)}, {JJ_20, LN * sizeof(double)},
                              {rates, (size_t)c->N * 6 * c->nlev * sizeof(double)}};
-    int rc = portal::run_solve_se(c, kmax, &nsing, rates != nullptr, out, 3);
-    if (rc) return rc;
+    if (int rc = portal::enqueue_solve_se(c, kmax, rates != nullptr, false)) return rc;
+    touch_pages(out, 3);   // the caller's result arrays, while the kernel runs
+    // every copy behind the kernel, one wait for all
     if (pol_pops)
         PCHECK(c, cudaMemcpyAsync(pol_pops, c->pops.p, (size_t)c->N * 2 * c->nlev * sizeof(double),
                                   cudaMemcpyDeviceToHost, c->stream));
@@ -1582,7 +1581,10 @@ extern "C" int portal_solve_se(portal_ctx *c, int kmax, const double *J0, const 
     if (rates)
         PCHECK(c, cudaMemcpyAsync(rates, c->rates.p, (size_t)c->N * 3 * 2 * c->nlev * sizeof(double),
                                   cudaMemcpyDeviceToHost, c->stream));
+    int nsing = 0;
+    PCHECK(c, cudaMemcpyAsync(&nsing, c->counters.p + 2, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     PCHECK(c, cudaStreamSynchronize(c->stream));
+    timer_collect(c, T_SE);
     if (nsing) return set_err(c, PORTAL_ERR_SINGULAR, std::to_string(nsing) + " singular SE systems");
     return PORTAL_OK;
 }
