@@ -16,8 +16,9 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "_build")
 LIB = os.path.join(OUT, "libportal_gb300.so")
-SOURCES = ["ctx.cu", "rf.cu", "rf_one.cu", "rf_even.cu", "rf_even_split.cu",
-           "rf_any.cu", "rf_dust.cu", "rf_batch.cu", "rf_batch_even.cu",
+SOURCES = ["ctx.cu", "rf.cu", "rf_one.cu", "rf_one_flat.cu", "rf_even.cu", "rf_even_flat.cu",
+           "rf_even_split.cu", "rf_even_split_flat.cu", "rf_any.cu", "rf_any_flat.cu",
+           "rf_dust.cu", "rf_dust_flat.cu", "rf_batch.cu", "rf_batch_even.cu",
            "rf_batch_any.cu", "rf_static.cu", "se.cu", "image.cu", "lambda.cu", "mlp.cu",
            "warmstart.cu", "batch.cu", "adjacency.cu", "wigner.cpp"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]

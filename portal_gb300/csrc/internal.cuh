@@ -38,11 +38,10 @@ struct RFArgs {
     float *kmom;                      // (6, N) second moment sum w I n n of line 1 (xx yy zz xy xz yz) or null
     int2 *walk;
     unsigned long long *counters;
-    // ray-range items (small clouds): rays per item (0: one item per node), and
-    // what the items leave for k_rf_finish -- per (node, ray, line) channel sums
-    // (three planes with a split field), ray directions, segments per item (-1:
-    // a walk past n_depth)
-    int rays_per_item;
+    // items of rays (small clouds), and what they leave for k_rf_finish -- per
+    // (node, ray, line) channel sums (three planes with a split field), ray
+    // directions, segments per ray (-1: a walk past n_depth)
+    int items32, items16;   // items of rays: so many of 32, then of 16, the rest of 8
     float *vray;
     float4 *dray;
     int *iseg;
@@ -126,12 +125,23 @@ struct SEBatch {
 int rf_prepare(portal_ctx *c, int nth, int nph, int nvel, const double *gvec, double dx, int n_depth,
                bool split, RFArgs *a);
 int rf_pass(portal_ctx *c, const RFArgs &a, cudaStream_t s);
-// the single-model kernel for groups of nlg lines (1..10, with dust 1..5):
-const void *rf_kernel_one(int nlg, bool split);    // one slot of channels
-const void *rf_kernel_even(int nlg);               // an even number of slots
-const void *rf_kernel_even_split(int nlg);
-const void *rf_kernel_any(int nlg);                // any, split or not
-const void *rf_kernel_dust(int nlg, int slots);    // slots 1: one, 2: an even number, 0: any
+// the single-model kernel for groups of nlg lines (1..10, with dust 1..5); FLAT:
+// its items are ranges of rays, not nodes
+template <bool FLAT> const void *rf_kernel_one(int nlg, bool split);    // one slot of channels
+template <bool FLAT> const void *rf_kernel_even(int nlg);               // an even number of slots
+template <bool FLAT> const void *rf_kernel_even_split(int nlg);
+template <bool FLAT> const void *rf_kernel_any(int nlg);                // any, split or not
+template <bool FLAT> const void *rf_kernel_dust(int nlg, int slots);    // slots 1: one, 2: an even number, 0: any
+template <> const void *rf_kernel_one<false>(int nlg, bool split);
+template <> const void *rf_kernel_one<true>(int nlg, bool split);
+template <> const void *rf_kernel_even<false>(int nlg);
+template <> const void *rf_kernel_even<true>(int nlg);
+template <> const void *rf_kernel_even_split<false>(int nlg);
+template <> const void *rf_kernel_even_split<true>(int nlg);
+template <> const void *rf_kernel_any<false>(int nlg);
+template <> const void *rf_kernel_any<true>(int nlg);
+template <> const void *rf_kernel_dust<false>(int nlg, int slots);
+template <> const void *rf_kernel_dust<true>(int nlg, int slots);
 const void *rf_batch_even();                       // the batched kernel's instantiations
 const void *rf_batch_any(bool dust, bool one_slot, bool split);
 size_t rf_walk_records(int n_depth);     // walk scratch per warp, int2 records

@@ -5,14 +5,16 @@
 // check_neigh_fast miscellaneous.f90:1017-1076, pos_quadratic :1078-1098),
 // ray_in :217-344, find_dir miscellaneous.f90:48-82.
 //
-// Two kernels:
+// Kernels:
 //   k_line_table   per (node, line): the opacity / emissivity factors that
 //                  ray_in rebuilds for every (direction, channel, cell):
 //                  A = kv * c/nu / (sqrt(pi) b) * tx*dx   (optical depth per
 //                  trace step per unit Gaussian profile value), E the same
 //                  for the emissivity, and the dust terms.  HBM-bound, tiny.
-//   k_radiation_field  one warp per node (persistent warps, node queue);
-//                  the directions of legendre_all in batches of 32 rays:
+//   k_radiation_field  one warp per node (persistent warps, node queue) or,
+//                  for small clouds, per range of rays, whose sums
+//                  k_rf_finish adds per node; the directions of
+//                  legendre_all in batches of 32 rays:
 //                   (1) FP64 set-up, one lane per ray: the direction
 //                       (find_dir's rotation in closed form) and the
 //                       sphere-exit distance (pos_quadratic from the node,
@@ -105,20 +107,20 @@ inline int max_line_group() {
     return RF_MAX_GROUP;
 }
 
-// Ray-range items: sums the items' per-ray channel sums of every node in ray
-// order (one warp per node, lane = line), as the whole-node items do.
-__global__ void __launch_bounds__(128) k_rf_finish(RFArgs a, int per_node, int split) {
+// Items of rays: sums the rays' channel sums of every node in ray order (one
+// warp per node, lane = line), as the whole-node items do.
+__global__ void __launch_bounds__(128) k_rf_finish(RFArgs a, int split) {
     const int lane = threadIdx.x & 31;
     const int node = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
     if (node >= a.bulk) return;
     int st = 0, seg = 0;
-    for (int p = 0; p < per_node; p++) {
-        const int s = a.iseg[(size_t)node * per_node + p];
-        if (s < 0) {   // the walks stop at this item, as the whole-node loop does
+    for (int r0 = 0; r0 < a.ndir; r0 += 32) {
+        const int s = (r0 + lane < a.ndir) ? a.iseg[(size_t)node * a.ndir + r0 + lane] : 0;
+        if (__any_sync(0xffffffffu, s < 0)) {   // the walks stop at these rays, as the whole-node loop does
             st = PORTAL_NODE_DEPTH;
             break;
         }
-        seg += s;
+        seg += __reduce_add_sync(0xffffffffu, s);
     }
     const bool on = st == 0 && a.ab[node] > 0.0;
     const int L = a.L;
@@ -161,28 +163,45 @@ __global__ void __launch_bounds__(128) k_rf_finish(RFArgs a, int per_node, int s
     }
 }
 
-// Rays per item: 0 (a warp per node) for clouds of many nodes; smaller ones
-// are split into ray ranges, so that every resident warp has several items
-// and the last ones to finish do not leave the GPU idle.
-inline int rays_per_item(const RFArgs &a, bool split, long long resident) {
-    if (a.bulk >= 16 * resident || a.ndir <= 8) return 0;
-    if ((double)a.bulk * a.ndir * (a.L * (split ? 3 : 1) * 4 + 16) > 2e9) return 0;   // scratch limit
-    for (int r : {32, 16})
-        if ((long long)a.bulk * ((a.ndir + r - 1) / r) >= 4 * resident) return r;
-    return 8;
+// Whether the items are rays, not nodes, and how many of 32, 16 and 8 rays:
+// full walks first, shorter ones behind, so that the last items to finish do
+// not leave the GPU idle; 16 rays a resident warp in sixteens, 4 in eights
+// (measured from 0 to 32 and 2 to 16 of each: 1,024 points 0.148 ms (0.216
+// with thirty-twos to the end), 4,096 points 1.69 (1.73), 6,001 with dust 4.85
+// (5.10), 34 passes over 2,500 16.3 (16.3; in eights alone 20.2)).  No more
+// than a node's rays, so that an item has two nodes at most.  From 16 nodes a
+// resident warp on the nodes themselves balance.
+bool ray_items(RFArgs &a, bool split, long long resident) {
+    if (a.bulk >= 16 * resident || a.ndir <= 8) return false;
+    const long long rays = (long long)a.bulk * a.ndir;
+    if ((double)rays * (a.L * (split ? 3 : 1) * 4 + 20) > 2e9) return false;   // scratch limit
+    const long long eights = std::min(rays, 4 * resident), sixteens = std::min(rays - eights, 16 * resident);
+    a.items32 = a.ndir >= 32 ? (int)((rays - eights - sixteens) / 32) : 0;
+    a.items16 = a.ndir >= 16 ? (int)((rays - eights - 32LL * a.items32) / 16) : 0;
+    return true;
+}
+
+template <bool FLAT>
+const void *rf_kernel(const RFShape &sh, bool dust, bool split) {
+    const int slots = sh.nslot == 1 ? 1 : sh.nslot % 2 == 0 ? 2 : 0;
+    return dust         ? rf_kernel_dust<FLAT>(sh.nlg, slots)
+           : slots == 1 ? rf_kernel_one<FLAT>(sh.nlg, split)
+           : slots == 0 ? rf_kernel_any<FLAT>(sh.nlg)
+           : split      ? rf_kernel_even_split<FLAT>(sh.nlg)
+                        : rf_kernel_even<FLAT>(sh.nlg);
 }
 
 int launch_rf(portal_ctx *c, RFArgs &a, int n_depth) {
     const bool dust = c->has_dust, split = a.JE != nullptr;
     const int rt = rf_remainder(a.nch, dust, a.L);
-    RFShape sh = rf_shape(a.L, max_line_group(), a.nch, dust, rt, split);
-    const int slots = sh.nslot == 1 ? 1 : sh.nslot % 2 == 0 ? 2 : 0;
-    const void *kern = dust         ? rf_kernel_dust(sh.nlg, slots)
-                       : slots == 1 ? rf_kernel_one(sh.nlg, split)
-                       : slots == 0 ? rf_kernel_any(sh.nlg)
-                       : split      ? rf_kernel_even_split(sh.nlg)
-                                    : rf_kernel_even(sh.nlg);
     const size_t table = (a.nch * sizeof(float2) + 15) & ~(size_t)15;
+    RFShape sh = rf_shape(a.L, max_line_group(), a.nch, dust, rt, split);
+    // about the warps resident: what the registers (the kernel's launch bounds)
+    // and shared memory leave room for
+    const long long fit = std::max<long long>(1, (224LL * 1024) / (sh.bytes + (long long)table / 4));
+    const bool flat = ray_items(a, split, c->sm_count * std::min(fit, sh.nlg <= 4 ? 24LL : 16LL));
+    if (flat) sh = rf_shape(a.L, max_line_group(), a.nch, dust, rt, split, 2);
+    const void *kern = flat ? rf_kernel<true>(sh, dust, split) : rf_kernel<false>(sh, dust, split);
     int wpb = rf_warps();
     while (wpb > 1 && table + (size_t)wpb * sh.bytes > 200 * 1024) wpb--;   // many lines and channels
     const size_t dyn = table + (size_t)wpb * sh.bytes;
@@ -196,14 +215,10 @@ int launch_rf(portal_ctx *c, RFArgs &a, int n_depth) {
         if (--nb < 1) return set_err(c, PORTAL_ERR_NOMEM, "walk scratch allocation failed");
     }
     const int grid = nb * c->sm_count;
-    const size_t nslots = (size_t)grid * wpb;
     a.walk = c->walk.p;
-    a.rays_per_item = rays_per_item(a, split, (long long)nslots);
-    const int per_node = a.rays_per_item ? (a.ndir + a.rays_per_item - 1) / a.rays_per_item : 1;
-    if (a.rays_per_item) {
+    if (flat) {
         const size_t rays = (size_t)a.bulk * a.ndir;
-        if (c->vray.reserve(rays * a.L * (split ? 3 : 1)) || c->dray.reserve(rays) ||
-            c->iseg.reserve((size_t)a.bulk * per_node))
+        if (c->vray.reserve(rays * a.L * (split ? 3 : 1)) || c->dray.reserve(rays) || c->iseg.reserve(rays))
             return set_err(c, PORTAL_ERR_NOMEM, "ray sums");
         a.vray = c->vray.p; a.dray = c->dray.p; a.iseg = c->iseg.p;
     }
@@ -211,7 +226,7 @@ int launch_rf(portal_ctx *c, RFArgs &a, int n_depth) {
     RFBatch none{};
     void *args[] = {&a, &none, &sh};
     PCHECK(c, cudaLaunchKernel(kern, dim3(grid), dim3(32 * wpb), args, dyn, c->stream));
-    if (a.rays_per_item && a.bulk > 0) k_rf_finish<<<(a.bulk + 3) / 4, 128, 0, c->stream>>>(a, per_node, split);
+    if (flat && a.bulk > 0) k_rf_finish<<<(a.bulk + 3) / 4, 128, 0, c->stream>>>(a, split);
     timer_stop(c, T_RF);
     PCHECK(c, cudaGetLastError());
     return PORTAL_OK;
@@ -360,7 +375,7 @@ int rf_prepare(portal_ctx *c, int nth, int nph, int nvel, const double *gvec, do
     a.LS = split ? c->LS.p : nullptr;
     a.walk = nullptr;
     a.frames = c->frames.p;
-    a.rays_per_item = 0;
+    a.items32 = a.items16 = 0;
     a.vray = nullptr; a.dray = nullptr; a.iseg = nullptr;
     // the line table's transfer step (main_para.f90:135 dx times r_max)
     c->rf_dxp = c->tx * dx;

@@ -2,19 +2,24 @@
 // (compiled apart so that the instantiations build in parallel).
 #include "rf_kernel.cuh"
 
+#ifndef RF_FLAT
+#define RF_FLAT false
+#endif
+
 namespace portal {
-const void *rf_kernel_even(int nlg) {
+template <>
+const void *rf_kernel_even<RF_FLAT>(int nlg) {
     switch (nlg) {
-    case 1: return (const void *)k_radiation_field<1, false, false, 2, false>;
-    case 2: return (const void *)k_radiation_field<2, false, false, 2, false>;
-    case 3: return (const void *)k_radiation_field<3, false, false, 2, false>;
-    case 4: return (const void *)k_radiation_field<4, false, false, 2, false>;
-    case 5: return (const void *)k_radiation_field<5, false, false, 2, false>;
-    case 6: return (const void *)k_radiation_field<6, false, false, 2, false>;
-    case 7: return (const void *)k_radiation_field<7, false, false, 2, false>;
-    case 8: return (const void *)k_radiation_field<8, false, false, 2, false>;
-    case 9: return (const void *)k_radiation_field<9, false, false, 2, false>;
-    default: return (const void *)k_radiation_field<10, false, false, 2, false>;
+    case 1: return (const void *)k_radiation_field<1, false, false, 2, false, RF_FLAT>;
+    case 2: return (const void *)k_radiation_field<2, false, false, 2, false, RF_FLAT>;
+    case 3: return (const void *)k_radiation_field<3, false, false, 2, false, RF_FLAT>;
+    case 4: return (const void *)k_radiation_field<4, false, false, 2, false, RF_FLAT>;
+    case 5: return (const void *)k_radiation_field<5, false, false, 2, false, RF_FLAT>;
+    case 6: return (const void *)k_radiation_field<6, false, false, 2, false, RF_FLAT>;
+    case 7: return (const void *)k_radiation_field<7, false, false, 2, false, RF_FLAT>;
+    case 8: return (const void *)k_radiation_field<8, false, false, 2, false, RF_FLAT>;
+    case 9: return (const void *)k_radiation_field<9, false, false, 2, false, RF_FLAT>;
+    default: return (const void *)k_radiation_field<10, false, false, 2, false, RF_FLAT>;
     }
 }
 }  // namespace portal

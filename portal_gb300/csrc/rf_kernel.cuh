@@ -320,7 +320,8 @@ __host__ __device__ inline int rf_remainder(int nch, bool dust, int max_lines) {
     return (!dust && max_lines <= 32 && nch % 32 == 1 && (k == 1 || k == 2 || k == 4 || k == 8)) ? 1 : 0;
 }
 
-__host__ __device__ inline RFShape rf_shape(int L, int max_group, int nch, bool dust, int rt, bool split) {
+__host__ __device__ inline RFShape rf_shape(int L, int max_group, int nch, bool dust, int rt, bool split,
+                                                    int rows = 1) {
     RFShape s;
     const int cap = dust ? (max_group < RF_MAX_GROUP_DUST ? max_group : RF_MAX_GROUP_DUST) : max_group;
     s.L = L;
@@ -338,7 +339,7 @@ __host__ __device__ inline RFShape rf_shape(int L, int max_group, int nch, bool 
     s.o_qd = o; o += 32 * 16;
     s.o_I = o; o += ((s.nslot / 2) * s.nlg + (s.nslot & 1) * s.npk) * 32 * 8;
     s.o_part = o; o += nq * s.npk * 32 * 8;
-    s.o_row = o; o += s.groups * (dust ? 2 : 1) * s.npk * 16;
+    s.o_row = o; o += rows * s.groups * (dust ? 2 : 1) * s.npk * 16;
     s.o_bb = o; o += 2 * s.groups * 2 * s.npk * 4;
     s.o_om = o; o += rt ? 32 * s.om_ld * 4 : 0;
     s.o_v = o; o += nq * 32 * L * 4;
@@ -484,7 +485,7 @@ struct WarpMem {
 template <int NLG, int NSL, bool DUST, bool SPLIT>
 __device__ __forceinline__ void channel_pass(const RFShape &sh, const WarpMem &m, const float2 *chtab, int nch,
                                              int nvel, int lane, int g, int s0, int nc, int tk, bool fast, bool first,
-                                             bool last, const float *bb, float fst0) {
+                                             bool last, const float *bb, const float4 *row0, float fst0) {
     constexpr int NP = NLG / 2, ODD = NLG & 1, NPK = NP + ODD;
     const bool split = SPLIT && sh.split;
     float2 I[NSL][NP > 0 ? NP : 1], Io;   // Io: the odd line's slots
@@ -586,7 +587,7 @@ __device__ __forceinline__ void channel_pass(const RFShape &sh, const WarpMem &m
     // central cell (inverse_rt.f90:320-339): no gate, profile at the node's own
     // b, then the weighted channel sum, slot by slot
     float2 *part = m.part(sh) + lane;
-    const float4 *row = m.row(sh) + g * (DUST ? 2 : 1) * NPK;
+    const float4 *row = row0 + g * (DUST ? 2 : 1) * NPK;
     const int np32 = sh.npk * 32;
     // the intensity after the cell; om and Ie: what L* and J_eff sum
     auto weigh = [&](float2 &I2, int k, float2 g0, float2 &om, float2 &Ie) {
@@ -658,14 +659,21 @@ __device__ __forceinline__ void channel_pass(const RFShape &sh, const WarpMem &m
     }
 }
 
+// The nodes of a batch of rays: one, or (FLAT) two, the second's from ray
+// `split` on, with its line row behind the first's.
+struct BatchNodes {
+    float dqfac[2];
+    int split;
+};
+
 // The channel integration of a warp's batch of nr walked rays: per ray and
 // line the weighted channel sum at the node (v), with split also those of
 // J_eff and L*.  One chunk of up to 32 cells at a time is staged in shared
 // memory (lane = cell); then lanes run over channels, pass by pass.
-template <int NLG, bool DUST, bool STAR, int SLOTS, bool SPLIT>
+template <int NLG, bool DUST, bool STAR, int SLOTS, bool SPLIT, bool FLAT>
 __device__ __forceinline__ void integrate_batch(const RFArgs &a, const RFShape &sh, const WarpMem &m,
                                                 const RayBatch &B, unsigned smask, const float2 *chtab,
-                                                const int2 *walk, int nr, float dqfac, int lane) {
+                                                const int2 *walk, int nr, const BatchNodes &bn, int lane) {
     const unsigned FULL = 0xffffffffu;
     const bool split = SPLIT && sh.split;
     constexpr int NP = NLG / 2, ODD = NLG & 1, NPK = NP + ODD;
@@ -681,6 +689,9 @@ __device__ __forceinline__ void integrate_batch(const RFArgs &a, const RFShape &
     for (int rr = 0; rr < nr; rr++) {
         const int Kr = B.K[rr];
         const float4 d4 = B.dir[rr];
+        const bool second = FLAT && rr >= bn.split;
+        const float dqfac = second ? bn.dqfac[1] : bn.dqfac[0];
+        const float4 *row0 = m.row(sh) + (second ? sh.groups * (DUST ? 2 : 1) * NPK : 0);
         const float fst0 = (float)B.st0[rr];
         const float *bb0 = m.bb(sh) + ((STAR && ((smask >> rr) & 1u)) ? sh.groups * 2 * NPK : 0);
         for (int g = 0; g < sh.groups; g++) {
@@ -795,11 +806,11 @@ __device__ __forceinline__ void integrate_batch(const RFArgs &a, const RFShape &
                 if constexpr (SLOTS != 1)
                     for (; s0 + 1 < sh.nslot; s0 += 2)
                         channel_pass<NLG, 2, DUST, SPLIT>(sh, m, chtab, nch, nvel, lane, g, s0, nc, tk, fast, first,
-                                                          last, bb, fst0);
+                                                          last, bb, row0, fst0);
                 if constexpr (SLOTS != 2)
                     if (s0 < sh.nslot)
                         channel_pass<NLG, 1, DUST, SPLIT>(sh, m, chtab, nch, nvel, lane, g, s0, nc, tk, fast, first,
-                                                          last, bb, fst0);
+                                                          last, bb, row0, fst0);
                 if (last) break;
             }
             // the channel sums over the lanes, the remainder channel's share
@@ -821,7 +832,7 @@ __device__ __forceinline__ void integrate_batch(const RFArgs &a, const RFShape &
                 if (!DUST && sh.rt) {
                     __syncwarp();
                     if (lane < NLG && l0 + lane < L) {
-                        const float *row = reinterpret_cast<const float *>(m.row(sh) + g * NPK + (lane >> 1)) + (lane & 1);
+                        const float *row = reinterpret_cast<const float *>(row0 + g * NPK + (lane >> 1)) + (lane & 1);
                         const float2 ct = chtab[nch - 1];
                         const float x = row[0] * ct.x * fst0 * LOG2E_F;
                         const float om = one_minus_exp(x, ex2(-x));
@@ -839,9 +850,9 @@ __device__ __forceinline__ void integrate_batch(const RFArgs &a, const RFShape &
 // any line count in one launch)
 template <int NLG, bool DUST, int SLOTS, bool SPLIT>
 __device__ __noinline__ void integrate_any_width(const RFArgs &a, const RFShape &sh, const WarpMem &m, const RayBatch &B,
-                                        unsigned smask, const float2 *chtab, const int2 *walk, int nr, float dqfac,
-                                        int lane) {
-    integrate_batch<NLG, DUST, true, SLOTS, SPLIT>(a, sh, m, B, smask, chtab, walk, nr, dqfac, lane);
+                                        unsigned smask, const float2 *chtab, const int2 *walk, int nr,
+                                        const BatchNodes &bn, int lane) {
+    integrate_batch<NLG, DUST, true, SLOTS, SPLIT, false>(a, sh, m, B, smask, chtab, walk, nr, bn, lane);
 }
 
 // FP32 sums over rays, in ray order.
@@ -874,13 +885,20 @@ __device__ __forceinline__ float moment_add(float km, int k, float w, float v, f
 // 0.498 -> 0.455).
 // BATCH: the work items are (model, node) pairs of many models (RFBatch);
 // each warp copies the argument block of its current model into shared
-// memory.  Otherwise the nodes of the one model a0, or -- a0.rays_per_item >
-// 0 -- their ray ranges: small clouds have too few nodes to fill the GPU with
-// a warp per node, so each item is a part of a node's rays and stores their
-// per-line channel sums, which k_rf_finish adds up in ray order afterwards
-// (the same sums in the same order).
-template <int NLG, bool DUST, bool BATCH, int SLOTS, bool SPLIT>
+// memory.  Otherwise the nodes of the one model a0.
+// FLAT: small clouds have too few nodes to fill the GPU with a warp per node.
+// The items are 32, 16 or 8 consecutive rays of all nodes' rays in a row (of
+// two nodes at most) and store the rays' per-line channel sums, which
+// k_rf_finish adds up in ray order afterwards (the same sums in the same
+// order).  Cut across the nodes the walk's lanes are full: as ranges of one
+// node's rays, 2,500 points of 44 directions had to be cut into eights to
+// balance, which walk with 8 lanes of 32 (0.512 -> 0.480 ms a pass).
+// What bounds it there (4,096 points, 4 lines, 65 channels): the load/store
+// unit, 70 % of its cycles (the walk's scattered 16-byte loads and the staged
+// cells), and issue, 71 %; the FMA pipe 51 %.
+template <int NLG, bool DUST, bool BATCH, int SLOTS, bool SPLIT, bool FLAT = false>
 __global__ void __launch_bounds__(256, (NLG >= 1 && NLG <= 4) ? 3 : 2) k_radiation_field(RFArgs a0, RFBatch bw, RFShape sh0) {
+    static_assert(!(BATCH && FLAT), "batched items are whole nodes");
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
@@ -915,12 +933,12 @@ __global__ void __launch_bounds__(256, (NLG >= 1 && NLG <= 4) ? 3 : 2) k_radiati
     if (!BATCH) fill_bb(a0, sh0);
     __syncthreads();
 
-    const int rpi = BATCH ? 0 : a0.rays_per_item;
-    const int per_node = rpi ? (a0.ndir + rpi - 1) / rpi : 1;
     unsigned long long nseg = 0;
     int cur_model = -1;
     for (;;) {
-        int node = 0, part = 0;
+        int node = 0;
+        long long ray0 = 0;   // FLAT: the item's first ray,
+        int item_rays = 0;    // and rays
         if (BATCH) {
             long long item = 0;
             if (lane == 0) item = (long long)atomicAdd(&bw.queue[0], 1ULL);
@@ -943,18 +961,30 @@ __global__ void __launch_bounds__(256, (NLG >= 1 && NLG <= 4) ? 3 : 2) k_radiati
             long long item = 0;
             if (lane == 0) item = (long long)atomicAdd(&a0.counters[0], 1ULL);
             item = __shfl_sync(FULL, item, 0);
-            if (item >= (long long)a0.bulk * per_node) break;
-            node = (int)(item / per_node);
-            part = (int)(item - (long long)node * per_node);
+            if constexpr (FLAT) {
+                const long long i16 = item - a0.items32, i8 = i16 - a0.items16, all = (long long)a0.bulk * a0.ndir;
+                item_rays = i16 < 0 ? 32 : i8 < 0 ? 16 : 8;
+                ray0 = i16 < 0 ? 32 * item : 32LL * a0.items32 + (i8 < 0 ? 16 * i16 : 16LL * a0.items16 + 8 * i8);
+                if (ray0 >= all) break;
+                item_rays = (int)min((long long)item_rays, all - ray0);
+                node = (int)(ray0 / a0.ndir);
+            } else {
+                if (item >= a0.bulk) break;
+                node = (int)item;
+            }
         }
         const RFArgs &a = BATCH ? margs[wib] : a0;
         const RFShape &sh = BATCH ? mshape[wib] : sh0;
         int st = 0;
         int node_seg = 0;   // the item's ray segments (sum of node_count over its rays)
-        if (a.ab[node] > 0.0) {
-            if (lane < FRAME_N) B.frame[lane] = a.frames[FRAME_N * (size_t)node + lane];
-            if (lane < 6) B.km[lane] = 0.f;
-            __syncwarp();
+        BatchNodes bn;
+        bn.split = FLAT ? (int)min(32LL, (long long)(node + 1) * a.ndir - ray0) : 32;
+        if (FLAT || a.ab[node] > 0.0) {
+            if (!FLAT) {
+                if (lane < FRAME_N) B.frame[lane] = a.frames[FRAME_N * (size_t)node + lane];
+                if (lane < 6) B.km[lane] = 0.f;
+                __syncwarp();
+            }
             if constexpr (BATCH) {
                 if (lane == 0) {
                     if (a.star) {
@@ -967,9 +997,9 @@ __global__ void __launch_bounds__(256, (NLG >= 1 && NLG <= 4) ? 3 : 2) k_radiati
                 }
             }
             // the node's own line row, packed as the staged cells are
-            {
-                const float4 *lt = a.ltab + (size_t)node * sh.L;
-                float4 *row = m.row(sh);
+            for (int second = 0; second < (FLAT && bn.split < item_rays ? 2 : 1); second++) {
+                const float4 *lt = a.ltab + (size_t)(node + second) * sh.L;
+                float4 *row = m.row(sh) + second * sh.groups * (DUST ? 2 : 1) * sh.npk;
                 for (int i = lane; i < sh.groups * sh.npk; i += 32) {
                     const int l0 = (i / sh.npk) * sh.nlg, k = i % sh.npk;
                     const float4 v = lt[min(l0 + 2 * k, sh.L - 1)];
@@ -977,20 +1007,28 @@ __global__ void __launch_bounds__(256, (NLG >= 1 && NLG <= 4) ? 3 : 2) k_radiati
                     row[DUST ? 2 * i : i] = make_float4(v.x, w.x, v.y, w.y);
                     if (DUST) row[2 * i + 1] = make_float4(v.z, w.z, v.w, w.w);
                 }
-                for (int i = lane; i < ((SPLIT && sh.split) ? 8 : 4) * sh.L; i += 32) m.acc(sh)[i] = 0.f;
             }
+            if (!FLAT)
+                for (int i = lane; i < ((SPLIT && sh.split) ? 8 : 4) * sh.L; i += 32) m.acc(sh)[i] = 0.f;
             __syncwarp();
             int n_rays = a.ndir;
             if constexpr (BATCH) {
                 n_rays = B.sn[1];
                 if (n_rays < 0) st |= PORTAL_NODE_STAR;
             }
-            const float4 cvn = a.cellv[node];
-            const float dqfac = 2.f * cvn.w / (float)a.nvel;
-            const int kfirst = part * rpi, kend = rpi ? min(n_rays, kfirst + rpi) : n_rays;
-
-            for (int k0 = kfirst; st == 0 && k0 < kend; k0 += 32) {
-                const int nr = min(32, kend - k0);
+            // the ray's node (FLAT: of this lane's ray)
+            const int node_l = FLAT ? min(node + (lane >= bn.split), a.bulk - 1) : node;
+            const float4 cvn = a.cellv[node_l];
+            if constexpr (FLAT) {
+                const float q = 2.f * cvn.w / (float)a.nvel;
+                bn.dqfac[0] = __shfl_sync(FULL, q, 0);
+                bn.dqfac[1] = __shfl_sync(FULL, q, 31);
+                n_rays = item_rays;
+            } else {
+                bn.dqfac[0] = bn.dqfac[1] = 2.f * cvn.w / (float)a.nvel;
+            }
+            for (int k0 = 0; st == 0 && k0 < n_rays; k0 += 32) {
+                const int nr = min(32, n_rays - k0);
                 // ---- (1)+(2) set-up and walk, one lane per ray ----
                 int K = 0;
                 bool over = false;
@@ -1000,8 +1038,12 @@ __global__ void __launch_bounds__(256, (NLG >= 1 && NLG <= 4) ? 3 : 2) k_radiati
                     sray = a.star && lane < nr && k0 + lane < B.sn[0];
                     smask = __ballot_sync(FULL, sray);
                 }
-                if (lane < nr) {
-                    const double *f = B.frame;
+                if (FLAT && lane < nr) {
+                    B.dir[lane] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    B.st0[lane] = B.K[lane] = 0;
+                }
+                if (lane < nr && (!FLAT || a.ab[node_l] > 0.0)) {
+                    const double *f = FLAT ? a.frames + FRAME_N * (size_t)node_l : B.frame;
                     double mu, sth, cph, sph;
                     bool tab = true;
                     if constexpr (BATCH) {
@@ -1013,7 +1055,8 @@ __global__ void __launch_bounds__(256, (NLG >= 1 && NLG <= 4) ? 3 : 2) k_radiati
                         }
                     }
                     if (tab) {
-                        const double *dr = a.dirs + 6 * (size_t)(k0 + lane);
+                        const double *dr =
+                            a.dirs + 6 * (FLAT ? (size_t)(ray0 + lane - (long long)node_l * a.ndir) : (size_t)(k0 + lane));
                         mu = dr[0]; sth = dr[1]; cph = dr[2]; sph = dr[3];
                         B.wts[lane] = make_float2((float)dr[4], (float)dr[5]);
                     }
@@ -1031,7 +1074,7 @@ __global__ void __launch_bounds__(256, (NLG >= 1 && NLG <= 4) ? 3 : 2) k_radiati
                     float rh = (float)sexit, rl = (float)(sexit - (double)rh);
                     float rx = 0.f, ry = 0.f, rz = 0.f;
                     const bool step_ok = a.dx32 > 1e-20f && a.dx32 < 1e20f;   // quot_rn's range
-                    int wg = a.wstart[node];
+                    int wg = a.wstart[node_l];
                     for (;;) {
                         // the cell's block of the walk tables: its header, the first 12
                         // edges and where their neighbours' blocks start, all in
@@ -1103,25 +1146,30 @@ __global__ void __launch_bounds__(256, (NLG >= 1 && NLG <= 4) ? 3 : 2) k_radiati
                     }
                     B.K[lane] = K;
                 }
-                if (__any_sync(FULL, over)) { st |= PORTAL_NODE_DEPTH; break; }
-                node_seg += __reduce_add_sync(FULL, lane < nr ? K : 0);
+                if constexpr (FLAT) {   // (a walk past n_depth: its node's field is not used)
+                    if (over) B.K[lane] = 0;
+                    if (lane < nr) a.iseg[ray0 + lane] = over ? -1 : K;
+                } else {
+                    if (__any_sync(FULL, over)) { st |= PORTAL_NODE_DEPTH; break; }
+                    node_seg += __reduce_add_sync(FULL, lane < nr ? K : 0);
+                }
                 __syncwarp();
 
                 // ---- (3)+(4) channel integration of the batch's rays ----
                 if constexpr (NLG > 0) {
-                    integrate_batch<NLG, DUST, BATCH, SLOTS, SPLIT>(a, sh, m, B, smask, chtab, walk, nr, dqfac, lane);
+                    integrate_batch<NLG, DUST, BATCH, SLOTS, SPLIT, FLAT>(a, sh, m, B, smask, chtab, walk, nr, bn, lane);
                 } else {
                     switch (sh.nlg) {
 #define RF_WIDTH(n)                                                                                        \
-    case n: integrate_any_width<n, DUST, SLOTS, SPLIT>(a, sh, m, B, smask, chtab, walk, nr, dqfac, lane); break;
+    case n: integrate_any_width<n, DUST, SLOTS, SPLIT>(a, sh, m, B, smask, chtab, walk, nr, bn, lane); break;
                         RF_WIDTH(1) RF_WIDTH(2) RF_WIDTH(3) RF_WIDTH(4)
                     default:
                         if constexpr (DUST) {
-                            integrate_any_width<5, DUST, SLOTS, SPLIT>(a, sh, m, B, smask, chtab, walk, nr, dqfac, lane);
+                            integrate_any_width<5, DUST, SLOTS, SPLIT>(a, sh, m, B, smask, chtab, walk, nr, bn, lane);
                         } else {
                             switch (sh.nlg) {
                                 RF_WIDTH(5) RF_WIDTH(6) RF_WIDTH(7) RF_WIDTH(8) RF_WIDTH(9)
-                            default: integrate_any_width<10, DUST, SLOTS, SPLIT>(a, sh, m, B, smask, chtab, walk, nr, dqfac, lane);
+                            default: integrate_any_width<10, DUST, SLOTS, SPLIT>(a, sh, m, B, smask, chtab, walk, nr, bn, lane);
                             }
                         }
                     }
@@ -1129,8 +1177,8 @@ __global__ void __launch_bounds__(256, (NLG >= 1 && NLG <= 4) ? 3 : 2) k_radiati
                 }
                 const float *v = m.v(sh);
                 const int L = sh.L;
-                if (rpi) {   // the rays' channel sums and directions for k_rf_finish
-                    const size_t ray0 = (size_t)node * a.ndir + k0, plane = (size_t)a.bulk * a.ndir * L;
+                if constexpr (FLAT) {   // the rays' channel sums and directions for k_rf_finish
+                    const size_t plane = (size_t)a.bulk * a.ndir * L;
                     for (int q = 0; q < ((SPLIT && sh.split) ? 3 : 1); q++)
                         for (int i = lane; i < nr * L; i += 32) a.vray[q * plane + ray0 * L + i] = v[q * 32 * L + i];
                     if (lane < nr) a.dray[ray0 + lane] = B.dir[lane];
@@ -1157,12 +1205,7 @@ __global__ void __launch_bounds__(256, (NLG >= 1 && NLG <= 4) ? 3 : 2) k_radiati
                 __syncwarp();
             }
         }
-        if (rpi) {
-            if (lane == 0) a.iseg[(size_t)node * per_node + part] = st ? -1 : node_seg;
-            __syncwarp();
-            continue;
-        }
-        {
+        if constexpr (!FLAT) {
             const int L = a.L;
             const bool on = st == 0 && a.ab[node] > 0.0;
             const float *acc = m.acc(sh);
@@ -1185,8 +1228,8 @@ __global__ void __launch_bounds__(256, (NLG >= 1 && NLG <= 4) ? 3 : 2) k_radiati
         nseg += (unsigned long long)node_seg;
         __syncwarp();
     }
-    // segment count (every lane holds the same count; k_rf_finish counts ray-range items)
-    if (lane == 0 && !rpi) atomicAdd(BATCH ? &bw.queue[1] : &a0.counters[1], nseg);
+    // segment count (every lane holds the same count; k_rf_finish counts rays' items)
+    if (lane == 0 && !FLAT) atomicAdd(BATCH ? &bw.queue[1] : &a0.counters[1], nseg);
 }
 
 
