@@ -92,7 +92,7 @@ RFBatch rf_batch(portal_batch *b, const int2 *items, long long n_items, int nlg)
 int enqueue_pass(portal_batch *b, const int2 *items, long long n_items) {
     int rc;
     for (size_t m = 0; m < b->models.size(); m++)
-        if ((rc = rf_pass(b->models[m], b->rf[m], b->stream)))
+        if ((rc = rf_pass(b->models[m], b->rf[m], b->nlg, b->dust, b->stream)))
             return bfail(b, rc, "model " + std::to_string(m) + ": " + b->models[m]->err);
     BCHECK(b, cudaMemsetAsync(b->queue.p, 0, 2 * sizeof(unsigned long long), b->stream));
     const RFBatch rb = rf_batch(b, items, n_items, b->nlg);
@@ -281,12 +281,13 @@ extern "C" int portal_batch_prepare(portal_batch *b, int nth, int nph, int nvel,
 
     b->tune.clear();
     if (autotune) {
-        // line tables for the trials (the trials' results are overwritten by
-        // every later pass)
-        for (int m = 0; m < M; m++)
-            if (int rc = rf_pass(b->models[m], b->rf[m], b->stream)) return bfail(b, rc, b->models[m]->err);
         double best = 1e300;
         for (const RFC &c : rfc) {
+            // this trial's line tables (the results are overwritten by every
+            // later pass)
+            for (int m = 0; m < M; m++)
+                if (int rc = rf_pass(b->models[m], b->rf[m], c.nlg, b->dust, b->stream))
+                    return bfail(b, rc, b->models[m]->err);
             const RFBatch rb = rf_batch(b, b->sample.p, b->n_sample, c.nlg);
             double ms = 0.0;
             int rc = time_launch(b, [&]() { return rf_batch_launch(b->stream, c.bps * b->sm_count, b->dust, rb); }, &ms);

@@ -124,7 +124,7 @@ struct SEBatch {
 // rf.cu
 int rf_prepare(portal_ctx *c, int nth, int nph, int nvel, const double *gvec, double dx, int n_depth,
                bool split, RFArgs *a);
-int rf_pass(portal_ctx *c, const RFArgs &a, cudaStream_t s);
+int rf_pass(portal_ctx *c, const RFArgs &a, int max_group, bool dust, cudaStream_t s);
 // the single-model kernel for groups of nlg lines (1..10, with dust 1..5); FLAT:
 // its items are ranges of rays, not nodes
 template <bool FLAT> const void *rf_kernel_one(int nlg, bool split);    // one slot of channels

@@ -283,6 +283,14 @@ int dispatch_rf(portal_ctx *c, RFArgs &a, int n_depth) {
 
 namespace portal {
 
+// float4 per node of the widest line table any launch asks for
+static size_t ltab_width(int L) {
+    int w = 0;
+    for (int group : {3, 4, 5, RF_MAX_GROUP})
+        for (bool dust : {false, true}) w = std::max(w, tab_shape(L, group, dust).width);
+    return (size_t)w;
+}
+
 size_t rf_walk_records(int n_depth) { return (size_t)1024 * (size_t)((n_depth + 31) / 32); }
 
 // Validates the call, uploads the molecule's line constants and the
@@ -339,7 +347,7 @@ int rf_prepare(portal_ctx *c, int nth, int nph, int nvel, const double *gvec, do
         }
     }
     if (c->dirtab.reserve(6 * (size_t)ndir) || c->chtab.reserve(2 * (size_t)nch) ||
-        c->ltab.reserve((size_t)L * N) || c->J0.reserve((size_t)L * N) || c->J2.reserve((size_t)L * N) ||
+        c->ltab.reserve((size_t)N * ltab_width(L)) || c->J0.reserve((size_t)L * N) || c->J2.reserve((size_t)L * N) ||
         c->nodeseg.reserve((size_t)N) || c->frames.reserve(FRAME_N * (size_t)N) || c->kmom.reserve((size_t)6 * N))
         return set_err(c, PORTAL_ERR_NOMEM, "radiation-field buffers");
     if (split && (c->JE.reserve((size_t)L * N) || c->LS.reserve((size_t)L * N)))
@@ -385,13 +393,15 @@ int rf_prepare(portal_ctx *c, int nth, int nph, int nvel, const double *gvec, do
 
 // The per-pass device work before the walk: zeroed outputs and counters, node
 // frames and the line table from the current populations.  Stream-ordered only (capturable).
-int rf_pass(portal_ctx *c, const RFArgs &a, cudaStream_t s) {
+// max_group (0: the model's own launch) and dust: the launch the table is for.
+int rf_pass(portal_ctx *c, const RFArgs &a, int max_group, bool dust, cudaStream_t s) {
     const int L = c->r_num, N = c->N;
     const long long tot = (long long)N * L;
     const int table_blocks = (int)((tot + 255) / 256);
     k_line_table<<<table_blocks + (std::max(N, 8) + 255) / 256, 256, 0, s>>>(
         N, L, c->rf_dxp, reinterpret_cast<const LineConst *>(c->linebuf.p), c->levp.p, c->nlev, c->b64.p,
-        c->dustp.p, c->tdust.p, c->ltab.p, a, table_blocks);
+        c->dustp.p, c->tdust.p, c->ltab.p, tab_shape(L, max_group ? max_group : max_line_group(), dust), a,
+        table_blocks);
     PCHECK(c, cudaGetLastError());
     return PORTAL_OK;
 }
@@ -406,7 +416,7 @@ int enqueue_radiation_field(portal_ctx *c, int nth, int nph, int nvel, const dou
     if (rc) return rc;
     c->ali_valid = false;
     timer_start(c, T_LINETAB);
-    if ((rc = rf_pass(c, a, c->stream))) return rc;
+    if ((rc = rf_pass(c, a, 0, c->has_dust, c->stream))) return rc;
     timer_stop(c, T_LINETAB);
     return dispatch_rf(c, a, n_depth);
 }

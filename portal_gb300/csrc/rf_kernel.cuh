@@ -107,6 +107,29 @@ __device__ __forceinline__ double sphere_exit_unit(double px, double py, double 
     return __fma_rn(__fma_rn(-q, a2, n), 0.5, q);
 }
 
+constexpr int RF_MAX_GROUP = 10;          // lines per group without dust
+constexpr int RF_MAX_GROUP_DUST = 5;      // with dust (a wider body costs more in registers than it gains)
+
+// The line table's layout: a node's row holds its lines as the cells are staged,
+// group by group in packs of two lines, (A, A', S, S') and, with dust, (Ad,
+// Ad', Jd, Jd'): one 16-byte load a pack where (A, S, Ad, Jd) per line took
+// two of 8, half of the bytes unused.  (Field kernels: 65,536 points x 9 lines
+// 309 -> 305 ms, 8,192 x 19 76.6 -> 75.2, 4,096 x 4 1.69 -> 1.67, 6,001 x 7 with
+// dust 4.83 -> 4.72.)
+struct TabShape {
+    int nlg, npk, dust, width;   // width: float4 per node
+};
+__host__ __device__ inline TabShape tab_shape(int L, int max_group, bool dust) {
+    TabShape t;
+    const int cap = (dust && max_group > RF_MAX_GROUP_DUST) ? RF_MAX_GROUP_DUST : max_group;
+    const int groups = (L + cap - 1) / cap;
+    t.nlg = (L + groups - 1) / groups;
+    t.npk = (t.nlg + 1) / 2;
+    t.dust = dust;
+    t.width = groups * (dust ? 2 : 1) * t.npk;
+    return t;
+}
+
 // Line table and zeroed fields, one thread per (node, line), and -- the blocks
 // after its own -- the node frames and what else a pass starts from zero, one
 // thread per node.  (One launch instead of nine: at 1,700 nodes the memsets
@@ -114,7 +137,7 @@ __device__ __forceinline__ double sphere_exit_unit(double px, double py, double 
 __global__ void k_line_table(int N, int L, double dxp, const LineConst *__restrict__ lines,
                              const double *__restrict__ levp, int nlev, const double *__restrict__ b,
                              const double *__restrict__ dustp, const double *__restrict__ tdust,
-                             float4 *__restrict__ ltab, RFArgs a, int table_blocks) {
+                             float4 *__restrict__ ltab, TabShape ts, RFArgs a, int table_blocks) {
     if ((int)blockIdx.x >= table_blocks) {
         const int node = (int)((blockIdx.x - table_blocks) * blockDim.x + threadIdx.x);
         if (node < 8) a.counters[node] = 0;
@@ -149,12 +172,25 @@ __global__ void k_line_table(int N, int L, double dxp, const LineConst *__restri
         double c2b = 4.79924e-11 / Td;
         Ibb = 1.4744995e-50 * lc.nu * lc.nu * lc.nu / (exp(c2b * lc.nu) - 1.0);
     }
-    // (optical depth per trace step at unit profile, line source function
-    // ev/kv, dust optical depth per step, dust emissivity per step): the
-    // source function is stored as the FP64 ratio, not the emissivity, so a
-    // weak line's S keeps full FP32 precision where kv and ev alone would be
-    // FP32 denormals
-    ltab[t] = make_float4((float)(kv * phif), (float)(kv != 0.0 ? ev / kv : 0.0), (float)Ad, (float)(Ad * Ibb));
+    // optical depth per trace step at unit profile, line source function
+    // ev/kv and, with dust, dust optical depth per step, dust emissivity per
+    // step: the source function is stored as the FP64 ratio, not the
+    // emissivity, so a weak line's S keeps full FP32 precision where kv and ev
+    // alone would be FP32 denormals
+    const float A = (float)(kv * phif), S = (float)(kv != 0.0 ? ev / kv : 0.0);
+    const int g = l / ts.nlg, i0 = l - g * ts.nlg;
+    // (an odd group's last pack and a last group's padding repeat the line)
+    const int i1 = (l == L - 1 || i0 == ts.nlg - 1) ? 2 * ts.npk : i0 + 1;
+    float *row = reinterpret_cast<float *>(ltab + (size_t)n * ts.width);
+    for (int i = i0; i < i1; i++) {
+        float *p = row + 4 * ((ts.dust ? 2 : 1) * (g * ts.npk + i / 2)) + (i & 1);
+        p[0] = A;
+        p[2] = S;
+        if (ts.dust) {
+            p[4] = (float)Ad;
+            p[6] = (float)(Ad * Ibb);
+        }
+    }
 }
 
 constexpr double PI_D = 3.141592653589793;  // acos(-1.d0)
@@ -309,9 +345,6 @@ struct RFShape {
     int rec_ld, om_ld;                    // row strides: float4 per cell, float per cell
     int o_rec, o_qd, o_om, o_I, o_part, o_v, o_acc, o_row, o_bb, bytes;   // byte offsets in the warp's block
 };
-constexpr int RF_MAX_GROUP = 10;          // lines per group without dust
-constexpr int RF_MAX_GROUP_DUST = 5;      // with dust (a wider body costs more in registers than it gains)
-
 // The remainder channel: 2 nvel + 1 channels with nvel a multiple of 16 are
 // whole slots and one channel more, which the lanes-over-lines pass takes (no
 // dust, at most 32 lines); any other count is padded to whole slots.
@@ -323,11 +356,11 @@ __host__ __device__ inline int rf_remainder(int nch, bool dust, int max_lines) {
 __host__ __device__ inline RFShape rf_shape(int L, int max_group, int nch, bool dust, int rt, bool split,
                                                     int rows = 1) {
     RFShape s;
-    const int cap = dust ? (max_group < RF_MAX_GROUP_DUST ? max_group : RF_MAX_GROUP_DUST) : max_group;
+    const TabShape t = tab_shape(L, max_group, dust);
     s.L = L;
-    s.groups = (L + cap - 1) / cap;
-    s.nlg = (L + s.groups - 1) / s.groups;
-    s.npk = (s.nlg + 1) / 2;
+    s.groups = t.width / ((dust ? 2 : 1) * t.npk);
+    s.nlg = t.nlg;
+    s.npk = t.npk;
     s.rt = rt;
     s.split = split;
     s.nslot = (nch - rt + 31) / 32;
@@ -679,6 +712,7 @@ __device__ __forceinline__ void integrate_batch(const RFArgs &a, const RFShape &
     constexpr int NP = NLG / 2, ODD = NLG & 1, NPK = NP + ODD;
     const int L = a.L, nch = a.nch, nvel = a.nvel;
     float4 *rec = m.rec(sh) + lane * sh.rec_ld;
+    const int width = sh.groups * (DUST ? 2 : 1) * NPK;   // the line table's
     // walk records of a chunk (lane = cell), the next chunk's -- of this ray,
     // the next line group or the next ray -- loaded while one is integrated
     int2 wcp = make_int2(0, 0);
@@ -720,19 +754,20 @@ __device__ __forceinline__ void integrate_batch(const RFArgs &a, const RFShape &
                 bool in_range = true;               // dust: the fast quotient serves this cell
                 if (lane < nc) {
                     const float4 cv = a.cellv[wc.x];
-                    const float4 *lt = a.ltab + (size_t)wc.x * L;
+                    const float4 *lt = a.ltab + (size_t)wc.x * width + g * (DUST ? 2 : 1) * NPK;
                     const float fst = (float)wc.y;
                     const float vp = fmaf(cv.z, d4.z, fmaf(cv.y, d4.y, __fmul_rn(cv.x, d4.x)));
                     const float ib = SQL2E_F * (1.f / cv.w);
                     const float2 qdl = make_float2((d4.w - vp) * ib, dqfac * ib);
                     m.qd(sh)[lane] = make_float4(qdl.x, qdl.x, qdl.y, qdl.y);
                     if constexpr (DUST) {
-                        float4 v[2 * NPK];
+                        float4 p[2 * NPK], v[2 * NPK];
 #pragma unroll
-                        for (int l = 0; l < NLG; l++) v[l] = lt[min(l0 + l, L - 1)];
+                        for (int k = 0; k < 2 * NPK; k++) p[k] = lt[k];
 #pragma unroll
                         for (int l = 0; l < NLG; l++) {
-                            const float4 t = v[l];
+                            const float4 q = p[l & ~1], r = p[l | 1];
+                            const float4 t = (l & 1) ? make_float4(q.y, q.w, r.y, r.w) : make_float4(q.x, q.z, r.x, r.z);
                             v[l] = make_float4(t.x * fst, t.y * t.x * fst, t.z * fst, t.w * fst);
                             in_range = in_range && dust_in_range(v[l]);
                             // |tau| <= |A| + |Ad|: the Taylor form in every channel
@@ -753,21 +788,19 @@ __device__ __forceinline__ void integrate_batch(const RFArgs &a, const RFShape &
                         // 0 < tau < 2^-54 rounds to a zero weight as in FP64, so
                         // the gate needs no test.  (The padding lines of a last group
                         // repeat its last line; nothing reads their sums.)
-                        float2 v[NLG];
+                        float4 v[NPK];   // (A, A', S, S')
 #pragma unroll
-                        for (int l = 0; l < NLG; l++)
-                            v[l] = *reinterpret_cast<const float2 *>(lt + min(l0 + l, L - 1));
+                        for (int k = 0; k < NPK; k++) v[k] = lt[k];
 #pragma unroll
-                        for (int l = 0; l < NLG; l++) {
-                            const bool on = v[l].x > 0.f;
-                            v[l].x = on ? v[l].x * fst * LOG2E_F : 0.f;
-                            v[l].y = on ? v[l].y : 0.f;
-                            if (!(v[l].x < OM_THIN_A)) thin &= ~(1u << (l / 2));
+                        for (int k = 0; k < NPK; k++) {
+                            const bool on0 = v[k].x > 0.f, on1 = v[k].y > 0.f;
+                            v[k].x = on0 ? v[k].x * fst * LOG2E_F : 0.f;
+                            v[k].y = on1 ? v[k].y * fst * LOG2E_F : 0.f;
+                            v[k].z = on0 ? v[k].z : 0.f;
+                            v[k].w = on1 ? v[k].w : 0.f;
+                            if (!(v[k].x < OM_THIN_A) || !(v[k].y < OM_THIN_A)) thin &= ~(1u << k);
+                            rec[k] = v[k];
                         }
-#pragma unroll
-                        for (int k = 0; k < NP; k++)
-                            rec[k] = make_float4(v[2 * k].x, v[2 * k + 1].x, v[2 * k].y, v[2 * k + 1].y);
-                        if (ODD) rec[NP] = make_float4(v[NLG - 1].x, v[NLG - 1].x, v[NLG - 1].y, v[NLG - 1].y);
                         if (sh.rt) {
                             // the remainder channel's transfer weight of this
                             // cell for the group's lines
@@ -776,13 +809,13 @@ __device__ __forceinline__ void integrate_batch(const RFArgs &a, const RFShape &
                             float *om = m.om(sh) + lane * sh.om_ld;
 #pragma unroll
                             for (int k = 0; k < NP; k++) {
-                                const float2 x = __fmul2_rn(make_float2(v[2 * k].x, v[2 * k + 1].x), make_float2(gr, gr));
+                                const float2 x = __fmul2_rn(make_float2(v[k].x, v[k].y), make_float2(gr, gr));
                                 const float2 w = one_minus_exp2(x, ex2(-x.x), ex2(-x.y));
                                 om[2 * k] = w.x;
                                 om[2 * k + 1] = w.y;
                             }
                             if (ODD) {
-                                const float x = v[NLG - 1].x * gr;
+                                const float x = v[NP].x * gr;
                                 om[NLG - 1] = one_minus_exp(x, ex2(-x));
                             }
                         }
@@ -996,17 +1029,11 @@ __global__ void __launch_bounds__(256, (NLG >= 1 && NLG <= 4) ? 3 : 2) k_radiati
                     }
                 }
             }
-            // the node's own line row, packed as the staged cells are
+            // the node's own line row
             for (int second = 0; second < (FLAT && bn.split < item_rays ? 2 : 1); second++) {
-                const float4 *lt = a.ltab + (size_t)(node + second) * sh.L;
-                float4 *row = m.row(sh) + second * sh.groups * (DUST ? 2 : 1) * sh.npk;
-                for (int i = lane; i < sh.groups * sh.npk; i += 32) {
-                    const int l0 = (i / sh.npk) * sh.nlg, k = i % sh.npk;
-                    const float4 v = lt[min(l0 + 2 * k, sh.L - 1)];
-                    const float4 w = lt[min(l0 + min(2 * k + 1, sh.nlg - 1), sh.L - 1)];
-                    row[DUST ? 2 * i : i] = make_float4(v.x, w.x, v.y, w.y);
-                    if (DUST) row[2 * i + 1] = make_float4(v.z, w.z, v.w, w.w);
-                }
+                const int width = sh.groups * (DUST ? 2 : 1) * sh.npk;
+                const float4 *lt = a.ltab + (size_t)(node + second) * width;
+                for (int i = lane; i < width; i += 32) m.row(sh)[second * width + i] = lt[i];
             }
             if (!FLAT)
                 for (int i = lane; i < ((SPLIT && sh.split) ? 8 : 4) * sh.L; i += 32) m.acc(sh)[i] = 0.f;
