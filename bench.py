@@ -93,7 +93,7 @@ def profile_constant(key):
 
 def traffic_per_segment():
     """DRAM bytes per ray segment of the radiation-field kernel (ncu)."""
-    return profile_constant("dram_bytes_per_segment")
+    return profile_constant("current_dram_bytes_per_segment")
 
 
 class ClockSampler:
@@ -733,7 +733,7 @@ def gpu_arm(args, rank, world, local_rank):
     # the kernel's actual bound is instruction issue (its data is L2-resident):
     # warp instructions per segment (ncu, profiles/) x segments / launch time
     # against one warp instruction per SMSP per cycle at the sampled SM clock
-    wips = profile_constant("warp_instructions_per_segment")
+    wips = profile_constant("current_warp_instructions_per_segment")
     if wips and clk and clk.get("sm_mhz"):
         import torch
         sms = torch.cuda.get_device_properties(0).multi_processor_count

@@ -229,15 +229,16 @@ __device__ bool team_lu(int n, T *M, int *piv, int tid, double *red_v, int *red_
     }
 }
 
-// Dynamic shared memory per team (one warp, or the block's team of warps):
+// Dynamic shared memory per team of the LU form (the inverses': GaussMem):
 //   feat [n_feat] double | x, r [n] double | LU32 [n*n] float | d32 [n] float
 //   | scale [n] float | piv [n] int
 // The FP64 matrix is kept as its entries only, row by row (a fifth of the
 // 74 x 74 systems, a third of the 34 x 34: collisions couple the K = 0
 // components of all levels, radiation only neighbouring levels): assembly, row
-// scaling and the refinement's residuals run over them.  They sit in a
+// scaling and the refinement's residuals run over them.  Here they sit in a
 // per-team slot of global memory, followed by the dense matrix of the FP64
-// fallback: kept out of shared memory they let 3x more warps share an SM.
+// fallback; the inverses, which need no dense copy, keep the entries in shared
+// memory.
 constexpr int NF = 7;  // features per transition
 constexpr int SE_GAUSS_DIM = 96;   // largest system inverted,
 constexpr int SE_WARP_DIM = 32;    // and by one warp in registers
