@@ -272,10 +272,11 @@ __host__ __device__ inline size_t se_warp_bytes(int n, int n_feat) {
 // slot is worked on without a test (branches a group of slots made it twice as
 // long), so the instances hold the next larger number of slots.
 // Measured, LU -> this (with the assembly in order of terms and the work of
-// the temperature once a node): 8,192 systems of 74 unknowns 2.29 -> 0.95 ms,
-// 8,192 of 39 1.51 -> 0.44 ms, 1,024 of 14 72 -> 29 us.  Of the 74 x 74
-// systems' time two thirds are the elimination (issue slots: 60 multiply-adds
-// in some 200 instructions a warp and step), the rest FP64 work.
+// the temperature once a node): 8,192 systems of 74 unknowns 2.29 -> 0.84 ms,
+// 8,192 of 39 1.51 -> 0.44 ms, 1,024 of 14 72 -> 26 us.  Of the 74 x 74
+// systems' time some two thirds are the elimination (issue slots; with its 60
+// multiply-adds a warp and step in packed pairs 0.92 -> 0.84 ms), the rest
+// FP64 work.
 //
 // Every form below (one warp or four, registers or shared memory) does the
 // same operations per element, so that their inverses are the same.
@@ -342,11 +343,14 @@ template <int MR, int NC>
 __device__ __forceinline__ void update_group(float (&a)[NC][MR], const float (&l)[MR], const float *row, int g) {
     const float4 s = *reinterpret_cast<const float4 *>(row + g);
 #pragma unroll
-    for (int m = 0; m < MR; m++) {
-        a[g][m] = fmaf(-l[m], s.x, a[g][m]);
-        a[g + 1][m] = fmaf(-l[m], s.y, a[g + 1][m]);
-        a[g + 2][m] = fmaf(-l[m], s.z, a[g + 2][m]);
-        a[g + 3][m] = fmaf(-l[m], s.w, a[g + 3][m]);
+    for (int m = 0; m < MR; m++) {   // (packed pairs: one issue slot for two multiply-adds)
+        const float2 ml = make_float2(-l[m], -l[m]);
+        const float2 p = __ffma2_rn(ml, make_float2(s.x, s.y), make_float2(a[g][m], a[g + 1][m]));
+        const float2 q = __ffma2_rn(ml, make_float2(s.z, s.w), make_float2(a[g + 2][m], a[g + 3][m]));
+        a[g][m] = p.x;
+        a[g + 1][m] = p.y;
+        a[g + 2][m] = q.x;
+        a[g + 3][m] = q.y;
     }
 }
 // slots [0, na) turn by R (na a multiple of R)
@@ -1483,7 +1487,7 @@ int se_batch_launch(cudaStream_t s, int grid, int warps_per_block, const SEBatch
 // the columns save it while one warp's registers hold them: 1,024 systems of
 // 14 unknowns 29 us by one warp, 41 by a team; 1,700 of 19 49 and 98 us.
 // Beyond its registers one warp works in shared memory: 8,192 of 39 0.86 ms,
-// a team 0.44; of 74 3.4 and 0.95.
+// a team 0.44; of 74 3.4 and 0.84.
 inline int se_team_warps(int n) {
     const char *e = getenv("PORTAL_SE_TEAM");
     if (e) {
