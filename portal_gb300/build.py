@@ -36,6 +36,8 @@ def _compile(src: str, verbose: bool) -> str:
     path = os.path.join(CSRC, src)
     deps = [path] + [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))]
     deps.append(os.path.join(ROOT, "include", "portal_gb300.h"))
+    if src.endswith("_flat.cu"):   # includes the source it is named after
+        deps.append(path.replace("_flat.cu", ".cu"))
     if os.path.exists(obj) and os.path.getmtime(obj) >= max(os.path.getmtime(d) for d in deps):
         return obj
     # host code uncontracted like the oracle (aarch64 g++ fuses a*b+c by default)
