@@ -704,10 +704,14 @@ struct BatchNodes {
 // J_eff and L*.  One chunk of up to 32 cells at a time is staged in shared
 // memory (lane = cell); then lanes run over channels, pass by pass.
 template <int NLG, bool DUST, bool STAR, int SLOTS, bool SPLIT, bool FLAT>
-__device__ __forceinline__ void integrate_batch(const RFArgs &a, const RFShape &sh, const WarpMem &m,
+__device__ __forceinline__ void integrate_batch(const RFArgs &a, const RFShape &shape, const WarpMem &m,
                                                 const RayBatch &B, unsigned smask, const float2 *chtab,
                                                 const int2 *walk, int nr, const BatchNodes &bn, int lane) {
     const unsigned FULL = 0xffffffffu;
+    // (copies: the batched kernel has both in shared memory, where every store
+    // to it would have them read again: six clouds in a batch 23.2 -> 22.6 ms)
+    const RFShape sh = shape;
+    const float4 *const cellv = a.cellv, *const ltab = a.ltab;
     const bool split = SPLIT && sh.split;
     constexpr int NP = NLG / 2, ODD = NLG & 1, NPK = NP + ODD;
     const int L = a.L, nch = a.nch, nvel = a.nvel;
@@ -753,8 +757,8 @@ __device__ __forceinline__ void integrate_batch(const RFArgs &a, const RFShape &
                 unsigned thin = (1u << NPK) - 1u;   // the packs thin in this cell
                 bool in_range = true;               // dust: the fast quotient serves this cell
                 if (lane < nc) {
-                    const float4 cv = a.cellv[wc.x];
-                    const float4 *lt = a.ltab + (size_t)wc.x * width + g * (DUST ? 2 : 1) * NPK;
+                    const float4 cv = cellv[wc.x];
+                    const float4 *lt = ltab + (size_t)wc.x * width + g * (DUST ? 2 : 1) * NPK;
                     const float fst = (float)wc.y;
                     const float vp = fmaf(cv.z, d4.z, fmaf(cv.y, d4.y, __fmul_rn(cv.x, d4.x)));
                     const float ib = SQL2E_F * (1.f / cv.w);
