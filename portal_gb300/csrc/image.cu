@@ -843,7 +843,6 @@ static int image_call(portal_ctx *c, const double *pol_pops, int nlines, const i
     long long batches = std::max(1, (nrays + 31) / 32);
     batches = std::min(batches, std::max<long long>(c->sm_count, (long long)(6e9 / (list * sizeof(int2)))));
     while (c->walk.reserve(batches * list) != cudaSuccess) {
-        cudaGetLastError();
         if ((batches /= 2) < 1) return set_err(c, PORTAL_ERR_NOMEM, "image walk scratch");
     }
     if (cnt.reserve(32 * batches) || on_star.reserve(32 * batches))

@@ -211,7 +211,6 @@ int launch_rf(portal_ctx *c, RFArgs &a, int n_depth) {
     if (nb < 1) nb = 1;
     // fewer blocks per SM where the device cannot hold the walk scratch of all
     while (c->walk.reserve((size_t)nb * c->sm_count * wpb * rf_walk_records(n_depth)) != cudaSuccess) {
-        cudaGetLastError();
         if (--nb < 1) return set_err(c, PORTAL_ERR_NOMEM, "walk scratch allocation failed");
     }
     const int grid = nb * c->sm_count;

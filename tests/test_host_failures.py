@@ -1,0 +1,88 @@
+"""What the library's host code does when a call of the CUDA runtime fails.
+
+Runs on the CPU: tests/fake_cudart.cpp stands in for the runtime (preloaded in
+a process of its own), kernels do nothing, and the failure is the error code
+that the stand-in returns."""
+import os
+import subprocess
+import sys
+import textwrap
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+PREAMBLE = """
+import ctypes as C, os, re
+import numpy as np
+import portal_gb300 as pg
+from portal_gb300 import synth
+
+fake = C.CDLL(os.environ["LD_PRELOAD"])
+fake.fake_log.restype = fake.fake_live_bytes.restype = C.c_size_t
+UNLIMITED = 2**64 - 1
+
+def memory(single=UNLIMITED, total=UNLIMITED):
+    fake.fake_memory(C.c_size_t(single), C.c_size_t(total))
+
+def live():
+    return fake.fake_live_bytes()
+
+def log(clear=True):
+    n = fake.fake_log(None, C.c_size_t(0))
+    b = C.create_string_buffer(n + 1)
+    fake.fake_log(b, C.c_size_t(n + 1))
+    if clear:
+        fake.fake_log_clear()
+    return b.value.decode().splitlines()
+
+def fails(code, f, *a, **k):
+    try:
+        f(*a, **k)
+    except pg.PortalError as e:
+        assert e.code == code, e
+        return
+    raise AssertionError("the call succeeded")
+
+CUDA_ERR, STATE, DEPTH, NOMEM = -1, -3, -4, -6
+
+def model(points=600, levels=4, seed=1):
+    mol = synth.linear_rotor(levels)
+    c = pg.Context(0)
+    c.set_molecule(mol)
+    c.set_cloud(synth.power_law_sphere(points, seed, mol))
+    return c
+
+def run(nth=6, nvel=8, kmax=2, n_depth=32):
+    return synth.RunConfig(nth=nth, nph=nth, nvel=nvel, kmax=kmax, n_depth=n_depth, gvec=synth.gauge_vector(3))
+"""
+
+
+@pytest.fixture(scope="session")
+def fake_cuda(built_lib, tmp_path_factory):
+    from portal_gb300 import build
+    inc = os.path.join(os.path.dirname(os.path.dirname(build._nvcc())), "include")
+    so = str(tmp_path_factory.mktemp("fake") / "fake_cudart.so")
+    subprocess.run([os.environ.get("CXX", "g++"), "-std=c++17", "-O1", "-fPIC", "-shared", "-I", inc,
+                    os.path.join(ROOT, "tests", "fake_cudart.cpp"), "-o", so], check=True)
+
+    def script(body, **env):
+        r = subprocess.run([sys.executable, "-c", PREAMBLE + textwrap.dedent(body)], cwd=ROOT, text=True,
+                           capture_output=True, timeout=120,
+                           env={**os.environ, "PYTHONPATH": ROOT, "LD_PRELOAD": so, "OMP_NUM_THREADS": "2", **env})
+        assert r.returncode == 0, r.stdout + r.stderr
+    return script
+
+
+def test_failed_allocation_does_not_fail_the_next_call(fake_cuda):
+    fake_cuda("""
+        c = model()
+        memory(single=14399)            # J0 takes 8 x 3 x 600 bytes
+        fails(NOMEM, c.radiation_field, run())
+        memory()
+        c.radiation_field(run())
+        memory(single=1 << 20)          # the FP64 matrices of the solve
+        fails(NOMEM, c.solve_se, 2)
+        memory()
+        c.solve_se(2)
+    """)
