@@ -345,14 +345,16 @@ int rf_prepare(portal_ctx *c, int nth, int nph, int nvel, const double *gvec, do
             ct[nch + i] = (float)(std::exp(-q0 * q0) * 2.0 / (spi * nvel));
         }
     }
+    // what is replaced is not kept: a growing buffer loses its contents, and a
+    // call that fails further down must not leave them marked as held
+    if (new_dirs) c->tab_nth = 0;
+    if (new_ch) c->tab_nvel = 0;
     if (c->dirtab.reserve(6 * (size_t)ndir) || c->chtab.reserve(2 * (size_t)nch) ||
         c->ltab.reserve((size_t)N * ltab_width(L)) || c->J0.reserve((size_t)L * N) || c->J2.reserve((size_t)L * N) ||
         c->nodeseg.reserve((size_t)N) || c->frames.reserve(FRAME_N * (size_t)N) || c->kmom.reserve((size_t)6 * N))
         return set_err(c, PORTAL_ERR_NOMEM, "radiation-field buffers");
     if (split && (c->JE.reserve((size_t)L * N) || c->LS.reserve((size_t)L * N)))
         return set_err(c, PORTAL_ERR_NOMEM, "split-field buffers");
-    c->tab_nth = c->tab_nvel = 0;   // (until the copies below are made)
-    c->lines_ready = false;
     if (new_dirs)
         PCHECK(c, cudaMemcpyAsync(c->dirtab.p, dt.data(), dt.size() * sizeof(double), cudaMemcpyHostToDevice,
                                   c->stream));

@@ -86,3 +86,22 @@ def test_failed_allocation_does_not_fail_the_next_call(fake_cuda):
         memory()
         c.solve_se(2)
     """)
+
+
+@pytest.mark.parametrize("nth,nvel", [(10, 8), (6, 60), (10, 60)])
+def test_failed_call_does_not_keep_tables_it_replaced(fake_cuda, nth, nvel):
+    """More angles or channels, then no memory for the split field: the tables
+    are new and empty by then, so the next call uploads its own again."""
+    fake_cuda(f"""
+        c = model()
+        c.radiation_field(run())
+        dirs, channels = [l for l in log() if l.startswith("h2d")][-2:]
+        memory(single=14399)            # J_eff takes 8 x 3 x 600 bytes
+        fails(NOMEM, c.radiation_field_split, run({nth}, {nvel}))
+        memory()
+        log()
+        c.radiation_field(run())
+        sent = log()
+        assert {nth} == 6 or dirs in sent, sent
+        assert {nvel} == 8 or channels in sent, sent
+    """)
