@@ -1289,7 +1289,7 @@ void build_program(const portal_ctx *c, int kmax, Program &P) {
 namespace portal {
 
 int prepare_se(portal_ctx *c, int kmax) {
-    if (c->se_kmax == kmax) return PORTAL_OK;
+    if (c->se_kmax == kmax && c->se_built) return PORTAL_OK;
     if (c->depol)
         for (int i = 0; i < c->nlev; i++)
             if (c->j_lev[i] != i)
@@ -1351,12 +1351,14 @@ int prepare_se(portal_ctx *c, int kmax) {
     const size_t o_asm = putI(sp_rec);
     size_t o_nu = putD(P.tr_nu), o_A = putD(P.tr_A), o_B = putD(P.tr_B21), o_tc = putD(P.term_c),
            o_nv = putD(norm_val), o_ct = putD(c->col_temps), o_C = putD(c->Cji), o_dep = putD(P.dep_tab);
+    c->se_built = false;   // (a growing buffer loses the program it held)
     if (c->se_ints.reserve(I.size()) || c->se_dbls.reserve(D.size()))
         return set_err(c, PORTAL_ERR_NOMEM, "SE program");
     PCHECK(c, cudaMemcpyAsync(c->se_ints.p, I.data(), I.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
     PCHECK(c, cudaMemcpyAsync(c->se_dbls.p, D.data(), D.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
     PCHECK(c, cudaStreamSynchronize(c->stream));
     c->se_kmax = kmax;
+    c->se_built = true;
     c->c_dim = P.c_dim;
     c->n_trans = P.n_trans;
     c->count_array = P.count_array;

@@ -105,3 +105,24 @@ def test_failed_call_does_not_keep_tables_it_replaced(fake_cuda, nth, nvel):
         assert {nth} == 6 or dirs in sent, sent
         assert {nvel} == 8 or channels in sent, sent
     """)
+
+
+def test_failed_solve_does_not_keep_a_program_it_replaced(fake_cuda):
+    """Memory for the larger program's integers, not for its coefficients: the
+    smaller one is uploaded again."""
+    fake_cuda("""
+        c, other = model(), model()
+        sizes = []
+        for ctx, kmax in ((other, 6), (c, 2)):
+            ctx.radiation_field(run(kmax=kmax))
+            log()
+            ctx.solve_se(kmax)
+            sizes.append([int(l.split()[1]) for l in log() if l.startswith("h2d")])
+        (big_i, big_d), (small_i, small_d) = sizes
+        memory(total=live() + big_i + big_d - small_i - small_d - 1)
+        fails(NOMEM, c.solve_se, 6)
+        memory()
+        log()
+        c.solve_se(2)
+        assert [int(l.split()[1]) for l in log() if l.startswith("h2d")] == [small_i, small_d]
+    """)
