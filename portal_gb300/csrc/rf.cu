@@ -245,6 +245,7 @@ int launch_rf_star(portal_ctx *c, RFArgs &a, int n_depth) {
     const int grid = nb * c->sm_count;
     if (c->walk.reserve((size_t)grid * RF_BATCH_WARPS * rf_walk_records(n_depth)) != cudaSuccess)
         return set_err(c, PORTAL_ERR_NOMEM, "walk scratch allocation failed");
+    if (c->star_items_n != c->bulk) c->star_items_n = -1;   // (a growing buffer loses its items)
     if (c->star_model.reserve(sizeof(RFArgs)) || c->star_items.reserve(c->bulk > 0 ? c->bulk : 1))
         return set_err(c, PORTAL_ERR_NOMEM, "star-mode work items");
     if (c->star_items_n != c->bulk) {

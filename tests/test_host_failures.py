@@ -126,3 +126,34 @@ def test_failed_solve_does_not_keep_a_program_it_replaced(fake_cuda):
         c.solve_se(2)
         assert [int(l.split()[1]) for l in log() if l.startswith("h2d")] == [small_i, small_d]
     """)
+
+
+def test_failed_star_call_does_not_keep_items_it_replaced(fake_cuda):
+    """A larger cloud whose star-mode items do not fit, then the first cloud
+    again: its items are uploaded again."""
+    fake_cuda("""
+        star = (5000.0, 1e9, (0.0, 0.0, 0.0))
+        mol = synth.linear_rotor(4)
+        small, large = (synth.power_law_sphere(n, 1, mol) for n in (600, 900))
+        c = pg.Context(0)
+        c.set_molecule(mol)
+        c.set_cloud(large)
+        c.set_star(star)
+        c.set_star(None)
+        c.radiation_field(run())
+        c.set_cloud(small)
+        c.set_star(star)
+        log()
+        c.radiation_field(run())
+        assert "h2d 4800" in [l.split(" stream")[0] for l in log()]
+        c.set_star(None)
+        c.set_cloud(large)
+        c.set_star(star)
+        memory(single=7199)
+        fails(NOMEM, c.radiation_field, run())
+        memory()
+        c.set_cloud(small)
+        log()
+        c.radiation_field(run())
+        assert "h2d 4800" in [l.split(" stream")[0] for l in log()]
+    """)
