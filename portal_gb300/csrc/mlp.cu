@@ -982,6 +982,7 @@ size_t work_floats(const portal_mlp *m, int B) {
 
 int ensure_batch(portal_mlp *m, int B) {
     if (B <= m->cap_batch) return PORTAL_OK;
+    m->cap_batch = 0;   // (buffers that grow are freed first)
     if (m->act.reserve(work_floats(m, B)) || m->xbuf.reserve((size_t)B * m->n_in) ||
         m->ybuf.reserve((size_t)B * m->n_out) || m->idx.reserve(B) || m->part.reserve((size_t)B * m->n_out / 256 + 2))
         return mlp_fail(m, PORTAL_ERR_NOMEM, "MLP workspace");

@@ -157,3 +157,19 @@ def test_failed_star_call_does_not_keep_items_it_replaced(fake_cuda):
         c.radiation_field(run())
         assert "h2d 4800" in [l.split(" stream")[0] for l in log()]
     """)
+
+
+def test_failed_batch_does_not_keep_a_workspace_it_freed(fake_cuda):
+    """A network wider than the whole-network kernels: a batch that does not
+    fit, then the earlier one, whose workspace is allocated again."""
+    fake_cuda("""
+        with pg.MLP(4, 300, 1, 3) as net:
+            X, T = np.zeros((4096, 4)), np.zeros((4096, 3))
+            net.gradients(X[:32], T[:32])
+            memory(single=1 << 20)
+            fails(NOMEM, net.gradients, X, T)
+            memory()
+            log()
+            net.gradients(X[:32], T[:32])
+            assert any(l.startswith("malloc") for l in log())
+    """)
