@@ -290,7 +290,10 @@ __global__ void k_star_mask(int N, double R, const double *__restrict__ pos, con
 // The abundances with the star's interior masked out (star mode, with a cloud).
 static int star_refresh(portal_ctx *c) {
     if (!c->star_mode || !c->have_cloud) return PORTAL_OK;
-    if (c->ab_star.reserve(c->N)) return set_err(c, PORTAL_ERR_NOMEM, "star mask");
+    if (c->ab_star.reserve(c->N)) {
+        c->have_cloud = false;   // (no mask: nothing may run on this cloud in star mode)
+        return set_err(c, PORTAL_ERR_NOMEM, "star mask");
+    }
     k_star_mask<<<(c->N + 255) / 256, 256, 0, c->stream>>>(c->N, c->R_star(), c->pos64.p, c->ab.p, c->ab_star.p);
     PCHECK(c, cudaGetLastError());
     PCHECK(c, cudaStreamSynchronize(c->stream));
@@ -304,6 +307,7 @@ extern "C" int portal_set_star(portal_ctx *c, int star_mod, double T_star, doubl
     if (star_mod == 1 && (!X_star || !(R_star > 0.0) || !(T_star >= 0.0)))
         return set_err(c, PORTAL_ERR_ARG, "portal_set_star: R_star > 0, T_star >= 0 and X_star(3) needed");
     cudaSetDevice(c->device);
+    if (star_mod && c->have_cloud && c->ab_star.reserve(c->N)) return set_err(c, PORTAL_ERR_NOMEM, "star mask");
     c->lines_ready = false;
     c->star_mode = star_mod;
     c->T_star = star_mod ? T_star : 0.0;

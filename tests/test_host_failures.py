@@ -173,3 +173,31 @@ def test_failed_batch_does_not_keep_a_workspace_it_freed(fake_cuda):
             net.gradients(X[:32], T[:32])
             assert any(l.startswith("malloc") for l in log())
     """)
+
+
+def test_star_mask_that_does_not_fit(fake_cuda):
+    """No memory for the mask: set_star leaves the context as it was, a new
+    cloud in star mode is refused as a whole."""
+    fake_cuda("""
+        star = (5000.0, 1e9, (0.0, 0.0, 0.0))
+        mol = synth.linear_rotor(4)
+        small, large = (synth.power_law_sphere(n, 1, mol) for n in (600, 900))
+        c = model()
+        memory(single=4799)
+        fails(NOMEM, c.set_star, star)
+        memory()
+        c.radiation_field(run())        # without a star
+        c.set_cloud(large)
+        c.set_cloud(small)
+        c.set_star(star)
+        log()
+        c.set_star(None)
+        c.set_cloud(large)
+        staging = [int(l.split()[1]) for l in log() if l.startswith("malloc")][-1]
+        c.set_cloud(small)
+        c.set_star(star)
+        memory(total=live() + staging + 2399)
+        fails(NOMEM, c.set_cloud, large)
+        memory()
+        fails(STATE, c.radiation_field, run())
+    """)
