@@ -89,6 +89,7 @@ struct SEArgs {
     double *rates;                      // (N, 3, 2 nlev) column-major or null
     int *status;
     int *nfail;
+    const unsigned long long *skip;     // the solve is left out where this is not 0 (null: never)
     double *a64;                        // FP64 matrices (entries, then dense), one slot of a64_stride doubles per team
     size_t a64_stride;
     int fp64_only;                      // factorise every system in FP64 (no FP32 LU)

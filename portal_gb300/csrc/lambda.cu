@@ -64,13 +64,13 @@ __global__ void k_rho_to_pops(int N, int bulk, int nlev, const double *__restric
 }
 
 // populations from the SE solution, and the residual (max relative change);
-// nothing where the pass failed (fail: singular systems, failed walks)
+// nothing where the pass failed (counters: singular systems, failed walks)
 __global__ void k_update(int N, int bulk, int nlev, const double *__restrict__ pops,
                          const double *__restrict__ nmol, const double *__restrict__ ab,
                          const int *__restrict__ jl, double *__restrict__ levp,
-                         double *__restrict__ rho_prev, const unsigned long long *__restrict__ fail,
-                         unsigned long long *__restrict__ resid) {
-    if (*fail) return;
+                         double *__restrict__ rho_prev, unsigned long long *counters) {
+    if (counters[2] || counters[RF_FAILED]) return;
+    unsigned long long *resid = counters + 3;
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     double r = 0.0;
     if (n < bulk && ab[n] > 0.0) {
@@ -216,22 +216,25 @@ extern "C" int portal_lambda_iterate(portal_ctx *c, int nth, int nph, int nvel, 
         const bool j_before = c->j_valid;
         c->j_valid = true;
         c->ali_valid = split;
-        if ((rc = enqueue_solve_se(c, kmax, false, true))) return rc;
-        k_update<<<nb, tb, 0, c->stream>>>(N, c->bulk, nlev, c->pops.p, c->nmol.p, c->active_ab(), jl.p, c->levp.p,
-                                           rho_prev.p, c->counters.p + 2, c->counters.p + 3);
-        PCHECK(c, cudaGetLastError());
-        unsigned long long cnt[4];
+        const int se_rc = enqueue_solve_se(c, kmax, false, true);
+        if (!se_rc) {
+            k_update<<<nb, tb, 0, c->stream>>>(N, c->bulk, nlev, c->pops.p, c->nmol.p, c->active_ab(), jl.p, c->levp.p,
+                                               rho_prev.p, c->counters.p);
+            PCHECK(c, cudaGetLastError());
+        }
+        unsigned long long cnt[RF_FAILED + 1];
         PCHECK(c, cudaMemcpyAsync(cnt, c->counters.p, sizeof cnt, cudaMemcpyDeviceToHost, c->stream));
         PCHECK(c, cudaStreamSynchronize(c->stream));
         timer_collect(c, T_LINETAB);
         timer_collect(c, T_RF);
-        timer_collect(c, T_SE);
-        nseg_tot += (long long)cnt[1];
-        if (cnt[2] >> 32) {
+        if (cnt[RF_FAILED]) {
             c->j_valid = j_before;
             c->ali_valid = false;
             return failed_nodes(c);
         }
+        if (se_rc) return se_rc;
+        timer_collect(c, T_SE);
+        nseg_tot += (long long)cnt[1];
         if (cnt[2]) return set_err(c, PORTAL_ERR_SINGULAR, std::to_string(cnt[2]) + " singular SE systems");
         const unsigned long long rb = cnt[3];
         double rv;

@@ -158,6 +158,7 @@ __global__ void __launch_bounds__(128) k_rf_finish(RFArgs a, int split) {
     if (a.kmom && lane < 6) a.kmom[(size_t)lane * a.N + node] = on ? km : 0.f;
     if (lane == 0) {
         a.status[node] = st;
+        if (st) atomicAdd(&a.counters[RF_FAILED], 1ULL);
         if (a.segs) a.segs[node] = seg;
         atomicAdd(&a.counters[1], (unsigned long long)seg);
     }

@@ -1251,6 +1251,7 @@ __global__ void __launch_bounds__(256, (NLG >= 1 && NLG <= 4) ? 3 : 2) k_radiati
             }
             if (lane == 0) {
                 a.status[node] = st;
+                if (st) atomicAdd(&a.counters[RF_FAILED], 1ULL);
                 if (a.segs) a.segs[node] = node_seg;
                 if (a.kmom)
                     for (int k = 0; k < 6; k++) a.kmom[(size_t)k * a.N + node] = on ? B.km[k] : 0.f;

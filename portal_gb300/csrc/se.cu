@@ -609,6 +609,9 @@ __global__ void __launch_bounds__(TW == 1 ? 256 : 32 * TW, se_min_blocks<TW, MR,
     double *const slot = (BATCH ? bw.a64 : a0.a64) +
                          (size_t)((long long)blockIdx.x * teams + team) * (BATCH ? bw.a64_stride : a0.a64_stride);
     int cur_model = -1;
+    // a pass of the iterated node loop with failed walks: the last good pass's
+    // populations stay
+    if (!BATCH && a0.skip && *a0.skip) return;
 
     // (nodes go to the blocks in turn, so that few nodes spread over the SMs)
     for (long long item = (long long)team * gridDim.x + blockIdx.x; item < n_items; item += (long long)gridDim.x * teams) {
@@ -638,8 +641,6 @@ __global__ void __launch_bounds__(TW == 1 ? 256 : 32 * TW, se_min_blocks<TW, MR,
         float *d32 = LU + (size_t)n * n;
         float *scl = GAUSS ? gm.scl : d32 + n;
         int *piv = GAUSS ? gm.kof : (int *)(scl + n);
-        // (a failed walk of the iterated node loop: counted, its update stops)
-        if (!BATCH && tid == 0 && (a.status[node] & (PORTAL_NODE_DEPTH | PORTAL_NODE_STAR))) atomicAdd(a.nfail + 1, 1);
         if (!(a.ab[node] > 0.0)) {  // main_para.f90:213 (pops and alignments stay 0)
             if (!BATCH) {
                 for (int c2 = tid; c2 < 2 * a.nlev; c2 += TS) a.pops[(size_t)node + (size_t)a.N * c2] = 0.0;
@@ -1414,6 +1415,7 @@ int se_prepare(portal_ctx *c, int kmax, SEArgs *out, size_t *warp_bytes) {
     a.pops = c->pops.p; a.jj20 = c->jj20.p; a.status = c->status.p;
     a.rates = nullptr;
     a.nfail = (int *)(c->counters.p + 2);
+    a.skip = nullptr;
     // PORTAL_SE_FP64=1: every system factorised in FP64 (the refinement's
     // fallback path), flagged PORTAL_NODE_REFINE
     {
@@ -1522,9 +1524,9 @@ int launch_se(portal_ctx *c, SEArgs &a) {
 }
 
 // Enqueues the solve: results in c->pops, c->jj20, c->rates, c->status; the
-// numbers of singular systems and of nodes with failed walks in c->counters[2]
-// (its lower and upper half), zeroed here or, after a radiation field
-// enqueued before (fresh), with its counters.
+// number of singular systems in c->counters[2], zeroed here or, after a
+// radiation field enqueued before (fresh), with its counters.  fresh: nothing
+// is solved where that field has failed walks.
 int enqueue_solve_se(portal_ctx *c, int kmax, bool rates, bool fresh) {
     SEArgs a;
     int rc = se_prepare(c, kmax, &a, nullptr);
@@ -1535,7 +1537,8 @@ int enqueue_solve_se(portal_ctx *c, int kmax, bool rates, bool fresh) {
         PCHECK(c, cudaMemsetAsync(c->rates.p, 0, nr * sizeof(double), c->stream));
         a.rates = c->rates.p;
     }
-    if (!fresh && (rc = se_pass(c, c->stream))) return rc;
+    if (fresh) a.skip = c->counters.p + RF_FAILED;
+    else if ((rc = se_pass(c, c->stream))) return rc;
     a.a64_stride = se_matrix_doubles(c);
     const int n = c->c_dim;
     if (se_team_warps(n) == 4)
