@@ -360,7 +360,7 @@ extern "C" int portal_batch_run(portal_batch *b, int use_graph, long long *n_seg
     if (ms) *ms = t;
     if (n_segments) *n_segments = (long long)q[1];
     for (auto *c : b->models) {
-        c->j_valid = true;
+        c->j_valid = c->pops_valid = true;
         c->ali_valid = false;
     }
     return PORTAL_OK;

@@ -346,7 +346,7 @@ extern "C" int portal_get_results(portal_ctx *c, double *J0, double *J2, double 
     if (J0) PCHECK(c, cudaMemcpyAsync(J0, c->J0.p, LN * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     if (J2) PCHECK(c, cudaMemcpyAsync(J2, c->J2.p, LN * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     if (pol_pops) {
-        if (!c->pops.p || c->se_kmax < 0) return set_err(c, PORTAL_ERR_STATE, "no device-resident populations");
+        if (!c->have_pops() || c->se_kmax < 0) return set_err(c, PORTAL_ERR_STATE, "no device-resident populations");
         PCHECK(c, cudaMemcpyAsync(pol_pops, c->pops.p, (size_t)c->N * 2 * c->nlev * sizeof(double),
                                   cudaMemcpyDeviceToHost, c->stream));
     }

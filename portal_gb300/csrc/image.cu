@@ -713,7 +713,7 @@ static int image_call(portal_ctx *c, const double *pol_pops, int nlines, const i
     if (mode == 0 && im_size * im_size * 2.0 >= 1.0)
         return set_err(c, PORTAL_ERR_ARG, "portal_image: im_size must keep the image corners inside "
                                           "the unit sphere (im_size < 1/sqrt(2))");
-    if (!pol_pops && !c->pops.p)
+    if (!pol_pops && !c->have_pops())
         return set_err(c, PORTAL_ERR_STATE, std::string(fn) + ": no pol_pops (pass them or run portal_solve_se)");
     cudaSetDevice(c->device);
     timers_reset(c);

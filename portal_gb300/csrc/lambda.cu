@@ -177,7 +177,7 @@ extern "C" int portal_lambda_iterate(portal_ctx *c, int nth, int nph, int nvel, 
     const int N = c->N, nlev = c->nlev;
     DevBuf<int> jl;
     DevBuf<double> rho_prev;
-    if (jl.reserve(nlev) || rho_prev.reserve((size_t)nlev * N) || c->pops.reserve((size_t)N * 2 * nlev))
+    if (jl.reserve(nlev) || rho_prev.reserve((size_t)nlev * N) || c->reserve_pops())
         return set_err(c, PORTAL_ERR_NOMEM, "lambda buffers");
     PCHECK(c, cudaMemcpyAsync(jl.p, c->j_lev.data(), nlev * sizeof(int), cudaMemcpyHostToDevice, c->stream));
     const int tb = 256, nb = (N + tb - 1) / tb;
@@ -233,6 +233,7 @@ extern "C" int portal_lambda_iterate(portal_ctx *c, int nth, int nph, int nvel, 
             return failed_nodes(c);
         }
         if (se_rc) return se_rc;
+        c->pops_valid = true;
         timer_collect(c, T_SE);
         nseg_tot += (long long)cnt[1];
         if (cnt[2]) return set_err(c, PORTAL_ERR_SINGULAR, std::to_string(cnt[2]) + " singular SE systems");

@@ -1389,7 +1389,7 @@ int se_prepare(portal_ctx *c, int kmax, SEArgs *out, size_t *warp_bytes) {
     const size_t wb = se_warp_bytes(n, c->n_feat);
     if (wb > 200 * 1024 || n > 32 * SE_MAX_ROWS)
         return set_err(c, PORTAL_ERR_ARG, "SE system too large for shared memory");
-    if (c->pops.reserve((size_t)c->N * 2 * c->nlev) || c->jj20.reserve((size_t)c->N * c->r_num))
+    if (c->reserve_pops() || c->jj20.reserve((size_t)c->N * c->r_num))
         return set_err(c, PORTAL_ERR_NOMEM, "SE outputs");
     SEArgs a;
     a.N = c->N; a.bulk = c->bulk; a.c_dim = n; a.n_trans = c->n_trans; a.nlev = c->nlev; a.L = c->r_num;
@@ -1595,6 +1595,7 @@ extern "C" int portal_solve_se(portal_ctx *c, int kmax, const double *J0, const 
     PCHECK(c, cudaMemcpyAsync(&nsing, c->counters.p + 2, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     PCHECK(c, cudaStreamSynchronize(c->stream));
     timer_collect(c, T_SE);
+    c->pops_valid = true;
     if (nsing) return set_err(c, PORTAL_ERR_SINGULAR, std::to_string(nsing) + " singular SE systems");
     return PORTAL_OK;
 }

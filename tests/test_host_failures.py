@@ -201,3 +201,29 @@ def test_star_mask_that_does_not_fit(fake_cuda):
         memory()
         fails(STATE, c.radiation_field, run())
     """)
+
+
+def test_only_populations_of_a_solve_are_used(fake_cuda):
+    """An image without pol_pops after an iteration that solved nothing, and
+    after a solve for a smaller cloud or molecule, is refused."""
+    fake_cuda("""
+        def image(c):
+            return c.image([1], [2], 0.3, 0.2, 4, 300.0, 0.0, 4, 0.4)
+        c = model()
+        memory(single=14399)            # J0 takes 8 x 3 x 600 bytes
+        fails(NOMEM, c.lambda_iterate, run())
+        memory()
+        fails(STATE, image, c)
+        c.radiation_field(run())
+        fails(STATE, c.results)
+        c.solve_se(2)
+        image(c)
+        c.results()
+        mol = synth.linear_rotor(4)
+        c.set_cloud(synth.power_law_sphere(900, 1, mol))
+        fails(STATE, image, c)
+        c.set_cloud(synth.power_law_sphere(600, 1, mol))
+        image(c)
+        c.lambda_iterate(run(), max_iter=1)
+        image(c)
+    """)
