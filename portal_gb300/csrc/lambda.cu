@@ -211,9 +211,9 @@ extern "C" int portal_lambda_iterate(portal_ctx *c, int nth, int nph, int nvel, 
     bool verify = false;  // this pass is the plain pass that decides convergence
     while (it < max_iter) {
         const bool split = local_operator && !verify;
+        const bool j_before = c->j_valid;
         // the pass enqueued as a whole, one wait (on its counters) at its end
         if ((rc = enqueue_radiation_field(c, nth, nph, nvel, gvec, dx, n_depth, split))) return rc;
-        const bool j_before = c->j_valid;
         c->j_valid = true;
         c->ali_valid = split;
         const int se_rc = enqueue_solve_se(c, kmax, false, true);

@@ -417,7 +417,7 @@ int enqueue_radiation_field(portal_ctx *c, int nth, int nph, int nvel, const dou
     RFArgs a;
     int rc = rf_prepare(c, nth, nph, nvel, gvec, dx, n_depth, split, &a);
     if (rc) return rc;
-    c->ali_valid = false;
+    c->j_valid = c->ali_valid = false;   // (the pass starts by clearing the field)
     timer_start(c, T_LINETAB);
     if ((rc = rf_pass(c, a, 0, c->has_dust, c->stream))) return rc;
     timer_stop(c, T_LINETAB);

@@ -227,3 +227,19 @@ def test_only_populations_of_a_solve_are_used(fake_cuda):
         c.lambda_iterate(run(), max_iter=1)
         image(c)
     """)
+
+
+def test_field_that_a_failed_call_cleared_is_not_used(fake_cuda):
+    """No memory for the walks: the field of the call before is gone by then."""
+    fake_cuda("""
+        c = model()
+        c.radiation_field(run())
+        c.solve_se(2)
+        memory(single=1 << 20)
+        fails(NOMEM, c.radiation_field, run(n_depth=3200))
+        memory()
+        fails(STATE, c.solve_se, 2)
+        fails(STATE, c.results)
+        c.radiation_field(run())
+        c.solve_se(2)
+    """)
