@@ -253,22 +253,9 @@ extern "C" int portal_batch_prepare(portal_batch *b, int nth, int nph, int nvel,
         rf_grid = std::max(rf_grid, (size_t)mx * b->sm_count);
     }
     if (rfc.empty()) return bfail(b, PORTAL_ERR_CUDA, "radiation-field kernel does not fit on an SM");
-    // the dynamic shared-memory limit of the largest candidate
-    auto raise_rf_limit = [&]() {
-        int most = 0;
-        for (const RFC &c : rfc)
-            if (rf_batch(b, nullptr, 0, c.nlg).warp_bytes > rf_batch(b, nullptr, 0, rfc[most].nlg).warp_bytes)
-                most = (int)(&c - rfc.data());
-        int mx = 0;
-        return rf_batch_blocks_per_sm(rf_batch(b, nullptr, 0, rfc[most].nlg), b->dust, &mx);
-    };
-    if (raise_rf_limit()) return bfail(b, PORTAL_ERR_CUDA, "occupancy query");
     std::vector<int> sec;
     for (int w : {2, 4, 8})
         if (team > 1 ? w == team : wb * w <= 200 * 1024) sec.push_back(w);
-    int dummy = 0;
-    if (se_batch_blocks_per_sm(sec.back(), wb, b->se_max_dim, b->se_gauss, &dummy))  // raises the smem limit to the largest candidate
-        return bfail(b, PORTAL_ERR_CUDA, "SE occupancy query");
     // FP64 matrix slots for the largest SE grid among the candidates
     {
         size_t most = 0;
@@ -277,7 +264,6 @@ extern "C" int portal_batch_prepare(portal_batch *b, int nth, int nph, int nvel,
             if (se_batch_blocks_per_sm(w, wb, b->se_max_dim, b->se_gauss, &bps)) return bfail(b, PORTAL_ERR_CUDA, "SE occupancy query");
             most = std::max(most, (size_t)std::max(1, bps) * b->sm_count * w);
         }
-        se_batch_blocks_per_sm(sec.back(), wb, b->se_max_dim, b->se_gauss, &dummy);
         if (b->se_a64.reserve(most * b->se_a64_stride)) return bfail(b, PORTAL_ERR_NOMEM, "SE matrix scratch");
     }
     // walk scratch for the largest grid
@@ -311,7 +297,6 @@ extern "C" int portal_batch_prepare(portal_batch *b, int nth, int nph, int nvel,
             b->tune.insert(b->tune.end(), {(double)w, (double)bps, ms});
             if (ms < best) { best = ms; b->se_warps = w; b->se_bps = bps; }
         }
-        se_batch_blocks_per_sm(sec.back(), wb, b->se_max_dim, b->se_gauss, &dummy);
     } else {
         b->nlg = rfc[0].nlg;
         b->rf_bps = rfc[0].bps;

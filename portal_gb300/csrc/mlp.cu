@@ -949,11 +949,7 @@ void gemm_tc(cudaStream_t s, int M, int N, int K, const float *A, const float *W
     uint32_t tcols = 32;
     while ((int)tcols < Np) tcols <<= 1;
     const size_t smem = tc_smem_bytes(Np, Kp);
-    static size_t raised = 0;
-    if (smem > raised) {
-        cudaFuncSetAttribute(k_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem_bytes(256, 256));
-        raised = tc_smem_bytes(256, 256);
-    }
+    allow_dyn_smem((const void *)k_gemm_tc);
     static int nsm = 0;
     if (!nsm) {
         int dev = 0;
@@ -1076,7 +1072,7 @@ int launch_rows(portal_mlp *m, int B, const int *idx, const float *X, const floa
                 float scale) {
     const size_t smem = m->net.wbuf + (size_t)NB * FU_MAX * 2 + 3 * 8 + 16 * 8 + (TRAIN ? sizeof(float) * NB * m->n_out : 0);
     auto k = k_mlp_rows<NB, TRAIN>;
-    MCHECK(m, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    MCHECK(m, allow_dyn_smem((const void *)k));
     k<<<(B + NB - 1) / NB, FU_THREADS, smem, m->stream>>>(m->net, B, idx, X, T, st, m->params.p, m->pk.p, Y,
                                                                    m->fb, scale, m->tc_err.p);
     MCHECK(m, cudaGetLastError());
@@ -1143,8 +1139,7 @@ int fused_step(portal_mlp *m, int B, const int *idx, const float *X, const float
         blocks += tm * ((m->fin[l] + 63) / 64) + tm;
     }
     const int n_loss = (B + TRAIN_NB - 1) / TRAIN_NB;
-    MCHECK(m, cudaFuncSetAttribute(ad ? (const void *)k_mlp_grads<true> : (const void *)k_mlp_grads<false>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DW_SMEM));
+    MCHECK(m, allow_dyn_smem(ad ? (const void *)k_mlp_grads<true> : (const void *)k_mlp_grads<false>));
     if (ad)
         k_mlp_grads<true><<<blocks, 128, DW_SMEM, m->stream>>>(m->net, B, m->fb, nullptr, *ad, n_loss, loss_acc);
     else

@@ -206,7 +206,7 @@ int launch_rf(portal_ctx *c, RFArgs &a, int n_depth) {
     int wpb = rf_warps();
     while (wpb > 1 && table + (size_t)wpb * sh.bytes > 200 * 1024) wpb--;   // many lines and channels
     const size_t dyn = table + (size_t)wpb * sh.bytes;
-    PCHECK(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+    PCHECK(c, allow_dyn_smem(kern));
     int nb = 0;
     PCHECK(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, 32 * wpb, dyn));
     if (nb < 1) nb = 1;

@@ -34,14 +34,13 @@ void rf_batch_shape(RFBatch *bw, const int *lines, int n_models, int nch, bool d
                                   (size_t)rf_shape(lines[m], max_group, nch, dust, bw->rt, split).bytes);
 }
 
-// Also raises the kernel's dynamic shared-memory limit: called for every
-// candidate before the pass is captured.
+// Also sets the kernel's dynamic shared-memory limit: called before the pass is
+// captured.
 int rf_batch_blocks_per_sm(const RFBatch &bw, bool dust, int *blocks) {
     const void *k = batch_kernel(bw, dust);
     const size_t dyn = batch_dyn_smem(bw);
     *blocks = 0;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn) != cudaSuccess)
-        return PORTAL_ERR_CUDA;
+    if (allow_dyn_smem(k) != cudaSuccess) return PORTAL_ERR_CUDA;
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, k, 32 * RF_BATCH_WARPS, dyn);
     return e == cudaSuccess ? PORTAL_OK : PORTAL_ERR_CUDA;
 }

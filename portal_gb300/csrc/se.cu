@@ -1466,15 +1466,14 @@ int se_batch_blocks_per_sm(int warps_per_block, size_t team_bytes, int max_dim, 
     const size_t smem = team_bytes * (warps_per_block / se_batch_team(max_dim, gauss));
     const void *k = se_batch_kernel(max_dim, gauss);
     *blocks = 0;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-        return PORTAL_ERR_CUDA;
+    if (allow_dyn_smem(k) != cudaSuccess) return PORTAL_ERR_CUDA;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, k, 32 * warps_per_block, smem) == cudaSuccess
                ? PORTAL_OK
                : PORTAL_ERR_CUDA;
 }
 
-// (the kernel's dynamic shared memory limit must have been raised by
-// se_batch_blocks_per_sm for at least this many warps)
+// (the kernel's dynamic shared memory limit must have been set by
+// se_batch_blocks_per_sm)
 int se_batch_launch(cudaStream_t s, int grid, int warps_per_block, const SEBatch &bw) {
     const size_t smem = bw.team_bytes * (warps_per_block / se_batch_team(bw.max_dim, bw.gauss));
     SEArgs a0{};
@@ -1509,7 +1508,7 @@ int launch_se(portal_ctx *c, SEArgs &a) {
     const size_t wb = NC >= 0 ? se_gauss_bytes(a.c_dim, a.n_feat, a.nnz, gauss_quads<TW, NC>, NC == 0) : se_warp_bytes(a.c_dim, a.n_feat);
     const int teams = (TW == 1) ? (int)std::min<size_t>(8, (200 * 1024) / wb) : 1;
     const size_t smem = wb * teams;
-    PCHECK(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PCHECK(c, allow_dyn_smem((const void *)kern));
     int nb = 0;
     PCHECK(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, 32 * TW * teams, smem));
     const int grid = c->sm_count * std::max(1, nb);

@@ -198,6 +198,7 @@ cudaError_t cudaFuncSetAttribute(const void *f, cudaFuncAttribute a, int v) {
     if (a == cudaFuncAttributeMaxDynamicSharedMemorySize) {
         if (v > 232448) return fail(cudaErrorInvalidValue);
         limits[f] = v;
+        note("limit " + names[f] + " " + std::to_string(v));
     }
     return cudaSuccess;
 }

@@ -243,3 +243,51 @@ def test_field_that_a_failed_call_cleared_is_not_used(fake_cuda):
         c.radiation_field(run())
         c.solve_se(2)
     """)
+
+
+def test_prepared_batch_runs_after_smaller_calls(fake_cuda):
+    """A prepared batch's launches are not refused because a smaller batch, or a
+    star-mode call, has used the same kernels since."""
+    fake_cuda("""
+        rc = run(nvel=64, kmax=6)
+        large, small, star = model(600, 20), model(600, 14), model(600, 3)
+        star.set_star((5000.0, 1e9, (0.0, 0.0, 0.0)))
+        with pg.Batch(0) as a, pg.Batch(0) as b:
+            a.add(large)
+            a.prepare(rc)
+            b.add(small)
+            b.prepare(rc)
+            star.radiation_field(rc)
+            star.solve_se(6)
+            log()
+            a.run(use_graph=False)
+            b.run(use_graph=False)
+        launched = [l.split()[1] for l in log() if l.startswith("launch")]
+        assert sum("k_radiation_field" in l for l in launched) == 2
+        assert sum("k_solve_se" in l for l in launched) == 2
+    """)
+
+
+def test_shared_memory_limits_are_not_lowered(fake_cuda):
+    """A kernel's limit is one value in every call: what one thread has set for
+    its launch, another thread's call for a smaller one leaves."""
+    fake_cuda("""
+        for levels in (4, 14, 20):
+            c = model(600, levels)
+            for nvel in (8, 40, 64):
+                for kmax in (2, 6):
+                    c.radiation_field(run(nvel=nvel))
+                    c.radiation_field_split(run(nvel=nvel))
+                    c.solve_se(kmax)
+        for shape in ((4, 32, 2, 3), (8, 256, 3, 40), (8, 200, 1, 250), (4, 300, 1, 3)):
+            with pg.MLP(*shape) as net:
+                X, T = np.zeros((70, shape[0])), np.zeros((70, shape[3]))
+                net.gradients(X, T)
+                net.predict(X)
+        seen = {}
+        for l in log():
+            if l.startswith("limit"):
+                seen.setdefault(l.split()[1], set()).add(int(l.split()[2]))
+        assert len(seen) > 10
+        assert all(len(v) == 1 for v in seen.values()), seen
+    """)
