@@ -174,6 +174,7 @@ extern "C" int portal_lambda_iterate(portal_ctx *c, int nth, int nph, int nvel, 
         return set_err(c, PORTAL_ERR_ARG, "portal_lambda_iterate: max_iter >= 1, tol > 0, ng_period 0 or >= 3");
     cudaSetDevice(c->device);
     timers_reset(c);
+    const RayItems give_back(c);
     const int N = c->N, nlev = c->nlev;
     DevBuf<int> jl;
     DevBuf<double> rho_prev;

@@ -182,6 +182,12 @@ bool ray_items(RFArgs &a, bool split, long long resident) {
     return true;
 }
 
+bool reserve_ray_items(portal_ctx *c, size_t rays, int values) {
+    if (!c->vray.reserve(rays * values) && !c->dray.reserve(rays) && !c->iseg.reserve(rays)) return true;
+    c->release_ray_items();
+    return false;
+}
+
 template <bool FLAT>
 const void *rf_kernel(const RFShape &sh, bool dust, bool split) {
     const int slots = sh.nslot == 1 ? 1 : sh.nslot % 2 == 0 ? 2 : 0;
@@ -197,29 +203,38 @@ int launch_rf(portal_ctx *c, RFArgs &a, int n_depth) {
     const int rt = rf_remainder(a.nch, dust, a.L);
     const size_t table = (a.nch * sizeof(float2) + 15) & ~(size_t)15;
     RFShape sh = rf_shape(a.L, max_line_group(), a.nch, dust, rt, split);
+    const void *kern = nullptr;
+    int wpb = 0, nb = 0;
+    size_t dyn = 0;
+    auto set_up = [&](bool flat) -> int {
+        sh = rf_shape(a.L, max_line_group(), a.nch, dust, rt, split, flat ? 2 : 1);
+        kern = flat ? rf_kernel<true>(sh, dust, split) : rf_kernel<false>(sh, dust, split);
+        wpb = rf_warps();
+        while (wpb > 1 && table + (size_t)wpb * sh.bytes > 200 * 1024) wpb--;   // many lines and channels
+        dyn = table + (size_t)wpb * sh.bytes;
+        PCHECK(c, allow_dyn_smem(kern));
+        PCHECK(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, 32 * wpb, dyn));
+        if (nb < 1) nb = 1;
+        // where the device cannot hold the walk scratch of all blocks: without
+        // the rays' sums of a call before, then fewer blocks per SM
+        while (c->walk.reserve((size_t)nb * c->sm_count * wpb * rf_walk_records(n_depth)) != cudaSuccess) {
+            if (c->vray.p) c->release_ray_items();
+            else if (--nb < 1) return set_err(c, PORTAL_ERR_NOMEM, "walk scratch allocation failed");
+        }
+        return PORTAL_OK;
+    };
     // about the warps resident: what the registers (the kernel's launch bounds)
     // and shared memory leave room for
     const long long fit = std::max<long long>(1, (224LL * 1024) / (sh.bytes + (long long)table / 4));
-    const bool flat = ray_items(a, split, c->sm_count * std::min(fit, sh.nlg <= 4 ? 24LL : 16LL));
-    if (flat) sh = rf_shape(a.L, max_line_group(), a.nch, dust, rt, split, 2);
-    const void *kern = flat ? rf_kernel<true>(sh, dust, split) : rf_kernel<false>(sh, dust, split);
-    int wpb = rf_warps();
-    while (wpb > 1 && table + (size_t)wpb * sh.bytes > 200 * 1024) wpb--;   // many lines and channels
-    const size_t dyn = table + (size_t)wpb * sh.bytes;
-    PCHECK(c, allow_dyn_smem(kern));
-    int nb = 0;
-    PCHECK(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, 32 * wpb, dyn));
-    if (nb < 1) nb = 1;
-    // fewer blocks per SM where the device cannot hold the walk scratch of all
-    while (c->walk.reserve((size_t)nb * c->sm_count * wpb * rf_walk_records(n_depth)) != cudaSuccess) {
-        if (--nb < 1) return set_err(c, PORTAL_ERR_NOMEM, "walk scratch allocation failed");
+    bool flat = ray_items(a, split, c->sm_count * std::min(fit, sh.nlg <= 4 ? 24LL : 16LL));
+    if (int rc = set_up(flat)) return rc;
+    if (flat && !reserve_ray_items(c, (size_t)a.bulk * a.ndir, a.L * (split ? 3 : 1))) {
+        flat = false;   // whole nodes need no rays' sums
+        if (int rc = set_up(flat)) return rc;
     }
     const int grid = nb * c->sm_count;
     a.walk = c->walk.p;
     if (flat) {
-        const size_t rays = (size_t)a.bulk * a.ndir;
-        if (c->vray.reserve(rays * a.L * (split ? 3 : 1)) || c->dray.reserve(rays) || c->iseg.reserve(rays))
-            return set_err(c, PORTAL_ERR_NOMEM, "ray sums");
         a.vray = c->vray.p; a.dray = c->dray.p; a.iseg = c->iseg.p;
     }
     timer_start(c, T_RF);
@@ -452,6 +467,7 @@ int radiation_field_call(portal_ctx *c, int nth, int nph, int nvel, const double
                          long long *n_segments) {
     if (!c) return PORTAL_ERR_ARG;
     timers_reset(c);
+    const RayItems give_back(c);
     const size_t LN = (size_t)c->r_num * c->N;
     if (int rc = portal::enqueue_radiation_field(c, nth, nph, nvel, gvec, dx, n_depth, split)) return rc;
     const HostSpan out[4] = {{J0, LN * sizeof(double)}, {J2, LN * sizeof(double)}, {JE, LN * sizeof(double)},

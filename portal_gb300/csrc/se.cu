@@ -1526,7 +1526,7 @@ int launch_se(portal_ctx *c, SEArgs &a) {
 // number of singular systems in c->counters[2], zeroed here or, after a
 // radiation field enqueued before (fresh), with its counters.  fresh: nothing
 // is solved where that field has failed walks.
-int enqueue_solve_se(portal_ctx *c, int kmax, bool rates, bool fresh) {
+static int try_solve_se(portal_ctx *c, int kmax, bool rates, bool fresh) {
     SEArgs a;
     int rc = se_prepare(c, kmax, &a, nullptr);
     if (rc) return rc;
@@ -1551,6 +1551,16 @@ int enqueue_solve_se(portal_ctx *c, int kmax, bool rates, bool fresh) {
              : n <= 24          ? launch_se<1, 1, 24>(c, a)
              : n <= SE_WARP_DIM ? launch_se<1, 1, SE_WARP_DIM>(c, a)
                                 : launch_se<1, 3, 0>(c, a);
+    return rc;
+}
+
+int enqueue_solve_se(portal_ctx *c, int kmax, bool rates, bool fresh) {
+    int rc = try_solve_se(c, kmax, rates, fresh);
+    if (rc == PORTAL_ERR_NOMEM && c->vray.p) {   // the rays' sums of the field, summed once its kernels are done
+        PCHECK(c, cudaStreamSynchronize(c->stream));
+        c->release_ray_items();
+        rc = try_solve_se(c, kmax, rates, fresh);
+    }
     return rc;
 }
 

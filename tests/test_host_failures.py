@@ -291,3 +291,57 @@ def test_shared_memory_limits_are_not_lowered(fake_cuda):
         assert len(seen) > 10
         assert all(len(v) == 1 for v in seen.values()), seen
     """)
+
+
+def test_scratch_of_ray_items_refuses_no_call(fake_cuda):
+    """Items of rays (small clouds) need a scratch for the rays' sums that whole
+    nodes do not: where it does not fit the call runs whole nodes, and what it
+    holds does not keep the walks or the solve after it from fitting."""
+    fake_cuda("""
+        def kernels():
+            return [l.split()[1] for l in log() if l.startswith("launch")]
+        c = model()
+        c.radiation_field(run())
+        walk = max(int(l.split()[1]) for l in log(False) if l.startswith("malloc"))
+        assert any("k_rf_finish" in k for k in kernels())
+        # the sums (540 kB) do not fit
+        c = model()
+        memory(total=live() + walk + 200000)
+        c.radiation_field(run())
+        k = kernels()
+        assert any("k_radiation_field" in x for x in k) and not any("k_rf_finish" in x for x in k)
+        memory()
+        c.radiation_field(run())
+        assert any("k_rf_finish" in x for x in kernels())
+        # kept sums in the way of a solve, and of a walk of twice the cells
+        model_2 = model()
+        model_2.radiation_field(run())
+        used = live()
+        model_2.solve_se(2)
+        solve = live() - used
+        c.close()
+        model_2.close()
+        c = model()
+        c.radiation_field(run())
+        memory(total=live() + solve - 300000)
+        c.solve_se(2)
+        memory()
+        c.radiation_field(run())
+        memory(total=live() + walk - 300000)
+        log()
+        c.radiation_field(run(n_depth=64))
+        assert max(int(l.split()[1]) for l in log() if l.startswith("free")) == walk
+        assert live() > 2 * walk
+        memory()
+        # not held above 256 MB
+        mol = synth.linear_rotor(20)
+        c.set_molecule(mol)
+        c.set_cloud(synth.power_law_sphere(4096, 1, mol))
+        log()
+        before = live()
+        rc = run(nth=40)
+        c.radiation_field(rc)
+        sums = max(int(l.split()[1]) for l in log(False) if l.startswith("malloc"))
+        assert sums > 256 << 20 and any("k_rf_finish" in x for x in kernels())
+        assert live() < before + sums
+    """)
