@@ -62,7 +62,10 @@ int bfail(portal_batch *b, int code, const std::string &m) {
 #define BCHECK(b, call)                                                                                  \
     do {                                                                                                 \
         cudaError_t _e = (call);                                                                         \
-        if (_e != cudaSuccess) return bfail((b), PORTAL_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(_e)); \
+        if (_e != cudaSuccess) {                                                                         \
+            cudaGetLastError(); /* reported here, not by the next call's launch check */                 \
+            return bfail((b), PORTAL_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(_e));      \
+        }                                                                                                \
     } while (0)
 
 void drop_graph(portal_batch *b) {

@@ -924,7 +924,10 @@ int mlp_fail(portal_mlp *m, int code, const std::string &msg) {
 #define MCHECK(m, call)                                                                  \
     do {                                                                                 \
         cudaError_t _e = (call);                                                         \
-        if (_e != cudaSuccess) return mlp_fail((m), PORTAL_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(_e)); \
+        if (_e != cudaSuccess) {                                                         \
+            cudaGetLastError(); /* reported here, not by the next call's launch check */ \
+            return mlp_fail((m), PORTAL_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(_e)); \
+        }                                                                                \
     } while (0)
 
 // after a stream synchronize: did a tensor-core GEMM give up waiting?

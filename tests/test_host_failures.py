@@ -345,3 +345,23 @@ def test_scratch_of_ray_items_refuses_no_call(fake_cuda):
         assert sums > 256 << 20 and any("k_rf_finish" in x for x in kernels())
         assert live() < before + sums
     """)
+
+
+def test_failed_copy_does_not_fail_the_next_call(fake_cuda):
+    fake_cuda("""
+        c = model()
+        fake.fake_refuse_d2h(1)
+        fails(CUDA_ERR, c.radiation_field, run())
+        c.radiation_field(run())
+        with pg.MLP(4, 32, 1, 3) as net, pg.Batch(0) as b:
+            X = np.zeros((16, 4))
+            fake.fake_refuse_d2h(1)
+            fails(CUDA_ERR, net.predict, X)
+            net.predict(X)
+            b.add(c)
+            b.prepare(run())
+            fake.fake_refuse_d2h(1)
+            fails(CUDA_ERR, b.run)
+            b.run()
+            c.radiation_field(run())
+    """)
