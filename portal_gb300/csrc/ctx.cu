@@ -17,10 +17,12 @@
 //                       radiation field's walk
 //   levp   (nlev,N) FP64 level populations, plus the per-node scalars
 //                       (b, T_kin, T_dust, dust, n_H2, abundance) in FP64.
+#include <sys/mman.h>
 #include <unistd.h>
 
 #include <algorithm>
 #include <cmath>
+#include <cstdint>
 #include <cstring>
 #include <thread>
 
@@ -367,7 +369,8 @@ extern "C" int portal_last_kernel_times(const portal_ctx *c, double *times_ms, i
 
 namespace portal {
 
-void touch_pages(const HostSpan *spans, int n) {
+void map_pages(const HostSpan *spans, int n) {
+#ifdef MADV_POPULATE_WRITE
     const size_t page = (size_t)std::max<long>(4096, sysconf(_SC_PAGESIZE));
     size_t pages = 0;
     for (int i = 0; i < n; i++)
@@ -376,18 +379,22 @@ void touch_pages(const HostSpan *spans, int n) {
     const int nt = pages < 64 ? 1 : 4;
     auto work = [&](int t) {
         for (int i = 0; i < n; i++) {
-            if (!spans[i].p) continue;
-            volatile char *b = static_cast<volatile char *>(spans[i].p);
-            for (size_t o = (size_t)t * page; o < spans[i].bytes; o += (size_t)nt * page) b[o] = 0;
+            if (!spans[i].p || !spans[i].bytes) continue;
+            // whole pages from the first to the last byte, a part per thread
+            const uintptr_t b = reinterpret_cast<uintptr_t>(spans[i].p) / page,
+                            e = (reinterpret_cast<uintptr_t>(spans[i].p) + spans[i].bytes - 1) / page + 1;
+            const uintptr_t lo = b + (e - b) * t / nt, hi = b + (e - b) * (t + 1) / nt;
+            if (hi > lo) madvise(reinterpret_cast<void *>(lo * page), (hi - lo) * page, MADV_POPULATE_WRITE);
         }
     };
     std::vector<std::thread> th;
     try {
         for (int t = 1; t < nt; t++) th.emplace_back(work, t);
-    } catch (...) {   // no thread to be had: the pages not touched here fault in the copy
+    } catch (...) {   // no thread to be had: the pages not mapped here fault in the copy
     }
     work(0);
     for (auto &x : th) x.join();
+#endif
 }
 
 void gauss_legendre(int n, double *x, double *w) {

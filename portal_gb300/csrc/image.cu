@@ -878,7 +878,7 @@ static int image_call(portal_ctx *c, const double *pol_pops, int nlines, const i
     HostSpan spans[9];
     for (int q = 0; q < 8; q++) spans[q] = {dout[q], cube * sizeof(float)};
     spans[8] = {xy, 2 * (size_t)nrays * sizeof(double)};
-    touch_pages(spans, 9);   // while the kernels run
+    map_pages(spans, 9);   // while the kernels run
     for (int q = 0; q < 8; q++)
         if (dout[q])
             PCHECK(c, cudaMemcpyAsync(dout[q], ia.out[q], cube * sizeof(float), cudaMemcpyDeviceToHost, c->stream));

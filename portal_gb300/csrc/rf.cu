@@ -472,7 +472,7 @@ int radiation_field_call(portal_ctx *c, int nth, int nph, int nvel, const double
     if (int rc = portal::enqueue_radiation_field(c, nth, nph, nvel, gvec, dx, n_depth, split)) return rc;
     const HostSpan out[4] = {{J0, LN * sizeof(double)}, {J2, LN * sizeof(double)}, {JE, LN * sizeof(double)},
                              {LS, LN * sizeof(double)}};
-    touch_pages(out, 4);   // the caller's result arrays, while the kernel runs
+    map_pages(out, 4);   // the caller's result arrays, while the kernel runs
     // every copy behind the kernels, one wait for all
     if (J0) PCHECK(c, cudaMemcpyAsync(J0, c->J0.p, LN * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     if (J2) PCHECK(c, cudaMemcpyAsync(J2, c->J2.p, LN * sizeof(double), cudaMemcpyDeviceToHost, c->stream));

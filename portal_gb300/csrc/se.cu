@@ -1588,7 +1588,7 @@ extern "C" int portal_solve_se(portal_ctx *c, int kmax, const double *J0, const 
     const HostSpan out[3] = {{pol_pops, (size_t)c->N * 2 * c->nlev * sizeof(double)}, {JJ_20, LN * sizeof(double)},
                              {rates, (size_t)c->N * 6 * c->nlev * sizeof(double)}};
     if (int rc = portal::enqueue_solve_se(c, kmax, rates != nullptr, false)) return rc;
-    touch_pages(out, 3);   // the caller's result arrays, while the kernel runs
+    map_pages(out, 3);   // the caller's result arrays, while the kernel runs
     // every copy behind the kernel, one wait for all
     if (pol_pops)
         PCHECK(c, cudaMemcpyAsync(pol_pops, c->pops.p, (size_t)c->N * 2 * c->nlev * sizeof(double),

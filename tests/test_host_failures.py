@@ -365,3 +365,64 @@ def test_failed_copy_does_not_fail_the_next_call(fake_cuda):
             b.run()
             c.radiation_field(run())
     """)
+
+
+def test_failed_call_leaves_the_result_arrays(fake_cuda):
+    """A copy to the host that fails: the caller's arrays keep what they held
+    (large enough for their pages to be mapped ahead of the copies)."""
+    fake_cuda("""
+        mol = synth.linear_rotor(5)
+        N = 4096
+        c = pg.Context(0)
+        c.set_molecule(mol)
+        c.set_cloud(synth.power_law_sphere(N, 1, mol))
+        rc = run()
+        g = np.ascontiguousarray(rc.gvec)
+        L = pg.lib()
+        a = [np.full((N, 4), 0.1) for _ in range(4)]
+        P = pg._p
+        fake.fake_refuse_d2h(1)
+        assert L.portal_radiation_field_split(c._h, rc.nth, rc.nph, rc.nvel, P(g), rc.dx, rc.n_depth, P(a[0]), P(a[1]),
+                                              P(a[2]), P(a[3]), None, None) == CUDA_ERR
+        assert all((x == 0.1).all() for x in a)
+        c.radiation_field(rc)
+        pops = np.full((10, N), 0.1)
+        rates = np.full((10, 3, N), 0.1)
+        fake.fake_refuse_d2h(1)
+        assert L.portal_solve_se(c._h, 2, None, None, P(pops), P(rates), None, None) == CUDA_ERR
+        assert (pops == 0.1).all() and (rates == 0.1).all()
+        c.radiation_field(rc)
+        c.solve_se(2)
+        out = np.full((8, 1, 41, 31, 31), 0.1, dtype=np.float32)
+        l1, l2 = np.array([1], dtype=np.int32), np.array([2], dtype=np.int32)
+        fake.fake_refuse_d2h(1)
+        ptrs = [out[q].ctypes.data_as(pg.P_F) for q in range(8)]
+        assert L.portal_image(c._h, None, 1, P(l1, pg.P_I), P(l2, pg.P_I), 0.3, 0.2, 20, 300.0, 0.0, 15, 0.4, 0.15, 1e-4,
+                              1000, *ptrs, None) == CUDA_ERR
+        assert (out == np.float32(0.1)).all()
+    """)
+
+
+def test_result_in_the_place_of_an_input(fake_cuda):
+    """Pinned memory, where the upload is still on its way when the kernel has
+    been launched: JJ_20 in the array of J2 leaves the J2 that is solved for."""
+    fake_cuda("""
+        mol = synth.linear_rotor(5)
+        cloud = synth.power_law_sphere(2048, 1, mol)
+        c = pg.Context(0)
+        c.set_molecule(mol)
+        c.set_cloud(cloud)
+        c.radiation_field(run())
+        c.solve_se(2)
+        rng = np.random.default_rng(1)
+        J0, J2 = rng.random((2048, 4)) + 1.0, rng.random((2048, 4)) + 1.0
+        keep = J2.copy()
+        pops = np.zeros((10, 2048))
+        rates = np.zeros((10, 3, 2048))
+        P = pg._p
+        fake.fake_deferred(1)
+        assert pg.lib().portal_solve_se(c._h, 2, P(J0), P(J2), P(pops), P(rates), P(J2), None) == 0
+        fake.fake_deferred(0)
+        _, sent, _ = c.results(pops=False)
+        np.testing.assert_array_equal(sent, keep)
+    """)
