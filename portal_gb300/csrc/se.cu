@@ -609,9 +609,6 @@ __global__ void __launch_bounds__(TW == 1 ? 256 : 32 * TW, se_min_blocks<TW, MR,
     double *const slot = (BATCH ? bw.a64 : a0.a64) +
                          (size_t)((long long)blockIdx.x * teams + team) * (BATCH ? bw.a64_stride : a0.a64_stride);
     int cur_model = -1;
-    // a pass of the iterated node loop with failed walks: the last good pass's
-    // populations stay
-    if (!BATCH && a0.skip && *a0.skip) return;
 
     // (nodes go to the blocks in turn, so that few nodes spread over the SMs)
     for (long long item = (long long)team * gridDim.x + blockIdx.x; item < n_items; item += (long long)gridDim.x * teams) {
@@ -641,6 +638,10 @@ __global__ void __launch_bounds__(TW == 1 ? 256 : 32 * TW, se_min_blocks<TW, MR,
         float *d32 = LU + (size_t)n * n;
         float *scl = GAUSS ? gm.scl : d32 + n;
         int *piv = GAUSS ? gm.kof : (int *)(scl + n);
+        // a pass of the iterated node loop with failed walks: the last good
+        // pass's populations stay (asked once a node: before the loop it cost the
+        // 74 x 74 systems' registers, 0.84 -> 0.88 ms)
+        if (!BATCH && a.skip && *a.skip) return;
         if (!(a.ab[node] > 0.0)) {  // main_para.f90:213 (pops and alignments stay 0)
             if (!BATCH) {
                 for (int c2 = tid; c2 < 2 * a.nlev; c2 += TS) a.pops[(size_t)node + (size_t)a.N * c2] = 0.0;
@@ -1048,7 +1049,7 @@ __global__ void __launch_bounds__(TW == 1 ? 256 : 32 * TW, se_min_blocks<TW, MR,
         }
         tsync();
     }
-    if (!BATCH) {
+    if (!BATCH && !(a0.skip && *a0.skip)) {
         // the boundary nodes' rows are 0
         const int nb = a0.N - a0.bulk, cols = 2 * a0.nlev + a0.L;
         const long long total = (long long)nb * cols;
