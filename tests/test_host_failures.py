@@ -333,16 +333,16 @@ def test_scratch_of_ray_items_refuses_no_call(fake_cuda):
         assert max(int(l.split()[1]) for l in log() if l.startswith("free")) == walk
         assert live() > 2 * walk
         memory()
-        # not held above 256 MB
+        # not held above 1 GB
         mol = synth.linear_rotor(20)
         c.set_molecule(mol)
-        c.set_cloud(synth.power_law_sphere(4096, 1, mol))
+        c.set_cloud(synth.power_law_sphere(14000, 1, mol))
         log()
         before = live()
         rc = run(nth=40)
         c.radiation_field(rc)
         sums = max(int(l.split()[1]) for l in log(False) if l.startswith("malloc"))
-        assert sums > 256 << 20 and any("k_rf_finish" in x for x in kernels())
+        assert sums > 1 << 30 and any("k_rf_finish" in x for x in kernels())
         assert live() < before + sums
     """)
 
