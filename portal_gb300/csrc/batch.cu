@@ -248,6 +248,11 @@ extern "C" int portal_batch_prepare(portal_batch *b, int nth, int nph, int nvel,
     std::vector<RFC> rfc;
     size_t rf_grid = 0;
     for (int nlg : {5, 10}) {
+        // (with dust, or five lines at most, both give the same groups: one launch to time)
+        bool same = !rfc.empty();
+        for (int lines : b->lines)
+            same = same && rf_line_group(lines, nlg, b->dust) == rf_line_group(lines, rfc[0].nlg, b->dust);
+        if (same) continue;
         int mx = 0;
         if (rf_batch_blocks_per_sm(rf_batch(b, nullptr, 0, nlg), b->dust, &mx))
             return bfail(b, PORTAL_ERR_CUDA, "occupancy query");

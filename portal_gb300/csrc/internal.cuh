@@ -149,6 +149,7 @@ size_t rf_walk_records(int n_depth);     // walk scratch per warp, int2 records
 // the batched launch: its shape for these models (max_group: the widest line
 // group wanted), and the blocks per SM the kernel reaches with it
 void rf_batch_shape(RFBatch *bw, const int *lines, int n_models, int nch, bool dust, int max_group, bool split);
+int rf_line_group(int lines, int max_group, bool dust);   // the groups' width for a model of so many lines
 int rf_batch_blocks_per_sm(const RFBatch &bw, bool dust, int *blocks);
 int rf_batch_launch(cudaStream_t s, int grid, bool dust, const RFBatch &bw);
 constexpr int RF_BATCH_WARPS = 4;        // warps per block of the batched launch

@@ -34,6 +34,8 @@ void rf_batch_shape(RFBatch *bw, const int *lines, int n_models, int nch, bool d
                                   (size_t)rf_shape(lines[m], max_group, nch, dust, bw->rt, split).bytes);
 }
 
+int rf_line_group(int lines, int max_group, bool dust) { return tab_shape(lines, max_group, dust).nlg; }
+
 // Also sets the kernel's dynamic shared-memory limit: called before the pass is
 // captured.
 int rf_batch_blocks_per_sm(const RFBatch &bw, bool dust, int *blocks) {

@@ -426,3 +426,26 @@ def test_result_in_the_place_of_an_input(fake_cuda):
         _, sent, _ = c.results(pops=False)
         np.testing.assert_array_equal(sent, keep)
     """)
+
+
+def test_batch_times_no_launch_twice(fake_cuda):
+    """Line groups of 5 and of 10 are one launch with dust or five lines at most."""
+    fake_cuda("""
+        def candidates(levels, dust=False):
+            mol = synth.linear_rotor(levels)
+            cloud = synth.power_law_sphere(600, 1, mol)
+            if dust:
+                cloud.dust_p = cloud.h2_dens * synth.F4(2.32e-27) / 100.0
+            c = pg.Context(0)
+            c.set_molecule(mol)
+            c.set_cloud(cloud)
+            with pg.Batch(0) as b:
+                b.add(c)
+                b.prepare(run())
+                rows = b.config()[1]
+            fake.fake_log_clear()
+            return [int(r[0]) for r in rows]
+        assert candidates(4)[:2] == [5, 2]            # the second row is the solve's
+        assert candidates(12, dust=True)[:2] == [5, 2]
+        assert candidates(12)[:3] == [5, 10, 2]
+    """)
