@@ -200,6 +200,9 @@ extern "C" int portal_batch_prepare(portal_batch *b, int nth, int nph, int nvel,
         size_t w = 0;
         if ((rc = se_prepare(c, kmax, &b->se[m], &w)))
             return bfail(b, rc, "model " + std::to_string(m) + ": " + c->err);
+        // (a call of the model that failed may have left kernels on its stream;
+        // with its tables kept, nothing above waits for them)
+        BCHECK(b, cudaStreamSynchronize(c->stream));
         wb = std::max(wb, w);
         b->se_a64_stride = std::max(b->se_a64_stride, se_matrix_doubles(c));
         b->se_max_dim = std::max(b->se_max_dim, c->c_dim);

@@ -449,3 +449,26 @@ def test_batch_times_no_launch_twice(fake_cuda):
         assert candidates(12, dust=True)[:2] == [5, 2]
         assert candidates(12)[:3] == [5, 10, 2]
     """)
+
+
+def test_batch_waits_for_its_models(fake_cuda):
+    """A model's call that fails after its first launch (no memory for the walks)
+    leaves kernels on its stream: the batch's own launches come after them,
+    also where the model's tables are kept from before."""
+    fake_cuda("""
+        c = model()
+        with pg.Batch(0) as b:
+            b.add(c)
+            b.prepare(run())
+            memory(single=300 << 20)
+            log()
+            fails(NOMEM, c.radiation_field, run(n_depth=3200000))
+            launches = [l for l in log() if l.startswith("launch")]
+            memory()
+            stream = launches[-1].split("stream ")[1]
+            b.prepare(run())
+            ops = [l for l in log() if l.startswith(("launch", "sync"))]
+            first = next(i for i, l in enumerate(ops) if l.startswith("launch"))
+            assert "sync stream " + stream in ops[:first]
+            assert not ops[first].endswith("stream " + stream)
+    """)
