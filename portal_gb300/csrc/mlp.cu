@@ -1242,9 +1242,8 @@ extern "C" int portal_mlp_gradients(portal_mlp *m, const float *X, const float *
                                     float *loss) {
     if (!m || !X || !T || B < 1) return PORTAL_ERR_ARG;
     cudaSetDevice(m->device);
-    if (m->fused) {
-        int rc = fused_reserve(m, B);
-        if (rc) return rc;
+    if (m->fused && !fused_reserve(m, B)) {   // (layer by layer where its buffers do not fit)
+        int rc = PORTAL_OK;
         if (m->xbuf.reserve((size_t)B * m->n_in) || m->ybuf.reserve((size_t)B * m->n_out))
             return mlp_fail(m, PORTAL_ERR_NOMEM, "MLP workspace");
         MCHECK(m, cudaMemcpyAsync(m->xbuf.p, X, (size_t)B * m->n_in * sizeof(float), cudaMemcpyHostToDevice, m->stream));
@@ -1318,10 +1317,15 @@ extern "C" int portal_mlp_train(portal_mlp *m, const float *X, const float *Y, i
     MCHECK(m, cudaMemcpyAsync(dX.p, X, (size_t)M * nin * sizeof(float), cudaMemcpyHostToDevice, m->stream));
     MCHECK(m, cudaMemcpyAsync(dY.p, Y, (size_t)M * nout * sizeof(float), cudaMemcpyHostToDevice, m->stream));
     const int B = std::min(batch, M);
-    int rc = m->fused ? fused_reserve(m, B) : ensure_batch(m, B);
-    if (rc || (m->fused && (rc = fused_pack(m)))) return rc;
+    // (layer by layer where the whole-network kernels' buffers do not fit)
+    const bool fused = m->fused && !fused_reserve(m, B);
+    int rc = fused ? fused_pack(m) : ensure_batch(m, B);
+    if (rc) return rc;
     Work w;
-    if (!m->fused) w = layout(m, B);
+    if (!fused) {
+        w = layout(m, B);
+        m->packed = false;   // (k_adam updates the parameters alone)
+    }
     std::mt19937_64 rng(seed);
     std::vector<int> perm(M);
     for (int i = 0; i < M; i++) perm[i] = i;
@@ -1337,7 +1341,7 @@ extern "C" int portal_mlp_train(portal_mlp *m, const float *X, const float *Y, i
             MCHECK(m, cudaMemsetAsync(m->lossacc.p, 0, sizeof(double), m->stream));
         }
         MCHECK(m, cudaStreamSynchronize(m->stream));  // perm is rewritten next epoch
-        for (int b0 = 0; m->fused && b0 + B <= M; b0 += B, nbatch++) {
+        for (int b0 = 0; fused && b0 + B <= M; b0 += B, nbatch++) {
             m->step++;
             const AdamArgs ad{m->params.p, m->adam_m.p, m->adam_v.p, m->pk.p, lr, b1, b2, eps,
                               1.f - std::pow(b1, (float)m->step), 1.f - std::pow(b2, (float)m->step)};
@@ -1345,7 +1349,7 @@ extern "C" int portal_mlp_train(portal_mlp *m, const float *X, const float *Y, i
                                  loss_per_epoch ? m->lossacc.p : nullptr)))
                 return rc;
         }
-        for (int b0 = 0; !m->fused && b0 + B <= M; b0 += B) {
+        for (int b0 = 0; !fused && b0 + B <= M; b0 += B) {
             k_gather<<<(B + 127) / 128, 128, 0, m->stream>>>(B, nin, nout, pidx.p + b0, dX.p, dY.p, m->stats.p, w.X,
                                                              m->ybuf.p);
             forward(m, B, w);

@@ -472,3 +472,25 @@ def test_batch_waits_for_its_models(fake_cuda):
             assert "sync stream " + stream in ops[:first]
             assert not ops[first].endswith("stream " + stream)
     """)
+
+
+def test_batch_too_large_for_the_whole_network_kernels(fake_cuda):
+    """Their buffers take more memory a row than the layers' one by one: where
+    they do not fit, the call runs layer by layer, and the weights it leaves
+    are the ones that are packed for the next."""
+    fake_cuda("""
+        def kernels():
+            return [l.split()[1] for l in log() if l.startswith("launch")]
+        with pg.MLP(8, 256, 16, 40) as net:
+            X, T = np.zeros((20000, 8)), np.zeros((20000, 40))
+            rows = 4 * (16 * 256 + 40)
+            memory(single=int(20000 * 2.6 * rows))     # whole network 3 x, layers 2.1 x
+            net.gradients(X, T)
+            assert any("k_gemm_tc" in k for k in kernels())
+            net.train(X, T, 1, 20000, 1e-3)
+            assert any("k_adam" in k for k in kernels())
+            memory()
+            net.train(X, T, 1, 20000, 1e-3)
+            k = kernels()
+            assert any("k_mlp_rows" in x for x in k) and any("k_pack_weights" in x for x in k)
+    """)
