@@ -778,11 +778,11 @@ static int image_call(portal_ctx *c, const double *pol_pops, int nlines, const i
     DevBuf<float4> &cellv = c->im_cellv, &cellb = c->im_cellb, &coef = c->im_coef;
     DevBuf<float> &outd = c->im_out;
     DevBuf<unsigned char> &on_star = c->im_star;
-    // the cubes are kept for the next call up to 1 GB
+    // the cubes are kept for the next call up to KEEP_BYTES
     struct KeepSmall {
         DevBuf<float> &b;
         ~KeepSmall() {
-            if (b.n * sizeof(float) > (size_t)1 << 30) b.release();
+            if (b.n * sizeof(float) > KEEP_BYTES) b.release();
         }
     } keep{outd};
     const size_t cube = (size_t)nrays * nch * nlines;

@@ -1313,6 +1313,17 @@ extern "C" int portal_mlp_train(portal_mlp *m, const float *X, const float *Y, i
     column_stats(Y, nout, st.data() + 2 * nin, st.data() + 2 * nin + nout);
     MCHECK(m, cudaMemcpyAsync(m->stats.p, st.data(), st.size() * sizeof(float), cudaMemcpyHostToDevice, m->stream));
     DevBuf<float> &dX = m->train_x, &dY = m->train_y;
+    // the rows are kept for the next call up to KEEP_BYTES
+    struct KeepSmall {
+        portal_mlp *m;
+        ~KeepSmall() {
+            if (sizeof(float) * (m->train_x.n + m->train_y.n) + sizeof(int) * m->train_perm.n <= KEEP_BYTES) return;
+            cudaStreamSynchronize(m->stream);
+            m->train_x.release();
+            m->train_y.release();
+            m->train_perm.release();
+        }
+    } keep{m};
     if (dX.reserve((size_t)M * nin) || dY.reserve((size_t)M * nout)) return mlp_fail(m, PORTAL_ERR_NOMEM, "MLP data");
     MCHECK(m, cudaMemcpyAsync(dX.p, X, (size_t)M * nin * sizeof(float), cudaMemcpyHostToDevice, m->stream));
     MCHECK(m, cudaMemcpyAsync(dY.p, Y, (size_t)M * nout * sizeof(float), cudaMemcpyHostToDevice, m->stream));

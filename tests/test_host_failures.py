@@ -494,3 +494,16 @@ def test_batch_too_large_for_the_whole_network_kernels(fake_cuda):
             k = kernels()
             assert any("k_mlp_rows" in x for x in k) and any("k_pack_weights" in x for x in k)
     """)
+
+
+def test_training_rows_are_not_held_above_the_bound(fake_cuda):
+    fake_cuda("""
+        with pg.MLP(8, 16, 1, 200) as net:
+            X, T = np.zeros((1400000, 8), dtype=np.float32), np.zeros((1400000, 200), dtype=np.float32)
+            net.train(X[:1000], T[:1000], 1, 1000, 1e-3)
+            held = live()
+            net.train(X[:1000], T[:1000], 1, 1000, 1e-3)
+            assert live() == held
+            net.train(X, T, 1, 1000, 1e-3)      # 1.16 GB
+            assert live() <= held
+    """)
