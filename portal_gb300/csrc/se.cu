@@ -230,7 +230,7 @@ __device__ bool team_lu(int n, T *M, int *piv, int tid, double *red_v, int *red_
 }
 
 // Dynamic shared memory per team of the LU form (the inverses': GaussMem):
-//   feat [n_feat] double | x, r [n] double | LU32 [n*n] float | d32 [n] float
+//   feat [n_feat] double | x [n] double | LU32 [n*n] float | d32 [n] float
 //   | scale [n] float | piv [n] int
 // The FP64 matrix is kept as its entries only, row by row (a fifth of the
 // 74 x 74 systems, a third of the 34 x 34: collisions couple the K = 0
@@ -245,7 +245,7 @@ constexpr int SE_WARP_DIM = 32;    // and by one warp in registers
 
 __host__ __device__ inline size_t se_warp_bytes(int n, int n_feat) {
     size_t b = 0;
-    b += sizeof(double) * ((size_t)n_feat + 2 * (size_t)n);
+    b += sizeof(double) * ((size_t)n_feat + (size_t)n);
     b += sizeof(float) * ((size_t)n * n + 2 * (size_t)n);
     b += sizeof(int) * (size_t)n;
     return (b + 15) & ~(size_t)15;
@@ -376,7 +376,7 @@ __device__ __forceinline__ void turn_slots(float (&a)[NC][MR], int na) {
 struct GaussMem {
     float *row;    // [8 nq] staged pivot rows, two per warp
     float *z;      // [4 nq] permuted residual
-    double *feat, *x, *r, *val;
+    double *feat, *x, *val;
     float *valf;   // [nnz + 1] scaled entries, 0
     float *scl;    // [n]
     float *part;   // [4 n] partial products
@@ -391,7 +391,7 @@ template <int TW, int NC>
 constexpr int gauss_quads = NC == 0 ? SE_GAUSS_DIM / 4 : NC * TW / 4;
 __host__ __device__ inline size_t se_gauss_bytes(int n, int n_feat, int nnz, int nq, bool dense) {
     size_t b = sizeof(float) * 12 * (size_t)nq;
-    b += sizeof(double) * ((size_t)n_feat + 2 * (size_t)n + (size_t)nnz);
+    b += sizeof(double) * ((size_t)n_feat + (size_t)n + (size_t)nnz);
     b += sizeof(float) * ((size_t)nnz + 1 + 7 * (size_t)n + 2 * (size_t)((n + 31) & ~31) + 8);
     if (dense) b += sizeof(float) * (size_t)n * n;
     return (b + 15) & ~(size_t)15;
@@ -402,8 +402,7 @@ __device__ __forceinline__ GaussMem gauss_mem(unsigned char *base, int n, int n_
     g.z = g.row + 8 * nq;
     g.feat = (double *)(g.z + 4 * nq);
     g.x = g.feat + n_feat;
-    g.r = g.x + n;
-    g.val = g.r + n;
+    g.val = g.x + n;
     g.valf = (float *)(g.val + nnz);
     g.scl = g.valf + nnz + 1;
     g.part = g.scl + n;
@@ -632,9 +631,8 @@ __global__ void __launch_bounds__(TW == 1 ? 256 : 32 * TW, se_min_blocks<TW, MR,
         const GaussMem gm = GAUSS ? gauss_mem(base, n, a.n_feat, a.nnz, nq) : GaussMem{};
         double *feat = GAUSS ? gm.feat : (double *)base;
         double *x = GAUSS ? gm.x : feat + (size_t)a.n_feat;
-        double *r = x + n;   // scratch (the rates)
         double *val = GAUSS ? gm.val : slot;
-        float *LU = (float *)(r + n);
+        float *LU = (float *)(x + n);
         float *d32 = LU + (size_t)n * n;
         float *scl = GAUSS ? gm.scl : d32 + n;
         int *piv = GAUSS ? gm.kof : (int *)(scl + n);
@@ -996,47 +994,49 @@ __global__ void __launch_bounds__(TW == 1 ? 256 : 32 * TW, se_min_blocks<TW, MR,
             // k (spontaneous, radiative, collisional), sum_j |M_k(i,j)| rho_j,
             // M_k the part of setup_stateq's matrix from A, from B J, from C
             // (pop_eqs.f90:424-426, 510-512, 558-559, 599-645); the unsplit
-            // field's values (f0, f2) stand for f5, f6.  Row by row in
-            // ascending column order, as the reference sums.
-            for (int k = 0; k < 3; k++) {
-                for (int i = tid; i < n; i += TS) {
-                    double acc = 0.0;
-                    if (!(st & PORTAL_NODE_SINGULAR))
-                        for (int q = a.row_off[i]; q < a.row_off[i + 1]; q++) {
-                            const int e = a.row_ent[q];
-                            double v = 0.0;
-                            for (int t = a.ent_off[e]; t < a.ent_off[e + 1]; t++) {
-                                const int tf = a.term_f[t];
-                                if (tf >= NF * a.n_trans) {
-                                    // depolarisation: C_mat where col_dep is assigned; the
-                                    // carried copies (mode 2) are in Amat only
-                                    if (k == 2 && tf < NF * a.n_trans + a.n_dep) v += a.term_c[t] * feat[tf];
-                                    continue;
-                                }
-                                const int f = tf % NF, base = tf - f;
-                                const int kind = (f == 2 || f == 6) ? 0 : (f == 3 || f == 4) ? 2 : 1;
-                                if (kind != k) continue;
-                                const int fu = (f == 5) ? 0 : (f == 6) ? 2 : f;
-                                v += a.term_c[t] * feat[base + fu];
+            // field's values (f0, f2) stand for f5, f6.  Each sum in ascending
+            // column order, as the reference's; the three kinds' sums together over
+            // the team's threads (4,000 systems of 33 unknowns with rates 0.73 ms;
+            // kind by kind, 95 of 128 threads idle, 1.55, one warp a node 1.48).
+            double *r3 = slot + a.nnz;   // (the FP64 fallback is done with it)
+            for (int q3 = tid; q3 < 3 * n; q3 += TS) {
+                const int k = q3 / n, i = q3 - k * n;
+                double acc = 0.0;
+                if (!(st & PORTAL_NODE_SINGULAR))
+                    for (int q = a.row_off[i]; q < a.row_off[i + 1]; q++) {
+                        const int e = a.row_ent[q];
+                        double v = 0.0;
+                        for (int t = a.ent_off[e]; t < a.ent_off[e + 1]; t++) {
+                            const int tf = a.term_f[t];
+                            if (tf >= NF * a.n_trans) {
+                                // depolarisation: C_mat where col_dep is assigned; the
+                                // carried copies (mode 2) are in Amat only
+                                if (k == 2 && tf < NF * a.n_trans + a.n_dep) v += a.term_c[t] * feat[tf];
+                                continue;
                             }
-                            acc += fabs(v) * x[a.ent_pos[e] / n];
+                            const int f = tf % NF, base = tf - f;
+                            const int kind = (f == 2 || f == 6) ? 0 : (f == 3 || f == 4) ? 2 : 1;
+                            if (kind != k) continue;
+                            const int fu = (f == 5) ? 0 : (f == 6) ? 2 : f;
+                            v += a.term_c[t] * feat[base + fu];
                         }
-                    r[i] = acc;
-                }
-                tsync();
-                // packing as the populations (main_sub.f90:116-135): K = 2
-                // components of J = 0 levels are 0; a NaN population zeroes the
-                // K = 2 rate entry (twice, as in the reference)
-                for (int c2 = tid; c2 < 2 * a.nlev; c2 += TS) {
-                    const int pidx = a.pack[c2];
-                    double v = (pidx >= 0) ? r[pidx] : 0.0;
-                    if (c2 & 1) {
-                        const double p0 = x[a.pack[c2 - 1]];
-                        if (p0 != p0) v = 0.0;
+                        acc += fabs(v) * x[a.ent_pos[e] / n];
                     }
-                    a.rates[(size_t)node + (size_t)a.N * (k + 3 * (size_t)c2)] = v;
+                r3[q3] = acc;
+            }
+            tsync();
+            // packing as the populations (main_sub.f90:116-135): K = 2
+            // components of J = 0 levels are 0; a NaN population zeroes the
+            // K = 2 rate entry (twice, as in the reference)
+            for (int q3 = tid; q3 < 6 * a.nlev; q3 += TS) {
+                const int k = q3 / (2 * a.nlev), c2 = q3 - k * 2 * a.nlev;
+                const int pidx = a.pack[c2];
+                double v = (pidx >= 0) ? r3[k * n + pidx] : 0.0;
+                if (c2 & 1) {
+                    const double p0 = x[a.pack[c2 - 1]];
+                    if (p0 != p0) v = 0.0;
                 }
-                tsync();
+                a.rates[(size_t)node + (size_t)a.N * (k + 3 * (size_t)c2)] = v;
             }
         }
         if (a.jj20)
@@ -1442,7 +1442,8 @@ int se_batch_pass(portal_ctx *c, cudaStream_t s) {
     return se_pass(c, s);
 }
 
-size_t se_matrix_doubles(const portal_ctx *c) { return (size_t)c->se_nnz + (size_t)c->c_dim * c->c_dim; }
+// (the rates' 3 n sums take the dense matrix's place)
+size_t se_matrix_doubles(const portal_ctx *c) { return (size_t)c->se_nnz + (size_t)c->c_dim * std::max(c->c_dim, 3); }
 
 // Whether the prepared system is inverted, and the inversion's shared memory
 // per warp.  The limit is on the largest form, the same for every launch.
