@@ -131,20 +131,34 @@ extern "C" int portal_set_molecule(portal_ctx *c, int nlev, const int *j_lev, co
     return PORTAL_OK;
 }
 
-// Edge geometry from the FP64 positions; one thread per (node, slot).
-__global__ void k_build_edges(int N, int maxne, const int *__restrict__ del_ne,
+constexpr int WALK_TAIL = 16;   // slots behind the last block of the walk tables
+
+// Edge geometry from the FP64 positions; one thread per (node, slot of its walk
+// block, padding included), and one per slot of the walk tables' tail.
+__global__ void k_build_edges(int N, int slots, const int *__restrict__ del_ne,
                               const int *__restrict__ off, const double *__restrict__ pos,
                               int *__restrict__ nb_idx, float4 *__restrict__ edge, const int *__restrict__ wstart,
                               int2 *__restrict__ whead, float4 *__restrict__ wedge, int *__restrict__ wnext) {
     long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    long long tot = (long long)N * maxne;
+    const size_t end = 4 * (size_t)wstart[N];
+    if (tid < WALK_TAIL) {
+        wedge[end + tid] = make_float4(0.f, 0.f, 0.f, 0.f);
+        wnext[end + tid] = 0;
+    }
+    long long tot = (long long)N * slots;
     if (tid >= tot) return;
     int s = (int)(tid / N);
     int i = (int)(tid - (long long)s * N);
     int o = off[i], deg = off[i + 1] - o;
     const size_t w = 4 * (size_t)wstart[i];
     if (s == 0) whead[wstart[i]] = make_int2(deg, i);
-    if (s >= deg) return;
+    if (s >= deg) {   // (slots past the degree are loaded, never used)
+        if (w + s < 4 * (size_t)wstart[i + 1]) {
+            wedge[w + s] = make_float4(0.f, 0.f, 0.f, 0.f);
+            wnext[w + s] = 0;
+        }
+        return;
+    }
     int nb = del_ne[(size_t)i + (size_t)N * s] - 1;
     double ex = pos[3 * (size_t)nb] - pos[3 * (size_t)i];
     double ey = pos[3 * (size_t)nb + 1] - pos[3 * (size_t)i + 1];
@@ -187,8 +201,11 @@ extern "C" int portal_set_cloud(portal_ctx *c, int N, int bulk, int nlev, const 
     cudaSetDevice(c->device);
     // CSR offsets + validation on the host (cheap, and fails loudly before
     // any kernel can read out of bounds)
-    std::vector<int> off(N + 1);
-    off[0] = 0;
+    std::vector<int> off(2 * ((size_t)N + 1));   // and the walk blocks' first groups
+    // (degrees rounded up to groups of 4 slots, at least one -- an isolated node
+    // has a header too -- and a tail that the first loads of the last blocks may
+    // run into)
+    int *ws = off.data() + N + 1;
     int maxdeg = 0;
     for (int i = 0; i < N; i++) {
         int d = del_num_ne[i];
@@ -197,6 +214,7 @@ extern "C" int portal_set_cloud(portal_ctx *c, int N, int bulk, int nlev, const 
         if ((long long)off[i] + d > 2000000000LL)
             return set_err(c, PORTAL_ERR_ARG, "portal_set_cloud: more than 2e9 neighbour entries");
         off[i + 1] = off[i] + d;
+        ws[i + 1] = ws[i] + std::max(1, (d + 3) / 4);
         if (d > maxdeg) maxdeg = d;
         for (int s = 0; s < d; s++) {
             int nb = del_ne[(size_t)i + (size_t)N * s];
@@ -205,25 +223,15 @@ extern "C" int portal_set_cloud(portal_ctx *c, int N, int bulk, int nlev, const 
         }
     }
     int nnz = off[N];
-    // the walk tables' blocks: degrees rounded up to groups of 4 slots, at least
-    // one (an isolated node has a header too), and a tail that the first
-    // loads of the last blocks may run into
-    std::vector<int> ws(N);
-    size_t groups = 0;
-    for (int i = 0; i < N; i++) {
-        ws[i] = (int)groups;
-        groups += std::max(1, (off[i + 1] - off[i] + 3) / 4);
-    }
-    groups += 4;
-    const size_t slots = 4 * groups;
+    const size_t groups = ws[N], slots = 4 * groups + WALK_TAIL;
     c->have_cloud = false;
     c->j_valid = false;
     c->ali_valid = false;
     if (c->pos64.reserve(3 * (size_t)N) || c->bvec64.reserve(3 * (size_t)N) ||
-        c->cellv.reserve(N) || c->nb_off.reserve(N + 1) || c->nb_idx.reserve(nnz) ||
+        c->cellv.reserve(N) || c->nb_off.reserve(off.size()) || c->nb_idx.reserve(nnz) ||
         c->edge.reserve(nnz) || c->levp.reserve((size_t)nlev * N) || c->b64.reserve(N) ||
         c->tkin.reserve(N) || c->tdust.reserve(N) || c->dustp.reserve(N) || c->h2.reserve(N) ||
-        c->ab.reserve(N) || c->status.reserve(N) || c->nmol.reserve(N) || c->wstart.reserve(N) ||
+        c->ab.reserve(N) || c->status.reserve(N) || c->nmol.reserve(N) ||
         c->whead.reserve(groups) || c->wedge.reserve(slots) || c->wnext.reserve(slots))
         return set_err(c, PORTAL_ERR_NOMEM, "portal_set_cloud: device allocation failed");
     std::vector<double> tk(N), td(N), nm(N);
@@ -247,12 +255,9 @@ extern "C" int portal_set_cloud(portal_ctx *c, int N, int bulk, int nlev, const 
     if ((rc = upload(c, c->h2.p, h2_dens, N))) return rc;
     if ((rc = upload(c, c->ab.p, ab_all, N))) return rc;
     if ((rc = upload(c, c->nmol.p, nm.data(), N))) return rc;
-    PCHECK(c, cudaMemcpyAsync(c->nb_off.p, off.data(), (N + 1) * sizeof(int),
+    c->wstart = c->nb_off.p + N + 1;
+    PCHECK(c, cudaMemcpyAsync(c->nb_off.p, off.data(), off.size() * sizeof(int),
                               cudaMemcpyHostToDevice, c->stream));
-    PCHECK(c, cudaMemcpyAsync(c->wstart.p, ws.data(), N * sizeof(int), cudaMemcpyHostToDevice, c->stream));
-    // (slots past a node's degree are loaded, never used)
-    PCHECK(c, cudaMemsetAsync(c->wedge.p, 0, slots * sizeof(float4), c->stream));
-    PCHECK(c, cudaMemsetAsync(c->wnext.p, 0, slots * sizeof(int), c->stream));
     DevBuf<int> dne;
     if (dne.reserve((size_t)N * maxne) || c->vel64.reserve(3 * (size_t)N))
         return set_err(c, PORTAL_ERR_NOMEM, "portal_set_cloud: staging allocation failed");
@@ -260,10 +265,10 @@ extern "C" int portal_set_cloud(portal_ctx *c, int N, int bulk, int nlev, const 
                               cudaMemcpyHostToDevice, c->stream));
     PCHECK(c, cudaMemcpyAsync(c->vel64.p, vel_all, 3 * (size_t)N * sizeof(double),
                               cudaMemcpyHostToDevice, c->stream));
-    long long tot = (long long)N * maxne;
-    k_build_edges<<<(unsigned)((tot + 255) / 256), 256, 0, c->stream>>>(N, maxne, dne.p, c->nb_off.p,
-                                                                      c->pos64.p, c->nb_idx.p,
-                                                                      c->edge.p, c->wstart.p, c->whead.p,
+    const int per = 4 * std::max(1, (maxdeg + 3) / 4);
+    const long long tot = std::max((long long)N * per, (long long)WALK_TAIL);
+    k_build_edges<<<(unsigned)((tot + 255) / 256), 256, 0, c->stream>>>(N, per, dne.p, c->nb_off.p, c->pos64.p,
+                                                                      c->nb_idx.p, c->edge.p, c->wstart, c->whead.p,
                                                                       c->wedge.p, c->wnext.p);
     PCHECK(c, cudaGetLastError());
     k_cellv<<<(N + 255) / 256, 256, 0, c->stream>>>(N, c->vel64.p, c->b64.p, c->cellv.p);

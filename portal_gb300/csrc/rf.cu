@@ -386,7 +386,7 @@ int rf_prepare(portal_ctx *c, int nth, int nph, int nvel, const double *gvec, do
     a.N = N; a.bulk = c->bulk; a.L = L; a.nvel = nvel; a.nch = nch; a.ndir = ndir; a.n_depth = n_depth;
     a.dx32 = (float)dx;
     a.pos = c->pos64.p; a.bvec = c->bvec64.p; a.ab = c->ab.p; a.cellv = c->cellv.p;
-    a.wstart = c->wstart.p; a.whead = c->whead.p; a.wedge = c->wedge.p; a.wnext = c->wnext.p; a.ltab = c->ltab.p;
+    a.wstart = c->wstart; a.whead = c->whead.p; a.wedge = c->wedge.p; a.wnext = c->wnext.p; a.ltab = c->ltab.p;
     a.dirs = c->dirtab.p; a.chq = c->chtab.p; a.chw = c->chtab.p + nch; a.bb = c->bbcmb.p;
     a.gx = gvec[0]; a.gy = gvec[1]; a.gz = gvec[2];
     a.ab = c->active_ab();

@@ -186,6 +186,7 @@ cudaError_t cudaGetSymbolAddress(void **p, const void *sym) {
 cudaError_t cudaMemset(void *p, int v, size_t n) { std::memset(p, v, n); return cudaSuccess; }
 cudaError_t cudaMemsetAsync(void *p, int v, size_t n, cudaStream_t s) {
     std::lock_guard<std::recursive_mutex> g(mu);
+    note("memset " + std::to_string(n));
     if (capturing) return cudaSuccess;
     if (deferred) pending[s].push_back([=] { std::memset(p, v, n); });
     else std::memset(p, v, n);

@@ -507,3 +507,19 @@ def test_training_rows_are_not_held_above_the_bound(fake_cuda):
             net.train(X, T, 1, 1000, 1e-3)      # 1.16 GB
             assert live() <= held
     """)
+
+
+def test_set_cloud_makes_no_more_calls_than_the_cloud_needs(fake_cuda):
+    """The walk tables come with the cloud's: one upload for both offsets, their
+    padding written by the kernel that fills them."""
+    fake_cuda("""
+        mol = synth.linear_rotor(4)
+        c = pg.Context(0)
+        c.set_molecule(mol)
+        cloud = synth.power_law_sphere(600, 1, mol)
+        c.set_cloud(cloud)
+        log()
+        c.set_cloud(cloud)
+        calls = [l.split()[0] for l in log()]
+        assert calls.count("h2d") == 13 and calls.count("launch") == 2 and calls.count("memset") == 0, calls
+    """)
