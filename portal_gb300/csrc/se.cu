@@ -897,12 +897,11 @@ __global__ void __launch_bounds__(TW == 1 ? 256 : 32 * TW, se_min_blocks<TW, MR,
                     if (kd >= 0x7f800000u || kx >= 0x7ff00000u) break;  // infinite or NaN
                     const double dm = (double)__uint_as_float(kd), xmax = __hiloint2double((int)kx, 0);
                     // converged: the correction is at the level FP64 residuals can
-                    // resolve (~cond(SA) * eps), or it stopped shrinking there, or
-                    // the next one, dm / dprev of this one's size, would be below
-                    // half a unit in the last place
+                    // resolve (~cond(SA) * eps), or it stopped shrinking there.  (The
+                    // norms are compared only: |x| by its upper word, the correction as
+                    // the FP32 number it is.)
                     if (dm <= 2e-14 * xmax) { conv = true; break; }
                     if (it >= 2 && dm <= 1e-12 * xmax && dm > 0.5 * dprev) { conv = true; break; }
-                    if (it >= 2 && dm <= 1e-3 * dprev && dm * dm <= 1e-16 * xmax * dprev) { conv = true; break; }
                     dprev = dm;
                 }
             }
