@@ -88,8 +88,9 @@ __device__ __forceinline__ void node_frame(int node, const double *__restrict__ 
 // |d|^2 = 1 + e, e a few ulp, sqrt(s) = 1 + e/2 - e^2/8 lies just below 1 +
 // e/2, which is a double or halfway between two: rounding 1 + e/2 downwards
 // rounds sqrt(s) correctly.  The quotient by 2 a = 2 (1 + h), h a few ulp, is
-// q = n/2 corrected by its exact residual (n - 2 a q)/2; and of the two roots
-// only the one taken is divided.
+// q - q (h - h^2) with q = n/2, rounded once (h^2 decides where q - q h lies
+// halfway between two doubles: rays that leave a node on the sphere at once
+// have an n of few bits); and of the two roots only the one taken is divided.
 __device__ __forceinline__ double sphere_exit_unit(double px, double py, double pz, double c, double dx, double dy,
                                                    double dz) {
     const double s = dsum3sq(dx, dy, dz), e = __dsub_rn(s, 1.0);
@@ -101,10 +102,9 @@ __device__ __forceinline__ double sphere_exit_unit(double px, double py, double 
     if (!(dis > 0.0)) return 0.0;
     const double sq = __dsqrt_rn(dis);
     const double n2 = __dsub_rn(-b, sq), n = (n2 > 0.0) ? n2 : __dadd_rn(-b, sq);
-    const double a2 = __dmul_rn(2.0, a);
-    if (!unit) return __ddiv_rn(n, a2);
-    const double q = __dmul_rn(0.5, n);
-    return __fma_rn(__fma_rn(-q, a2, n), 0.5, q);
+    if (!unit) return __ddiv_rn(n, __dmul_rn(2.0, a));
+    const double q = __dmul_rn(0.5, n), h = __dsub_rn(a, 1.0);
+    return __fma_rn(-q, __fma_rn(-h, h, h), q);
 }
 
 constexpr int RF_MAX_GROUP = 10;          // lines per group without dust
