@@ -584,9 +584,11 @@ def reduce_replicas(t, units, dist=None):
 
 
 def lu_rates(nodes, n, launch_ms, sms=None, sm_mhz=None):
-    """FP32 factorisation flop rate of an SE launch (2/3 n^3 per node of n
-    unknowns) and, given the SM count and the sampled clock, its fraction of
-    the FP32 FMA peak (SMs x 128 lanes x 2 flop x clock)."""
+    """The rate at which an SE launch gets through the operations that a solve
+    of n unknowns cannot do without, an LU factorisation's 2/3 n^3 per node,
+    and, given the SM count and the sampled clock, its fraction of the FP32
+    FMA peak (SMs x 128 lanes x 2 flop x clock).  (The kernel inverts systems
+    of up to 96 unknowns, three times these operations.)"""
     r = {"fp32_lu_flop_per_s": nodes * (2.0 / 3.0) * n ** 3 / (launch_ms * 1e-3)}
     if sms and sm_mhz:
         peak = sms * 128 * 2 * float(sm_mhz) * 1e6
@@ -746,7 +748,7 @@ def gpu_arm(args, rank, world, local_rank):
 
     line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": t_total_ms / args.steps, "higher_is_better": True,
-            "scaling": "weak", "vs_baseline": None, "dtype": "f32 ray integration, f32 LU + f64 refinement",
+            "scaling": "weak", "vs_baseline": None, "dtype": "f32 ray integration, f32 inverse + f64 refinement",
             "data": "synthetic", "config": workload_config(cloud, mol, rc, N),
             "e2e": {"value": e2e_val, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
             "gpu_launches": launches, "roofline": roof, "clocks": clk, "stages": stages}

@@ -23,6 +23,9 @@
  *     portal_radiation_field with J0 = J2 = NULL followed by
  *     portal_solve_se with J0 = J2 = NULL runs the whole node loop of
  *     main_portal.x without a host round trip).
+ *   - A context's calls write an output array by a copy once the device's
+ *     work is done, and nothing before: it may be an input's array of the
+ *     same shape (JJ_20 in the place of J2).
  */
 #ifndef PORTAL_GB300_H
 #define PORTAL_GB300_H
@@ -179,7 +182,8 @@ int portal_set_depolarization(portal_ctx *ctx, int mode);
  * decides convergence.  Outputs (any may be NULL): the last
  * pol_pops(N, 2*nlev), the final lev_p(nlev, N) (they also become the
  * context's populations), the number of passes, residuals(max_iter) per
- * pass, and the total ray segments walked. */
+ * pass, and the total ray segments walked.  A pass whose walks fail
+ * (PORTAL_ERR_DEPTH) leaves the populations of the pass before. */
 int portal_lambda_iterate(portal_ctx *ctx, int nth, int nph, int nvel, const double *gvec, double dx,
                           int n_depth, int kmax, double tol, int max_iter, int ng_period,
                           int local_operator, const double *start_pops,
@@ -193,7 +197,8 @@ int portal_lambda_iterate(portal_ctx *ctx, int nth, int nph, int nvel, const dou
  * (raytrace.f90:58-177) per pixel and ray_in_raytrace (:179-323) per pixel,
  * line and channel; star mode as set by portal_set_star.
  *   pol_pops(N, 2*nlev) as main_portal.x wrote it, or NULL for the
- *   device-resident result of portal_solve_se;
+ *   device-resident result of the last solve (PORTAL_ERR_STATE where there
+ *   is none for a cloud of this size);
  *   lines l1(nlines), l2(nlines) 1-based levels (at most 16 lines; as in
  *   the reference every line takes the frequency of the last pair,
  *   para_finish.f90:173-175); th_inc, ph_az inclination and azimuth

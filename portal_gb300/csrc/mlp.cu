@@ -1068,7 +1068,11 @@ void fused_setup(portal_mlp *m) {
 }
 
 // rows per CTA of a training step: few, as the step is one CTA's serial chain
-// (34 us with 32 rows, 25 with 16)
+// while every CTA has an SM of its own (8 -> 256 x 3 -> 40, one batch an epoch
+// with its wait and both launches: 32 to 512 rows 60-62 us, with 32 rows a CTA
+// 65-75; 2,048 rows 78 and 82).  From about 4,096 rows on, where the CTAs come
+// in several waves, 32 would be the better (118 and 107 us; 16,384 rows 364 and
+// 324); the warm start's batches are of 512.
 constexpr int TRAIN_NB = 16;
 template <int NB, bool TRAIN>
 int launch_rows(portal_mlp *m, int B, const int *idx, const float *X, const float *T, const float *st, float *Y,

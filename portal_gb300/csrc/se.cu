@@ -272,10 +272,10 @@ __host__ __device__ inline size_t se_warp_bytes(int n, int n_feat) {
 // slot is worked on without a test (branches a group of slots made it twice as
 // long), so the instances hold the next larger number of slots.
 // Measured, LU -> this (with the assembly in order of terms and the work of
-// the temperature once a node): 8,192 systems of 74 unknowns 2.29 -> 0.84 ms,
-// 8,192 of 39 1.51 -> 0.44 ms, 1,024 of 14 72 -> 26 us.  Of the 74 x 74
+// the temperature once a node): 8,192 systems of 74 unknowns 2.29 -> 0.85 ms,
+// 8,192 of 39 1.51 -> 0.43 ms, 1,024 of 14 72 -> 26 us.  Of the 74 x 74
 // systems' time some two thirds are the elimination (issue slots; with its 60
-// multiply-adds a warp and step in packed pairs 0.92 -> 0.84 ms), the rest
+// multiply-adds a warp and step in packed pairs 0.92 -> 0.84 ms at the time), the rest
 // FP64 work.
 //
 // Every form below (one warp or four, registers or shared memory) does the
@@ -1489,9 +1489,9 @@ int se_batch_launch(cudaStream_t s, int grid, int warps_per_block, const SEBatch
 // Warps per node: one up to SE_WARP_DIM unknowns, a team of four above
 // (PORTAL_SE_TEAM=1|4 overrides).  The barrier a step costs a team more than
 // the columns save it while one warp's registers hold them: 1,024 systems of
-// 14 unknowns 29 us by one warp, 41 by a team; 1,700 of 19 49 and 98 us.
-// Beyond its registers one warp works in shared memory: 8,192 of 39 0.86 ms,
-// a team 0.44; of 74 3.4 and 0.84.
+// 14 unknowns 26 us by one warp, 37 by a team; 1,700 of 19 43 and 66 us; 4,096
+// of 31 133 and 172.  Beyond its registers one warp works in shared memory:
+// 8,192 of 39 0.88 ms, a team 0.43; of 74 3.5 and 0.85.
 inline int se_team_warps(int n) {
     const char *e = getenv("PORTAL_SE_TEAM");
     if (e) {
