@@ -65,7 +65,6 @@ struct ImLine {
     int lo, up, j1, j2;  // 0-based levels
 };
 constexpr int IM_MAX_LINES = 16;
-__constant__ ImLine c_im[IM_MAX_LINES];
 
 struct ImNodeArgs {
     int N, bulk, nlev, nlines;
@@ -73,6 +72,7 @@ struct ImNodeArgs {
     double tdx;               // tx * dx
     const double *xyz, *vel, *bvec, *b, *tdust, *levp, *pops_in;
     const int *j_lev;
+    const ImLine *lines;      // (nlines) the context's own: contexts may run on several threads
     double *xyz_r;            // (3,N) rotated positions
     double *nrm2;             // (N) |X|^2 of the rotated positions (the march's predictions)
     float4 *cellv;            // (vz, 1/b, cos 2alpha, sin 2alpha)
@@ -130,7 +130,7 @@ __global__ void k_im_nodes(ImNodeArgs a) {
     for (int j = 0; j < a.nlines; j++) {
         float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
         if (n < a.bulk && pp0(0) != 0.0) {
-            const ImLine L = c_im[j];
+            const ImLine L = a.lines[j];
             const double r1_0 = pp0(L.lo), r2_0 = pp0(L.up);
             const double r1_2 = pp2(L.lo), r2_2 = pp2(L.up);
             const double g1 = 2.0 * L.j1 + 1.0, g2 = 2.0 * L.j2 + 1.0;
@@ -175,6 +175,7 @@ struct ImArgs {
     const int *off, *idx;    // neighbour CSR
     const float4 *edge;      // (e, |e|^2/2) per directed edge, unrotated
     const float4 *cellv, *cellb, *coef;
+    const ImLine *lines;     // (nlines)
     const double *dust_p, *ibb;   // dust density; Planck function of the dust (nlines, N)
     int ray0, rays;          // this launch's rays [ray0, ray0 + rays), of nrays
     int2 *walk;              // march lists, per batch of 32 rays of the launch: 32 x n_depth
@@ -240,10 +241,11 @@ __device__ double black_body(double T, double nu) {
 }
 
 // the dust's Planck function per (line, node)
-__global__ void k_im_dust(int N, int nlines, const double *__restrict__ tdust, double *__restrict__ ibb) {
+__global__ void k_im_dust(int N, int nlines, const ImLine *__restrict__ lines, const double *__restrict__ tdust,
+                          double *__restrict__ ibb) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (long long)N * nlines) return;
-    ibb[t] = black_body(tdust[t % N], c_im[t / N].nu0);
+    ibb[t] = black_body(tdust[t % N], lines[t / N].nu0);
 }
 
 // Index of record k of ray r (of its batch of 32) in the batch's march list:
@@ -523,7 +525,7 @@ __global__ void __launch_bounds__(64) k_im_march(ImArgs a, int per) {
 __global__ void __launch_bounds__(64) k_im_dust_maps(ImArgs a) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y;
     if (i >= a.rays) return;
-    const ImLine L = c_im[j];
+    const ImLine L = a.lines[j];
     const int ncr = a.cnt[i];
     const int2 *dl = march_list(a, i);
     const double Iin = a.on_star[i] ? L.bb_star : L.bb_cmb;
@@ -604,7 +606,7 @@ struct Stokes {
     }
     __device__ __forceinline__ void store(const ImArgs &a, int p, int ch, int j, bool bad) const {
         const size_t o = cube_at(a, p, ch, j);
-        const float v[4] = {bad ? NAN : (float)((double)I - c_im[j].bb_cmb), bad ? NAN : Q, bad ? NAN : U,
+        const float v[4] = {bad ? NAN : (float)((double)I - a.lines[j].bb_cmb), bad ? NAN : Q, bad ? NAN : U,
                             bad ? NAN : tau};
 #pragma unroll
         for (int q = 0; q < 4; q++)
@@ -629,7 +631,7 @@ __global__ void __launch_bounds__(32 * IM_WARPS) k_im_stokes(ImArgs a, int s0) {
     if (i >= a.rays) return;
     const int cnt = a.cnt[i], ncr = max(cnt, 0);
     const int2 *dl = march_list(a, i);
-    const float Iin = (float)(a.on_star[i] ? c_im[j].bb_star : c_im[j].bb_cmb);  // I_in (raytrace.f90:97-115)
+    const float Iin = (float)(a.on_star[i] ? a.lines[j].bb_star : a.lines[j].bb_cmb);  // I_in (raytrace.f90:97-115)
     Stokes st[NS];
     float vobs[NS];
 #pragma unroll
@@ -671,7 +673,7 @@ __global__ void __launch_bounds__(64) k_im_stokes_tail(ImArgs a, int ch0) {
     if (i >= a.rays) return;
     const int cnt = a.cnt[i], n = min(4, a.nch - c0);
     const int2 *dl = march_list(a, i);
-    const float Iin = (float)(a.on_star[i] ? c_im[j].bb_star : c_im[j].bb_cmb);
+    const float Iin = (float)(a.on_star[i] ? a.lines[j].bb_star : a.lines[j].bb_cmb);
     Stokes st[4];
     float vobs[4];
 #pragma unroll
@@ -752,7 +754,9 @@ static int image_call(portal_ctx *c, const double *pol_pops, int nlines, const i
                               std::pow(std::exp(4.79924e-11 / c->T_star * nu_last) - 1.0, -1.0)
                         : 0.0;
     }
-    PCHECK(c, cudaMemcpyToSymbolAsync(c_im, h, sizeof(ImLine) * nlines, 0, cudaMemcpyHostToDevice, c->stream));
+    if (c->im_lines.reserve(sizeof(ImLine) * IM_MAX_LINES)) return set_err(c, PORTAL_ERR_NOMEM, "image lines");
+    const ImLine *lines = reinterpret_cast<const ImLine *>(c->im_lines.p);
+    PCHECK(c, cudaMemcpyAsync(c->im_lines.p, h, sizeof(ImLine) * nlines, cudaMemcpyHostToDevice, c->stream));
     // rotation R_tot = R_z(ph_az) R_x(th_inc) (rotmat miscellaneous.f90:146-181)
     auto rotmat = [](const double *nv, double th, double *R) {
         double ct = std::cos(th), oc = 1.0 - ct, s = std::sin(th);
@@ -799,7 +803,7 @@ static int image_call(portal_ctx *c, const double *pol_pops, int nlines, const i
     PCHECK(c, cudaMemcpyAsync(jl.p, c->j_lev.data(), nlev * sizeof(int), cudaMemcpyHostToDevice, c->stream));
     na.N = N; na.bulk = c->bulk; na.nlev = nlev; na.nlines = nlines; na.tdx = c->tx * dx;
     na.xyz = c->pos64.p; na.vel = c->vel64.p; na.bvec = c->bvec64.p; na.b = c->b64.p;
-    na.tdust = c->tdust.p; na.levp = c->levp.p; na.pops_in = pops_src; na.j_lev = jl.p;
+    na.tdust = c->tdust.p; na.levp = c->levp.p; na.pops_in = pops_src; na.j_lev = jl.p; na.lines = lines;
     na.xyz_r = xyz_r.p; na.nrm2 = nrm2.p; na.cellv = cellv.p; na.cellb = cellb.p; na.coef = coef.p;
     timer_start(c, T_EMCOEF);
     k_im_nodes<<<(N + 127) / 128, 128, 0, c->stream>>>(na);
@@ -808,7 +812,7 @@ static int image_call(portal_ctx *c, const double *pol_pops, int nlines, const i
     if (c->has_dust) {
         if (ibb.reserve((size_t)nlines * N)) return set_err(c, PORTAL_ERR_NOMEM, "dust emission");
         const long long tot = (long long)nlines * N;
-        k_im_dust<<<(unsigned)((tot + 127) / 128), 128, 0, c->stream>>>(N, nlines, c->tdust.p, ibb.p);
+        k_im_dust<<<(unsigned)((tot + 127) / 128), 128, 0, c->stream>>>(N, nlines, lines, c->tdust.p, ibb.p);
         PCHECK(c, cudaGetLastError());
     }
     // outputs on the device
@@ -830,7 +834,7 @@ static int image_call(portal_ctx *c, const double *pol_pops, int nlines, const i
     }
     ia.n_depth = n_depth_rt; ia.im_size = im_size; ia.dx = dx; ia.tdx = c->tx * dx; ia.alpha = alpha; ia.dvel = dvel; ia.v0 = v0;
     ia.xyz = xyz_r.p; ia.nrm2 = nrm2.p; ia.off = c->nb_off.p; ia.idx = c->nb_idx.p; ia.cellv = cellv.p; ia.cellb = cellb.p;
-    ia.coef = coef.p; ia.dust_p = c->dustp.p; ia.ibb = ibb.p; ia.dust = c->has_dust; ia.status = stat.p;
+    ia.lines = lines; ia.coef = coef.p; ia.dust_p = c->dustp.p; ia.ibb = ibb.p; ia.dust = c->has_dust; ia.status = stat.p;
     ia.edge = c->edge.p; ia.inv_dx = 1.0 / dx;
     for (int i = 0; i < 9; i++) ia.R[i] = (float)na.R[i];
     {
